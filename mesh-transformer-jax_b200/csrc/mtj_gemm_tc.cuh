@@ -29,14 +29,14 @@
 
 namespace mtj {
 
-// mtj_gemm_tc_gptj.cu; map_x_lo as in launch_gemm_tc
+// mtj_gemm_tc_gptj.cu; map_x2: as map_x_lo in launch_gemm_tc, or (wide) the activations once more with 64-row boxes
 cudaError_t launch_gemm_tc_gptj(GemvEpilogue epi, bool wide, const CUtensorMap& map_w, const CUtensorMap& map_x,
-                                const CUtensorMap* map_x_lo, const GemmTcArgs& a, cudaStream_t s, bool pdl);
+                                const CUtensorMap* map_x2, const GemmTcArgs& a, cudaStream_t s, bool pdl);
 // mtj_gemm_tc_stack.cu
 cudaError_t launch_gemm_tc_stack(GemvEpilogue epi, bool wide, const CUtensorMap& map_w, const CUtensorMap& map_x,
-                                 const GemmTcArgs& a, cudaStream_t s, bool pdl);
+                                 const CUtensorMap* map_x64, const GemmTcArgs& a, cudaStream_t s, bool pdl);
 cudaError_t launch_gemm_tc_stack_post(GemvEpilogue epi, bool wide, const CUtensorMap& map_w, const CUtensorMap& map_x,
-                                 const GemmTcArgs& a, cudaStream_t s, bool pdl);
+                                 const CUtensorMap* map_x64, const GemmTcArgs& a, cudaStream_t s, bool pdl);
 
 namespace {
 
@@ -514,12 +514,12 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const __grid_consta
 // tile is 128 weight rows x 256 token rows (UMMA 128 x 256 x 16), and the accumulator is double
 // buffered in tensor memory (2 x 256 columns) so that the epilogue of tile i runs while the tensor
 // core works on tile i + 1.  Warp 0 = TMA producer, warp 1 = MMA issuer, warps 2-9 = epilogue
-// (lane quadrant = warp % 4, column half = (warp - 2) / 4).  Token tiles vary fastest in the tile
+// (lane quadrant = warp % 4; the two warps of a quadrant take 32-column chunks in turn).  Token tiles vary fastest in the tile
 // list, so the blocks that run together share weight tiles through L2.
 //
-// PAIR: the blocks come as clusters of 2 and a tile is 256 weight rows x 256 token rows, computed by
-// tcgen05.mma.cta_group::2 (UMMA 256 x 256 x 16).  Block r of the pair holds weight rows [128 r, 128 r + 128) and
-// token rows [128 r, 128 r + 128) of the tile in its shared memory and the accumulator of its own 128 weight
+// PAIR: the blocks come as clusters of 2 and a tile is 256 weight rows x bn token rows (at most 256), computed by
+// tcgen05.mma.cta_group::2 (UMMA 256 x bn x 16).  Block r of the pair holds weight rows [128 r, 128 r + 128) and
+// token rows [bn / 2 r, bn / 2 r + bn / 2) of the tile in its shared memory and the accumulator of its own 128 weight
 // rows in its tensor memory, so the epilogue is the same as without PAIR.  Both producers complete their bytes
 // on block 0's "full" barrier; block 0 issues the MMAs and its commits arrive on the "empty" and "accumulator
 // full" barriers of both blocks; the epilogue warps of both blocks arrive on block 0's "accumulator empty".
@@ -527,7 +527,7 @@ constexpr int kPBN = 256;
 constexpr int kPStages = 4;
 constexpr int kPEpiWarps = 8;
 constexpr int kPThreads = 64 + 32 * kPEpiWarps;
-constexpr int kPMaxStages = 6;
+constexpr int kPMaxStages = 9;
 template <int EPI, bool PAIR>
 struct PersistCfg {
   static constexpr int kStages = PAIR ? (EPI == kEpiLogitsCE ? 5 : 6) : kPStages;
@@ -551,11 +551,14 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
                                                                        const __grid_constant__ CUtensorMap map_x,
                                                                        const GemmTcArgs a) {
   using Cfg = PersistCfg<EPI, PAIR>;
-  constexpr int kStages = Cfg::kStages;
-  constexpr uint32_t kABytes = Cfg::kABytes, kStageBytes = Cfg::kStageBytes;
+  // with a 64-row activation box (tiles of at most 128 token rows) a stage is smaller and the ring deeper
+  const int kStages = PAIR ? a.stages : Cfg::kStages;
+  constexpr uint32_t kABytes = Cfg::kABytes;
+  const uint32_t kStageBytes = PAIR ? kABytes + static_cast<uint32_t>(a.x_box) * kBK * 2 : Cfg::kStageBytes;
   constexpr int kTileN = PAIR ? 2 * kBM : kBM;       // weight rows per tile (of the pair)
-  constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kPBN >> 3) << 17) |
-                              (static_cast<uint32_t>(kTileN >> 4) << 24);
+  const int bn = PAIR ? a.bn : kPBN;                 // token rows per tile
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(bn >> 3) << 17) |
+                         (static_cast<uint32_t>(kTileN >> 4) << 24);
   extern __shared__ unsigned char tc_smem_raw[];
   const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
   __shared__ __align__(8) uint64_t bars[2 * kPMaxStages + 4];
@@ -601,45 +604,62 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
   pdl_wait();
   pdl_launch_dependents();
 
-  const int m_tiles = (a.M + kPBN - 1) / kPBN;
+  const int m_tiles = (a.M + bn - 1) / bn;
   const int n_tiles = (a.N + kTileN - 1) / kTileN;
-  const int total = m_tiles * n_tiles;
-  const int nk = (a.K + kBK - 1) / kBK;
+  // split-K (PAIR, a.partial): piece z of a tile covers k-blocks [z * per_z, + per_z) and leaves a plane of partial sums
+  const int ks = PAIR && a.partial ? a.ksplit : 1;
+  const int total = m_tiles * ks * n_tiles;
+  const int nk_all = (a.K + kBK - 1) / kBK, per_z = (nk_all + ks - 1) / ks;
+  auto piece = [&](int t, int& m0, int& n0, int& z, int& kb0, int& nk) {
+    m0 = (t % m_tiles) * bn;
+    const int u = t / m_tiles;
+    z = u % ks;
+    n0 = (u / ks) * kTileN + static_cast<int>(crank) * kBM;
+    kb0 = z * per_z;
+    nk = min(per_z, nk_all - kb0);                   // at least 1 (checked at launch)
+  };
   const int tile_first = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
   const int tile_step = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
   if (warp == 0) {
     if (lane == 0) {
-      uint32_t it = 0;
+      const uint32_t box_bytes = static_cast<uint32_t>(a.x_box) * kBK * 2;   // rows past bn / 2 are not multiplied
+      int s = 0;
+      uint32_t phase = 0;
       bool alive = true;
       for (int t = tile_first; t < total && alive; t += tile_step) {
-        const int n0 = (t / m_tiles) * kTileN + static_cast<int>(crank) * kBM, m0 = (t % m_tiles) * kPBN;
-        for (int kb = 0; kb < nk; ++kb, ++it) {
-          const int s = it % kStages;
-          if (it >= kStages && !mbar_wait(empty_bar(s), ((it / kStages) - 1) & 1)) {
+        int m0, n0, z, kb0, nk;
+        piece(t, m0, n0, z, kb0, nk);
+        for (int kb = 0; kb < nk; ++kb) {
+          if (!mbar_wait(empty_bar(s), phase ^ 1u)) {        // passes in the ring's first round
             atomicOr(&failed, 1u);
             alive = false;
             break;
           }
           const uint32_t dst = smem_base + s * kStageBytes;
           if (PAIR) {
-            // block 0's barrier counts the bytes of both blocks; the activation box has 128 token rows
-            if (crank == 0) mbar_expect_tx(full_bar(s), 2 * kStageBytes);
+            // block 0's barrier counts the bytes of both blocks
+            if (crank == 0) mbar_expect_tx(full_bar(s), 2 * (kABytes + box_bytes));
             const uint32_t fb = tc_map_to_rank(full_bar(s), 0);
-            tma_load_2d_pair(dst, &map_w, kb * kBK, n0, fb);
-            tma_load_2d_pair(dst + kABytes, &map_x, kb * kBK, a.x_row0 + m0 + static_cast<int>(crank) * (kPBN / 2), fb);
+            tma_load_2d_pair(dst, &map_w, (kb0 + kb) * kBK, n0, fb);
+            tma_load_2d_pair(dst + kABytes, &map_x, (kb0 + kb) * kBK, a.x_row0 + m0 + static_cast<int>(crank) * (bn / 2), fb);
           } else {
             mbar_expect_tx(full_bar(s), kStageBytes);
             tma_load_2d(dst, &map_w, kb * kBK, n0, full_bar(s));
             tma_load_2d(dst + kABytes, &map_x, kb * kBK, a.x_row0 + m0, full_bar(s));
             tma_load_2d(dst + kABytes + (kPBN / 2) * kBK * 2, &map_x, kb * kBK, a.x_row0 + m0 + kPBN / 2, full_bar(s));
           }
+          if (++s == kStages) {
+            s = 0;
+            phase ^= 1u;
+          }
         }
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && crank == 0) {
-      uint32_t it = 0;
+      int s = 0;
+      uint32_t phase = 0;
       bool alive = true;
       int i = 0;
       for (int t = tile_first; t < total && alive; t += tile_step, ++i) {
@@ -650,9 +670,10 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
         }
         tc_fence_after();
         const uint32_t d = tmem_acc + static_cast<uint32_t>(b * kPBN);
-        for (int kb = 0; kb < nk; ++kb, ++it) {
-          const int s = it % kStages;
-          if (!mbar_wait(full_bar(s), (it / kStages) & 1)) {
+        int m0, n0, z, kb0, nk;
+        piece(t, m0, n0, z, kb0, nk);
+        for (int kb = 0; kb < nk; ++kb) {
+          if (!mbar_wait(full_bar(s), phase)) {
             atomicOr(&failed, 1u);
             alive = false;
             break;
@@ -662,11 +683,15 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
           const uint64_t adesc = smem_desc_sw128(sa), bdesc = smem_desc_sw128(sa + kABytes);
 #pragma unroll
           for (int k4 = 0; k4 < kBK / 16; ++k4) {
-            if (PAIR) tc_mma_bf16_pair(d, adesc + 2 * k4, bdesc + 2 * k4, kIdesc, (kb > 0 || k4 > 0) ? 1u : 0u);
-            else tc_mma_bf16(d, adesc + 2 * k4, bdesc + 2 * k4, kIdesc, (kb > 0 || k4 > 0) ? 1u : 0u);
+            if (PAIR) tc_mma_bf16_pair(d, adesc + 2 * k4, bdesc + 2 * k4, idesc, (kb > 0 || k4 > 0) ? 1u : 0u);
+            else tc_mma_bf16(d, adesc + 2 * k4, bdesc + 2 * k4, idesc, (kb > 0 || k4 > 0) ? 1u : 0u);
           }
           if (PAIR) tc_commit_pair(empty_bar(s));
           else tc_commit(empty_bar(s));
+          if (++s == kStages) {
+            s = 0;
+            phase ^= 1u;
+          }
         }
         if (alive) {
           if (PAIR) tc_commit_pair(acc_full(b));
@@ -677,19 +702,14 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
   } else {
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;
-    const int Tc = a.rows.Tc;
+    const int Tc = max(1, a.rows.Tc);
     int pos0 = 0;
     if (EPI == kEpiInProj) pos0 = a.rows.pos0_dev ? *a.rows.pos0_dev : a.rows.pos0_host;
     int i = 0;
     for (int t = tile_first; t < total; t += tile_step, ++i) {
       const int b = i & 1;
-      if (*failed_v || !mbar_wait(acc_full(b), (i >> 1) & 1)) {
-        atomicOr(&failed, 1u);
-        break;
-      }
-      tc_fence_after();
-      const int n0 = (t / m_tiles) * kTileN + static_cast<int>(crank) * kBM,
-                m0 = (t % m_tiles) * kPBN + half * (kPBN / 2);
+      int m0, n0, z, kb0, nk;
+      piece(t, m0, n0, z, kb0, nk);
       const int n = n0 + quad * 32 + lane;
       const bool n_ok = n < a.N;
       int region = 0, nn = 0, head = 0, j = 0;
@@ -710,24 +730,45 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
       } else if (n_ok && a.bias) {
         bias = a.bias[n];
       }
-      // (sequence, position) of the chunk's first row, advanced chunk by chunk (uniform over the warp)
-      int seq = 0, tin = 0;
-      if (EPI == kEpiInProj) {
-        seq = a.rows.b0 + m0 / Tc;
-        tin = m0 % Tc;
-      }
       const bool rotary = EPI == kEpiInProj && n_ok && region < 2 && j < a.rot;
       const bool any_rot = __any_sync(0xffffffffu, rotary);
+      const bool kv_lane = EPI == kEpiInProj && n_ok && (region == 1 || region == 2);
+      const bool kv_warp = __any_sync(0xffffffffu, kv_lane);
       const float sgn = (j & 1) ? 1.f : -1.f;
       const int half_rot = a.rot >> 1;
       const size_t ld_act = static_cast<size_t>(a.dl + a.ffl);
       const uint32_t tbase = tmem_acc + (static_cast<uint32_t>(quad * 32) << 16) +
-                             static_cast<uint32_t>(b * kPBN + half * (kPBN / 2));
+                             static_cast<uint32_t>(b * kPBN);
+      // the 32-column chunks of the tile that hold token rows alternate between the two warps of a lane quadrant
+      const int cols = min(bn, (a.M - m0 + 31) & ~31);
+      // of the row m that this lane looks after: its position, and its row of the cache slabs (-1: not stored)
+      auto row_of = [&](int m, int& row_pos, int& row_cache) {
+        row_pos = 0;
+        row_cache = -1;
+        if (m >= a.M) return;
+        const int seq = a.rows.b0 + m / Tc;
+        row_pos = pos0 + m % Tc;
+        if (kv_warp && row_pos >= a.kv.pad[seq])
+          row_cache = a.kv.page_table[static_cast<size_t>(seq) * a.kv.ring_pages + (row_pos / kPageTokens) % a.kv.ring_pages] * a.heads * kPageTokens +
+                      row_pos % kPageTokens;
+      };
+      int row_pos = 0, row_cache = -1, next_pos = 0, next_cache = -1;
+      if (EPI == kEpiInProj && (any_rot || kv_warp)) row_of(m0 + 32 * half + lane, next_pos, next_cache);
+      if (*failed_v || !mbar_wait(acc_full(b), (i >> 1) & 1)) {
+        atomicOr(&failed, 1u);
+        break;
+      }
+      tc_fence_after();
 #pragma unroll 1
-      for (int c0 = 0; c0 < kPBN / 2; c0 += 32) {
+      for (int c0 = 32 * half; c0 < cols || c0 == 32 * half; c0 += 64) {
         uint32_t r[32];
+        if (EPI == kEpiInProj) {
+          row_pos = next_pos;
+          row_cache = next_cache;
+          if (any_rot || kv_warp) row_of(m0 + c0 + 64 + lane, next_pos, next_cache);     // of the next chunk, a chunk ahead
+        }
         tmem_ld32(tbase + c0, r);
-        if (c0 + 32 == kPBN / 2) {
+        if (c0 + 64 >= cols) {
           // this warp has read its part of the accumulator: hand the buffer back to the MMA warp
           tc_fence_before();
           __syncwarp();
@@ -738,95 +779,74 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
         }
         const int mc = m0 + c0;                          // first token row of the chunk
         const int valid = min(32, a.M - mc);             // rows of the chunk that exist
-        if (EPI == kEpiInProj) {
-          if (valid == 32 && tin + 32 <= Tc) {
-            // all 32 rows exist and belong to one sequence: positions pos .. pos + 31
-            const int pos = pos0 + tin;
-            if (any_rot) {
-              const float2* sc = a.sincos + static_cast<size_t>(pos) * half_rot + (rotary ? (j >> 1) : 0);
-#pragma unroll
-              for (int q = 0; q < 32; ++q) {
-                const float v = __uint_as_float(r[q]);
-                const float partner = __shfl_xor_sync(0xffffffffu, v, 1);
-                if (rotary) {
-                  const float2 t = sc[q * half_rot];
-                  r[q] = __float_as_uint(fmaf(v, t.y, (sgn * partner) * t.x));
-                }
-              }
-            }
-            if (!n_ok) {
-            } else if (region == 3) {
-              __nv_bfloat16* dst = a.act_out + static_cast<size_t>(mc) * ld_act + a.dl + nn;
+        if (EPI == kEpiPlain || EPI == kEpiOut) {
+          if (a.partial) {
+            if (n_ok && valid > 0) {
+              float* dst = a.partial + (static_cast<size_t>(z) * a.M + mc) * a.N + n;
 #pragma unroll
               for (int q = 0; q < 32; ++q)
-                dst[q * ld_act] = __float2bfloat16_rn(gelu_tanh_fast(__uint_as_float(r[q]) + bias));
-            } else if (region == 0) {
-              if (a.q_bf16) {
-                __nv_bfloat16* dst = a.q_bf16 + static_cast<size_t>(mc) * a.dl + nn;
+                if (q < valid) dst[static_cast<size_t>(q) * a.N] = __uint_as_float(r[q]);
+            }
+            continue;
+          }
+        }
+        if (EPI == kEpiInProj) {
+          // what concerns a token row (position, cache row) was fetched by the lane of its number; 16 rotations' factors
+          // are in flight at a time (looked up row by row, a 256-row tile's rotation took longer than its main loop)
+          if (any_rot) {
+#pragma unroll
+            for (int q0 = 0; q0 < 32; q0 += 16) {
+              float2 f[16];
+#pragma unroll
+              for (int q = 0; q < 16; ++q) {
+                const int p = __shfl_sync(0xffffffffu, row_pos, q0 + q);
+                if (rotary) f[q] = __ldg(a.sincos + static_cast<size_t>(p) * half_rot + (j >> 1));
+              }
+#pragma unroll
+              for (int q = 0; q < 16; ++q) {
+                const float v = __uint_as_float(r[q0 + q]);
+                const float partner = __shfl_xor_sync(0xffffffffu, v, 1);
+                if (rotary) r[q0 + q] = __float_as_uint(fmaf(v, f[q].y, (sgn * partner) * f[q].x));
+              }
+            }
+          }
+          if (kv_warp) {
+            __nv_bfloat16* pool = (region == 1 ? a.kv.kpool : a.kv.vpool) + static_cast<size_t>(head) * kPageTokens * a.d_head + j;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) {
+              const int cr = __shfl_sync(0xffffffffu, row_cache, q);
+              if (kv_lane && cr >= 0) pool[static_cast<size_t>(cr) * a.d_head] = __float2bfloat16_rn(__uint_as_float(r[q]));
+            }
+          }
+          if (n_ok && valid > 0 && region == 3) {
+            __nv_bfloat16* dst = a.act_out + static_cast<size_t>(mc) * ld_act + a.dl + nn;
+            // (computed whether it is stored or not: a branch around each would serialise the exponentials)
+#pragma unroll
+            for (int q = 0; q < 32; ++q) r[q] = __float_as_uint(gelu_tanh_fast(__uint_as_float(r[q]) + bias));
+            if (valid == 32) {
+#pragma unroll
+              for (int q = 0; q < 32; ++q) dst[q * ld_act] = __float2bfloat16_rn(__uint_as_float(r[q]));
+            } else {
+#pragma unroll
+              for (int q = 0; q < 32; ++q)
+                if (q < valid) dst[q * ld_act] = __float2bfloat16_rn(__uint_as_float(r[q]));
+            }
+          } else if (n_ok && valid > 0 && region == 0) {
+            if (a.q_bf16) {
+              __nv_bfloat16* dst = a.q_bf16 + static_cast<size_t>(mc) * a.dl + nn;
+              if (valid == 32) {
 #pragma unroll
                 for (int q = 0; q < 32; ++q) dst[static_cast<size_t>(q) * a.dl] = __float2bfloat16_rn(__uint_as_float(r[q]));
               } else {
-                float* dst = a.q_out + static_cast<size_t>(mc) * a.dl + nn;
 #pragma unroll
-                for (int q = 0; q < 32; ++q) dst[static_cast<size_t>(q) * a.dl] = __uint_as_float(r[q]);
+                for (int q = 0; q < 32; ++q)
+                  if (q < valid) dst[static_cast<size_t>(q) * a.dl] = __float2bfloat16_rn(__uint_as_float(r[q]));
               }
             } else {
-              __nv_bfloat16* pool = (region == 1 ? a.kv.kpool : a.kv.vpool) + j;
-              const int32_t* trow = a.kv.page_table + static_cast<size_t>(seq) * a.kv.ring_pages;
-              const int padv = a.kv.pad[seq];
-              const size_t slab = static_cast<size_t>(kPageTokens) * a.d_head;
-              int pg = pos / kPageTokens, off = pos % kPageTokens;
-              __nv_bfloat16* dst = pool + (static_cast<size_t>(trow[pg % a.kv.ring_pages]) * a.heads + head) * slab;
+              float* dst = a.q_out + static_cast<size_t>(mc) * a.dl + nn;
 #pragma unroll
-              for (int q = 0; q < 32; ++q) {
-                if (off == kPageTokens) {
-                  off = 0;
-                  ++pg;
-                  dst = pool + (static_cast<size_t>(trow[pg % a.kv.ring_pages]) * a.heads + head) * slab;
-                }
-                if (pos + q >= padv) dst[off * a.d_head] = __float2bfloat16_rn(__uint_as_float(r[q]));
-                ++off;
-              }
-            }
-            tin += 32;
-            if (tin == Tc) {
-              tin = 0;
-              ++seq;
-            }
-          } else {
-            // ragged chunk (end of the rows, or a sequence boundary inside it): element by element
-#pragma unroll
-            for (int q = 0; q < 32; ++q) {
-              const int m = mc + q;
-              const float v = __uint_as_float(r[q]);
-              const float partner = __shfl_xor_sync(0xffffffffu, v, 1);
-              const int pos = pos0 + tin;
-              if (m < a.M && n_ok) {
-                if (region < 3) {
-                  float y = v;
-                  if (rotary) {
-                    const float2 t = a.sincos[static_cast<size_t>(pos) * half_rot + (j >> 1)];
-                    y = fmaf(v, t.y, (sgn * partner) * t.x);
-                  }
-                  if (region == 0) {
-                    if (a.q_bf16)
-                      a.q_bf16[static_cast<size_t>(m) * a.dl + nn] = __float2bfloat16_rn(y);
-                    else
-                      a.q_out[static_cast<size_t>(m) * a.dl + nn] = y;
-                  } else if (pos >= a.kv.pad[seq]) {
-                    __nv_bfloat16* pool = region == 1 ? a.kv.kpool : a.kv.vpool;
-                    const size_t o = kv_offset(a.kv.page_table + static_cast<size_t>(seq) * a.kv.ring_pages,
-                                               a.kv.ring_pages, a.heads, a.d_head, head, pos);
-                    pool[o + j] = __float2bfloat16_rn(y);
-                  }
-                } else {
-                  a.act_out[static_cast<size_t>(m) * ld_act + a.dl + nn] = __float2bfloat16_rn(gelu_tanh_fast(v + bias));
-                }
-              }
-              if (++tin == Tc) {
-                tin = 0;
-                ++seq;
-              }
+              for (int q = 0; q < 32; ++q)
+                if (q < valid) dst[static_cast<size_t>(q) * a.dl] = __uint_as_float(r[q]);
             }
           }
         } else if (EPI == kEpiLogitsCE) {
@@ -969,8 +989,16 @@ cudaError_t launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTc
   return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, STAGES, EPI, HILO>, mw, mx, mxlo ? *mxlo : mx, a);
 }
 
+// Token rows per tile of the pair kernel: the fewest tiles of at most 256, as even as 32-row chunks allow.  A k-block
+// costs 0.31 us at 64 rows and 0.36 at 256 (the round trip through the ring bounds it), so a lower tile never pays for
+// one more; evening out saves operand and epilogue work (300 rows: in-projection 108 us as 256 + 44, 95 as 160 + 140).
+inline int gemm_tc_wide_bn(int M) {
+  const int tiles = (M + kPBN - 1) / kPBN;
+  return std::max(64, ((M + tiles - 1) / tiles + 31) / 32 * 32);
+}
+
 template <int EPI>
-cudaError_t launch_tc_persist(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTcArgs& a, cudaStream_t s) {
+cudaError_t launch_tc_persist(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap* mx64, const GemmTcArgs& a, cudaStream_t s) {
   // the cross-entropy epilogue turns each epilogue warp's 32 x 32 block through 4 KB of shared memory
   constexpr int smem = PersistCfg<EPI, false>::kSmem, smem_pair = PersistCfg<EPI, true>::kSmem;
   static DeviceOnce once;
@@ -986,10 +1014,17 @@ cudaError_t launch_tc_persist(const CUtensorMap& mw, const CUtensorMap& mx, cons
     return cudaDeviceGetAttribute(&sms_of[dev], cudaDevAttrMultiProcessorCount, dev);
   });
   if (e != cudaSuccess) return e;
-  const int m_tiles = (a.M + kPBN - 1) / kPBN;
   if (a.pair && a.N >= 2 * kBM && sms_of[dev] >= 2) {
-    // clusters of 2 blocks, one 256 x 256 tile per pair at a time
-    const int total = m_tiles * ((a.N + 2 * kBM - 1) / (2 * kBM));
+    // clusters of 2 blocks, one tile of 256 weight rows per pair at a time
+    using Cfg = PersistCfg<EPI, true>;
+    GemmTcArgs b = a;
+    b.bn = gemm_tc_wide_bn(a.M);
+    b.x_box = b.bn <= 128 && mx64 ? 64 : 128;
+    b.stages = static_cast<int>(Cfg::kStages * Cfg::kStageBytes / (Cfg::kABytes + b.x_box * kBK * 2));
+    if (a.partial && (EPI != kEpiOut && EPI != kEpiPlain)) return cudaErrorInvalidValue;
+    const int nk = (a.K + kBK - 1) / kBK, ks = a.partial ? a.ksplit : 1;
+    if (ks < 1 || (ks - 1) * ((nk + ks - 1) / ks) >= nk) return cudaErrorInvalidValue;
+    const int total = (a.M + b.bn - 1) / b.bn * ((a.N + 2 * kBM - 1) / (2 * kBM)) * ks;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -1002,9 +1037,10 @@ cudaError_t launch_tc_persist(const CUtensorMap& mw, const CUtensorMap& mx, cons
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_tc_persist_kernel<EPI, true>, mw, mx, a);
+    return cudaLaunchKernelEx(&cfg, gemm_tc_persist_kernel<EPI, true>, mw, b.x_box == 64 ? *mx64 : mx, b);
   }
-  const int total = m_tiles * ((a.N + kBM - 1) / kBM);
+  if (a.partial) return cudaErrorInvalidValue;
+  const int total = (a.M + kPBN - 1) / kPBN * ((a.N + kBM - 1) / kBM);
   gemm_tc_persist_kernel<EPI, false><<<std::min(total, sms_of[dev]), kPThreads, smem, s>>>(mw, mx, a);
   return cudaGetLastError();
 }

@@ -7,12 +7,12 @@ cudaError_t launch_gemm_tc_gptj(GemvEpilogue epi, bool wide, const CUtensorMap& 
                                 const CUtensorMap* ml, const GemmTcArgs& a, cudaStream_t s, bool pdl) {
   if (wide) {
     switch (epi) {
-      case kEpiInProj: return launch_tc_persist<kEpiInProj>(mw, mx, a, s);
-      case kEpiOut: return launch_tc_persist<kEpiOut>(mw, mx, a, s);
+      case kEpiInProj: return launch_tc_persist<kEpiInProj>(mw, mx, ml, a, s);
+      case kEpiOut: return launch_tc_persist<kEpiOut>(mw, mx, ml, a, s);
       case kEpiLogitsCE:
         if (!a.ce_gmax || !a.ce_gsum || !a.ce_tlogit || !a.ce_hit || !a.ce_targets || a.ce_ld < a.M) return cudaErrorInvalidValue;
-        return launch_tc_persist<kEpiLogitsCE>(mw, mx, a, s);
-      default: return launch_tc_persist<kEpiLogits>(mw, mx, a, s);
+        return launch_tc_persist<kEpiLogitsCE>(mw, mx, ml, a, s);
+      default: return launch_tc_persist<kEpiLogits>(mw, mx, ml, a, s);
     }
   }
   if (ml) {

@@ -6,10 +6,10 @@
 namespace mtj {
 
 cudaError_t launch_gemm_tc_stack(GemvEpilogue epi, bool wide, const CUtensorMap& mw, const CUtensorMap& mx,
-                                 const GemmTcArgs& a, cudaStream_t s, bool pdl) {
+                                 const CUtensorMap* m64, const GemmTcArgs& a, cudaStream_t s, bool pdl) {
   if (epi == kEpiSwiGLU ? (!a.out_bf16 || (a.N & 1) || a.partial || a.bias) : (!a.out && !a.out_bf16 && !a.partial))
     return cudaErrorInvalidValue;
-  if (wide) return epi == kEpiPlain ? launch_tc_persist<kEpiPlain>(mw, mx, a, s) : launch_tc_persist<kEpiSwiGLU>(mw, mx, a, s);
+  if (wide) return epi == kEpiPlain ? launch_tc_persist<kEpiPlain>(mw, mx, m64, a, s) : launch_tc_persist<kEpiSwiGLU>(mw, mx, m64, a, s);
   switch (gemm_tc_token_tile_for(a.M)) {
     case 32: return epi == kEpiPlain ? launch_tc<32, 5, kEpiPlain>(mw, mx, a, s, pdl) : launch_tc<32, 5, kEpiSwiGLU>(mw, mx, a, s, pdl);
     case 64: return epi == kEpiPlain ? launch_tc<64, 4, kEpiPlain>(mw, mx, a, s, pdl) : launch_tc<64, 4, kEpiSwiGLU>(mw, mx, a, s, pdl);

@@ -113,6 +113,9 @@ struct mtj_handle {
                                     // arg-max to all ranks instead of gathering the logits (MTJ_NO_TP_TOKEN=1: off)
   bool tp_push = false;             // batched decode at mp > 1: push all-reduce fused with the split-K reduction and
                                     // the LayerNorm; default: from 4 shards on (MTJ_TP_PUSH=0 / 1 overrides)
+  // Evaluation: products keep one order of sums (no split along K, the same kernels at every row count).  The loss of a token
+  // that the model is sure of is the difference of two nearly equal numbers and shows every change of rounding.
+  bool same_sums = false;
   bool xn_ready = false;            // the bf16 operand of the next projection has already been written
   bool tc_cluster_k = true;         // batched decode: split K over block clusters when tiles are few (MTJ_NO_CLUSTER_K=1: off)
   float* uniforms = nullptr;        // [max_batch, V] sampler inputs of the current step
@@ -314,7 +317,7 @@ struct mtj_handle {
       logits_gather = c.take<float>(static_cast<int64_t>(max_batch) * V);
       part = c.take<float>(R * d);
     }
-    tc_partial = c.take<float>(static_cast<int64_t>(mtj::kTcSplitMax) * std::min<int64_t>(R, mtj::kTcSplitRows) * d);
+    tc_partial = c.take<float>(std::max(static_cast<int64_t>(mtj::kTcSplitMax) * std::min<int64_t>(R, mtj::kTcSplitRows) * d, mtj::kWidePlaneFloats));
     q_bf16 = c.take<__nv_bfloat16>(R * dl);
     xn_bf16 = c.take<__nv_bfloat16>(R * d);
     act_bf16 = c.take<__nv_bfloat16>(R * (dl + ffl));

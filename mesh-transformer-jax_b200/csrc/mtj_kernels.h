@@ -6,6 +6,21 @@
 
 namespace mtj {
 
+template <typename K, typename... A>
+cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Rows of a forward chunk: row m belongs to sequence b0 + m / Tc and sits at
 // absolute position pos0 + m % Tc, where pos0 = *pos0_dev when that pointer is
 // set (decode: the step counter lives on the device so that a captured graph
@@ -272,16 +287,33 @@ struct GemmTcArgs {
                                // to out_bf16; 0: every row to both
   float softcap;               // kEpiSoftcap
   int pair;                    // wide kernel only: 1 = clusters of 2 blocks on 256 x 256 tiles (tcgen05 cta_group::2)
+  int bn, x_box, stages;       // wide kernel with pair: token rows per tile and of the activation box, ring stages; set by the launch
   uint32_t* dev_err;
 };
+constexpr int64_t kWidePlaneFloats = 148LL * 256 * 256;   // most partial sums of a split launch_gemm_tc_wide: two waves of tiles
 int gemm_tc_token_tile();                 // widest token tile of launch_gemm_tc (128)
 // Token tile launch_gemm_tc uses for M rows (32, 64 or 128): map_x must have been made with this box_rows.
 int gemm_tc_token_tile_for(int M);
+// Whether M rows go through launch_gemm_tc_wide.
+bool gemm_tc_use_wide(int M, bool same_sums);
+// Pieces launch_gemm_tc_wide should cut K into (GemmTcArgs.partial, ksplit) when the caller can add planes; 1: none.
+int gemm_tc_wide_split(int M, int N, int K);
 // Cluster split-K factor (1, 2 or 4) launch_gemm_tc should be given for a decode-size GEMM (GemmTcArgs.cluster_k).
 int gemm_tc_decode_cluster_k(int weight_rows, int M, int K);
 cudaError_t launch_splitk_reduce(const float* partial, int ksplit, int M, int N, const float* bias,
                                  const float* residual, float* out, int ld_out, const uint32_t* slot_sel,
                                  size_t slot_stride, cudaStream_t s, bool pdl = false);
+// out[m] = sum of the planes + bias + residual[m] (out may be the residual); with scale also its layer norm in bf16
+struct ReduceLnArgs {
+  const float* partial;        // [planes, M, d]
+  int planes, M, d;
+  const float *bias, *residual;
+  float* out;
+  const float *scale, *offset; // or null: no norm
+  __nv_bfloat16 *xn, *xn_lo;   // xn_lo optional
+};
+bool reduce_ln_rows_ok(int d);
+cudaError_t launch_reduce_ln_rows(const ReduceLnArgs& a, cudaStream_t s, bool pdl);
 cudaError_t make_tensor_map_bf16(void* map_out_128B, const void* base, int64_t rows, int64_t K, int box_rows, int64_t ld = 0);   // ld: row stride in elements (0 = K)
 // map_x_lo (optional, M <= 64): a second activation view holding the bf16 rounding error of the first
 // (x = hi + lo); both are multiplied into the same accumulator.
@@ -290,7 +322,7 @@ cudaError_t launch_gemm_tc(GemvEpilogue epi, const void* map_w, const void* map_
 // Persistent variant for many token rows (tiles of 128 or, as block pairs, 256 weight rows x 256 token rows);
 // map_x must have been made with box_rows = gemm_tc_wide_token_tile().  No split-K.
 int gemm_tc_wide_token_tile();
-cudaError_t launch_gemm_tc_wide(GemvEpilogue epi, const void* map_w, const void* map_x, const GemmTcArgs& a,
+cudaError_t launch_gemm_tc_wide(GemvEpilogue epi, const void* map_w, const void* map_x, const void* map_x64, const GemmTcArgs& a,
                                 cudaStream_t s);
 cudaError_t launch_ln_rows(const float* x, const float* scale, const float* offset, __nv_bfloat16* out, int rows,
                            int d, cudaStream_t s, bool pdl = false, __nv_bfloat16* out_lo = nullptr);

@@ -245,22 +245,25 @@ int32_t run_layer(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, bool
 }
 
 int tc_tile_index(int M) { return mtj::gemm_tc_token_tile_for(M) == 32 ? 0 : (mtj::gemm_tc_token_tile_for(M) == 64 ? 1 : 2); }
-bool use_tc_wide(const mtj_handle* h, int M) { return h->tc_wide_ok && M > 192; }
+bool use_tc_wide(const mtj_handle* h, int M, bool same_sums) { return h->tc_wide_ok && mtj::gemm_tc_use_wide(M, same_sums); }
 
 // The same layer for many token rows on the tensor cores: LayerNorm to bf16, in-proj GEMM
-// (RoPE / KV / GELU epilogue), causal attention, out-proj GEMM (+ bias + residual).
+// (RoPE / KV / GELU epilogue), causal attention, out-proj GEMM (+ bias + residual).  chain: the next call is the following
+// layer's for the same rows (behind the last layer in decode, the logits), so its norm may be left ready here.
 int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, const int32_t* key_limit,
-                     cudaStream_t s, float* detached_out = nullptr, bool decode = false, bool defer_reduce = false) {
+                     cudaStream_t s, float* detached_out = nullptr, bool decode = false, bool defer_reduce = false, bool chain = false) {
   LayerWeights& lw = h->layers[layer];
   // decode (graph-replayed, launch-latency sensitive): every kernel of the chain waits on its predecessor with
   // griddepcontrol.wait, so each may be scheduled while the previous one drains
   const bool pdl = h->use_pdl && h->tc_pdl && decode;
   // few sequences: activations go through the GEMMs as hi + lo bf16 pairs
   const bool hilo = decode && h->hilo_ok && M <= h->tc_hilo_max_b;
-  if (h->xn_ready)
-    h->xn_ready = false;            // the previous exchange has already written this layer's operand
-  else
+  if (h->xn_ready) {
+    h->xn_ready = false;            // the previous exchange or reduction has already written this layer's operand
+  } else {
+    h->launches++;
     MTJ_CUDA(mtj::launch_ln_rows(h->x, lw.ln_scale, lw.ln_offset, h->xn_bf16, M, h->d, s, pdl, hilo ? h->xn_lo : nullptr));
+  }
   mtj::GemmTcArgs a = {};
   a.M = M;
   a.N = 3 * h->dl + h->ffl;
@@ -281,10 +284,10 @@ int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, c
   a.dev_err = h->dev_err;
   a.cluster_k = (decode && h->tc_cluster_k) ? mtj::gemm_tc_decode_cluster_k(a.N, M, a.K) : 1;
   h->prof_begin(MTJ_FAMILY_INPROJ, s);
-  const bool wide = use_tc_wide(h, M) && !decode;
+  const bool wide = !decode && use_tc_wide(h, M, h->same_sums);
   a.pair = h->tc_pair & 1;
   if (wide)
-    MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiInProj, &lw.map_in, &h->map_xn_wide, a, s));
+    MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiInProj, &lw.map_in, &h->map_xn_wide, &h->map_xn[1], a, s));
   else
     MTJ_CUDA(mtj::launch_gemm_tc(mtj::kEpiInProj, &lw.map_in, &h->map_xn[tc_tile_index(M)], a, s, pdl,
                                  hilo ? &h->map_xn_lo[tc_tile_index(M)] : nullptr));
@@ -351,7 +354,9 @@ int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, c
   // Few token rows give only d/128 tiles: split K over blocks so the whole GPU streams the weights.
   const int tiles = ((h->d + 127) / 128) * ((M + mtj::gemm_tc_token_tile() - 1) / mtj::gemm_tc_token_tile());
   int ksplit = 1;
-  if (M <= kTcSplitRows && tiles < 148) ksplit = std::max(1, std::min({kTcSplitMax, 296 / tiles, o.K / 64}));
+  const bool wide_out = wide && !to_slot;
+  if (!wide_out && M <= kTcSplitRows && tiles < 148) ksplit = std::max(1, std::min({kTcSplitMax, 296 / tiles, o.K / 64}));
+  if (wide_out && h->mp == 1 && !h->same_sums && mtj::reduce_ln_rows_ok(h->d)) ksplit = mtj::gemm_tc_wide_split(M, o.N, o.K);
   if (to_slot && ksplit == 1) ksplit = 2;          // the slot is selected by the reduction kernel
   const bool push = decode && !detached_out && !defer_reduce && use_push(h, M) && M <= kTcSplitRows;
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
@@ -374,20 +379,36 @@ int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, c
     const float* res = o.residual;
     o.partial = h->tc_partial;
     o.ksplit = ksplit;
-    MTJ_CUDA(mtj::launch_gemm_tc(mtj::kEpiOut, &lw.map_out, &h->map_act[tc_tile_index(M)], o, s, pdl,
-                                 hilo ? &h->map_act_lo[tc_tile_index(M)] : nullptr));
-    MTJ_CUDA(mtj::launch_splitk_reduce(h->tc_partial, ksplit, M, h->d, lw.b_out, res, dst, h->d,
-                                       to_slot ? partial_slot_sel(h, M) : nullptr, partial_slot_stride(h), s, pdl));
+    o.pair = 1;
+    if (wide_out) MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiOut, &lw.map_out, &h->map_act_wide, &h->map_act[1], o, s));
+    else MTJ_CUDA(mtj::launch_gemm_tc(mtj::kEpiOut, &lw.map_out, &h->map_act[tc_tile_index(M)], o, s, pdl,
+                                      hilo ? &h->map_act_lo[tc_tile_index(M)] : nullptr));
+    if (h->mp == 1 && res && !h->same_sums && mtj::reduce_ln_rows_ok(h->d)) {
+      // one kernel adds the planes and norms the rows for what follows: the next layer, or in decode the logits
+      const bool last = layer + 1 == h->L, norm = chain && (!last || decode);
+      mtj::ReduceLnArgs r = {h->tc_partial, ksplit, M, h->d, lw.b_out, res, dst};
+      if (norm) {
+        r.scale = last ? h->lnf_scale : h->layers[layer + 1].ln_scale;
+        r.offset = last ? h->lnf_offset : h->layers[layer + 1].ln_offset;
+        r.xn = h->xn_bf16;
+        r.xn_lo = hilo ? h->xn_lo : nullptr;
+      }
+      MTJ_CUDA(mtj::launch_reduce_ln_rows(r, s, pdl));
+      h->xn_ready = norm;
+    } else {
+      MTJ_CUDA(mtj::launch_splitk_reduce(h->tc_partial, ksplit, M, h->d, lw.b_out, res, dst, h->d,
+                                         to_slot ? partial_slot_sel(h, M) : nullptr, partial_slot_stride(h), s, pdl));
+    }
     h->launches++;
-  } else if (wide) {
+  } else if (wide_out) {
     o.pair = (h->tc_pair >> 1) & 1;
-    MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiOut, &lw.map_out, &h->map_act_wide, o, s));
+    MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiOut, &lw.map_out, &h->map_act_wide, &h->map_act[1], o, s));
   } else {
     MTJ_CUDA(mtj::launch_gemm_tc(mtj::kEpiOut, &lw.map_out, &h->map_act[tc_tile_index(M)], o, s, pdl,
                                  hilo ? &h->map_act_lo[tc_tile_index(M)] : nullptr));
   }
   h->prof_end(s);
-  h->launches += 4;
+  h->launches += 3;
   if (h->mp > 1 && detached_out) {
     std::string err;
     if (mtj::comm_all_reduce(h->comm, h->part, static_cast<size_t>(M) * h->d, false, s, &err))
@@ -403,12 +424,14 @@ int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, c
 int32_t run_logits_tc(mtj_handle* h, int M, int row0, float* out, cudaStream_t s, bool pdl = false,
                       bool decode = false) {
   const bool hilo = decode && row0 == 0 && h->hilo_ok && M <= h->tc_hilo_max_b;
-  if (h->xn_ready && decode && row0 == 0)
-    h->xn_ready = false;            // the last layer's exchange applied the final LayerNorm already
-  else
+  if (h->xn_ready && decode && row0 == 0) {
+    h->xn_ready = false;            // the last layer's exchange or reduction applied the final LayerNorm already
+  } else {
+    h->launches++;
     MTJ_CUDA(mtj::launch_ln_rows(h->x + static_cast<size_t>(row0) * h->d, h->lnf_scale, h->lnf_offset,
                                  h->xn_bf16 + static_cast<size_t>(row0) * h->d, M, h->d, s, pdl,
                                  hilo ? h->xn_lo : nullptr));
+  }
   mtj::GemmTcArgs a = {};
   a.M = M;
   a.N = h->Vl;
@@ -421,13 +444,13 @@ int32_t run_logits_tc(mtj_handle* h, int M, int row0, float* out, cudaStream_t s
   a.cluster_k = (decode && h->tc_cluster_k) ? mtj::gemm_tc_decode_cluster_k(a.N, M, a.K) : 1;
   h->prof_begin(MTJ_FAMILY_LOGITS, s);
   a.pair = (h->tc_pair >> 2) & 1;
-  if (use_tc_wide(h, M))
-    MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiLogits, &h->map_proj, &h->map_xn_wide, a, s));
+  if (use_tc_wide(h, M, decode || h->same_sums))
+    MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiLogits, &h->map_proj, &h->map_xn_wide, &h->map_xn[1], a, s));
   else
     MTJ_CUDA(mtj::launch_gemm_tc(mtj::kEpiLogits, &h->map_proj, &h->map_xn[tc_tile_index(M)], a, s, pdl,
                                  hilo ? &h->map_xn_lo[tc_tile_index(M)] : nullptr));
   h->prof_end(s);
-  h->launches += 2;
+  h->launches++;
   return MTJ_OK;
 }
 
@@ -457,7 +480,7 @@ int32_t run_loss_rows_fused(mtj_handle* h, int n, int row0, const mtj::CeArgs& c
   a.dev_err = h->dev_err;
   h->prof_begin(MTJ_FAMILY_LOGITS, s);
   a.pair = (h->tc_pair >> 2) & 1;
-  MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiLogitsCE, &h->map_proj, &h->map_xn_wide, a, s));
+  MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiLogitsCE, &h->map_proj, &h->map_xn_wide, &h->map_xn[1], a, s));
   h->prof_end(s);
   mtj::CeArgs c2 = ce;
   c2.row0 = row0;
@@ -472,6 +495,7 @@ bool use_tc_decode(const mtj_handle* h, int B) { return h->tc_ok && B >= h->tc_d
 
 int32_t run_embed(mtj_handle* h, const uint32_t* ids, int ids_ld, int M, const mtj::RowMap& rows,
                   bool decode, cudaStream_t s, bool tc_decode = false) {
+  h->xn_ready = false;
   // batched decode at mp > 1: the rows go through the push exchange, which also applies layer 0's LayerNorm
   const bool push = tc_decode && use_push(h, M) && M <= kTcSplitRows;
   mtj::EmbedArgs e = {};
@@ -611,7 +635,7 @@ int32_t forward_chunks(mtj_handle* h, const uint32_t* ids, int ids_ld, int batch
         rc = h->stack ? h->stack->forward(h, ids, ids_ld, rows, M, rows, c.t0 - t_begin, false, s)
                       : run_embed(h, ids, ids_ld, M, rows, false, s);
         for (int l = 0; l < h->L && !rc && !h->stack; ++l)
-          rc = use_tc(h, M) ? run_layer_tc(h, l, M, rows, key_limit, s) : run_layer(h, l, M, rows, false, key_limit, s);
+          rc = use_tc(h, M) ? run_layer_tc(h, l, M, rows, key_limit, s, nullptr, false, false, true) : run_layer(h, l, M, rows, false, key_limit, s);
         if (!rc) rc = after_chunk(c.b0, c.ns, c.t0, c.tc);
       }
       continue;
@@ -1232,7 +1256,7 @@ int32_t mtj_admit(mtj_handle* h, int32_t slot, const uint32_t* prompt, int32_t l
     }
     rc = run_embed(h, prompt + t0, 0, M, ids_rows, false, s);
     for (int l = 0; l < h->L && !rc; ++l)
-      rc = use_tc(h, M) ? run_layer_tc(h, l, M, rows, nullptr, s) : run_layer(h, l, M, rows, false, nullptr, s);
+      rc = use_tc(h, M) ? run_layer_tc(h, l, M, rows, nullptr, s, nullptr, false, false, true) : run_layer(h, l, M, rows, false, nullptr, s);
   }
   return rc;
 }
@@ -1394,7 +1418,7 @@ int32_t mtj_decode_step(mtj_handle* h, const uint32_t* tokens_in, const float* t
       h->launches++;
     }
     for (int l = 0; !mega && !h->stack && l < h->L; ++l) {
-      r = tc ? run_layer_tc(h, l, B, rows, nullptr, st, nullptr, true) : run_layer(h, l, B, rows, true, nullptr, st);
+      r = tc ? run_layer_tc(h, l, B, rows, nullptr, st, nullptr, true, false, true) : run_layer(h, l, B, rows, true, nullptr, st);
       if (r) return r;
     }
     if (!mega) {
@@ -1559,6 +1583,7 @@ int32_t mtj_eval_loss(mtj_handle* h, const uint32_t* obs, const uint32_t* target
   rc = setup_sequences(h, pad, limit, T, s);
   if (rc) return rc;
   h->prefilled = false;
+  h->same_sums = true;
   rc = forward_chunks(h, obs, T, batch, T, h->key_limit, s, [&](int b0, int ns, int t0, int tc) -> int32_t {
     const int M = ns * tc;
     mtj::CeArgs ce = {};
@@ -1576,7 +1601,7 @@ int32_t mtj_eval_loss(mtj_handle* h, const uint32_t* obs, const uint32_t* target
     const int step = fused ? h->ce_rows : h->eval_rows;
     for (int m0 = 0; m0 < M; m0 += step) {
       const int n = std::min(step, M - m0);
-      if (fused && use_tc_wide(h, n)) {
+      if (fused && use_tc_wide(h, n, true)) {
         int32_t r3 = run_loss_rows_fused(h, n, m0, ce, s);
         if (r3) return r3;
         continue;
@@ -1604,6 +1629,7 @@ int32_t mtj_eval_loss(mtj_handle* h, const uint32_t* obs, const uint32_t* target
     h->launches += 2;
     return MTJ_OK;
   });
+  h->same_sums = false;
   return rc;
 }
 
@@ -1755,6 +1781,7 @@ int32_t mtj_k_layer(mtj_handle* h, int32_t layer, const float* x_in, int32_t bat
   rc = setup_sequences(h, pad, limit, pos0, s);
   if (rc) return rc;
   h->prefilled = false;
+  h->xn_ready = false;
   // x <- x_in with its LayerNorm statistics
   MTJ_CUDA(mtj::launch_residual_stats(h->x, x_in, h->stats, static_cast<int>(M), h->d, false, s, false));
   h->launches++;
@@ -1803,7 +1830,7 @@ int32_t mtj_k_projection_loss(mtj_handle* h, const float* x_in, const uint32_t* 
   const int step = fused ? h->ce_rows : h->eval_rows;
   for (int m0 = 0; m0 < rows; m0 += step) {
     const int n = std::min(step, rows - m0);
-    if (fused && use_tc_wide(h, n)) {
+    if (fused && use_tc_wide(h, n, true)) {
       rc = run_loss_rows_fused(h, n, m0, ce, s);
       if (rc) return rc;
       continue;

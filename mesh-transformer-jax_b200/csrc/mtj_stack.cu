@@ -19,6 +19,7 @@ int up8(int64_t v) { return static_cast<int>(align_up(v, 8)); }
 int up4(int v) { return (v + 3) & ~3; }
 constexpr int kAbsorbRows = 256;       // rows of the absorbed attention's scratch
 constexpr int kSelectGemvRows = 4;
+constexpr int kSplitPlanes = 8;        // most pieces of an output projection cut along K
 constexpr int kChunkedRows = 2 * kMatrixChunk;   // rows of a sequence from which matrix-state mixers work in chunks
 }  // namespace
 
@@ -294,6 +295,8 @@ void LayerStack::carve_workspace(Carver& c) {
     cat_ = c.take<float>(R * 2 * ld_);
   }
   if (!f32_) {
+    y_planes_elems_ = std::max<int64_t>(kWidePlaneFloats, static_cast<int64_t>(kSplitPlanes) * std::min<int64_t>(R, 192) * ld_);
+    y_planes_ = c.take<float>(y_planes_elems_);
     xn_bf_ = c.take<__nv_bfloat16>(R * ld_);
     sel_bf_ = c.take<__nv_bfloat16>(R * ld_);
     if (loop_times_ > 0) cat_bf_ = c.take<__nv_bfloat16>(R * 2 * ld_);
@@ -555,7 +558,7 @@ bool LayerStack::use_tc(const mtj_handle* h, int M, bool decode) const {
   return !f32_ && M >= (decode ? h->tc_decode_min_b : tc_min_rows_);
 }
 
-const TensorMap* LayerStack::xmap(const __nv_bfloat16* buf, int K, int ld, int M) {
+const TensorMap* LayerStack::xmap(const __nv_bfloat16* buf, int K, int ld, int tile) {
   const auto key = std::make_tuple(static_cast<const void*>(buf), K, ld);
   auto it = xmaps_.find(key);
   if (it == xmaps_.end()) {
@@ -565,13 +568,14 @@ const TensorMap* LayerStack::xmap(const __nv_bfloat16* buf, int K, int ld, int M
       if (make_tensor_map_bf16(&maps[i], buf, rows, K, 32 << i, ld) != cudaSuccess) return nullptr;
     it = xmaps_.emplace(key, maps).first;
   }
-  const int tile = M > 192 ? gemm_tc_wide_token_tile() : gemm_tc_token_tile_for(M);
   return &it->second[tile == 32 ? 0 : tile == 64 ? 1 : 2];
 }
 
 int32_t LayerStack::gemm(mtj_handle* h, GemvEpilogue epi, const Linear& l, const __nv_bfloat16* x, int M, float* out, int ld_out,
                          __nv_bfloat16* out_bf16, int ld_bf16, bool decode, cudaStream_t s, int x_row0, int x_ld, int f32_from) {
-  const TensorMap* mx = xmap(x, l.K, x_ld > 0 ? x_ld : l.ld, M);
+  const bool wide = gemm_tc_use_wide(M, decode || h->same_sums);
+  const int ldx = x_ld > 0 ? x_ld : l.ld;
+  const TensorMap* mx = xmap(x, l.K, ldx, wide ? gemm_tc_wide_token_tile() : gemm_tc_token_tile_for(M));
   if (!mx) return fail(MTJ_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   GemmTcArgs a = {};
   a.M = M;
@@ -587,8 +591,41 @@ int32_t LayerStack::gemm(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
   a.f32_from = f32_from;
   a.pair = 1;
   a.cluster_k = h->tc_cluster_k ? gemm_tc_decode_cluster_k(l.N, M, l.K) : 1;
-  if (M > 192) MTJ_CUDA(launch_gemm_tc_wide(epi, &l.map, mx, a, s));
+  if (wide) MTJ_CUDA(launch_gemm_tc_wide(epi, &l.map, mx, xmap(x, l.K, ldx, 64), a, s));
   else MTJ_CUDA(launch_gemm_tc(epi, &l.map, mx, a, s, decode && h->use_pdl && h->tc_pdl));
+  h->launches++;
+  return MTJ_OK;
+}
+
+int32_t LayerStack::gemm_out(mtj_handle* h, const Linear& l, int M, bool decode, cudaStream_t s) {
+  const bool wide = gemm_tc_use_wide(M, decode || h->same_sums);
+  int ks = 1;
+  if (l.N == ld_ && !h->same_sums) {                                  // the planes have the residual rows' stride
+    if (wide) {
+      ks = gemm_tc_wide_split(M, l.N, l.K);
+    } else {
+      // few rows: two blocks per SM, each with at least four k-blocks
+      const int bn = gemm_tc_token_tile_for(M), tiles = (l.N + 127) / 128 * ((M + bn - 1) / bn), nk = (l.K + 63) / 64;
+      ks = std::max(1, std::min({kSplitPlanes, 296 / tiles, nk / 4}));
+      while (ks > 1 && (ks - 1) * ((nk + ks - 1) / ks) >= nk) --ks;
+    }
+    while (ks > 1 && static_cast<int64_t>(ks) * M * l.N > y_planes_elems_) --ks;
+  }
+  y_count_ = ks;
+  y_from_ = ks > 1 ? y_planes_ : y_;
+  if (ks == 1) return gemm(h, kEpiPlain, l, act_bf_, M, y_, ld_, nullptr, 0, decode, s);
+  const TensorMap* mx = xmap(act_bf_, l.K, l.ld, wide ? gemm_tc_wide_token_tile() : gemm_tc_token_tile_for(M));
+  if (!mx) return fail(MTJ_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+  GemmTcArgs a = {};
+  a.M = M;
+  a.N = l.N;
+  a.K = l.K;
+  a.partial = y_planes_;
+  a.ksplit = ks;
+  a.dev_err = h->dev_err;
+  a.pair = 1;
+  if (wide) MTJ_CUDA(launch_gemm_tc_wide(kEpiPlain, &l.map, mx, xmap(act_bf_, l.K, l.ld, 64), a, s));
+  else MTJ_CUDA(launch_gemm_tc(kEpiPlain, &l.map, mx, a, s, decode && h->use_pdl && h->tc_pdl));
   h->launches++;
   return MTJ_OK;
 }
@@ -597,7 +634,7 @@ int32_t LayerStack::gemm(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
 int32_t LayerStack::gemm_planes(mtj_handle* h, const Linear& l, const __nv_bfloat16* x, int M, int* planes, bool decode,
                                 cudaStream_t s) {
   const int bn = gemm_tc_token_tile_for(M);
-  const auto key = xmap(x, l.K, l.ld, std::min(M, 128));
+  const auto key = xmap(x, l.K, l.ld, bn);
   if (!key) return fail(MTJ_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   const int tiles = ((l.N + 127) / 128) * ((M + bn - 1) / bn);
   const int64_t fit = xp_planes_elems_ / (static_cast<int64_t>(M) * l.N);
@@ -728,7 +765,7 @@ int32_t LayerStack::mamba(mtj_handle* h, const Run& r, int M, const RowMap& rows
   h->launches++;
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
-  if (tc) MTJ_DO(gemm(h, kEpiPlain, l.out, act_bf_, M, y_, ld_, nullptr, 0, decode, s));
+  if (tc) MTJ_DO(gemm_out(h, l.out, M, decode, s));
   else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, nullptr, y_, ld_, &post, pdl, s));
   h->prof_end(s);
   return MTJ_OK;
@@ -818,7 +855,7 @@ int32_t LayerStack::latent(mtj_handle* h, const Run& r, int M, const RowMap& row
   }
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
-  if (tc) MTJ_DO(gemm(h, kEpiPlain, l.out, act_bf_, M, y_, ld_, nullptr, 0, decode, s));
+  if (tc) MTJ_DO(gemm_out(h, l.out, M, decode, s));
   else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, nullptr, y_, ld_, &post, pdl, s));
   h->prof_end(s);
   return MTJ_OK;
@@ -901,7 +938,7 @@ int32_t LayerStack::grouped(mtj_handle* h, const Run& r, int M, const RowMap& ro
   }
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
-  if (tc) MTJ_DO(gemm(h, kEpiPlain, l.out, act_bf_, M, y_, ld_, nullptr, 0, decode, s));
+  if (tc) MTJ_DO(gemm_out(h, l.out, M, decode, s));
   else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, nullptr, y_, ld_, &post, pdl, s));
   h->prof_end(s);
   return MTJ_OK;
@@ -1002,7 +1039,7 @@ int32_t LayerStack::matrix(mtj_handle* h, const Run& r, int M, const RowMap& row
   h->launches += (normed ? 1 : 2) + (!step && tc && rows.Tc >= kChunkedRows ? 1 : 0);
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
-  if (tc) MTJ_DO(gemm(h, kEpiPlain, l.out, act_bf_, M, y_, ld_, nullptr, 0, decode, s));
+  if (tc) MTJ_DO(gemm_out(h, l.out, M, decode, s));
   else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, nullptr, y_, ld_, &post, pdl, s));
   h->prof_end(s);
   return MTJ_OK;
@@ -1049,6 +1086,7 @@ int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, cons
       a.d = d_;
       a.ld = ld_;
       a.y = y;
+      a.planes = y ? y_count_ : 1;
       a.w = post.w;
       a.b = post.b;
       a.alpha = mult_;
@@ -1069,7 +1107,7 @@ int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, cons
     a.d = d_;
     a.ld = ld_;
     a.y = y;
-    a.planes = 1;
+    a.planes = y ? y_count_ : 1;
     a.w_post = post.w;
     a.mult = mult_;
     a.eps = eps_;
@@ -1087,7 +1125,7 @@ int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, cons
     return MTJ_OK;
   };
   auto after = [&](const Post& post, const Next& n) -> int32_t {
-    if (tc) return settle(y_, post, n);
+    if (tc) return settle(y_from_, post, n);
     return n.pass ? settle(nullptr, Post{}, n) : MTJ_OK;
   };
   if (!post_ln_) MTJ_DO(settle(nullptr, Post{}, next_run(0)));
@@ -1117,7 +1155,7 @@ int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, cons
       else MTJ_DO(gemv(h, act, l.gate_up, x_, ld_, M, post_ln_ ? nullptr : l.norm2, act_, l.down.ld, nullptr, pdl, s));
       h->prof_end(s);
       h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
-      if (tc) MTJ_DO(gemm(h, kEpiPlain, l.down, act_bf_, M, y_, ld_, nullptr, 0, decode, s));
+      if (tc) MTJ_DO(gemm_out(h, l.down, M, decode, s));
       else MTJ_DO(gemv(h, kEpiOut, l.down, act_, l.down.ld, M, nullptr, y_, ld_, &post2, pdl, s));
       h->prof_end(s);
       MTJ_DO(after(post2, after_layer));

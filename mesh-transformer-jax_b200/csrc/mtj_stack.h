@@ -100,9 +100,11 @@ class LayerStack {
   enum { kRows, kF32, kNegExp, kTransposeF32 };
 
   bool use_tc(const mtj_handle* h, int M, bool decode) const;
-  const TensorMap* xmap(const __nv_bfloat16* buf, int K, int ld, int M);
+  const TensorMap* xmap(const __nv_bfloat16* buf, int K, int ld, int tile);
   int32_t gemm(mtj_handle* h, GemvEpilogue epi, const Linear& l, const __nv_bfloat16* x, int M, float* out, int ld_out,
                __nv_bfloat16* out_bf16, int ld_bf16, bool decode, cudaStream_t s, int x_row0 = 0, int x_ld = 0, int f32_from = 0);
+  // a sublayer's output projection: into y_, or cut along K into planes that the residual kernel adds (y_from_, y_count_)
+  int32_t gemm_out(mtj_handle* h, const Linear& l, int M, bool decode, cudaStream_t s);
   int32_t gemm_planes(mtj_handle* h, const Linear& l, const __nv_bfloat16* x, int M, int* planes, bool decode, cudaStream_t s);
   int32_t gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const float* x, int ldx, int M, const float* norm, float* out,
                int ld_out, const Post* post, bool pdl, cudaStream_t s, const int32_t* select = nullptr,
@@ -136,7 +138,9 @@ class LayerStack {
   int rows_a_ = 0, lin_rows_ = 0, ld_p1_ = 0, ld_act_ = 0;
   int64_t xp_planes_elems_ = 0;
   bool last_tc_ = false;
-  float *x_ = nullptr, *x0_ = nullptr, *stats_ = nullptr, *cat_ = nullptr, *y_ = nullptr, *p1_ = nullptr, *u_ = nullptr, *xp_ = nullptr,
+  int y_count_ = 1;
+  int64_t y_planes_elems_ = 0;
+  float *x_ = nullptr, *x0_ = nullptr, *stats_ = nullptr, *cat_ = nullptr, *y_ = nullptr, *y_planes_ = nullptr, *y_from_ = nullptr, *p1_ = nullptr, *u_ = nullptr, *xp_ = nullptr,
         *dt_raw_ = nullptr, *gate_raw_ = nullptr, *aux_ = nullptr, *mix_ = nullptr, *q_f32_ = nullptr, *act_ = nullptr, *xp_planes_ = nullptr, *q_abs_ = nullptr, *part_o_ = nullptr, *part_ml_ = nullptr;
   __nv_bfloat16 *xn_bf_ = nullptr, *cat_bf_ = nullptr, *xz_bf_ = nullptr, *u_bf_ = nullptr, *dtr_bf_ = nullptr, *act_bf_ = nullptr,
                 *sel_bf_ = nullptr, *q_pack_ = nullptr, *c_lin_ = nullptr, *kr_lin_ = nullptr, *kv_lin_ = nullptr, *gate_bf_ = nullptr;

@@ -28,6 +28,163 @@ __device__ __forceinline__ uint2 pack4(const float4& v) {
   return make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
 }
 
+// The row kernels in two forms: rows of up to 8192 columns in registers (HOLD float4 a thread), every load of the row and
+// of the planes issued before the first sum, because with few rows the kernel is nothing but the latency of its loads
+// and sums (8 rows of 4096 in 8 planes: 12.4 us through shared memory); wider rows in shared memory.  Both add in the
+// same order.
+constexpr int kRegThreads = 256, kRegHold = 8;
+
+// the sum of the planes of row m, in order
+template <int HOLD>
+__device__ __forceinline__ void load_planes(const float* y, int planes, size_t m, int M, int ld, int n4, float4 (&v)[HOLD]) {
+  const size_t step = static_cast<size_t>(M) * ld / 4;
+  const float4* src = reinterpret_cast<const float4*>(y + m * ld);
+#pragma unroll
+  for (int i = 0; i < HOLD; ++i) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int p = 0; p < planes; ++p) {
+#pragma unroll
+    for (int i = 0; i < HOLD; ++i) {
+      const int c = i * kRegThreads + threadIdx.x;
+      const float4 w = c < n4 ? __ldcg(src + p * step + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[i].x += w.x; v[i].y += w.y; v[i].z += w.z; v[i].w += w.w;
+    }
+  }
+}
+template <int HOLD>
+__device__ __forceinline__ void load_row(const float* row, int n4, float4 (&v)[HOLD]) {
+#pragma unroll
+  for (int i = 0; i < HOLD; ++i) {
+    const int c = i * kRegThreads + threadIdx.x;
+    v[i] = row && c < n4 ? reinterpret_cast<const float4*>(row)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
+template <int HOLD>
+__global__ void __launch_bounds__(kRegThreads) residual_norm_reg_kernel(const ResidualNormArgs a) {
+  __shared__ float red[kRegThreads / 32];
+  const int n4 = a.ld >> 2;
+  const size_t m = blockIdx.x;
+  float4 wp[HOLD], wn[HOLD], x[HOLD];
+  load_row<HOLD>(a.y ? a.w_post : nullptr, n4, wp);          // weights do not depend on the predecessor
+  load_row<HOLD>(a.xn ? a.w_next : nullptr, n4, wn);
+  pdl_wait();
+  pdl_launch_dependents();
+  float4* xrow = reinterpret_cast<float4*>(a.x + m * a.ld);
+  load_row<HOLD>(a.x + m * a.ld, n4, x);
+  float ss = 0.f;
+  if (a.y) {
+    float4 y[HOLD];
+    load_planes<HOLD>(a.y, a.planes, m, a.M, a.ld, n4, y);
+    float ys = 0.f;
+#pragma unroll
+    for (int i = 0; i < HOLD; ++i) ys += dot4(y[i]);
+    const float rs = a.mult / sqrtf(rn_block_sum(ys, red) / static_cast<float>(a.d) + a.eps);
+#pragma unroll
+    for (int i = 0; i < HOLD; ++i) {
+      const int c = i * kRegThreads + threadIdx.x;
+      x[i] = make_float4(fmaf(y[i].x * rs, wp[i].x, x[i].x), fmaf(y[i].y * rs, wp[i].y, x[i].y), fmaf(y[i].z * rs, wp[i].z, x[i].z),
+                         fmaf(y[i].w * rs, wp[i].w, x[i].w));
+      if (c < n4) xrow[c] = x[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < HOLD; ++i) ss += dot4(x[i]);
+  const float rs = 1.0f / sqrtf(rn_block_sum(ss, red) / static_cast<float>(a.d) + a.eps);
+  if (a.stats && threadIdx.x == 0) {
+    a.stats[2 * m] = 0.f;
+    a.stats[2 * m + 1] = rs;
+  }
+#pragma unroll
+  for (int i = 0; i < HOLD; ++i) {
+    const int c = i * kRegThreads + threadIdx.x;
+    if (c >= n4) continue;
+    const float4 v = x[i], w = wn[i];
+    if (a.xn) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(make_float4(v.x * rs * w.x, v.y * rs * w.y, v.z * rs * w.z, v.w * rs * w.w));
+    if (a.cat_f32 || a.cat_bf16) {
+      const float4 e = reinterpret_cast<const float4*>(a.x0 + m * a.ld)[c];
+      if (a.cat_f32) {
+        float4* o = reinterpret_cast<float4*>(a.cat_f32 + m * 2 * a.ld);
+        o[c] = v;
+        o[n4 + c] = e;
+      }
+      if (a.cat_bf16) {
+        uint2* o = reinterpret_cast<uint2*>(a.cat_bf16 + m * 2 * a.ld);
+        o[c] = pack4(v);
+        o[n4 + c] = pack4(e);
+      }
+    }
+  }
+}
+
+template <int HOLD>
+__global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(const ResidualLayerNormArgs a) {
+  __shared__ float red[kRegThreads / 32];
+  const int n4 = a.ld >> 2;
+  const size_t m = blockIdx.x;
+  const float inv_n = 1.0f / static_cast<float>(a.d);
+  float4 w[HOLD], b[HOLD], x[HOLD];
+  load_row<HOLD>(a.y ? a.w : nullptr, n4, w);                // weights do not depend on the predecessor
+  load_row<HOLD>(a.y ? a.b : nullptr, n4, b);
+  pdl_wait();
+  pdl_launch_dependents();
+  float4* xrow = reinterpret_cast<float4*>(a.x + m * a.ld);
+  auto norm = [&](float* mu, float* rs) {
+    float s = 0.f, q = 0.f;
+#pragma unroll
+    for (int i = 0; i < HOLD; ++i) s += (x[i].x + x[i].y) + (x[i].z + x[i].w);
+    *mu = rn_block_sum(s, red) * inv_n;
+#pragma unroll
+    for (int i = 0; i < HOLD; ++i) {
+      const int left = a.d - 4 * (i * kRegThreads + static_cast<int>(threadIdx.x));      // columns that exist
+      q += dot4(make_float4(left > 0 ? x[i].x - *mu : 0.f, left > 1 ? x[i].y - *mu : 0.f, left > 2 ? x[i].z - *mu : 0.f, left > 3 ? x[i].w - *mu : 0.f));
+    }
+    *rs = 1.0f / sqrtf(rn_block_sum(q, red) * inv_n + a.eps);
+  };
+  auto scaled = [](const float4& z, float mu, float rs, const float4& w4, const float4& b4) {
+    return make_float4(fmaf((z.x - mu) * rs, w4.x, b4.x), fmaf((z.y - mu) * rs, w4.y, b4.y), fmaf((z.z - mu) * rs, w4.z, b4.z),
+                       fmaf((z.w - mu) * rs, w4.w, b4.w));
+  };
+  float mu, rs;
+  load_row<HOLD>(a.x + m * a.ld, n4, x);
+  if (a.y) {
+    float4 y[HOLD];
+    load_planes<HOLD>(a.y, a.planes, m, a.M, a.ld, n4, y);
+#pragma unroll
+    for (int i = 0; i < HOLD; ++i)
+      x[i] = make_float4(fmaf(a.alpha, x[i].x, y[i].x), fmaf(a.alpha, x[i].y, y[i].y), fmaf(a.alpha, x[i].z, y[i].z), fmaf(a.alpha, x[i].w, y[i].w));
+    norm(&mu, &rs);
+#pragma unroll
+    for (int i = 0; i < HOLD; ++i) {
+      const int c = i * kRegThreads + threadIdx.x;
+      x[i] = scaled(x[i], mu, rs, w[i], b[i]);               // w and b are zero in the padding and past the row
+      if (c < n4) xrow[c] = x[i];
+    }
+  }
+  if (a.xn && !a.w_next) {
+#pragma unroll
+    for (int i = 0; i < HOLD; ++i) {
+      const int c = i * kRegThreads + threadIdx.x;
+      if (c < n4) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(x[i]);
+    }
+  }
+  if (!a.w_next && !a.stats) return;
+  norm(&mu, &rs);
+  if (a.stats && threadIdx.x == 0) {
+    a.stats[2 * m] = mu;
+    a.stats[2 * m + 1] = rs;
+  }
+  if (a.xn && a.w_next) {
+    load_row<HOLD>(a.w_next, n4, w);
+    load_row<HOLD>(a.b_next, n4, b);
+#pragma unroll
+    for (int i = 0; i < HOLD; ++i) {
+      const int c = i * kRegThreads + threadIdx.x;
+      if (c < n4) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(scaled(x[i], mu, rs, w[i], b[i]));
+    }
+  }
+}
+
 // Norm after the sublayer, residual add and the norm before the next sublayer, one pass over the row.  Every thread
 // touches only the columns it owns, so the row lives in shared memory without barriers between the passes.
 __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const ResidualNormArgs a) {
@@ -44,6 +201,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const Residua
     float ys = 0.f;
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
       float4 v = reinterpret_cast<const float4*>(a.y + m * a.ld)[i];
+#pragma unroll 4
       for (int p = 1; p < a.planes; ++p) {
         const float4 w = reinterpret_cast<const float4*>(a.y + (static_cast<size_t>(p) * a.M + m) * a.ld)[i];
         v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
@@ -130,7 +288,12 @@ __global__ void __launch_bounds__(kRnThreads) residual_layernorm_kernel(const Re
   for (int i = threadIdx.x; i < n4; i += kRnThreads) {
     float4 x = xrow[i];
     if (a.y) {
-      const float4 y = reinterpret_cast<const float4*>(a.y + m * a.ld)[i];
+      float4 y = reinterpret_cast<const float4*>(a.y + m * a.ld)[i];
+#pragma unroll 4
+      for (int p = 1; p < a.planes; ++p) {
+        const float4 w = reinterpret_cast<const float4*>(a.y + (static_cast<size_t>(p) * a.M + m) * a.ld)[i];
+        y.x += w.x; y.y += w.y; y.z += w.z; y.w += w.w;
+      }
       x = make_float4(fmaf(a.alpha, x.x, y.x), fmaf(a.alpha, x.y, y.y), fmaf(a.alpha, x.z, y.z), fmaf(a.alpha, x.w, y.w));
     }
     rn_row[i] = x;
@@ -206,6 +369,10 @@ int load_grid(int64_t n) { return static_cast<int>(std::min<int64_t>((n + 255) /
 
 cudaError_t launch_residual_norm(const ResidualNormArgs& a, cudaStream_t s, bool pdl) {
   if (a.M <= 0 || a.d <= 0 || a.ld < a.d || (a.ld & 3)) return cudaErrorInvalidValue;
+  const dim3 grid(a.M), block(kRegThreads);
+  if (a.ld <= 8 * kRegThreads) return launch_pdl(residual_norm_reg_kernel<2>, grid, block, 0, s, pdl, a);
+  if (a.ld <= 16 * kRegThreads) return launch_pdl(residual_norm_reg_kernel<4>, grid, block, 0, s, pdl, a);
+  if (a.ld <= 4 * kRegHold * kRegThreads) return launch_pdl(residual_norm_reg_kernel<kRegHold>, grid, block, 0, s, pdl, a);
   const size_t smem = static_cast<size_t>(a.ld) * sizeof(float) * (a.y ? 2 : 1);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   static DeviceOnce once;
@@ -218,6 +385,10 @@ cudaError_t launch_residual_norm(const ResidualNormArgs& a, cudaStream_t s, bool
 
 cudaError_t launch_residual_layernorm(const ResidualLayerNormArgs& a, cudaStream_t s, bool pdl) {
   if (a.M <= 0 || a.d <= 0 || a.ld < a.d || (a.ld & 3) || (a.y && (!a.w || !a.b)) || (a.w_next && !a.b_next)) return cudaErrorInvalidValue;
+  const dim3 grid(a.M), block(kRegThreads);
+  if (a.ld <= 8 * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<2>, grid, block, 0, s, pdl, a);
+  if (a.ld <= 16 * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<4>, grid, block, 0, s, pdl, a);
+  if (a.ld <= 4 * kRegHold * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<kRegHold>, grid, block, 0, s, pdl, a);
   const size_t smem = static_cast<size_t>(a.ld) * sizeof(float);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   static DeviceOnce once;

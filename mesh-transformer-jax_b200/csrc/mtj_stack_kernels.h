@@ -9,21 +9,6 @@
 
 namespace mtj {
 
-template <typename K, typename... A>
-cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // ---- mtj_stack_kernels.cu
 // One row per block:  y = sum of the planes;  x += mult * RMSNorm(y) * w_post (y may be null);  then, of the new x:
 // stats = (0, 1 / rms), xn = RMSNorm(x) * w_next in bf16, and cat = [x | x0] for the projection at the start of a pass.
@@ -42,12 +27,13 @@ struct ResidualNormArgs {
   __nv_bfloat16* cat_bf16;     // [M, 2 ld] or null
 };
 cudaError_t launch_residual_norm(const ResidualNormArgs& a, cudaStream_t s, bool pdl);
-// One row per block:  x = LayerNorm(alpha * x + y) * w + b;  then xn = x in bf16, or, with w_next, the layer norm of the
+// One row per block:  y = sum of the planes;  x = LayerNorm(alpha * x + y) * w + b;  then xn = x in bf16, or, with w_next, the layer norm of the
 // new x in bf16, and its (mean, 1 / deviation) into stats.  y == null: x stays, only what follows is done.
 struct ResidualLayerNormArgs {
   float* x;                    // [M, ld]; columns d .. ld - 1 of every buffer here are zero
   int M, d, ld;
-  const float* y;              // [M, ld] or null
+  const float* y;              // [planes, M, ld] or null
+  int planes;
   const float *w, *b;          // [ld]
   float alpha, eps;
   __nv_bfloat16* xn;           // [M, ld] or null
