@@ -98,6 +98,13 @@ struct GemvArgs {
 
 cudaError_t launch_gemv(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl);
 
+// The same product for 5 rows and more on the CUDA cores, fp32 activations and sums (mtj_gemm_rows.cu): every epilogue but
+// the in-projection's, no residual, no norm behind it.  planes and counters (zero between launches) are scratch of
+// kGemmRowsPlaneFloats and kGemmRowsCounters elements; one launch at a time may use them.
+constexpr int64_t kGemmRowsPlaneFloats = 4 << 20;
+constexpr int kGemmRowsCounters = 1024, kGemmRowsMin = 5;
+cudaError_t launch_gemm_rows(GemvEpilogue epi, const GemvArgs& a, float* planes, uint32_t* counters, cudaStream_t s, bool pdl);
+
 struct EmbedArgs {
   // id of row m = ids[(rows.b0 + m / rows.Tc) * ids_ld + rows.pos0_host + m % rows.Tc]
   const uint32_t* ids;

@@ -289,6 +289,8 @@ void LayerStack::carve_workspace(Carver& c) {
   part_o_ = c.take<float>(std::max((rows_a_ + kLatentBlocks) * po, gpo));
   part_ml_ = c.take<float>(std::max((rows_a_ + kLatentBlocks) * ml * 2, gml));
   counters_ = c.take<uint32_t>(R);
+  rows_planes_ = c.take<float>(kGemmRowsPlaneFloats);
+  rows_counters_ = c.take<uint32_t>(kGemmRowsCounters);
   attn_counters_ = c.take<uint32_t>(cnt);
   if (loop_times_ > 0) {
     x0_ = c.take<float>(R * ld_);
@@ -672,6 +674,42 @@ int32_t LayerStack::gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
   if (epi == kEpiSwiGLU || epi == kEpiRelu2) a.act2 = out;
   else if (epi == kEpiLogits) { a.logits = out; a.ld_logits = ld_out; a.softcap = l.w == head_.w ? softcap_ : 0.f; }
   else a.out = out;
+  if (M >= kGemmRowsMin) {
+    MTJ_CUDA(launch_gemm_rows(epi, a, rows_planes_, rows_counters_, s, pdl));
+    h->launches++;
+    if (!post) return MTJ_OK;
+    // what the GEMV's last block does behind the product
+    if (post->b) {
+      ResidualLayerNormArgs r = {};
+      r.x = x_;
+      r.M = M;
+      r.d = d_;
+      r.ld = ld_;
+      r.y = out;
+      r.planes = 1;
+      r.w = post->w;
+      r.b = post->b;
+      r.alpha = mult_;
+      r.eps = eps_;
+      r.stats = post->stats ? stats_ : nullptr;
+      MTJ_CUDA(launch_residual_layernorm(r, s, pdl));
+    } else {
+      ResidualNormArgs r = {};
+      r.x = x_;
+      r.M = M;
+      r.d = d_;
+      r.ld = ld_;
+      r.y = out;
+      r.planes = 1;
+      r.w_post = post->w;
+      r.mult = mult_;
+      r.eps = eps_;
+      r.stats = stats_;
+      MTJ_CUDA(launch_residual_norm(r, s, pdl));
+    }
+    h->launches++;
+    return MTJ_OK;
+  }
   if (post) {
     a.post_w = post->w;
     a.post_b = post->b;
@@ -694,6 +732,12 @@ int32_t LayerStack::gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
     if (_rc) return _rc;                   \
   } while (0)
 
+namespace {
+// Kernels chained by programmatic launch: in decode, and wherever few rows make a pass of 47 short kernels (5 to 20 rows of
+// width 2048: 3 us between kernels without).
+bool chained(const mtj_handle* h, bool tc, bool decode) { return h->use_pdl && (decode || !tc); }
+}  // namespace
+
 int32_t LayerStack::project_in(mtj_handle* h, const Linear& l, const float* norm, int M, float* out, int ld_out, bool pdl, cudaStream_t s) {
   return post_ln_ ? gemv(h, kEpiOut, l, x_, ld_, M, nullptr, out, ld_out, nullptr, pdl, s)
                   : gemv(h, kEpiLogits, l, x_, ld_, M, norm, out, ld_out, nullptr, pdl, s);
@@ -702,7 +746,7 @@ int32_t LayerStack::project_in(mtj_handle* h, const Linear& l, const float* norm
 int32_t LayerStack::mamba(mtj_handle* h, const Run& r, int M, const RowMap& rows, bool tc, bool decode, const Post& post, cudaStream_t s) {
   Layer& l = layers_[r.layer];
   const mtj_layer_desc& m = l.d;
-  const bool pdl = decode && h->use_pdl;
+  const bool pdl = chained(h, tc, decode);
   SsmArgs a = {};
   a.M = M;
   a.inner = m.inner;
@@ -775,7 +819,7 @@ int32_t LayerStack::latent(mtj_handle* h, const Run& r, int M, const RowMap& row
                            cudaStream_t s) {
   Layer& l = layers_[r.layer];
   const mtj_layer_desc& m = l.d;
-  const bool pdl = decode && h->use_pdl;
+  const bool pdl = chained(h, tc, decode);
   LatentArgs a = {};
   a.M = M;
   a.heads = m.heads;
@@ -864,7 +908,7 @@ int32_t LayerStack::latent(mtj_handle* h, const Run& r, int M, const RowMap& row
 int32_t LayerStack::grouped(mtj_handle* h, const Run& r, int M, const RowMap& rows, bool tc, bool decode, const Post& post, cudaStream_t s) {
   Layer& l = layers_[r.layer];
   const mtj_layer_desc& m = l.d;
-  const bool pdl = decode && h->use_pdl;
+  const bool pdl = chained(h, tc, decode);
   GroupedAttnArgs a = {};
   a.M = M;
   a.heads = m.heads;
@@ -947,7 +991,7 @@ int32_t LayerStack::grouped(mtj_handle* h, const Run& r, int M, const RowMap& ro
 int32_t LayerStack::matrix(mtj_handle* h, const Run& r, int M, const RowMap& rows, bool tc, bool decode, const Post& post, cudaStream_t s) {
   Layer& l = layers_[r.layer];
   const mtj_layer_desc& m = l.d;
-  const bool pdl = decode && h->use_pdl, ssd = m.mixer == MTJ_MIXER_MATRIX_STATE_SSD;
+  const bool pdl = chained(h, tc, decode), ssd = m.mixer == MTJ_MIXER_MATRIX_STATE_SSD;
   const int ld_p = up8(l.in.N), inner = m.heads * m.vdim, keys = m.kv_heads * m.dim;
   // the input projection: convolution inputs, gates and low-rank parts in bf16, step sizes and update strengths in fp32
   const float* aux = tc ? aux_ : p1_ + l.aux0;
@@ -1049,7 +1093,7 @@ int32_t LayerStack::matrix(mtj_handle* h, const Run& r, int M, const RowMap& row
 int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, const RowMap& id_rows, int M, const RowMap& rows,
                             int hist, bool decode, cudaStream_t s) {
   if (M <= 0 || M > R_ || M % rows.Tc) return fail(MTJ_ERR_INVALID, "rows exceed max_rows");
-  const bool tc = use_tc(h, M, decode), pdl = decode && h->use_pdl;
+  const bool tc = use_tc(h, M, decode), pdl = chained(h, tc, decode);
   last_tc_ = tc;
   EmbedArgs e = {};
   e.ids = ids;

@@ -138,6 +138,8 @@ class LayerStack {
   int rows_a_ = 0, lin_rows_ = 0, ld_p1_ = 0, ld_act_ = 0;
   int64_t xp_planes_elems_ = 0;
   bool last_tc_ = false;
+  float* rows_planes_ = nullptr;       // scratch of launch_gemm_rows
+  uint32_t* rows_counters_ = nullptr;
   int y_count_ = 1;
   int64_t y_planes_elems_ = 0;
   float *x_ = nullptr, *x0_ = nullptr, *stats_ = nullptr, *cat_ = nullptr, *y_ = nullptr, *y_planes_ = nullptr, *y_from_ = nullptr, *p1_ = nullptr, *u_ = nullptr, *xp_ = nullptr,
