@@ -98,6 +98,9 @@ struct GemvArgs {
 
 cudaError_t launch_gemv(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl);
 
+// The same for one row and long weight rows, streamed by one block per SM (mtj_gemv_stream.cu).
+bool gemv_stream_ok(GemvEpilogue epi, const GemvArgs& a);
+cudaError_t launch_gemv_stream(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl);
 // The same product for 5 rows and more on the CUDA cores, fp32 activations and sums (mtj_gemm_rows.cu): every epilogue but
 // the in-projection's, no residual, no norm behind it.  planes and counters (zero between launches) are scratch of
 // kGemmRowsPlaneFloats and kGemmRowsCounters elements; one launch at a time may use them.

@@ -720,7 +720,8 @@ int32_t LayerStack::gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
     a.stats_out = post->stats ? stats_ : nullptr;
     a.counters = counters_;
   }
-  MTJ_CUDA(launch_gemv(epi, a, s, pdl));
+  if (gemv_stream_ok(epi, a)) MTJ_CUDA(launch_gemv_stream(epi, a, s, pdl));
+  else MTJ_CUDA(launch_gemv(epi, a, s, pdl));
   h->launches++;
   return MTJ_OK;
 }
