@@ -28,6 +28,13 @@ __device__ __forceinline__ uint2 pack4(const float4& v) {
   return make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
 }
 
+// Columns from `left` on are padding and stay zero for good, whatever the row holds: a norm of a row that is not finite
+// would make them NaN, and the embedding, which opens the next call, writes the columns that exist only.
+__device__ __forceinline__ float4 keep(float4 v, int left) {
+  if (left < 4) v = make_float4(left > 0 ? v.x : 0.f, left > 1 ? v.y : 0.f, left > 2 ? v.z : 0.f, 0.f);
+  return v;
+}
+
 // The row kernels in two forms: rows of up to 8192 columns in registers (HOLD float4 a thread), every load of the row and
 // of the planes issued before the first sum, because with few rows the kernel is nothing but the latency of its loads
 // and sums (8 rows of 4096 in 8 planes: 12.4 us through shared memory); wider rows in shared memory.  Both add in the
@@ -83,8 +90,8 @@ __global__ void __launch_bounds__(kRegThreads) residual_norm_reg_kernel(const Re
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
       const int c = i * kRegThreads + threadIdx.x;
-      x[i] = make_float4(fmaf(y[i].x * rs, wp[i].x, x[i].x), fmaf(y[i].y * rs, wp[i].y, x[i].y), fmaf(y[i].z * rs, wp[i].z, x[i].z),
-                         fmaf(y[i].w * rs, wp[i].w, x[i].w));
+      x[i] = keep(make_float4(fmaf(y[i].x * rs, wp[i].x, x[i].x), fmaf(y[i].y * rs, wp[i].y, x[i].y), fmaf(y[i].z * rs, wp[i].z, x[i].z),
+                              fmaf(y[i].w * rs, wp[i].w, x[i].w)), a.d - 4 * c);
       if (c < n4) xrow[c] = x[i];
     }
   }
@@ -100,7 +107,7 @@ __global__ void __launch_bounds__(kRegThreads) residual_norm_reg_kernel(const Re
     const int c = i * kRegThreads + threadIdx.x;
     if (c >= n4) continue;
     const float4 v = x[i], w = wn[i];
-    if (a.xn) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(make_float4(v.x * rs * w.x, v.y * rs * w.y, v.z * rs * w.z, v.w * rs * w.w));
+    if (a.xn) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(keep(make_float4(v.x * rs * w.x, v.y * rs * w.y, v.z * rs * w.z, v.w * rs * w.w), a.d - 4 * c));
     if (a.cat_f32 || a.cat_bf16) {
       const float4 e = reinterpret_cast<const float4*>(a.x0 + m * a.ld)[c];
       if (a.cat_f32) {
@@ -141,9 +148,9 @@ __global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(con
     }
     *rs = 1.0f / sqrtf(rn_block_sum(q, red) * inv_n + a.eps);
   };
-  auto scaled = [](const float4& z, float mu, float rs, const float4& w4, const float4& b4) {
-    return make_float4(fmaf((z.x - mu) * rs, w4.x, b4.x), fmaf((z.y - mu) * rs, w4.y, b4.y), fmaf((z.z - mu) * rs, w4.z, b4.z),
-                       fmaf((z.w - mu) * rs, w4.w, b4.w));
+  auto scaled = [&](int c, const float4& z, float mu, float rs, const float4& w4, const float4& b4) {
+    return keep(make_float4(fmaf((z.x - mu) * rs, w4.x, b4.x), fmaf((z.y - mu) * rs, w4.y, b4.y), fmaf((z.z - mu) * rs, w4.z, b4.z),
+                            fmaf((z.w - mu) * rs, w4.w, b4.w)), a.d - 4 * c);
   };
   float mu, rs;
   load_row<HOLD>(a.x + m * a.ld, n4, x);
@@ -157,7 +164,7 @@ __global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(con
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
       const int c = i * kRegThreads + threadIdx.x;
-      x[i] = scaled(x[i], mu, rs, w[i], b[i]);               // w and b are zero in the padding and past the row
+      x[i] = scaled(c, x[i], mu, rs, w[i], b[i]);
       if (c < n4) xrow[c] = x[i];
     }
   }
@@ -180,7 +187,7 @@ __global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(con
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
       const int c = i * kRegThreads + threadIdx.x;
-      if (c < n4) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(scaled(x[i], mu, rs, w[i], b[i]));
+      if (c < n4) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(scaled(c, x[i], mu, rs, w[i], b[i]));
     }
   }
 }
@@ -218,6 +225,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const Residua
       x.y = fmaf(y.y * rs, w.y, x.y);
       x.z = fmaf(y.z * rs, w.z, x.z);
       x.w = fmaf(y.w * rs, w.w, x.w);
+      x = keep(x, a.d - 4 * i);
       rn_row[i] = x;
       xrow[i] = x;
       ss += dot4(x);
@@ -238,7 +246,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const Residua
     uint2* o = reinterpret_cast<uint2*>(a.xn + m * a.ld);
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
       const float4 x = rn_row[i], w = reinterpret_cast<const float4*>(a.w_next)[i];
-      o[i] = pack4(make_float4(x.x * rs * w.x, x.y * rs * w.y, x.z * rs * w.z, x.w * rs * w.w));
+      o[i] = pack4(keep(make_float4(x.x * rs * w.x, x.y * rs * w.y, x.z * rs * w.z, x.w * rs * w.w), a.d - 4 * i));
     }
   }
   if (a.cat_f32 || a.cat_bf16) {
@@ -281,8 +289,8 @@ __global__ void __launch_bounds__(kRnThreads) residual_layernorm_kernel(const Re
   };
   auto scaled = [&](int i, float mu, float rs, const float* w, const float* b) {
     const float4 z = rn_row[i], w4 = reinterpret_cast<const float4*>(w)[i], b4 = reinterpret_cast<const float4*>(b)[i];
-    return make_float4(fmaf((z.x - mu) * rs, w4.x, b4.x), fmaf((z.y - mu) * rs, w4.y, b4.y), fmaf((z.z - mu) * rs, w4.z, b4.z),
-                       fmaf((z.w - mu) * rs, w4.w, b4.w));
+    return keep(make_float4(fmaf((z.x - mu) * rs, w4.x, b4.x), fmaf((z.y - mu) * rs, w4.y, b4.y), fmaf((z.z - mu) * rs, w4.z, b4.z),
+                            fmaf((z.w - mu) * rs, w4.w, b4.w)), a.d - 4 * i);
   };
   float sum = 0.f, mu, rs;
   for (int i = threadIdx.x; i < n4; i += kRnThreads) {
@@ -303,7 +311,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_layernorm_kernel(const Re
     norm(sum, &mu, &rs);
     sum = 0.f;
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
-      const float4 x = scaled(i, mu, rs, a.w, a.b);       // w and b are zero in the padding
+      const float4 x = scaled(i, mu, rs, a.w, a.b);
       rn_row[i] = x;
       xrow[i] = x;
       sum += (x.x + x.y) + (x.z + x.w);
