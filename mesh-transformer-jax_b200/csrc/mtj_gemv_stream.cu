@@ -107,7 +107,8 @@ __global__ void __launch_bounds__(kStreamThreads, 2) gemv_stream_kernel(const Ge
       uint4 v[NCH];
 #pragma unroll
       for (int c = 0; c < NCH; ++c) v[c] = c * 32 + lane < mine ? rowp[c * 32 + lane] : make_uint4(0u, 0u, 0u, 0u);
-      ok = __all_sync(0xffffffffu, ok);                          // every lane has read the slot
+      ok = __all_sync(0xffffffffu, ok);
+      __syncwarp();                                              // every lane has read the slot (a vote orders no memory)
       if (lane == 0) arrive(empty(slot));
       if (++slot == ring) {
         slot = 0;
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) gemv_stream_kernel(const Ge
       }
       return s0 + s1;
     };
-    // two rows' sums at a time; after a failed wait the rows left are only waited for (each wait is bounded)
+    // two rows' sums at a time; a wait that ran out ends the loop
     for (int r = r0; r < r1; r += 2) {
       float p0 = dot(), p1 = dot();
       if (!ok) break;
