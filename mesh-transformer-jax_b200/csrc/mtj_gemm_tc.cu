@@ -19,20 +19,30 @@ __device__ __forceinline__ float row_sum(float v, float* red) {
 }
 
 // LayerNorm of fp32 rows into bf16 (the GEMM's activation operand: hi, and lo where asked for), layers.py:17-36.  HOLD > 0:
-// rows of up to 256 HOLD columns stay in registers, one read of the row with all loads in flight instead of three; 0:
-// wider rows.  Both add in the same order.
+// rows of up to 256 HOLD columns stay in registers, one read of the row with all loads in flight instead of three, and the
+// weights before it; 0: wider rows, three reads.  Both add in the same order.  Few rows are bound by the loads' latency (33 of
+// 4096: 5.2 us in three reads, 3.0 from registers; 33 of 1024: 2.7 and 2.2), many by how many blocks an SM holds.
 template <int HOLD>
 __global__ void __launch_bounds__(256) ln_rows_kernel(const float* __restrict__ x, const float* __restrict__ scale,
                                                       const float* __restrict__ offset,
                                                       __nv_bfloat16* __restrict__ out, __nv_bfloat16* out_lo, int d) {
   __shared__ float red[8];
+  float sc[HOLD > 0 ? HOLD : 1], of[HOLD > 0 ? HOLD : 1];
+  if constexpr (HOLD > 0) {                              // weights do not depend on the predecessor
+#pragma unroll
+    for (int k = 0; k < HOLD; ++k) {
+      const int i = k * 256 + static_cast<int>(threadIdx.x);
+      sc[k] = i < d ? scale[i] : 0.f;
+      of[k] = i < d ? offset[i] : 0.f;
+    }
+  }
   pdl_wait();
   pdl_launch_dependents();
   const float* xr = x + static_cast<size_t>(blockIdx.x) * d;
   __nv_bfloat16* o = out + static_cast<size_t>(blockIdx.x) * d;
   __nv_bfloat16* ol = out_lo ? out_lo + static_cast<size_t>(blockIdx.x) * d : nullptr;
-  auto put = [&](int i, float xi, float mu, float rstd) {
-    const float y = fmaf(scale[i] * rstd, xi - mu, offset[i]);
+  auto put = [&](int i, float xi, float mu, float rstd, float w, float b) {
+    const float y = fmaf(w * rstd, xi - mu, b);
     const __nv_bfloat16 hi = __float2bfloat16_rn(y);
     o[i] = hi;
     if (ol) ol[i] = __float2bfloat16_rn(y - __bfloat162float(hi));
@@ -53,7 +63,7 @@ __global__ void __launch_bounds__(256) ln_rows_kernel(const float* __restrict__ 
     const float rstd = 1.0f / sqrtf(row_sum<256>(v, red) / static_cast<float>(d) + 1e-5f);
 #pragma unroll
     for (int k = 0; k < HOLD; ++k)
-      if (k * 256 + static_cast<int>(threadIdx.x) < d) put(k * 256 + threadIdx.x, r[k], mu, rstd);
+      if (k * 256 + static_cast<int>(threadIdx.x) < d) put(k * 256 + threadIdx.x, r[k], mu, rstd, sc[k], of[k]);
   } else {
     for (int i = threadIdx.x; i < d; i += 256) s += xr[i];
     const float mu = row_sum<256>(s, red) / static_cast<float>(d);
@@ -62,22 +72,33 @@ __global__ void __launch_bounds__(256) ln_rows_kernel(const float* __restrict__ 
       v = fmaf(t, t, v);
     }
     const float rstd = 1.0f / sqrtf(row_sum<256>(v, red) / static_cast<float>(d) + 1e-5f);
-    for (int i = threadIdx.x; i < d; i += 256) put(i, xr[i], mu, rstd);
+    for (int i = threadIdx.x; i < d; i += 256) put(i, xr[i], mu, rstd, scale[i], offset[i]);
   }
 }
 
 // x = sum of split-K planes (in order) + bias + residual, and from the finished row the next projection's operand, the
 // layer norm in bf16 (hi, and lo where asked for).  One block per row, the row in registers (HOLD float4 a thread), every
 // load issued before the first sum.  The planes are in L2; bound by the latency of one round of loads and two block sums
-// up to about 300 rows, by L2 above.  It replaces two kernels: 56 rows of 4096 in 4 planes 5.4 us against 5.1 + 4.4, 700
-// rows in 3 planes 14 us against 35 + 6.
+// up to about 300 rows, by L2 above; the weights come before the wait.  It replaces two kernels: 56 rows of 4096 in 4
+// planes 5.4 us against 5.1 + 4.4, 700 rows in 3 planes 14 us against 35 + 6, 8 rows in 8 planes 5.1 us against 2.4 + 4.6.
 constexpr int kRowThreads = 512;
 template <int HOLD>
 __global__ void __launch_bounds__(kRowThreads) reduce_ln_rows_kernel(const ReduceLnArgs a) {
   __shared__ float red[kRowThreads / 32];
+  const int n4 = a.d >> 2;
+  auto weights = [&](const float* w, float4 (&v)[HOLD]) {
+#pragma unroll
+    for (int i = 0; i < HOLD; ++i) {
+      const int c = i * kRowThreads + threadIdx.x;
+      v[i] = w && c < n4 ? reinterpret_cast<const float4*>(w)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  float4 b[HOLD], sc[HOLD], of[HOLD];                    // they do not depend on the predecessor
+  weights(a.bias, b);
+  weights(a.scale, sc);
+  weights(a.offset, of);
   pdl_wait();
   pdl_launch_dependents();
-  const int n4 = a.d >> 2;
   const size_t row4 = static_cast<size_t>(blockIdx.x) * n4, plane4 = static_cast<size_t>(a.M) * n4;
   const float4* res = reinterpret_cast<const float4*>(a.residual) + row4;
   const float4* part = reinterpret_cast<const float4*>(a.partial) + row4;
@@ -89,7 +110,7 @@ __global__ void __launch_bounds__(kRowThreads) reduce_ln_rows_kernel(const Reduc
     v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     r[i] = c < n4 ? res[c] : v[i];
   }
-#pragma unroll 4
+#pragma unroll (HOLD > 2 ? 4 : 8)
   for (int z = 0; z < a.planes; ++z) {
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
@@ -102,8 +123,7 @@ __global__ void __launch_bounds__(kRowThreads) reduce_ln_rows_kernel(const Reduc
   for (int i = 0; i < HOLD; ++i) {
     const int c = i * kRowThreads + threadIdx.x;
     if (c >= n4) continue;
-    const float4 b = reinterpret_cast<const float4*>(a.bias)[c];
-    v[i].x = v[i].x + b.x + r[i].x; v[i].y = v[i].y + b.y + r[i].y; v[i].z = v[i].z + b.z + r[i].z; v[i].w = v[i].w + b.w + r[i].w;
+    v[i].x = v[i].x + b[i].x + r[i].x; v[i].y = v[i].y + b[i].y + r[i].y; v[i].z = v[i].z + b[i].z + r[i].z; v[i].w = v[i].w + b[i].w + r[i].w;
     reinterpret_cast<float4*>(a.out)[row4 + c] = v[i];
   }
   if (!a.scale) return;
@@ -122,9 +142,8 @@ __global__ void __launch_bounds__(kRowThreads) reduce_ln_rows_kernel(const Reduc
   for (int i = 0; i < HOLD; ++i) {
     const int c = i * kRowThreads + threadIdx.x;
     if (c >= n4) continue;
-    const float4 sc = reinterpret_cast<const float4*>(a.scale)[c], of = reinterpret_cast<const float4*>(a.offset)[c];
-    const float y[4] = {fmaf(sc.x * rstd, v[i].x - mu, of.x), fmaf(sc.y * rstd, v[i].y - mu, of.y),
-                        fmaf(sc.z * rstd, v[i].z - mu, of.z), fmaf(sc.w * rstd, v[i].w - mu, of.w)};
+    const float y[4] = {fmaf(sc[i].x * rstd, v[i].x - mu, of[i].x), fmaf(sc[i].y * rstd, v[i].y - mu, of[i].y),
+                        fmaf(sc[i].z * rstd, v[i].z - mu, of[i].z), fmaf(sc[i].w * rstd, v[i].w - mu, of[i].w)};
     reinterpret_cast<uint2*>(a.xn)[row4 + c] = make_uint2(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]));
     if (a.xn_lo) {
       float e[4];
@@ -289,8 +308,11 @@ cudaError_t launch_ln_rows(const float* x, const float* scale, const float* offs
                            int d, cudaStream_t s, bool pdl, __nv_bfloat16* out_lo) {
   const dim3 grid(rows), block(256);
   if (d <= 1024) return launch_pdl(ln_rows_kernel<4>, grid, block, 0, s, pdl, x, scale, offset, out, out_lo, d);
-  if (d <= 4096) return launch_pdl(ln_rows_kernel<16>, grid, block, 0, s, pdl, x, scale, offset, out, out_lo, d);
-  if (d <= 8192) return launch_pdl(ln_rows_kernel<32>, grid, block, 0, s, pdl, x, scale, offset, out, out_lo, d);
+  if (d <= 2048) return launch_pdl(ln_rows_kernel<8>, grid, block, 0, s, pdl, x, scale, offset, out, out_lo, d);
+  // wide rows take the registers of more than one block in two: 512 rows of 4096 6.3 us in three reads and 5.3, 1000 7.5 and 8.7
+  const bool few = rows <= 512;
+  if (few && d <= 4096) return launch_pdl(ln_rows_kernel<16>, grid, block, 0, s, pdl, x, scale, offset, out, out_lo, d);
+  if (few && d <= 8192) return launch_pdl(ln_rows_kernel<32>, grid, block, 0, s, pdl, x, scale, offset, out, out_lo, d);
   return launch_pdl(ln_rows_kernel<0>, grid, block, 0, s, pdl, x, scale, offset, out, out_lo, d);
 }
 
