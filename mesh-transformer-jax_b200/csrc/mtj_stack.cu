@@ -573,9 +573,19 @@ const TensorMap* LayerStack::xmap(const __nv_bfloat16* buf, int K, int ld, int t
   return &it->second[tile == 32 ? 0 : tile == 64 ? 1 : 2];
 }
 
+namespace {
+// Whole-K products of a prompt's 33 to 192 rows: on the pair kernel or on the small tiles.  Up to 64 rows the small tiles cut K
+// over clusters and keep every SM on the weights; a pair walks all of K.  48 rows, us, small tiles and pairs: 4096 x 8192
+// weights 19 and 41, 2048 x 4096 12 and 23, 22528 x 4096 41 and 52, 8192 x 2048 15 and 9.  Above, the small tiles have whole
+// K too and lose except where few pairs would be busy for a short time (192 rows: 512 x 1024 8.7 and 10.1, 1024 x 512 7.0
+// and 8.7; 2048 x 512 9.3 and 8.7).
+bool pair_pays(int M, int N, int K) { return M > 192 || (M > 64 && (N >= 2048 || K > 1024)); }
+constexpr double kSplitLeastUs = 3.6;   // a cut of K that saves less is not seen: 1500 rows of 512 x 1536 11.2 whole, 9.1 + 1.9 in pieces
+}  // namespace
+
 int32_t LayerStack::gemm(mtj_handle* h, GemvEpilogue epi, const Linear& l, const __nv_bfloat16* x, int M, float* out, int ld_out,
                          __nv_bfloat16* out_bf16, int ld_bf16, bool decode, cudaStream_t s, int x_row0, int x_ld, int f32_from) {
-  const bool wide = gemm_tc_use_wide(M, decode || h->same_sums);
+  const bool wide = gemm_tc_use_wide(M, decode || h->same_sums) && pair_pays(M, l.N, l.K);
   const int ldx = x_ld > 0 ? x_ld : l.ld;
   const TensorMap* mx = xmap(x, l.K, ldx, wide ? gemm_tc_wide_token_tile() : gemm_tc_token_tile_for(M));
   if (!mx) return fail(MTJ_ERR_CUDA, "cuTensorMapEncodeTiled failed");
@@ -604,7 +614,7 @@ int32_t LayerStack::gemm_out(mtj_handle* h, const Linear& l, int M, bool decode,
   int ks = 1;
   if (l.N == ld_ && !h->same_sums) {                                  // the planes have the residual rows' stride
     if (wide) {
-      ks = gemm_tc_wide_split(M, l.N, l.K);
+      ks = gemm_tc_wide_split(M, l.N, l.K, kSplitLeastUs);
     } else {
       // few rows: two blocks per SM, each with at least four k-blocks
       const int bn = gemm_tc_token_tile_for(M), tiles = (l.N + 127) / 128 * ((M + bn - 1) / bn), nk = (l.K + 63) / 64;
