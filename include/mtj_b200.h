@@ -132,9 +132,9 @@ typedef struct mtj_stack_desc {
 } mtj_stack_desc;
 
 const char* mtj_last_error(void);
-/* ABI revision: 5 (2: mtj_config with the tuning fields, mtj_generate, mtj_start_batch / mtj_admit;
+/* ABI revision: 6 (2: mtj_config with the tuning fields, mtj_generate, mtj_start_batch / mtj_admit;
  * 3: top_k in mtj_sample_top_p / mtj_nucleus_filter, mtj_set_top_k; 4: layer-stack models, mtj_extend,
- * mtj_release; 5: more mixers and residual forms in mtj_stack_desc). */
+ * mtj_release; 5: more mixers and residual forms in mtj_stack_desc; 6: mtj_k_out_projection_pieces). */
 int32_t mtj_version(void);
 
 /* CausalTransformerShard.__init__ (transformer_shard.py:21-45): validates the
@@ -332,6 +332,11 @@ int32_t mtj_k_embed(mtj_handle* h, const uint32_t* ids_dev, int32_t rows,
 int32_t mtj_k_layer(mtj_handle* h, int32_t layer, const float* x_dev, int32_t batch, int32_t T, int32_t pos0,
                     const int32_t* pad_host, const int32_t* key_limit_host, int32_t decode,
                     float* out_dev, mtj_stream s);
+
+/* Pieces that K is cut into in the output projection of a layer over `rows` rows of a prompt, or of an evaluation
+ * (layers.py:285-297), where the shard's sums do not go to a peer slot; 1: whole.  A pure function of the sizes: the
+ * handle need not be bound. */
+int32_t mtj_k_out_projection_pieces(const mtj_handle* h, int32_t rows, int32_t evaluation);
 
 /* ProjectionShard.__call__ before the all-gather (layers.py:561-564):
  * logits_out_dev [rows, n_vocab/mp] of this shard. */

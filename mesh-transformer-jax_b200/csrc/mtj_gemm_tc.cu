@@ -193,10 +193,11 @@ int gemm_tc_token_tile_for(int M) { return M <= 32 ? 32 : (M <= 64 ? 64 : 128); 
 bool gemm_tc_use_wide(int M, bool same_sums) { return M > (same_sums ? 192 : 32); }
 // Pieces that K is cut into, each leaving a plane of partial sums: as many as shorten the critical path by more than
 // writing and adding the planes takes.  One unit is a k-block of 64, 0.36 us at any tile height (a pair keeps 192 KB of
-// operands in flight, and that round trip is what a k-block waits for); planes move at about 8 TB/s through L2.  4096 x
+// operands in flight, and that round trip is what a k-block waits for); a number of a plane costs 1 ps to write and add
+// where the following kernel adds the planes, and 4 ps with a kernel for it (own_sum).  4096 x
 // 20480 weights: 136 rows 104 us whole, 37 us in 4 pieces; 448 rows 110 and 58 in 2; 700 rows 114 and 78 in 3; from 998
 // rows on whole tiles are best.
-int gemm_tc_wide_split(int M, int N, int K, double least_us) {
+int gemm_tc_wide_split(int M, int N, int K, bool own_sum, double least_us) {
   if (N < 2 * kBM) return 1;                           // the pair kernel's tile
   const int tiles = (M + kPBN - 1) / kPBN * ((N + 2 * kBM - 1) / (2 * kBM)), pairs = std::max(1, sm_count() / 2), nk = (K + kBK - 1) / kBK;
   int best = 1;
@@ -204,7 +205,7 @@ int gemm_tc_wide_split(int M, int N, int K, double least_us) {
   for (int s = 1; s <= 8 && (s == 1 || nk / s >= 8); ++s) {
     if ((s - 1) * ((nk + s - 1) / s) >= nk || (s > 1 && static_cast<int64_t>(s) * M * N > kWidePlaneFloats)) continue;
     const int waves = (tiles * s + pairs - 1) / pairs;
-    const double planes = s > 1 ? 8e-6 / 8.0 * s * M * N / 0.36 : 0.0;
+    const double planes = s > 1 ? (own_sum ? 4e-6 : 1e-6) * s * M * N / 0.36 : 0.0;
     const double cost = static_cast<double>(waves) * ((nk + s - 1) / s) + planes;
     if (s == 1) whole = cost;
     if (cost < 0.97 * best_cost && (s == 1 || 0.36 * (whole - cost) >= least_us)) {

@@ -306,9 +306,9 @@ int gemm_tc_token_tile();                 // widest token tile of launch_gemm_tc
 int gemm_tc_token_tile_for(int M);
 // Whether M rows go through launch_gemm_tc_wide.
 bool gemm_tc_use_wide(int M, bool same_sums);
-// Pieces launch_gemm_tc_wide should cut K into (GemmTcArgs.partial, ksplit) when the caller can add planes; 1: none, also
-// where the pieces would save less than least_us.
-int gemm_tc_wide_split(int M, int N, int K, double least_us = 0.0);
+// Pieces launch_gemm_tc_wide should cut K into (GemmTcArgs.partial, ksplit) when the caller can add planes, in the kernel that
+// follows or (own_sum) in launch_splitk_reduce; 1: none, also where the pieces would save less than least_us.
+int gemm_tc_wide_split(int M, int N, int K, bool own_sum, double least_us = 0.0);
 // Cluster split-K factor (1, 2 or 4) launch_gemm_tc should be given for a decode-size GEMM (GemmTcArgs.cluster_k).
 int gemm_tc_decode_cluster_k(int weight_rows, int M, int K);
 cudaError_t launch_splitk_reduce(const float* partial, int ksplit, int M, int N, const float* bias,

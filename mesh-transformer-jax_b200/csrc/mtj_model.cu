@@ -247,6 +247,26 @@ int32_t run_layer(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, bool
 int tc_tile_index(int M) { return mtj::gemm_tc_token_tile_for(M) == 32 ? 0 : (mtj::gemm_tc_token_tile_for(M) == 64 ? 1 : 2); }
 bool use_tc_wide(const mtj_handle* h, int M, bool same_sums) { return h->tc_wide_ok && mtj::gemm_tc_use_wide(M, same_sums); }
 
+// How a layer's output projection over M rows runs: on the pair kernel (wide) or the small tiles, the pieces that K is cut into,
+// and whether the kernel that adds them also norms the rows for what follows (else launch_splitk_reduce adds them).
+struct OutPlan {
+  bool wide, fused;
+  int pieces;
+};
+OutPlan plan_out(const mtj_handle* h, int M, bool wide, bool to_slot, bool detached, bool same_sums) {
+  const int K = h->dl + h->ffl;
+  OutPlan p = {wide && !to_slot, h->mp == 1 && !detached && !same_sums && mtj::reduce_ln_rows_ok(h->d), 1};
+  if (p.wide) {
+    if (!same_sums) p.pieces = mtj::gemm_tc_wide_split(M, h->d, K, !p.fused);
+  } else {
+    // Few token rows give only d/128 tiles: split K over blocks so the whole GPU streams the weights.
+    const int tiles = ((h->d + 127) / 128) * ((M + mtj::gemm_tc_token_tile() - 1) / mtj::gemm_tc_token_tile());
+    if (M <= kTcSplitRows && tiles < 148) p.pieces = std::max(1, std::min({kTcSplitMax, 296 / tiles, K / 64}));
+  }
+  if (to_slot && p.pieces == 1) p.pieces = 2;          // the slot is selected by the reduction kernel
+  return p;
+}
+
 // The same layer for many token rows on the tensor cores: LayerNorm to bf16, in-proj GEMM
 // (RoPE / KV / GELU epilogue), causal attention, out-proj GEMM (+ bias + residual).  chain: the next call is the following
 // layer's for the same rows (behind the last layer in decode, the logits), so its norm may be left ready here.
@@ -351,13 +371,9 @@ int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, c
   o.out = h->mp == 1 ? (detached_out ? detached_out : h->x) : (to_slot ? partial_dst(h, M) : h->part);
   o.ld_out = h->d;
   o.dev_err = h->dev_err;
-  // Few token rows give only d/128 tiles: split K over blocks so the whole GPU streams the weights.
-  const int tiles = ((h->d + 127) / 128) * ((M + mtj::gemm_tc_token_tile() - 1) / mtj::gemm_tc_token_tile());
-  int ksplit = 1;
-  const bool wide_out = wide && !to_slot;
-  if (!wide_out && M <= kTcSplitRows && tiles < 148) ksplit = std::max(1, std::min({kTcSplitMax, 296 / tiles, o.K / 64}));
-  if (wide_out && h->mp == 1 && !h->same_sums && mtj::reduce_ln_rows_ok(h->d)) ksplit = mtj::gemm_tc_wide_split(M, o.N, o.K);
-  if (to_slot && ksplit == 1) ksplit = 2;          // the slot is selected by the reduction kernel
+  const OutPlan plan = plan_out(h, M, wide, to_slot, detached_out != nullptr, h->same_sums);
+  const bool wide_out = plan.wide;
+  const int ksplit = plan.pieces;
   const bool push = decode && !detached_out && !defer_reduce && use_push(h, M) && M <= kTcSplitRows;
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
   if (push) {
@@ -383,7 +399,7 @@ int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, c
     if (wide_out) MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiOut, &lw.map_out, &h->map_act_wide, &h->map_act[1], o, s));
     else MTJ_CUDA(mtj::launch_gemm_tc(mtj::kEpiOut, &lw.map_out, &h->map_act[tc_tile_index(M)], o, s, pdl,
                                       hilo ? &h->map_act_lo[tc_tile_index(M)] : nullptr));
-    if (h->mp == 1 && res && !h->same_sums && mtj::reduce_ln_rows_ok(h->d)) {
+    if (plan.fused) {
       // one kernel adds the planes and norms the rows for what follows: the next layer, or in decode the logits
       const bool last = layer + 1 == h->L, norm = chain && (!last || decode);
       mtj::ReduceLnArgs r = {h->tc_partial, ksplit, M, h->d, lw.b_out, res, dst};
@@ -723,7 +739,7 @@ int32_t mtj_set_error(int32_t code, const char* msg) {
   g_last_error = msg ? msg : "";
   return code;
 }
-int32_t mtj_version(void) { return 5; }
+int32_t mtj_version(void) { return 6; }
 
 int32_t mtj_create(const mtj_config* c, mtj_handle** out) {
   if (!c || !out) return fail(MTJ_ERR_INVALID, "null argument");
@@ -1790,6 +1806,11 @@ int32_t mtj_k_layer(mtj_handle* h, int32_t layer, const float* x_in, int32_t bat
   if (!decode && use_tc(h, static_cast<int>(M)))
     return run_layer_tc(h, layer, static_cast<int>(M), rows, key_limit_host ? h->key_limit : nullptr, s, out);
   return run_layer(h, layer, static_cast<int>(M), rows, decode != 0, key_limit_host ? h->key_limit : nullptr, s, out);
+}
+
+int32_t mtj_k_out_projection_pieces(const mtj_handle* h, int32_t rows, int32_t evaluation) {
+  if (!h || h->stack || rows <= 0) return -1;
+  return plan_out(h, rows, mtj::gemm_tc_use_wide(rows, evaluation != 0), false, false, evaluation != 0).pieces;
 }
 
 int32_t mtj_k_projection(mtj_handle* h, const float* x_in, int32_t rows, float* logits_out, mtj_stream stream) {

@@ -614,7 +614,7 @@ int32_t LayerStack::gemm_out(mtj_handle* h, const Linear& l, int M, bool decode,
   int ks = 1;
   if (l.N == ld_ && !h->same_sums) {                                  // the planes have the residual rows' stride
     if (wide) {
-      ks = gemm_tc_wide_split(M, l.N, l.K, kSplitLeastUs);
+      ks = gemm_tc_wide_split(M, l.N, l.K, false, kSplitLeastUs);
     } else {
       // few rows: two blocks per SM, each with at least four k-blocks
       const int bn = gemm_tc_token_tile_for(M), tiles = (l.N + 127) / 128 * ((M + bn - 1) / bn), nk = (l.K + 63) / 64;
