@@ -257,7 +257,7 @@ OutPlan plan_out(const mtj_handle* h, int M, bool wide, bool to_slot, bool detac
   const int K = h->dl + h->ffl;
   OutPlan p = {wide && !to_slot, h->mp == 1 && !detached && !same_sums && mtj::reduce_ln_rows_ok(h->d), 1};
   if (p.wide) {
-    if (!same_sums) p.pieces = mtj::gemm_tc_wide_split(M, h->d, K, !p.fused);
+    if (!same_sums && (h->tc_pair >> 1 & 1)) p.pieces = mtj::gemm_tc_wide_split(M, h->d, K, !p.fused);   // only pairs cut K
   } else {
     // Few token rows give only d/128 tiles: split K over blocks so the whole GPU streams the weights.
     const int tiles = ((h->d + 127) / 128) * ((M + mtj::gemm_tc_token_tile() - 1) / mtj::gemm_tc_token_tile());
@@ -714,6 +714,7 @@ void read_switches(mtj_handle* h, const mtj_config& c) {
   h->tp_token = !(e && e[0] == '1');
   e = getenv("MTJ_NO_CLUSTER_K");
   h->tc_cluster_k = !(e && e[0] == '1');
+  if (const char* mask = getenv("MTJ_TC_PAIR")) h->tc_pair = atoi(mask) & 7;
   e = getenv("MTJ_NO_FUSED_CE");
   h->fused_ce = !(e && e[0] == '1');
   e = getenv("MTJ_NO_FORK");
@@ -942,7 +943,6 @@ int32_t mtj_bind_arenas(mtj_handle* h, void* wdev, int64_t wbytes, void* sdev, i
     ok = ok && mtj::make_tensor_map_bf16(&h->map_xn_wide, h->xn_bf16, h->max_rows, h->d, bw) == cudaSuccess;
     ok = ok && mtj::make_tensor_map_bf16(&h->map_act_wide, h->act_bf16, h->max_rows, h->dl + h->ffl, bw) == cudaSuccess;
     h->tc_wide_ok = ok && !getenv("MTJ_NO_TC_WIDE");
-    if (const char* e = getenv("MTJ_TC_PAIR")) h->tc_pair = atoi(e) & 7;
     {
       const int64_t rl = std::min<int64_t>(h->max_rows, kHiLoRows);
       bool okl = ok;

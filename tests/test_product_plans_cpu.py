@@ -40,3 +40,12 @@ def test_evaluation_keeps_whole_k_from_129_rows_on(lib):
     assert [lib.lib.mtj_k_out_projection_pieces(h, rows, 1) for rows in (33, 128, 129, 192, 193, 700, 2048)] == [8, 8, 1, 1, 1, 1, 1]
     assert lib.lib.mtj_k_out_projection_pieces(h, 0, 0) < 0
     lib.lib.mtj_destroy(h)
+
+
+def test_the_pair_mask_reaches_the_output_projection(lib, monkeypatch):
+    """Only block pairs cut K: with them switched off at that call site its K stays whole."""
+    for mask, whole in (("7", False), ("5", True), ("2", False), ("0", True)):
+        monkeypatch.setenv("MTJ_TC_PAIR", mask)
+        h = _handle(lib)
+        assert (lib.lib.mtj_k_out_projection_pieces(h, 136, 0) == 1) == whole, mask
+        lib.lib.mtj_destroy(h)
