@@ -113,8 +113,10 @@ struct mtj_handle {
                                     // arg-max to all ranks instead of gathering the logits (MTJ_NO_TP_TOKEN=1: off)
   bool tp_push = false;             // batched decode at mp > 1: push all-reduce fused with the split-K reduction and
                                     // the LayerNorm; default: from 4 shards on (MTJ_TP_PUSH=0 / 1 overrides)
-  // Evaluation: products keep one order of sums (no split along K, the same kernels at every row count).  The loss of a token
-  // that the model is sure of is the difference of two nearly equal numbers and shows every change of rounding.
+  // Evaluation: products run as they did before prompts of 33 to 192 rows went to the pair kernel and long K was cut for it:
+  // small tiles up to 192 rows (GPT-J cuts K in the output projection up to 128, stacks over clusters up to 64 and where weight
+  // rows are few), pairs on whole K above.  The loss of a token that the model is sure of is the difference of two nearly equal
+  // numbers and shows every change of rounding, the one between those row counts too.  Set through SameSums.
   bool same_sums = false;
   bool xn_ready = false;            // the bf16 operand of the next projection has already been written
   bool tc_cluster_k = true;         // batched decode: split K over block clusters when tiles are few (MTJ_NO_CLUSTER_K=1: off)

@@ -247,6 +247,13 @@ int32_t run_layer(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, bool
 int tc_tile_index(int M) { return mtj::gemm_tc_token_tile_for(M) == 32 ? 0 : (mtj::gemm_tc_token_tile_for(M) == 64 ? 1 : 2); }
 bool use_tc_wide(const mtj_handle* h, int M, bool same_sums) { return h->tc_wide_ok && mtj::gemm_tc_use_wide(M, same_sums); }
 
+// Evaluation's products (mtj_handle::same_sums) for the length of a call, however it ends.
+struct SameSums {
+  mtj_handle* h;
+  explicit SameSums(mtj_handle* handle) : h(handle) { h->same_sums = true; }
+  ~SameSums() { h->same_sums = false; }
+};
+
 // How a layer's output projection over M rows runs: on the pair kernel (wide) or the small tiles, the pieces that K is cut into,
 // and whether the kernel that adds them also norms the rows for what follows (else launch_splitk_reduce adds them).
 struct OutPlan {
@@ -1599,7 +1606,7 @@ int32_t mtj_eval_loss(mtj_handle* h, const uint32_t* obs, const uint32_t* target
   rc = setup_sequences(h, pad, limit, T, s);
   if (rc) return rc;
   h->prefilled = false;
-  h->same_sums = true;
+  const SameSums sums(h);
   rc = forward_chunks(h, obs, T, batch, T, h->key_limit, s, [&](int b0, int ns, int t0, int tc) -> int32_t {
     const int M = ns * tc;
     mtj::CeArgs ce = {};
@@ -1617,7 +1624,7 @@ int32_t mtj_eval_loss(mtj_handle* h, const uint32_t* obs, const uint32_t* target
     const int step = fused ? h->ce_rows : h->eval_rows;
     for (int m0 = 0; m0 < M; m0 += step) {
       const int n = std::min(step, M - m0);
-      if (fused && use_tc_wide(h, n, true)) {
+      if (fused && use_tc_wide(h, n, h->same_sums)) {
         int32_t r3 = run_loss_rows_fused(h, n, m0, ce, s);
         if (r3) return r3;
         continue;
@@ -1645,7 +1652,6 @@ int32_t mtj_eval_loss(mtj_handle* h, const uint32_t* obs, const uint32_t* target
     h->launches += 2;
     return MTJ_OK;
   });
-  h->same_sums = false;
   return rc;
 }
 
@@ -1834,6 +1840,7 @@ int32_t mtj_k_projection_loss(mtj_handle* h, const float* x_in, const uint32_t* 
   if (!x_in || !targets || !loss_out || !correct_out || rows <= 0 || rows > h->max_rows)
     return fail(MTJ_ERR_INVALID, "bad argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const SameSums sums(h);
   MTJ_CUDA(mtj::launch_residual_stats(h->x, x_in, h->stats, rows, h->d, false, s, false));
   h->launches++;
   mtj::CeArgs ce = {};
@@ -1851,7 +1858,7 @@ int32_t mtj_k_projection_loss(mtj_handle* h, const float* x_in, const uint32_t* 
   const int step = fused ? h->ce_rows : h->eval_rows;
   for (int m0 = 0; m0 < rows; m0 += step) {
     const int n = std::min(step, rows - m0);
-    if (fused && use_tc_wide(h, n, true)) {
+    if (fused && use_tc_wide(h, n, h->same_sums)) {
       rc = run_loss_rows_fused(h, n, m0, ce, s);
       if (rc) return rc;
       continue;
