@@ -215,6 +215,14 @@ int gemm_tc_wide_split(int M, int N, int K, bool own_sum, double least_us) {
   }
   return best;
 }
+int64_t gemm_tc_wide_plane_floats(int max_rows, int N, int K, bool own_sum, double least_us) {
+  int64_t most = 0;
+  for (int M = 33; M <= max_rows && 2LL * M * N <= kWidePlaneFloats; ++M) {
+    const int s = gemm_tc_wide_split(M, N, K, own_sum, least_us);
+    if (s > 1) most = std::max(most, static_cast<int64_t>(s) * M * N);
+  }
+  return most;
+}
 int gemm_tc_wide_token_tile() { return kPBN / 2; }     // rows of the activation box: a tile takes two of them
 
 cudaError_t launch_gemm_tc_wide(GemvEpilogue epi, const void* map_w, const void* map_x, const void* map_x64, const GemmTcArgs& a,

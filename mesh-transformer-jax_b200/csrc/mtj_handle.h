@@ -143,7 +143,10 @@ struct mtj_handle {
   int tc_pair = 7;           // ... as block pairs on 256 x 256 tiles: bit 0 in-projection, 1 out-projection, 2 logits
                              // (MTJ_TC_PAIR=<mask> overrides, for measurement)
   bool mega_push = true;     // per-block push exchange inside the persistent decode kernel (MTJ_NO_MEGA_PUSH=1: slot protocol)
-  float* tc_partial = nullptr;        // [kTcSplitMax, kTcSplitRows, d] split-K partial sums of small-M out-projections
+  // partial sums of out-projections cut along K: [kTcSplitMax, up to kTcSplitRows, d] of the small tiles, or what the pair
+  // kernel's pieces need for any number of rows; set when the handle is made
+  float* tc_partial = nullptr;
+  int64_t tc_partial_floats = 0;
   int eval_rows = 0;                // rows of logits materialised at a time by the loss path
   float* eval_logits = nullptr;     // [eval_rows, Vl]
   // loss path on the persistent GEMM: the logits are never stored, its epilogue leaves per (32-entry vocabulary
@@ -319,7 +322,7 @@ struct mtj_handle {
       logits_gather = c.take<float>(static_cast<int64_t>(max_batch) * V);
       part = c.take<float>(R * d);
     }
-    tc_partial = c.take<float>(std::max(static_cast<int64_t>(mtj::kTcSplitMax) * std::min<int64_t>(R, mtj::kTcSplitRows) * d, mtj::kWidePlaneFloats));
+    tc_partial = c.take<float>(tc_partial_floats);
     q_bf16 = c.take<__nv_bfloat16>(R * dl);
     xn_bf16 = c.take<__nv_bfloat16>(R * d);
     act_bf16 = c.take<__nv_bfloat16>(R * (dl + ffl));

@@ -103,8 +103,9 @@ bool gemv_stream_ok(GemvEpilogue epi, const GemvArgs& a);
 cudaError_t launch_gemv_stream(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl);
 // The same product for 5 rows and more on the CUDA cores, fp32 activations and sums (mtj_gemm_rows.cu): every epilogue but
 // the in-projection's, no residual, no norm behind it.  planes and counters (zero between launches) are scratch of
-// kGemmRowsPlaneFloats and kGemmRowsCounters elements; one launch at a time may use them.
-constexpr int64_t kGemmRowsPlaneFloats = 4 << 20;
+// kGemmRowsPlaneFloats and kGemmRowsCounters elements; one launch at a time may use them.  (K is cut until there are four
+// blocks per SM, each with a tile of 64 x 16.)
+constexpr int64_t kGemmRowsPlaneFloats = 4 * 148 * 64 * 16;
 constexpr int kGemmRowsCounters = 1024, kGemmRowsMin = 5;
 cudaError_t launch_gemm_rows(GemvEpilogue epi, const GemvArgs& a, float* planes, uint32_t* counters, cudaStream_t s, bool pdl);
 
@@ -300,7 +301,7 @@ struct GemmTcArgs {
   int bn, x_box, stages;       // wide kernel with pair: token rows per tile and of the activation box, ring stages; set by the launch
   uint32_t* dev_err;
 };
-constexpr int64_t kWidePlaneFloats = 148LL * 256 * 256;   // most partial sums of a split launch_gemm_tc_wide: two waves of tiles
+constexpr int64_t kWidePlaneFloats = 148LL * 256 * 256;   // most partial sums of any split launch_gemm_tc_wide: two waves of tiles
 int gemm_tc_token_tile();                 // widest token tile of launch_gemm_tc (128)
 // Token tile launch_gemm_tc uses for M rows (32, 64 or 128): map_x must have been made with this box_rows.
 int gemm_tc_token_tile_for(int M);
@@ -309,6 +310,8 @@ bool gemm_tc_use_wide(int M, bool same_sums);
 // Pieces launch_gemm_tc_wide should cut K into (GemmTcArgs.partial, ksplit) when the caller can add planes, in the kernel that
 // follows or (own_sum) in launch_splitk_reduce; 1: none, also where the pieces would save less than least_us.
 int gemm_tc_wide_split(int M, int N, int K, bool own_sum, double least_us = 0.0);
+// The most partial sums that those pieces leave for products of up to max_rows rows.
+int64_t gemm_tc_wide_plane_floats(int max_rows, int N, int K, bool own_sum, double least_us = 0.0);
 // Cluster split-K factor (1, 2 or 4) launch_gemm_tc should be given for a decode-size GEMM (GemmTcArgs.cluster_k).
 int gemm_tc_decode_cluster_k(int weight_rows, int M, int K);
 cudaError_t launch_splitk_reduce(const float* partial, int ksplit, int M, int N, const float* bias,

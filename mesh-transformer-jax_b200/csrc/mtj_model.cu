@@ -265,6 +265,7 @@ OutPlan plan_out(const mtj_handle* h, int M, bool wide, bool to_slot, bool detac
   OutPlan p = {wide && !to_slot, h->mp == 1 && !detached && !same_sums && mtj::reduce_ln_rows_ok(h->d), 1};
   if (p.wide) {
     if (!same_sums && (h->tc_pair >> 1 & 1)) p.pieces = mtj::gemm_tc_wide_split(M, h->d, K, !p.fused);   // only pairs cut K
+    if (static_cast<int64_t>(p.pieces) * M * h->d > h->tc_partial_floats) p.pieces = 1;
   } else {
     // Few token rows give only d/128 tiles: split K over blocks so the whole GPU streams the weights.
     const int tiles = ((h->d + 127) / 128) * ((M + mtj::gemm_tc_token_tile() - 1) / mtj::gemm_tc_token_tile());
@@ -795,6 +796,11 @@ int32_t mtj_create(const mtj_config* c, mtj_handle** out) {
   h->n_pages = h->ring_pages * h->max_batch;
   h->max_splits = mtj::decode_attn_splits(h->W);
   h->expected = 2 + 10LL * h->L + 4;
+  h->tc_partial_floats = static_cast<int64_t>(kTcSplitMax) * std::min(h->max_rows, kTcSplitRows) * h->d;
+  if (mp > 1)                                          // rows of a peer slot: two pieces at least (plan_out)
+    h->tc_partial_floats = std::max<int64_t>(h->tc_partial_floats, 2LL * std::min(h->max_rows, h->max_batch) * h->d);
+  for (const bool own_sum : {false, true})
+    h->tc_partial_floats = std::max(h->tc_partial_floats, mtj::gemm_tc_wide_plane_floats(h->max_rows, h->d, h->dl + h->ffl, own_sum));
   read_switches(h, *c);
   *out = h;
   return MTJ_OK;

@@ -12,6 +12,8 @@
 #include <math.h>
 #include <stdlib.h>
 
+#include <set>
+
 namespace mtj {
 
 namespace {
@@ -297,7 +299,7 @@ void LayerStack::carve_workspace(Carver& c) {
     cat_ = c.take<float>(R * 2 * ld_);
   }
   if (!f32_) {
-    y_planes_elems_ = std::max<int64_t>(kWidePlaneFloats, static_cast<int64_t>(kSplitPlanes) * std::min<int64_t>(R, 192) * ld_);
+    y_planes_elems_ = out_plane_floats();
     y_planes_ = c.take<float>(y_planes_elems_);
     xn_bf_ = c.take<__nv_bfloat16>(R * ld_);
     sel_bf_ = c.take<__nv_bfloat16>(R * ld_);
@@ -609,20 +611,35 @@ int32_t LayerStack::gemm(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
   return MTJ_OK;
 }
 
+int LayerStack::out_pieces(const Linear& l, int M, bool wide) const {
+  if (l.N != ld_) return 1;                                            // the planes have the residual rows' stride
+  if (wide) return gemm_tc_wide_split(M, l.N, l.K, false, kSplitLeastUs);
+  // few rows: two blocks per SM, each with at least four k-blocks
+  const int bn = gemm_tc_token_tile_for(M), tiles = (l.N + 127) / 128 * ((M + bn - 1) / bn), nk = (l.K + 63) / 64;
+  int ks = std::max(1, std::min({kSplitPlanes, 296 / tiles, nk / 4}));
+  while (ks > 1 && (ks - 1) * ((nk + ks - 1) / ks) >= nk) --ks;
+  return ks;
+}
+
+int64_t LayerStack::out_plane_floats() const {
+  int64_t most = 0;
+  std::set<int> seen;
+  for (const Layer& l : layers_)
+    for (const Linear* w : {&l.out, &l.down}) {
+      if (w->N != ld_ || !seen.insert(w->K).second) continue;
+      most = std::max(most, gemm_tc_wide_plane_floats(R_, w->N, w->K, false, kSplitLeastUs));
+      for (int M = 1; M <= std::min(R_, 192); ++M) {
+        const int ks = out_pieces(*w, M, false);
+        if (ks > 1) most = std::max(most, static_cast<int64_t>(ks) * M * w->N);
+      }
+    }
+  return most;
+}
+
 int32_t LayerStack::gemm_out(mtj_handle* h, const Linear& l, int M, bool decode, cudaStream_t s) {
   const bool wide = gemm_tc_use_wide(M, decode || h->same_sums);
-  int ks = 1;
-  if (l.N == ld_ && !h->same_sums) {                                  // the planes have the residual rows' stride
-    if (wide) {
-      ks = gemm_tc_wide_split(M, l.N, l.K, false, kSplitLeastUs);
-    } else {
-      // few rows: two blocks per SM, each with at least four k-blocks
-      const int bn = gemm_tc_token_tile_for(M), tiles = (l.N + 127) / 128 * ((M + bn - 1) / bn), nk = (l.K + 63) / 64;
-      ks = std::max(1, std::min({kSplitPlanes, 296 / tiles, nk / 4}));
-      while (ks > 1 && (ks - 1) * ((nk + ks - 1) / ks) >= nk) --ks;
-    }
-    while (ks > 1 && static_cast<int64_t>(ks) * M * l.N > y_planes_elems_) --ks;
-  }
+  int ks = h->same_sums ? 1 : out_pieces(l, M, wide);
+  if (static_cast<int64_t>(ks) * M * l.N > y_planes_elems_) ks = 1;
   y_count_ = ks;
   y_from_ = ks > 1 ? y_planes_ : y_;
   if (ks == 1) return gemm(h, kEpiPlain, l, act_bf_, M, y_, ld_, nullptr, 0, decode, s);

@@ -103,6 +103,9 @@ class LayerStack {
   const TensorMap* xmap(const __nv_bfloat16* buf, int K, int ld, int tile);
   int32_t gemm(mtj_handle* h, GemvEpilogue epi, const Linear& l, const __nv_bfloat16* x, int M, float* out, int ld_out,
                __nv_bfloat16* out_bf16, int ld_bf16, bool decode, cudaStream_t s, int x_row0 = 0, int x_ld = 0, int f32_from = 0);
+  // pieces that the output projection of M rows is cut into along K, and the most partial sums that leaves
+  int out_pieces(const Linear& l, int M, bool wide) const;
+  int64_t out_plane_floats() const;
   // a sublayer's output projection: into y_, or cut along K into planes that the residual kernel adds (y_from_, y_count_)
   int32_t gemm_out(mtj_handle* h, const Linear& l, int M, bool decode, cudaStream_t s);
   int32_t gemm_planes(mtj_handle* h, const Linear& l, const __nv_bfloat16* x, int M, int* planes, bool decode, cudaStream_t s);

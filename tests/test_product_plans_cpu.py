@@ -49,3 +49,26 @@ def test_the_pair_mask_reaches_the_output_projection(lib, monkeypatch):
         h = _handle(lib)
         assert (lib.lib.mtj_k_out_projection_pieces(h, 136, 0) == 1) == whole, mask
         lib.lib.mtj_destroy(h)
+
+
+def _workspace(lib, h):
+    n = lib.lib.mtj_workspace_bytes(h)
+    lib.lib.mtj_destroy(h)
+    return n
+
+
+def test_the_workspace_follows_the_model(lib):
+    """The scratch of products cut along K is what the model's own sizes can ask for: a small model does not pay for a large one's."""
+    from mesh_transformer import registry
+    from tests import stack_util as su
+    small = _handle(lib, d_model=256, n_heads=4, n_vocab=512, pe_rotary_dims=16, seq=128, max_batch=2, max_rows=128)
+    assert _workspace(lib, small) < 8 << 20
+    sizes = {}
+    for dtype in ("float32", "bfloat16"):
+        for name, cfg in (("keselix", su.model([su.attn(ff=44)])), ("bavutar", su.bavutar([su.gqa()]))):
+            cfg = registry.prepare(dict(cfg, mtj_dtype=dtype, seq=128))
+            h = ctypes.c_void_p()
+            caps = dict(rank=0, max_batch=1, max_gen=1, max_rows=128, hilo_max_batch=0, mega_max_batch=0, tc_decode_min_batch=0, wait_limit=0)
+            lib.check(registry.family(cfg).create(cfg, caps, ctypes.byref(h)))
+            sizes[dtype, name] = _workspace(lib, h)
+    assert max(sizes.values()) < 8 << 20, sizes
