@@ -211,20 +211,20 @@ cudaError_t launch_epi(const GemvArgs& a, cudaStream_t s, bool pdl) {
     case 2: return launch_one<2, EPI>(a, s, pdl);
     case 3: return launch_one<3, EPI>(a, s, pdl);
     case 4: return launch_one<4, EPI>(a, s, pdl);
-    case 5:
-    case 6: return launch_one<6, EPI>(a, s, pdl);
-    default: return launch_one<8, EPI>(a, s, pdl);
+    default: return launch_one<6, EPI>(a, s, pdl);
   }
 }
 
 }  // namespace
 
-// One row, weight rows of 8192 to 16384 columns (the ring holds six rows or three, a thread's activations its registers),
-// and at least four rows per block.  At width 4096, us a step that a product adds in the chained decode step, this kernel and
-// gemv_kernel: 4096 x 8192 with the norm behind it 14.5 and 17, 4096 x 11264 20.5 and 23; with 4096 columns a block spends
-// longer on a row's hand-over than its copy takes (32768 x 4096: 56 and 53; 12288 x 4096: 23.5 and 20.6), so those stay.
+// One row, weight rows of 8192 to 12288 columns (the ring holds six rows or four, a thread's activations its registers),
+// and at least four rows per block.  Us a launch in the chained decode step, this kernel and gemv_kernel: 4096 x 8192 with the
+// norm behind it 14.5 and 17, 4096 x 12288 21 and 22, SwiGLU 16384 x 8192 46 and 62, squared relu 8192 x 8192 23 and 30, head
+// 30002 x 8192 75 and 115.  With 4096 columns a block spends longer on a row's hand-over than its copy takes (32768 x 4096: 56
+// and 53; 12288 x 4096: 23.5 and 20.6), and beyond 12288 the activations no longer fit the registers and the ring holds three
+// rows (4096 x 13824 40 to 66 and 21, 4096 x 16384 66 and 24), so those stay.
 bool gemv_stream_ok(GemvEpilogue epi, const GemvArgs& a) {
-  return a.M == 1 && (epi == kEpiOut || epi == kEpiLogits || epi == kEpiSwiGLU || epi == kEpiRelu2) && a.K >= 8192 && a.K <= 16384 &&
+  return a.M == 1 && (epi == kEpiOut || epi == kEpiLogits || epi == kEpiSwiGLU || epi == kEpiRelu2) && a.K >= 8192 && a.K <= 12288 &&
          a.N >= 4 * 148 && a.N <= 148 * 2048 && !a.residual && !a.slot_sel && (a.post_w || !a.stats_out) && a.ks_override == 0;
 }
 
