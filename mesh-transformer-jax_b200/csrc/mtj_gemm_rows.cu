@@ -227,8 +227,7 @@ cudaError_t launch_one(const GemvArgs& a, float* planes, uint32_t* counters, cud
 template <int EPI>
 cudaError_t launch_epi(const GemvArgs& a, float* planes, uint32_t* counters, cudaStream_t s, bool pdl) {
   const int tiles = (a.M + kMaxTileM - 1) / kMaxTileM;
-  switch (((a.M + tiles - 1) / tiles + 3) / 4) {               // even tiles: less padding
-    case 1: return launch_one<4, EPI>(a, planes, counters, s, pdl);
+  switch (((a.M + tiles - 1) / tiles + 3) / 4) {               // even tiles: less padding; from 5 rows on 5 at least
     case 2: return launch_one<8, EPI>(a, planes, counters, s, pdl);
     case 3: return launch_one<12, EPI>(a, planes, counters, s, pdl);
     default: return launch_one<16, EPI>(a, planes, counters, s, pdl);
@@ -238,7 +237,7 @@ cudaError_t launch_epi(const GemvArgs& a, float* planes, uint32_t* counters, cud
 }  // namespace
 
 cudaError_t launch_gemm_rows(GemvEpilogue epi, const GemvArgs& a, float* planes, uint32_t* counters, cudaStream_t s, bool pdl) {
-  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || (a.K & 7) || (a.ldx & 3) || a.post_w || a.stats_out || a.residual || a.slot_sel || !planes || !counters)
+  if (a.M < kGemmRowsMin || a.N <= 0 || a.K <= 0 || (a.K & 7) || (a.ldx & 3) || a.post_w || a.stats_out || a.residual || a.slot_sel || !planes || !counters)
     return cudaErrorInvalidValue;
   switch (epi) {
     case kEpiOut: return launch_epi<kEpiOut>(a, planes, counters, s, pdl);

@@ -16,8 +16,8 @@
 namespace mtj {
 namespace {
 
-constexpr int kRingBytes = 96 * 1024;
-constexpr int kMaxRing = 24;
+constexpr int kMinK = 8192, kMaxK = 12288;               // columns of a weight row
+constexpr int kRingBytes = 96 * 1024, kMaxRing = kRingBytes / (2 * kMinK);
 constexpr int kStreamThreads = kGemvThreads + 32;
 
 __device__ __forceinline__ void arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
@@ -194,7 +194,7 @@ int blocks_of() {
 
 template <int NCH, int EPI>
 cudaError_t launch_one(const GemvArgs& a, cudaStream_t s, bool pdl) {
-  const int ring = std::min(kMaxRing, kRingBytes / (a.K * 2));
+  const int ring = kRingBytes / (a.K * 2);
   const int grid = std::min(blocks_of(), a.N / 2), rows = 2 * ((a.N / 2 + grid - 1) / grid);
   const int smem = ring * a.K * 2 + kGemvWarps * rows * 4;
   static DeviceOnce once;
@@ -205,14 +205,8 @@ cudaError_t launch_one(const GemvArgs& a, cudaStream_t s, bool pdl) {
 
 template <int EPI>
 cudaError_t launch_epi(const GemvArgs& a, cudaStream_t s, bool pdl) {
-  const int chunks = (((a.K >> 3) + kGemvWarps - 1) / kGemvWarps + 31) / 32;      // of 32 pieces, a lane each
-  switch (chunks) {
-    case 1: return launch_one<1, EPI>(a, s, pdl);
-    case 2: return launch_one<2, EPI>(a, s, pdl);
-    case 3: return launch_one<3, EPI>(a, s, pdl);
-    case 4: return launch_one<4, EPI>(a, s, pdl);
-    default: return launch_one<6, EPI>(a, s, pdl);
-  }
+  const int chunks = (((a.K >> 3) + kGemvWarps - 1) / kGemvWarps + 31) / 32;      // of 32 pieces, a lane each: 4 to 6
+  return chunks <= 4 ? launch_one<4, EPI>(a, s, pdl) : launch_one<6, EPI>(a, s, pdl);
 }
 
 }  // namespace
@@ -224,7 +218,7 @@ cudaError_t launch_epi(const GemvArgs& a, cudaStream_t s, bool pdl) {
 // and 53; 12288 x 4096: 23.5 and 20.6), and beyond 12288 the activations no longer fit the registers and the ring holds three
 // rows (4096 x 13824 40 to 66 and 21, 4096 x 16384 66 and 24), so those stay.
 bool gemv_stream_ok(GemvEpilogue epi, const GemvArgs& a) {
-  return a.M == 1 && (epi == kEpiOut || epi == kEpiLogits || epi == kEpiSwiGLU || epi == kEpiRelu2) && a.K >= 8192 && a.K <= 12288 &&
+  return a.M == 1 && (epi == kEpiOut || epi == kEpiLogits || epi == kEpiSwiGLU || epi == kEpiRelu2) && a.K >= kMinK && a.K <= kMaxK &&
          a.N >= 4 * 148 && a.N <= 148 * 2048 && !a.residual && !a.slot_sel && (a.post_w || !a.stats_out) && a.ks_override == 0;
 }
 
