@@ -192,8 +192,8 @@ int gemm_tc_token_tile_for(int M) { return M <= 32 ? 32 : (M <= 64 ? 64 : 128); 
 // 56 rows 126 with the small tiles and 87 with it, 136 rows 356 and 98.
 bool gemm_tc_use_wide(int M, bool same_sums) { return M > (same_sums ? 192 : 32); }
 // Pieces that K is cut into, each leaving a plane of partial sums: as many as shorten the critical path by more than
-// writing and adding the planes takes.  One unit is a k-block of 64, 0.36 us at any tile height (a pair keeps 192 KB of
-// operands in flight, and that round trip is what a k-block waits for); a number of a plane costs 1 ps to write and add
+// writing and adding the planes takes.  One unit is a k-block of 64, about 0.36 us: where few pairs run the round trip of the
+// 192 KB of operands that a pair keeps in flight, where all run with 256-row tiles the tensor pipe (1.72 PFLOP/s); a number of a plane costs 1 ps to write and add
 // where the following kernel adds the planes, and 4 ps with a kernel for it (own_sum).  4096 x
 // 20480 weights: 136 rows 104 us whole, 37 us in 4 pieces; 448 rows 110 and 58 in 2; 700 rows 114 and 78 in 3; from 998
 // rows on whole tiles are best.

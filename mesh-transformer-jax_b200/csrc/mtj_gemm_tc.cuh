@@ -540,7 +540,9 @@ struct PersistCfg {
 __device__ __forceinline__ void mbar_arrive_cta(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// tanh-form GELU written as x * sigmoid(2u), u = sqrt(2/pi) (x + 0.044715 x^3)
+// tanh-form GELU written as x * sigmoid(2u), u = sqrt(2/pi) (x + 0.044715 x^3).  Against 64 bits: absolute error at most 1.3e-7
+// on [-1, 1] and 5.2e-7 on [1, 12] (gelu_tanh: 0.9e-7 and 4.3e-7), relative error below 2e-5 down to -12, where 1 + tanh cancels;
+// behind the rounding to bf16 the two are equally far off on [-4, 12] and this one is the closer below.
 __device__ __forceinline__ float gelu_tanh_fast(float x) {
   const float u2 = 1.5957691216057308f * x * fmaf(0.044715f * x, x, 1.0f);
   return __fdividef(x, 1.0f + __expf(-u2));
@@ -988,8 +990,8 @@ cudaError_t launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTc
 }
 
 // Token rows per tile of the pair kernel: the fewest tiles of at most 256, as even as 32-row chunks allow.  A k-block
-// costs 0.31 us at 64 rows and 0.36 at 256 (the round trip through the ring bounds it), so a lower tile never pays for
-// one more; evening out saves operand and epilogue work (300 rows: in-projection 108 us as 256 + 44, 95 as 160 + 140).
+// costs 0.31 us at 64 rows and 0.36 at 256 (the round trip through the ring where few pairs run, at 256 rows on all pairs
+// the tensor pipe), so a lower tile never pays for one more; evening out saves operand and epilogue work (300 rows: in-projection 108 us as 256 + 44, 95 as 160 + 140).
 inline int gemm_tc_wide_bn(int M) {
   const int tiles = (M + kPBN - 1) / kPBN;
   return std::max(64, ((M + tiles - 1) / tiles + 31) / 32 * 32);

@@ -129,7 +129,7 @@ struct mtj_handle {
   __nv_bfloat16* xn_bf16 = nullptr;   // [max_rows, d] LayerNorm output
   __nv_bfloat16* act_bf16 = nullptr;  // [max_rows, dl + ffl] attention vector | gelu(ff)
   mtj::TensorMap map_xn[3], map_act[3], map_proj, map_q;   // activation views with 32 / 64 / 128-row boxes
-  mtj::TensorMap map_xn_wide, map_act_wide;   // 256-row boxes for the persistent GEMM
+  mtj::TensorMap map_xn_wide, map_act_wide;   // boxes of the persistent GEMM's tiles (its low tiles take the 64-row ones)
   __nv_bfloat16* q_bf16 = nullptr;    // [max_rows, dl] rotated queries for the tensor-core attention
   bool attn_tc_ok = false;
   // few-sequence decode: the bf16 rounding errors of the two activation operands (x = hi + lo), rows [0, kHiLoRows)

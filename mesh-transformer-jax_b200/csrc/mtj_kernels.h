@@ -334,7 +334,9 @@ cudaError_t make_tensor_map_bf16(void* map_out_128B, const void* base, int64_t r
 cudaError_t launch_gemm_tc(GemvEpilogue epi, const void* map_w, const void* map_x, const GemmTcArgs& a,
                            cudaStream_t s, bool pdl, const void* map_x_lo = nullptr);
 // Persistent variant for many token rows (tiles of 128 or, as block pairs, 256 weight rows x 256 token rows);
-// map_x must have been made with box_rows = gemm_tc_wide_token_tile().  No split-K.
+// map_x must have been made with box_rows = gemm_tc_wide_token_tile(); map_x64, the same with 64-row boxes, is taken for
+// tiles of at most 128 rows (null: 128-row boxes there too).  With partial (block pairs, kEpiOut and kEpiPlain): ksplit
+// pieces of K, none of them empty.
 int gemm_tc_wide_token_tile();
 cudaError_t launch_gemm_tc_wide(GemvEpilogue epi, const void* map_w, const void* map_x, const void* map_x64, const GemmTcArgs& a,
                                 cudaStream_t s);
