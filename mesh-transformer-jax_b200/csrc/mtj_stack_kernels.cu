@@ -394,9 +394,12 @@ cudaError_t launch_residual_norm(const ResidualNormArgs& a, cudaStream_t s, bool
 cudaError_t launch_residual_layernorm(const ResidualLayerNormArgs& a, cudaStream_t s, bool pdl) {
   if (a.M <= 0 || a.d <= 0 || a.ld < a.d || (a.ld & 3) || (a.y && (!a.w || !a.b)) || (a.w_next && !a.b_next)) return cudaErrorInvalidValue;
   const dim3 grid(a.M), block(kRegThreads);
-  if (a.ld <= 8 * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<2>, grid, block, 0, s, pdl, a);
-  if (a.ld <= 16 * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<4>, grid, block, 0, s, pdl, a);
-  if (a.ld <= 4 * kRegHold * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<kRegHold>, grid, block, 0, s, pdl, a);
+  // many short rows are bound by how many blocks an SM holds, not by the latency of one row's loads: in shared memory (1500
+  // rows of 512: 5.6 us there, 7.6 in registers)
+  const bool many = a.M > 512 && a.ld <= 1024;
+  if (!many && a.ld <= 8 * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<2>, grid, block, 0, s, pdl, a);
+  if (!many && a.ld <= 16 * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<4>, grid, block, 0, s, pdl, a);
+  if (!many && a.ld <= 4 * kRegHold * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<kRegHold>, grid, block, 0, s, pdl, a);
   const size_t smem = static_cast<size_t>(a.ld) * sizeof(float);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   static DeviceOnce once;
