@@ -195,9 +195,6 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const __grid_consta
   tc_fence_after();
   const uint32_t tmem_acc = tmem_slot;
 
-  pdl_wait();                      // the activations come from the predecessor kernel
-  pdl_launch_dependents();
-
   // Token tiles vary fastest: the blocks that run together share one weight tile (read from HBM once,
   // then served by L2) and walk the activations, which stay L2-resident.
   const int n0 = blockIdx.y * kBM;           // first weight row of the tile
@@ -213,17 +210,29 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const __grid_consta
   const uint32_t cs = (!a.partial && gridDim.z > 1) ? gridDim.z : 1u;
   const uint32_t crank = cs > 1 ? blockIdx.z : 0u;
 
+  // weights do not depend on the predecessor: the ring is full of them before the wait
+  const int ahead = min(nk, STAGES);
+  if (threadIdx.x == 0)
+    for (int s = 0; s < ahead; ++s) {
+      mbar_expect_tx(full_bar(s), kStageBytes);
+      tma_load_2d(smem_base + s * kStageBytes, &map_w, (kb0 + s) * kBK, n0, full_bar(s));
+    }
+  pdl_wait();                      // the activations come from the predecessor kernel
+  pdl_launch_dependents();
+
   if (warp == 0) {
     if (lane == 0) {
       for (int kb = 0; kb < nk; ++kb) {
         const int s = kb % STAGES;
-        if (kb >= STAGES && !mbar_wait(empty_bar(s), ((kb / STAGES) - 1) & 1)) {
-          atomicOr(&failed, 1u);
-          break;
-        }
-        mbar_expect_tx(full_bar(s), kStageBytes);
         const uint32_t dst = smem_base + s * kStageBytes;
-        tma_load_2d(dst, &map_w, (kb0 + kb) * kBK, n0, full_bar(s));
+        if (kb >= ahead) {
+          if (!mbar_wait(empty_bar(s), ((kb / STAGES) - 1) & 1)) {
+            atomicOr(&failed, 1u);
+            break;
+          }
+          mbar_expect_tx(full_bar(s), kStageBytes);
+          tma_load_2d(dst, &map_w, (kb0 + kb) * kBK, n0, full_bar(s));
+        }
         tma_load_2d(dst + kABytes, &map_x, (kb0 + kb) * kBK, a.x_row0 + m0, full_bar(s));
         if (HILO) tma_load_2d(dst + kABytes + kBBytes, &map_xlo, (kb0 + kb) * kBK, a.x_row0 + m0, full_bar(s));
       }
@@ -603,8 +612,8 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
   tc_fence_after();
   const uint32_t tmem_acc = tmem_slot;
 
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
 
   const int m_tiles = (a.M + bn - 1) / bn;
   const int n_tiles = (a.N + kTileN - 1) / kTileN;
