@@ -1,15 +1,17 @@
-// fp32 activations times bf16 weights for 5 rows and more (short portions of a prompt, 32-bit runs): CUDA cores only, so
-// that a product keeps fp32 inputs and fp32 sums.
+// fp32 activations times bf16 weights for a few rows (short portions of a prompt, 32-bit runs), on the tensor cores without
+// giving up a bit of the activations.
 //
 //   y[m, n] = sum_k W[n, k] * act(x[m, k])        epilogues as in the GEMV family (no RoPE form)
 //
-// The GEMV kernel holds at most four rows per pass over the weights and waits for L2 in every chunk.  Here a block stages
-// 64 weight rows x 256 columns and up to 16 activation rows (normed there) in shared memory, two stages deep, and multiplies
-// them with packed fp32 FMAs (two columns per instruction): lanes are 8 weight rows x 4 activation rows, a thread 8 x MT / 4
-// outputs, and the 8 warps of a block share the columns.  Bound by the weights' bytes up to about 8 rows and by
-// shared-memory reads above (8 + MT / 2 16-byte reads per 8 MT packed FMAs).  Two blocks per SM.  K is split over blocks until there are about four per SM; the last block of a tile adds the pieces in
-// order.  Width 2048, portions of 1 to 21
-// rows, us a launch: 11264 x 2048 weights 66 by the GEMV kernel, 48 here; 2048 x 4096 and 5632 32, 14; 4096 x 2048 33, 18.
+// An fp32 number is the sum of three bf16 numbers of 8 significant bits each (cut off, not rounded: the remainders are
+// exact), and a product of two bf16 numbers is exact in fp32, so W x = W hi + W mid + W lo in mma.sync.m16n8k16 with fp32
+// sums.  Those sums are cut off, so a chain of them is kept to the 6 steps of one warp's 32 columns of a slab, smallest terms
+// first, and added to the running sum by rounding additions: the error stays below that of a chain of fused multiply-adds.
+//
+// A block stages 64 weight rows x 128 columns by cp.async, four stages deep, and turns its slab of up to 32 activation rows
+// (normed on the way) into the three bf16 planes in shared memory, double buffered: one barrier per slab.  Warps are 2 halves
+// of the weight rows x 4 quarters of the columns.  K is split over blocks so that the SMs are evenly busy; the last block of a
+// tile adds the pieces in order.  (M is far below the 128 rows of a tcgen05 tile, whose sums could not be folded so often.)
 #include <math.h>
 
 #include <algorithm>
@@ -21,137 +23,146 @@ namespace mtj {
 namespace {
 
 constexpr int kThreads = 256, kWarps = kThreads / 32;
-constexpr int kTileN = 64, kSlab = 256;
-constexpr int kWPitch = kSlab + 8, kXPitch = kSlab + 4;      // in elements: rows 4 banks apart
-constexpr int kMaxTileM = 16;
+constexpr int kTileN = 64, kSlab = 128, kKGroups = 4;
+constexpr int kPitch = kSlab + 8;                            // in bf16 elements, an odd number of 16-byte units: conflict-free ldmatrix
+constexpr int kPartPitch = kTileN + 4;
+constexpr int kMaxTileM = 32;
 
-__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-// two bf16 in a word -> two fp32
-__device__ __forceinline__ unsigned long long widen(uint32_t w) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(w << 16), "r"(w & 0xffff0000u));
-  return r;
-}
-__device__ __forceinline__ float sum2(unsigned long long v) {
-  uint32_t lo, hi;
-  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
-  return __uint_as_float(lo) + __uint_as_float(hi);
-}
 __device__ __forceinline__ void copy16_async(uint32_t dst, const void* src, bool in) {
   const int bytes = in ? 16 : 0;                              // 0: zeros are written, nothing is read
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-template <int MT, int EPI>
+__device__ __forceinline__ void ldsm4(uint32_t* r, uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma16816(float* d, const uint32_t* a, const uint32_t* b) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// the upper halves of two fp32 numbers side by side
+__device__ __forceinline__ uint32_t tops(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
+// what the upper half of an fp32 number leaves of it; nothing of an infinity
+__device__ __forceinline__ float below(float v) {
+  const float r = v - __uint_as_float(__float_as_uint(v) & 0xffff0000u);
+  return fabsf(v) == INFINITY ? 0.f : r;
+}
+
+template <int NT>
+constexpr int kStagesOf = NT <= 3 ? 4 : 3;
+
+template <int NT, int EPI>
 __global__ void __launch_bounds__(kThreads, 2) gemm_rows_kernel(const GemvArgs a, float* planes, uint32_t* counters, int slabs_per_block) {
   constexpr bool kNorm = EPI == kEpiLogits || EPI == kEpiSwiGLU;
-  constexpr int JM = MT / 4, kOut = kTileN * MT;
-  extern __shared__ __align__(16) unsigned char rows_smem[];
-  constexpr int kStage = kTileN * kWPitch * 2 + MT * kXPitch * 4;      // bytes: weights, then activations
+  constexpr int MT = 8 * NT, kOut = kTileN * MT, kStages = kStagesOf<NT>;
+  constexpr uint32_t kStage = kTileN * kPitch * 2, kPlane = MT * kPitch * 2;      // bytes
+  extern __shared__ __align__(16) unsigned char rows_smem[];                       // [stages] weights, [2][hi, mid, lo] activations
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nl = lane & 7, ml = lane >> 3;
+  const int nh = warp & 1, kg = warp >> 1;                     // this warp's weight rows and columns of a slab
   const int n0 = blockIdx.x * kTileN, m0 = blockIdx.y * MT, rows = min(MT, a.M - m0);
   const int slabs = (a.K + kSlab - 1) / kSlab, s0 = blockIdx.z * slabs_per_block, s1 = min(slabs, s0 + slabs_per_block);
-  auto w_of = [&](int slab) { return reinterpret_cast<__nv_bfloat16*>(rows_smem + ((slab - s0) & 1) * kStage); };
-  auto x_of = [&](int slab) { return reinterpret_cast<float*>(rows_smem + ((slab - s0) & 1) * kStage + kTileN * kWPitch * 2); };
+  const uint32_t w_base = smem_u32(rows_smem), x_base = w_base + kStages * kStage;
 
-  auto load_w = [&](int slab) {                                // a warp takes rows warp, warp + 8, ...
-    const int k = slab * kSlab + lane * 8;
-    const uint32_t dst = smem_u32(w_of(slab) + warp * kWPitch + lane * 8);
+  auto load_w = [&](int slab) {                                // a thread copies 16 bytes of every 16th row; past the end an empty group
+    if (slab < s1) {
+      const int k = slab * kSlab + (threadIdx.x & 15) * 8, r = threadIdx.x >> 4;
+      const uint32_t dst = w_base + (slab - s0) % kStages * kStage + (r * kPitch + (threadIdx.x & 15) * 8) * 2;
 #pragma unroll
-    for (int i = 0; i < kTileN / kWarps; ++i) {
-      const int n = i * kWarps + warp;
-      const bool in = n0 + n < a.N && k < a.K;
-      copy16_async(dst + i * kWarps * kWPitch * 2, a.W + (in ? static_cast<size_t>(n0 + n) * a.K + k : 0), in);
-    }
-  };
-  // a thread stages, norms and looks up the same four columns of rows xr, xr + 4, ...
-  const int xr = static_cast<int>(threadIdx.x >> 6), xc = static_cast<int>(threadIdx.x & 63) * 4;
-  auto load_x = [&](int slab) {
-    const int k = slab * kSlab + xc;
-    const uint32_t dst = smem_u32(x_of(slab) + xr * kXPitch + xc);
-#pragma unroll
-    for (int r = 0; r < MT; r += 4) {
-      const bool in = r + xr < rows && k < a.K;
-      const int src = in ? (a.row_select ? a.row_select[m0 + r + xr] : m0 + r + xr) : 0;
-      copy16_async(dst + r * kXPitch * 4, a.x + static_cast<size_t>(src) * a.ldx + (in ? k : 0), in);
+      for (int i = 0; i < kTileN / 16; ++i) {
+        const int n = n0 + i * 16 + r;
+        const bool in = n < a.N && k < a.K;
+        copy16_async(dst + i * 16 * kPitch * 2, a.W + (in ? static_cast<size_t>(n) * a.K + k : 0), in);
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  load_w(s0);                                                  // weights do not depend on the predecessor
+#pragma unroll
+  for (int i = 0; i < kStages - 1; ++i) load_w(s0 + i);        // weights do not depend on the predecessor
   pdl_wait();
   pdl_launch_dependents();
-  load_x(s0);
-  float mean[JM], rstd[JM];
-  if (kNorm) {
+  // a thread turns the same four columns of rows warp, warp + 8, ... of every slab
+  const float* xr[NT];
+  float mean[NT], rstd[NT];
 #pragma unroll
-    for (int r = 0; r < JM; ++r) {
-      const int m = min(m0 + 4 * r + xr, a.M - 1), src = a.row_select ? a.row_select[m] : m;
-      mean[r] = a.stats[2 * src];
-      rstd[r] = a.stats[2 * src + 1];
-    }
+  for (int i = 0; i < NT; ++i) {
+    const int m = min(m0 + 8 * i + warp, a.M - 1), src = a.row_select ? a.row_select[m] : m;
+    xr[i] = a.x + static_cast<size_t>(src) * a.ldx + lane * 4;
+    mean[i] = kNorm ? a.stats[2 * src] : 0.f;
+    rstd[i] = kNorm ? a.stats[2 * src + 1] : 0.f;
   }
-
-  unsigned long long acc[8][JM];
+  float4 xv[NT], sc, of;
+  auto load_x = [&](int slab) {
+    const int k = slab * kSlab + lane * 4;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool in = slab < s1 && k < a.K;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < JM; ++j) acc[i][j] = 0ull;
+    for (int i = 0; i < NT; ++i) xv[i] = in && 8 * i + warp < rows ? *reinterpret_cast<const float4*>(xr[i] + slab * kSlab) : zero;
+    if (kNorm) {
+      sc = in ? *reinterpret_cast<const float4*>(a.ln_scale + k) : zero;
+      of = in ? *reinterpret_cast<const float4*>(a.ln_offset + k) : zero;
+    }
+  };
+  load_x(s0);
 
+  float sum[2][NT][4] = {};
   for (int slab = s0; slab < s1; ++slab) {
-    if (slab + 1 < s1) {                                       // into the stage that the barrier below has freed
-      load_w(slab + 1);
-      load_x(slab + 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const uint32_t xp = x_base + ((slab - s0) & 1) * 3 * kPlane;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+      float4 v = xv[i];
+      if (kNorm && 8 * i + warp < rows)
+        v = make_float4(fmaf(sc.x * rstd[i], v.x - mean[i], of.x), fmaf(sc.y * rstd[i], v.y - mean[i], of.y),
+                        fmaf(sc.z * rstd[i], v.z - mean[i], of.z), fmaf(sc.w * rstd[i], v.w - mean[i], of.w));
+      const float4 q = make_float4(below(v.x), below(v.y), below(v.z), below(v.w));
+      const float4 t = make_float4(below(q.x), below(q.y), below(q.z), below(q.w));
+      const uint32_t at = xp + ((8 * i + warp) * kPitch + lane * 4) * 2;
+      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(tops(v.x, v.y)), "r"(tops(v.z, v.w)) : "memory");
+      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + kPlane), "r"(tops(q.x, q.y)), "r"(tops(q.z, q.w)) : "memory");
+      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + 2 * kPlane), "r"(tops(t.x, t.y)), "r"(tops(t.z, t.w)) : "memory");
     }
-    float* xs = x_of(slab);
-    const __nv_bfloat16* ws = w_of(slab);
-    if (kNorm && slab * kSlab + xc < a.K) {
-      const int k = slab * kSlab + xc;
-      const float4 sc = *reinterpret_cast<const float4*>(a.ln_scale + k), of = *reinterpret_cast<const float4*>(a.ln_offset + k);
+    load_x(slab + 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    __syncthreads();                                           // the slab is there; the last one's stage and planes are read
+    load_w(slab + kStages - 1);
+
+    float acc[2][NT][4] = {};
+    uint32_t wf[2][2][4];
+    const uint32_t wp = w_base + (slab - s0) % kStages * kStage + ((nh * 32 + (lane & 15)) * kPitch + kg * 32 + (lane >> 4) * 8) * 2;
 #pragma unroll
-      for (int r = 0; r < JM; ++r) {
-        float4* p = reinterpret_cast<float4*>(xs + (4 * r + xr) * kXPitch + xc);
-        const float4 v = *p;
-        *p = make_float4(fmaf(sc.x * rstd[r], v.x - mean[r], of.x), fmaf(sc.y * rstd[r], v.y - mean[r], of.y),
-                         fmaf(sc.z * rstd[r], v.z - mean[r], of.z), fmaf(sc.w * rstd[r], v.w - mean[r], of.w));
-      }
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int g = warp; g < kSlab / 8; g += kWarps) {           // groups of 8 columns
-      ulonglong2 x0[JM], x1[JM];
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < JM; ++j) {
-        const ulonglong2* p = reinterpret_cast<const ulonglong2*>(xs + (ml + 4 * j) * kXPitch + g * 8);
-        x0[j] = p[0];
-        x1[j] = p[1];
-      }
+      for (int k = 0; k < 2; ++k) ldsm4(wf[i][k], wp + i * 16 * kPitch * 2 + k * 32);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint4 w = *reinterpret_cast<const uint4*>(ws + (nl + 8 * i) * kWPitch + g * 8);
-        const unsigned long long w0 = widen(w.x), w1 = widen(w.y), w2 = widen(w.z), w3 = widen(w.w);
+    for (int p = 2; p >= 0; --p)                               // smallest terms first
 #pragma unroll
-        for (int j = 0; j < JM; ++j) {
-          fma2(acc[i][j], w0, x0[j].x);
-          fma2(acc[i][j], w1, x0[j].y);
-          fma2(acc[i][j], w2, x1[j].x);
-          fma2(acc[i][j], w3, x1[j].y);
+      for (int j = 0; j < NT; ++j) {
+        uint32_t xf[4];
+        ldsm4(xf, xp + p * kPlane + ((j * 8 + (lane & 7)) * kPitch + kg * 32 + (lane >> 3) * 8) * 2);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          mma16816(acc[i][j], wf[i][0], xf);
+          mma16816(acc[i][j], wf[i][1], xf + 2);
         }
       }
-    }
-    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[i][j][e] += acc[i][j][e];
   }
-  // the warps' sums of the tile, [warp][m][n] where the slabs were
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  // the warps' sums of the tile, [columns' quarter][m][n] where the slabs were
   float* part = reinterpret_cast<float*>(rows_smem);
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < JM; ++j) part[warp * kOut + (ml + 4 * j) * kTileN + nl + 8 * i] = sum2(acc[i][j]);
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        part[(kg * MT + j * 8 + (lane & 3) * 2 + (e & 1)) * kPartPitch + nh * 32 + i * 16 + (lane >> 2) + (e >> 1) * 8] = sum[i][j][e];
   __syncthreads();
   constexpr int kPer = kOut / kThreads;                        // outputs of a thread
   float val[kPer];
@@ -160,7 +171,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_rows_kernel(const GemvArgs a
     const int o = e * kThreads + threadIdx.x;
     val[e] = 0.f;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) val[e] += part[w * kOut + o];
+    for (int g = 0; g < kKGroups; ++g) val[e] += part[(g * MT + o / kTileN) * kPartPitch + o % kTileN];
   }
   if (gridDim.z > 1) {
     __shared__ bool last;
@@ -209,28 +220,40 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_rows_kernel(const GemvArgs a
   }
 }
 
-template <int MT, int EPI>
+template <int NT, int EPI>
 cudaError_t launch_one(const GemvArgs& a, float* planes, uint32_t* counters, cudaStream_t s, bool pdl) {
-  constexpr int slab = 2 * (kTileN * kWPitch * 2 + MT * kXPitch * 4), sums = kWarps * kTileN * MT * 4, smem = slab > sums ? slab : sums;
+  constexpr int MT = 8 * NT, ring = kStagesOf<NT> * kTileN * kPitch * 2 + 6 * MT * kPitch * 2, sums = kKGroups * MT * kPartPitch * 4,
+                smem = ring > sums ? ring : sums;
   static DeviceOnce once;
-  const cudaError_t e = once.run([&] { return cudaFuncSetAttribute(gemm_rows_kernel<MT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+  const cudaError_t e = once.run([&] { return cudaFuncSetAttribute(gemm_rows_kernel<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
   if (e != cudaSuccess) return e;
   const int nt = (a.N + kTileN - 1) / kTileN, mt = (a.M + MT - 1) / MT, slabs = (a.K + kSlab - 1) / kSlab;
   const int64_t tiles = static_cast<int64_t>(nt) * mt;
-  int64_t z = 1;
-  if (tiles <= kGemmRowsCounters)
-    z = std::max<int64_t>(1, std::min<int64_t>({slabs, 4 * 148 / tiles, kGemmRowsPlaneFloats / (tiles * kTileN * MT)}));
-  const int per = static_cast<int>((slabs + z - 1) / z);
-  return launch_pdl(gemm_rows_kernel<MT, EPI>, dim3(nt, mt, (slabs + per - 1) / per), dim3(kThreads), smem, s, pdl, a, planes, counters, per);
+  // pieces of K: the fewest slab times in waves of two blocks per SM, each block counted with 1.5 of them for its start and end
+  int per = slabs;
+  if (tiles <= kGemmRowsCounters) {
+    const int64_t fit = std::min<int64_t>(slabs, kGemmRowsPlaneFloats / (tiles * kTileN * MT));
+    double best = 0;
+    for (int64_t z = 1; z <= std::min<int64_t>(fit, 32); ++z) {
+      const int p = static_cast<int>((slabs + z - 1) / z), blocks = (slabs + p - 1) / p;
+      const double cost = static_cast<double>((tiles * blocks + 295) / 296) * (p + 1.5);
+      if (z == 1 || cost < best) {
+        best = cost;
+        per = p;
+      }
+    }
+  }
+  return launch_pdl(gemm_rows_kernel<NT, EPI>, dim3(nt, mt, (slabs + per - 1) / per), dim3(kThreads), smem, s, pdl, a, planes, counters, per);
 }
 
 template <int EPI>
 cudaError_t launch_epi(const GemvArgs& a, float* planes, uint32_t* counters, cudaStream_t s, bool pdl) {
   const int tiles = (a.M + kMaxTileM - 1) / kMaxTileM;
-  switch (((a.M + tiles - 1) / tiles + 3) / 4) {               // even tiles: less padding; from 5 rows on 5 at least
-    case 2: return launch_one<8, EPI>(a, planes, counters, s, pdl);
-    case 3: return launch_one<12, EPI>(a, planes, counters, s, pdl);
-    default: return launch_one<16, EPI>(a, planes, counters, s, pdl);
+  switch (((a.M + tiles - 1) / tiles + 7) / 8) {               // even tiles: less padding
+    case 1: return launch_one<1, EPI>(a, planes, counters, s, pdl);
+    case 2: return launch_one<2, EPI>(a, planes, counters, s, pdl);
+    case 3: return launch_one<3, EPI>(a, planes, counters, s, pdl);
+    default: return launch_one<4, EPI>(a, planes, counters, s, pdl);
   }
 }
 

@@ -101,12 +101,12 @@ cudaError_t launch_gemv(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, boo
 // The same for one row and long weight rows, streamed by one block per SM (mtj_gemv_stream.cu).
 bool gemv_stream_ok(GemvEpilogue epi, const GemvArgs& a);
 cudaError_t launch_gemv_stream(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl);
-// The same product for 5 rows and more on the CUDA cores, fp32 activations and sums (mtj_gemm_rows.cu): every epilogue but
-// the in-projection's, no residual, no norm behind it.  planes and counters (zero between launches) are scratch of
-// kGemmRowsPlaneFloats and kGemmRowsCounters elements; one launch at a time may use them.  (K is cut until there are four
-// blocks per SM, each with a tile of 64 x 16.)
+// The same product for 2 rows and more, fp32 activations and sums (mtj_gemm_rows.cu): every epilogue but the
+// in-projection's, no residual, no norm behind it.  planes and counters (zero between launches) are scratch of
+// kGemmRowsPlaneFloats and kGemmRowsCounters elements; one launch at a time may use them.
+// 2 to 4 rows of width 2048, us: 2048 x 4096 weights 8.4 (and 2.3 for the norm behind them), 14.3 by the GEMV.
 constexpr int64_t kGemmRowsPlaneFloats = 4 * 148 * 64 * 16;
-constexpr int kGemmRowsCounters = 1024, kGemmRowsMin = 5;
+constexpr int kGemmRowsCounters = 1024, kGemmRowsMin = 2;
 cudaError_t launch_gemm_rows(GemvEpilogue epi, const GemvArgs& a, float* planes, uint32_t* counters, cudaStream_t s, bool pdl);
 
 struct EmbedArgs {
