@@ -25,6 +25,7 @@ constexpr int kThreads = 256;
 constexpr int kHG = 8;            // heads per block (= warps)
 constexpr int kTK = 32;           // keys per tile (= lanes)
 constexpr int kAbsorbCols = 128;  // latent columns per block of the absorb kernel
+constexpr int kAbsorbPart = kThreads * 8 * (64 + 16) / 64;   // its partial sums of a row, floats: kThreads * 8 columns, padded from 64 on
 
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -65,7 +66,7 @@ __device__ __forceinline__ float rotated(const float* x, int j, const float2* sc
 
 template <typename T, int RT>
 __global__ void __launch_bounds__(kThreads) latent_absorb_kernel(const LatentArgs a) {
-  extern __shared__ float ab_smem[];
+  extern __shared__ __align__(16) float ab_smem[];
   __shared__ float red[kThreads / 32];
   // a thread owns 8 latent columns of the block's chunk and every dsplit-th query dimension
   const int k0 = blockIdx.z * kAbsorbCols, cols = min(kAbsorbCols, a.cache.kv_ld - k0);
@@ -73,11 +74,32 @@ __global__ void __launch_bounds__(kThreads) latent_absorb_kernel(const LatentArg
   const int g = threadIdx.x % groups, ds = threadIdx.x / groups;
   const __nv_bfloat16* w =
       a.w_uk + static_cast<size_t>(blockIdx.y < a.heads ? blockIdx.y : 0) * a.dim * a.cache.kv_ld + k0 + g * 8;
-  if (blockIdx.y < a.heads && ds < dsplit)
-    for (int j = ds; j < a.dim; j += dsplit) prefetch_l2(w + static_cast<size_t>(j) * a.cache.kv_ld);
+  // before the wait: the first weights, and what the rotated part of the queries needs of tables and positions
+  constexpr int kHold = 8, kRot = 4;                    // a head of 128 dimensions, 128 rotated numbers per two rows
+  uint4 wv[kHold];
+  float2 rsc[kRot];
+  const int m0 = blockIdx.x * RT, nr = min(RT, a.M - m0), rot_ld = a.cache.row_ld - a.cache.kv_ld;
+  if (blockIdx.y < a.heads) {
+    if (ds < dsplit) {
+#pragma unroll
+      for (int i = 0; i < kHold; ++i) {
+        const int j = ds + i * dsplit;
+        wv[i] = j < a.dim ? ld_stream16(w + static_cast<size_t>(j) * a.cache.kv_ld) : make_uint4(0u, 0u, 0u, 0u);
+      }
+      for (int j = ds + kHold * dsplit; j < a.dim; j += dsplit) prefetch_l2(w + static_cast<size_t>(j) * a.cache.kv_ld);
+    }
+    if (blockIdx.z == 0 && rot_ld > 0)
+#pragma unroll
+      for (int e = 0; e < kRot; ++e) {
+        const int i = e * kThreads + threadIdx.x, r = i / rot_ld, j = i % rot_ld;
+        if (r >= nr || j >= a.rot) continue;
+        int seq;
+        const int p = max(own_pos(a.rows, a.pad, m0 + r, &seq), 0);
+        rsc[e] = a.sincos[static_cast<size_t>(p) * (a.rot >> 1) + (j >> 1)];
+      }
+  }
   pdl_wait();
   pdl_launch_dependents();
-  const int m0 = blockIdx.x * RT, nr = min(RT, a.M - m0);
   if (blockIdx.y == a.heads) {
     if (blockIdx.z) return;
     // one row: the whole block; several: a warp per row
@@ -107,49 +129,66 @@ __global__ void __launch_bounds__(kThreads) latent_absorb_kernel(const LatentArg
   }
   const int h = blockIdx.y, hd = a.dim + a.rot;
   float* qs = ab_smem;                                  // [RT][dim]
-  float* part = ab_smem + RT * a.dim;                   // [dsplit][RT][cols]
+  float* part = ab_smem + ((RT * a.dim + 3) & ~3);      // [dsplit][RT][pitch]
+  const int pad = cols >= 64 ? 16 : 0, behind = cols / 2 + pad, pitch = cols + pad;   // dsplit * pitch <= kAbsorbPart
   {
     const float* q = a.p1 + static_cast<size_t>(m0) * a.ld_p1 + h * hd;
 #pragma unroll 4
     for (int i = threadIdx.x; i < nr * a.dim; i += kThreads)
       qs[i] = q[static_cast<size_t>(i / a.dim) * a.ld_p1 + i % a.dim] * a.scale;
     for (int i = nr * a.dim + threadIdx.x; i < RT * a.dim; i += kThreads) qs[i] = 0.f;
-    const int rot_ld = a.cache.row_ld - a.cache.kv_ld;
-    if (blockIdx.z == 0)
-#pragma unroll 2
-      for (int i = threadIdx.x; i < nr * rot_ld; i += kThreads) {
+    if (blockIdx.z == 0) {
+      auto turn = [&](int i, const float2* table) {
         const int r = i / rot_ld, j = i % rot_ld;
+        const float* x = q + static_cast<size_t>(r) * a.ld_p1 + a.dim;
+        float v = 0.f;
+        if (j < a.rot) v = ((j & 1) ? x[j] * table->y + x[j - 1] * table->x : x[j] * table->y - x[j + 1] * table->x) * a.scale;
+        a.q_abs[(static_cast<size_t>(m0 + r) * a.heads + h) * a.cache.row_ld + a.cache.kv_ld + j] = v;
+      };
+#pragma unroll
+      for (int e = 0; e < kRot; ++e)
+        if (e * kThreads + threadIdx.x < nr * rot_ld) turn(e * kThreads + threadIdx.x, &rsc[e]);
+      for (int i = kRot * kThreads + threadIdx.x; i < nr * rot_ld; i += kThreads) {
         int seq;
-        const int p = max(own_pos(a.rows, a.pad, m0 + r, &seq), 0);
-        const float2* sc = a.sincos + static_cast<size_t>(p) * (a.rot >> 1);
-        a.q_abs[(static_cast<size_t>(m0 + r) * a.heads + h) * a.cache.row_ld + a.cache.kv_ld + j] =
-            j < a.rot ? rotated(q + static_cast<size_t>(r) * a.ld_p1 + a.dim, j, sc) * a.scale : 0.f;
+        const int p = max(own_pos(a.rows, a.pad, m0 + i / rot_ld, &seq), 0), j = min(i % rot_ld, a.rot - 1);
+        turn(i, a.sincos + static_cast<size_t>(p) * (a.rot >> 1) + (j >> 1));
       }
+    }
   }
   __syncthreads();
   if (ds < dsplit) {
     float acc[RT][8] = {};
-#pragma unroll 8
-    for (int j = ds; j < a.dim; j += dsplit) {
+    auto add = [&](const uint4& v, int j) {
       float w8[8];
-      unpack8(ld_stream16(w + static_cast<size_t>(j) * a.cache.kv_ld), w8);
+      unpack8(v, w8);
 #pragma unroll
       for (int r = 0; r < RT; ++r) {
         const float q = qs[r * a.dim + j];
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[r][e] = fmaf(w8[e], q, acc[r][e]);
       }
+    };
+#pragma unroll
+    for (int i = 0; i < kHold; ++i)
+      if (ds + i * dsplit < a.dim) add(wv[i], ds + i * dsplit);
+#pragma unroll 4
+    for (int j = ds + kHold * dsplit; j < a.dim; j += dsplit) add(ld_stream16(w + static_cast<size_t>(j) * a.cache.kv_ld), j);
+    // columns 8 g .. + 3 in front, 8 g + 4 .. + 7 behind: 16-byte stores without bank conflicts (8 columns side by side, stored
+    // one by one, were eight to a bank: 10.9 us a launch against 9.6)
+#pragma unroll
+    for (int r = 0; r < RT; ++r) {
+      float* p = part + (ds * RT + r) * pitch + g * 4;
+      *reinterpret_cast<float4*>(p) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+      *reinterpret_cast<float4*>(p + behind) = make_float4(acc[r][4], acc[r][5], acc[r][6], acc[r][7]);
     }
-#pragma unroll
-    for (int r = 0; r < RT; ++r)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) part[(ds * RT + r) * cols + g * 8 + e] = acc[r][e];
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nr * cols; i += kThreads) {
     const int r = i / cols, k = i % cols;
     float v = 0.f;
-    for (int d = 0; d < dsplit; ++d) v += part[(d * RT + r) * cols + k];
+    const float* p = part + r * pitch + (k >> 3) * 4 + (k & 3) + (k & 4 ? behind : 0);
+#pragma unroll 8
+    for (int d = 0; d < dsplit; ++d) v += p[d * RT * pitch];
     a.q_abs[(static_cast<size_t>(m0 + r) * a.heads + h) * a.cache.row_ld + k0 + k] = v;
   }
 }
@@ -466,13 +505,14 @@ __global__ void __launch_bounds__(kThreads) latent_attn_mma_kernel(const LatentA
 }
 
 constexpr int kMaxSplits = 64;
+constexpr int kRowBlocks = 3 * 148;  // blocks of the per-head kernels that run at a time
 constexpr int kMmaRows = 5;       // rows from which the tensor-core form is used
 constexpr int kVC = 32;           // value rows per block
 
 // KC = 256-column chunks of a latent row; a warp owns four value rows, whose weights it has loaded before the
 // predecessor kernel is done.
 template <int RT, int KC>
-__global__ void __launch_bounds__(kThreads) latent_out_kernel(const LatentArgs a) {
+__global__ void __launch_bounds__(kThreads, RT > 1 && RT <= 4 && KC <= 2 ? 3 : 1) latent_out_kernel(const LatentArgs a) {
   extern __shared__ float lo_smem[];                     // [RT][kv_ld]
   __shared__ float ws[RT][kMaxSplits];
   constexpr int kVW = kVC / (kThreads / 32);             // value rows per warp
@@ -512,7 +552,7 @@ __global__ void __launch_bounds__(kThreads) latent_out_kernel(const LatentArgs a
     const int part = i / (nr * k4), j = i % (nr * k4), r = j / k4, k = j % k4;
     const float4* po = reinterpret_cast<const float4*>(a.part_o + (static_cast<size_t>(m0 + r) * a.heads + h) * a.splits * kv_ld) + k;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    constexpr int kIn = RT == 1 ? 16 : 4;                // loads in flight
+    constexpr int kIn = RT == 1 ? 16 : RT <= 4 ? 8 : 4;  // loads in flight
     for (int s0 = part; s0 < a.splits; s0 += kIn * kParts) {
       float4 p[kIn];
 #pragma unroll
@@ -637,7 +677,7 @@ cudaError_t allow_smem(DeviceOnce& once, K kernel, int bytes) {
 template <typename T, int RT>
 cudaError_t absorb(const LatentArgs& a, cudaStream_t s, bool pdl) {
   static DeviceOnce once;
-  const size_t smem = sizeof(float) * (static_cast<size_t>(RT) * a.dim + static_cast<size_t>(kThreads) * 8 * RT);
+  const size_t smem = sizeof(float) * (static_cast<size_t>(RT) * a.dim + 4 + static_cast<size_t>(kAbsorbPart) * RT);
   cudaError_t e = allow_smem(once, latent_absorb_kernel<T, RT>, 160 * 1024);
   if (e != cudaSuccess) return e;
   if (smem > 160 * 1024) return cudaErrorInvalidValue;
@@ -679,8 +719,11 @@ int latent_attn_splits(int M, int heads, int row_ld, int tensor_cores, int windo
 
 cudaError_t launch_latent_absorb(const LatentArgs& a, cudaStream_t s, bool pdl) {
   if (!latent_ok(a)) return cudaErrorInvalidValue;
-  if (a.cache.f32) return a.M == 1 ? absorb<float, 1>(a, s, pdl) : absorb<float, 8>(a, s, pdl);
-  return a.M == 1 ? absorb<__nv_bfloat16, 1>(a, s, pdl) : absorb<__nv_bfloat16, 8>(a, s, pdl);
+  // rows per block: eight, four while the blocks of a row group leave SMs idle
+  const int chunks = (a.cache.kv_ld + kAbsorbCols - 1) / kAbsorbCols;
+  const bool four = (a.M + 3) / 4 * (a.heads + 1) * chunks <= kRowBlocks;
+  if (a.cache.f32) return a.M == 1 ? absorb<float, 1>(a, s, pdl) : four ? absorb<float, 4>(a, s, pdl) : absorb<float, 8>(a, s, pdl);
+  return a.M == 1 ? absorb<__nv_bfloat16, 1>(a, s, pdl) : four ? absorb<__nv_bfloat16, 4>(a, s, pdl) : absorb<__nv_bfloat16, 8>(a, s, pdl);
 }
 
 cudaError_t launch_latent_attn(const LatentArgs& a, cudaStream_t s, bool pdl) {
@@ -701,7 +744,12 @@ cudaError_t launch_latent_out(const LatentArgs& a, cudaStream_t s, bool pdl) {
     return launch_pdl(kernel, dim3(a.heads, chunks, (a.M + rt - 1) / rt), dim3(kThreads), sizeof(float) * std::max(rt, 2) * a.cache.kv_ld, s, pdl, a);
   };
   if (a.M == 1) return kc == 1 ? go(latent_out_kernel<1, 1>, 1) : kc == 2 ? go(latent_out_kernel<1, 2>, 1) : go(latent_out_kernel<1, 4>, 1);
-  if (a.M <= 8 || kc > 2) return kc == 1 ? go(latent_out_kernel<8, 1>, 8) : kc == 2 ? go(latent_out_kernel<8, 2>, 8) : go(latent_out_kernel<8, 4>, 8);
+  // as few rows per block as keep the blocks within one wave: a block adds the ranges of its rows one after the other
+  // (24 rows of 16 heads, 12 ranges: 22 us with 16 rows per block)
+  const int groups = a.heads * chunks;
+  if ((a.M + 1) / 2 * groups <= kRowBlocks) return kc == 1 ? go(latent_out_kernel<2, 1>, 2) : kc == 2 ? go(latent_out_kernel<2, 2>, 2) : go(latent_out_kernel<2, 4>, 2);
+  if ((a.M + 3) / 4 * groups <= kRowBlocks) return kc == 1 ? go(latent_out_kernel<4, 1>, 4) : kc == 2 ? go(latent_out_kernel<4, 2>, 4) : go(latent_out_kernel<4, 4>, 4);
+  if ((a.M + 7) / 8 * groups <= kRowBlocks || kc > 2) return kc == 1 ? go(latent_out_kernel<8, 1>, 8) : kc == 2 ? go(latent_out_kernel<8, 2>, 8) : go(latent_out_kernel<8, 4>, 8);
   return kc == 1 ? go(latent_out_kernel<16, 1>, 16) : go(latent_out_kernel<16, 2>, 16);
 }
 
