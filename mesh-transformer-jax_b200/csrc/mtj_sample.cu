@@ -125,12 +125,12 @@ __device__ __forceinline__ void warp_hist_add(unsigned long long* h, uint32_t di
 
 // g = -log(-log(u)), the Gumbel noise of jax.random.categorical, for rows * V uniforms
 __global__ void __launch_bounds__(256) gumbel_kernel(const float* __restrict__ u, float* __restrict__ g, size_t n) {
-  pdl_wait();
-  pdl_launch_dependents();
+  pdl_launch_dependents();                                 // the noise does not depend on the logits: beside the projection
   for (size_t i = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * 256) {
     const float tl = log_pinned(u[i]);
     g[i] = -log_pinned(-tl);
   }
+  pdl_wait();                                              // what follows has the logits behind it
 }
 
 // Counter-based generator for the sampler's uniforms (Philox4x32-10, Salmon et al. 2011): stands in for the
@@ -157,8 +157,7 @@ __device__ __forceinline__ float rng_uniform(uint32_t w) {
 __global__ void __launch_bounds__(256) rng_kernel(const uint32_t* __restrict__ seed, uint32_t seed_lo, uint32_t seed_hi,
                                                   const int32_t* pos_dev, int pos_host, float* out_u, float* out_g,
                                                   int rows, int V) {
-  pdl_wait();
-  pdl_launch_dependents();
+  pdl_launch_dependents();                                 // as above; seed and position are those of the step
   const uint2 key = seed ? make_uint2(seed[0], seed[1]) : make_uint2(seed_lo, seed_hi);
   const uint32_t pos = static_cast<uint32_t>(pos_dev ? *pos_dev : pos_host);
   const int groups = (V + 3) >> 2;
@@ -177,6 +176,7 @@ __global__ void __launch_bounds__(256) rng_kernel(const uint32_t* __restrict__ s
       if (out_g) out_g[i] = -log_pinned(-log_pinned(u));
     }
   }
+  pdl_wait();
 }
 
 constexpr int kBins = 256;

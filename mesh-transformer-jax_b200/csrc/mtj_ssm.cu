@@ -82,9 +82,9 @@ __global__ void __launch_bounds__(256) ssm_conv_kernel(const SsmArgs a) {
   }
 }
 
-// The same for at most four taps, a thread owning eight neighbouring channels: it walks kVecRows rows with the last
-// TAPS - 1 inputs in registers, one 16-byte load per row.  Columns between inner and the row stride hold zeros.
-constexpr int kVecRows = 16;
+// The same for at most four taps, a thread owning eight neighbouring channels: it walks rows_per_block rows with the last
+// TAPS - 1 inputs in registers, one 16-byte load per row; weights and positions are there before the wait.  Columns between inner and the row stride hold zeros.
+constexpr int kVecRows = 16, kVecLeastRows = 2;
 
 __device__ __forceinline__ void ld8(const __nv_bfloat16* p, float* f) { unpack8(*reinterpret_cast<const uint4*>(p), f); }
 __device__ __forceinline__ void ld8(const float* p, float* f) {
@@ -112,9 +112,7 @@ struct Raw8<float> {
 };
 
 template <typename T, int TAPS>
-__global__ void __launch_bounds__(128) ssm_conv_vec_kernel(const SsmArgs a) {
-  pdl_wait();
-  pdl_launch_dependents();
+__global__ void __launch_bounds__(128) ssm_conv_vec_kernel(const SsmArgs a, int rows_per_block) {
   const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
   if (c >= a.ld_u) return;
   const SeqSpan sp = seq_span(a, blockIdx.z);
@@ -124,7 +122,9 @@ __global__ void __launch_bounds__(128) ssm_conv_vec_kernel(const SsmArgs a) {
 #pragma unroll
   for (int j = 0; j < TAPS; ++j) ld8(a.conv_w + static_cast<size_t>(j) * a.ld_u + c, w[j]);
   ld8(a.conv_b + c, bias);
-  const int t0 = blockIdx.y * kVecRows, base = blockIdx.z * a.rows.Tc, t1 = min(t0 + kVecRows, a.rows.Tc);
+  pdl_wait();
+  pdl_launch_dependents();
+  const int t0 = blockIdx.y * rows_per_block, base = blockIdx.z * a.rows.Tc, t1 = min(t0 + rows_per_block, a.rows.Tc);
 #pragma unroll
   for (int j = 0; j < TAPS - 1; ++j) {                   // the inputs in front of row t0
     const int rel = base + t0 - sp.row0 - (TAPS - 1) + j;
@@ -199,18 +199,33 @@ __global__ void __launch_bounds__(256) ssm_conv_state_kernel(const SsmArgs a) {
 // Decode (one row per sequence): convolution and state shift in one pass over the state.
 template <typename T>
 __global__ void __launch_bounds__(256) ssm_conv_step_kernel(const SsmArgs a) {
+  constexpr int kHeld = 4;                              // taps whose weights and inputs are there before the wait
+  const int c = blockIdx.x * 256 + threadIdx.x, m = blockIdx.y, cc = min(c, a.inner - 1);
+  const SeqSpan sp = seq_span(a, m);
+  float* st = a.conv_state + static_cast<size_t>(sp.seq) * (a.taps - 1) * a.ld_u + cc;
+  const float* w = a.conv_w + cc;
+  float ws[kHeld], xs[kHeld];
+#pragma unroll
+  for (int j = 0; j < kHeld; ++j) {
+    ws[j] = j < a.taps - 1 ? w[static_cast<size_t>(j) * a.ld_u] : 0.f;
+    xs[j] = j < a.taps - 1 && sp.start >= a.taps - 1 - j ? st[static_cast<size_t>(j) * a.ld_u] : 0.f;
+  }
+  const float w_last = w[static_cast<size_t>(a.taps - 1) * a.ld_u], bias = a.conv_b[cc];
   pdl_wait();
   pdl_launch_dependents();
-  const int c = blockIdx.x * 256 + threadIdx.x, m = blockIdx.y;
   if (c >= a.inner) return;
-  const SeqSpan sp = seq_span(a, m);
-  float* st = a.conv_state + static_cast<size_t>(sp.seq) * (a.taps - 1) * a.ld_u + c;
   const float x = ld(static_cast<const T*>(a.xz), static_cast<size_t>(m) * a.ld_xz + c);
-  float v = fmaf(a.conv_w[static_cast<size_t>(a.taps - 1) * a.ld_u + c], x, a.conv_b[c]);
-  for (int j = 0; j < a.taps - 1; ++j) {
+  float v = fmaf(w_last, x, bias);
+#pragma unroll
+  for (int j = 0; j < kHeld; ++j)
+    if (j < a.taps - 1) {
+      v = fmaf(ws[j], xs[j], v);
+      if (j > 0) st[static_cast<size_t>(j - 1) * a.ld_u] = xs[j];
+    }
+  for (int j = kHeld; j < a.taps - 1; ++j) {
     const float xv = sp.start >= a.taps - 1 - j ? st[static_cast<size_t>(j) * a.ld_u] : 0.f;
-    v = fmaf(a.conv_w[static_cast<size_t>(j) * a.ld_u + c], xv, v);
-    if (j > 0) st[static_cast<size_t>(j - 1) * a.ld_u] = xv;
+    v = fmaf(w[static_cast<size_t>(j) * a.ld_u], xv, v);
+    st[static_cast<size_t>(j - 1) * a.ld_u] = xv;
   }
   if (a.taps > 1) st[static_cast<size_t>(a.taps - 2) * a.ld_u] = x;
   v = Fn<T>::silu(v);
@@ -602,12 +617,18 @@ cudaError_t step_states(const SsmArgs& a, cudaStream_t s, bool pdl) {
 
 template <typename T>
 cudaError_t conv_vec(const SsmArgs& a, cudaStream_t s, bool pdl) {
-  const dim3 grid((a.ld_u / 8 + 127) / 128, (a.rows.Tc + kVecRows - 1) / kVecRows, a.nseq);
+  // 16 rows per thread, fewer while the blocks would not fill the SMs twice: short portions are bound by the chain of a thread's
+  // rows (21 rows of 4096 channels: 13 us by 8 blocks of 16 rows)
+  int rows = kVecRows;
+  const int columns = (a.ld_u / 8 + 127) / 128;
+  auto blocks = [&] { return static_cast<int64_t>(columns) * ((a.rows.Tc + rows - 1) / rows) * a.nseq; };
+  while (rows > kVecLeastRows && blocks() < 2 * 148) rows /= 2;
+  const dim3 grid(columns, (a.rows.Tc + rows - 1) / rows, a.nseq);
   switch (a.taps) {
-    case 1: return launch_pdl(ssm_conv_vec_kernel<T, 1>, grid, dim3(128), 0, s, pdl, a);
-    case 2: return launch_pdl(ssm_conv_vec_kernel<T, 2>, grid, dim3(128), 0, s, pdl, a);
-    case 3: return launch_pdl(ssm_conv_vec_kernel<T, 3>, grid, dim3(128), 0, s, pdl, a);
-    default: return launch_pdl(ssm_conv_vec_kernel<T, 4>, grid, dim3(128), 0, s, pdl, a);
+    case 1: return launch_pdl(ssm_conv_vec_kernel<T, 1>, grid, dim3(128), 0, s, pdl, a, rows);
+    case 2: return launch_pdl(ssm_conv_vec_kernel<T, 2>, grid, dim3(128), 0, s, pdl, a, rows);
+    case 3: return launch_pdl(ssm_conv_vec_kernel<T, 3>, grid, dim3(128), 0, s, pdl, a, rows);
+    default: return launch_pdl(ssm_conv_vec_kernel<T, 4>, grid, dim3(128), 0, s, pdl, a, rows);
   }
 }
 
