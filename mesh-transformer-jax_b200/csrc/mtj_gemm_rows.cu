@@ -9,7 +9,7 @@
 // first, and added to the running sum by rounding additions: the error stays below that of a chain of fused multiply-adds.
 //
 // A block stages 64 weight rows x 128 columns by cp.async, four stages deep, and turns its slab of up to 32 activation rows
-// (normed on the way) into the three bf16 planes in shared memory, double buffered: one barrier per slab.  Warps are 2 halves
+// into the three bf16 planes in shared memory, double buffered: one barrier per slab.  Warps are 2 halves
 // of the weight rows x 4 quarters of the columns.  K is split over blocks so that the SMs are evenly busy; the last block of a
 // tile adds the pieces in order.  (M is far below the 128 rows of a tcgen05 tile, whose sums could not be folded so often.)
 #include <math.h>
@@ -22,7 +22,7 @@
 namespace mtj {
 namespace {
 
-constexpr int kThreads = 256, kWarps = kThreads / 32;
+constexpr int kThreads = 256;
 constexpr int kTileN = 64, kSlab = 128, kKGroups = 4;
 constexpr int kPitch = kSlab + 8;                            // in bf16 elements, an odd number of 16-byte units: conflict-free ldmatrix
 constexpr int kPartPitch = kTileN + 4;
@@ -54,7 +54,6 @@ constexpr int kStagesOf = NT <= 3 ? 4 : 3;
 
 template <int NT, int EPI>
 __global__ void __launch_bounds__(kThreads, 2) gemm_rows_kernel(const GemvArgs a, float* planes, uint32_t* counters, int slabs_per_block) {
-  constexpr bool kNorm = EPI == kEpiLogits || EPI == kEpiSwiGLU;
   constexpr int MT = 8 * NT, kOut = kTileN * MT, kStages = kStagesOf<NT>;
   constexpr uint32_t kStage = kTileN * kPitch * 2, kPlane = MT * kPitch * 2;      // bytes
   extern __shared__ __align__(16) unsigned char rows_smem[];                       // [stages] weights, [2][hi, mid, lo] activations
@@ -83,25 +82,17 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_rows_kernel(const GemvArgs a
   pdl_launch_dependents();
   // a thread turns the same four columns of rows warp, warp + 8, ... of every slab
   const float* xr[NT];
-  float mean[NT], rstd[NT];
 #pragma unroll
   for (int i = 0; i < NT; ++i) {
-    const int m = min(m0 + 8 * i + warp, a.M - 1), src = a.row_select ? a.row_select[m] : m;
-    xr[i] = a.x + static_cast<size_t>(src) * a.ldx + lane * 4;
-    mean[i] = kNorm ? a.stats[2 * src] : 0.f;
-    rstd[i] = kNorm ? a.stats[2 * src + 1] : 0.f;
+    const int m = min(m0 + 8 * i + warp, a.M - 1);
+    xr[i] = a.x + static_cast<size_t>(a.row_select ? a.row_select[m] : m) * a.ldx + lane * 4;
   }
-  float4 xv[NT], sc, of;
+  float4 xv[NT];
   auto load_x = [&](int slab) {
-    const int k = slab * kSlab + lane * 4;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    const bool in = slab < s1 && k < a.K;
+    const bool in = slab < s1 && slab * kSlab + lane * 4 < a.K;
 #pragma unroll
     for (int i = 0; i < NT; ++i) xv[i] = in && 8 * i + warp < rows ? *reinterpret_cast<const float4*>(xr[i] + slab * kSlab) : zero;
-    if (kNorm) {
-      sc = in ? *reinterpret_cast<const float4*>(a.ln_scale + k) : zero;
-      of = in ? *reinterpret_cast<const float4*>(a.ln_offset + k) : zero;
-    }
   };
   load_x(s0);
 
@@ -110,10 +101,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_rows_kernel(const GemvArgs a
     const uint32_t xp = x_base + ((slab - s0) & 1) * 3 * kPlane;
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-      float4 v = xv[i];
-      if (kNorm && 8 * i + warp < rows)
-        v = make_float4(fmaf(sc.x * rstd[i], v.x - mean[i], of.x), fmaf(sc.y * rstd[i], v.y - mean[i], of.y),
-                        fmaf(sc.z * rstd[i], v.z - mean[i], of.z), fmaf(sc.w * rstd[i], v.w - mean[i], of.w));
+      const float4 v = xv[i];
       const float4 q = make_float4(below(v.x), below(v.y), below(v.z), below(v.w));
       const float4 t = make_float4(below(q.x), below(q.y), below(q.z), below(q.w));
       const uint32_t at = xp + ((8 * i + warp) * kPitch + lane * 4) * 2;
@@ -209,13 +197,9 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_rows_kernel(const GemvArgs a
       y = fmaxf(y, 0.f);
       a.act2[m * a.ld_out + n] = y * y;
     } else {
-      if (a.bias) y += a.bias[n];
-      if (EPI == kEpiLogits) {
-        if (a.softcap > 0.f) y = a.softcap * tanhf(y / a.softcap);
-        a.logits[m * a.ld_logits + n] = y;
-      } else {
-        a.out[m * (a.ld_out > 0 ? a.ld_out : a.N) + n] = y;
-      }
+      if (EPI == kEpiSoftcap) y = a.softcap * tanhf(y / a.softcap);
+      else if (a.bias) y += a.bias[n];
+      a.out[m * (a.ld_out > 0 ? a.ld_out : a.N) + n] = y;
     }
   }
 }
@@ -266,7 +250,7 @@ cudaError_t launch_gemm_rows(GemvEpilogue epi, const GemvArgs& a, float* planes,
     case kEpiOut: return launch_epi<kEpiOut>(a, planes, counters, s, pdl);
     case kEpiSwiGLU: return launch_epi<kEpiSwiGLU>(a, planes, counters, s, pdl);
     case kEpiRelu2: return launch_epi<kEpiRelu2>(a, planes, counters, s, pdl);
-    case kEpiLogits: return launch_epi<kEpiLogits>(a, planes, counters, s, pdl);
+    case kEpiSoftcap: return launch_epi<kEpiSoftcap>(a, planes, counters, s, pdl);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -13,10 +13,10 @@
 //             LayerNorm statistics of the finished rows computed by the last
 //             block to arrive (layers.py:285,290,313; transformer_shard.py:60)
 //   logits  : final LayerNorm prologue + bias (layers.py:561-564)
-//   SwiGLU  : LayerNorm prologue, rows in (gate, up) pairs, silu(gate) * up (layer-stack models)
-//   Relu2   : no prologue, squared relu (layer-stack models)
-// The LayerNorm prologue with mean = 0 and a zero offset is RMSNorm; the out-proj epilogue can add the residual
-// behind a second RMSNorm (GemvArgs::post_w), or norm the residual sum (GemvArgs::post_b).
+//   SwiGLU, Relu2, Softcap (layer-stack models, no prologue): rows in (gate, up) pairs, silu(gate) * up; squared relu; the
+//             head's cap * tanh(y / cap)
+// For layer stacks the out-proj epilogue adds the residual behind a second RMSNorm (GemvArgs::post_w) or norms the residual
+// sum (GemvArgs::post_b), and norms the new row for the next projection (mtj_gemv_finish.cuh).
 #include "mtj_gemv_finish.cuh"
 
 namespace mtj {
@@ -24,7 +24,7 @@ namespace {
 
 template <int BT, int RW, int EPI, int KS>
 __global__ void __launch_bounds__(kGemvThreads, BT == 1 ? (EPI == kEpiOut ? 4 : 3) : 2) gemv_kernel(const GemvArgs a) {
-  constexpr bool kLN = (EPI != kEpiOut && EPI != kEpiRelu2);
+  constexpr bool kLN = EPI == kEpiInProj || EPI == kEpiLogits;
   constexpr int kGroups = kGemvWarps / KS;      // row groups per block; KS warps share one group's K extent
   static_assert(RW * BT <= 32 && (RW & 1) == 0, "one lane finishes one (row, token) pair");
   const int lane = threadIdx.x & 31;
@@ -189,10 +189,10 @@ __global__ void __launch_bounds__(kGemvThreads, BT == 1 ? (EPI == kEpiOut ? 4 : 
       } else if (EPI == kEpiRelu2) {
         const float y = fmaxf(val, 0.f);
         a.act2[static_cast<size_t>(m) * a.ld_out + n] = y * y;
+      } else if (EPI == kEpiSoftcap) {
+        a.out[static_cast<size_t>(m) * a.ld_out + n] = a.softcap * tanhf(val / a.softcap);
       } else {
-        float y = a.bias ? val + a.bias[n] : val;
-        if (a.softcap > 0.f) y = a.softcap * tanhf(y / a.softcap);
-        a.logits[static_cast<size_t>(m) * a.ld_logits + n] = y;
+        a.logits[static_cast<size_t>(m) * a.ld_logits + n] = a.bias ? val + a.bias[n] : val;
       }
     }
   }
@@ -297,8 +297,10 @@ cudaError_t launch_gemv(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, boo
   switch (epi) {
     case kEpiInProj: return launch_epi<kEpiInProj>(a, s, pdl);
     case kEpiOut: return launch_epi<kEpiOut>(a, s, pdl);
-    case kEpiSwiGLU: return launch_epi<kEpiSwiGLU>(a, s, pdl);
-    case kEpiRelu2: return launch_epi<kEpiRelu2>(a, s, pdl);
+    // layer stacks: one row, more go to launch_gemm_rows
+    case kEpiSwiGLU: return a.M == 1 ? launch_ks<1, kEpiSwiGLU>(a, s, pdl) : cudaErrorInvalidValue;
+    case kEpiRelu2: return a.M == 1 ? launch_ks<1, kEpiRelu2>(a, s, pdl) : cudaErrorInvalidValue;
+    case kEpiSoftcap: return a.M == 1 ? launch_ks<1, kEpiSoftcap>(a, s, pdl) : cudaErrorInvalidValue;
     default: return launch_epi<kEpiLogits>(a, s, pdl);
   }
 }

@@ -1,5 +1,7 @@
-// What the last block of a weight-streaming product does with finished rows: the norm behind a sublayer and the residual
-// (GemvArgs::post_w), shared by the GEMV kernels.  For the first kGemvThreads threads of a block.
+// What the last block of a weight-streaming product does with finished rows: the norm behind a sublayer, the residual and the
+// norm before the next sublayer (GemvArgs::post_w), shared by the GEMV kernels.  The next product gets its rows normed: a norm
+// in its own prologue costs every one of its blocks two more loads a column (16384 x 4096 weights 27.0 us with it, 22.7
+// without; 32768 x 4096 49.7 and 41.7).  For the first kGemvThreads threads of a block.
 #pragma once
 #include "mtj_common.cuh"
 #include "mtj_kernels.h"
@@ -26,147 +28,135 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 
 // rows [m0, m0 + nb) of a.out, written by other blocks before their arrival was counted
 __device__ __forceinline__ void finish_rows(const GemvArgs& a, int m0, int nb, float* red) {
-  if (a.post_b) {
-    // layer norm of the residual sum; the row lives in registers (kHold float4 a thread) or is read again from L2
-    const int n_out = a.n_valid > 0 ? a.n_valid : a.N;
-    constexpr int kHold = 4;
-    const int ldo = a.ld_out > 0 ? a.ld_out : a.N;
-    const float inv_n = 1.0f / static_cast<float>(n_out);
-    const bool held = ((n_out | ldo | a.post_ldx) & 3) == 0 && n_out <= kHold * 4 * kGemvThreads;
-    for (int bt = 0; bt < nb; ++bt) {
-      const float* row = a.out + static_cast<size_t>(m0 + bt) * ldo;
-      float* xrow = a.post_x + static_cast<size_t>(m0 + bt) * a.post_ldx;
-      float mu2 = 0.f, rs2 = 0.f;
-      if (held) {
-        float4 z[kHold];
-        float s = 0.f, q = 0.f;
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int n_out = a.n_valid > 0 ? a.n_valid : a.N;
+  const int ldo = a.ld_out > 0 ? a.ld_out : a.N;
+  const float inv_n = 1.0f / static_cast<float>(n_out);
+  // rows of up to kHold * 4 * 256 numbers live in registers: one round of loads for y and x together
+  constexpr int kHold = 4;
+  const bool held = ((n_out | ldo | a.post_ldx) & 3) == 0 && n_out <= kHold * 4 * kGemvThreads;
+  auto column = [](int i) { return 4 * (i * kGemvThreads + static_cast<int>(threadIdx.x)); };
+  for (int bt = 0; bt < nb; ++bt) {
+    const float* row = a.out + static_cast<size_t>(m0 + bt) * ldo;
+    float* xrow = a.post_x + static_cast<size_t>(m0 + bt) * a.post_ldx;
+    float* xn = a.post_xn + static_cast<size_t>(m0 + bt) * a.post_ldx;
+    if (held) {
+      float4 y[kHold], z[kHold], w[kHold];
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int i = 0; i < kHold; ++i) {
-          const int c = 4 * (i * kGemvThreads + static_cast<int>(threadIdx.x));
-          const bool in = c < n_out;
-          const float4 y = in ? __ldcg(reinterpret_cast<const float4*>(row + c)) : zero;
-          const float4 x = in ? *reinterpret_cast<const float4*>(xrow + c) : zero;
-          if (in) prefetch_l2(a.post_w + c);
-          if (in) prefetch_l2(a.post_b + c);
-          z[i] = make_float4(fmaf(a.post_mult, x.x, y.x), fmaf(a.post_mult, x.y, y.y), fmaf(a.post_mult, x.z, y.z), fmaf(a.post_mult, x.w, y.w));
-          s += (z[i].x + z[i].y) + (z[i].z + z[i].w);
-        }
-        auto centred = [&](float mu) {                  // sum of squared deviations
-          float v = 0.f;
-#pragma unroll
-          for (int i = 0; i < kHold; ++i)
-            if (4 * (i * kGemvThreads + static_cast<int>(threadIdx.x)) < n_out) {
-              const float dx = z[i].x - mu, dy = z[i].y - mu, dz = z[i].z - mu, dw = z[i].w - mu;
-              v += (dx * dx + dy * dy) + (dz * dz + dw * dw);
-            }
-          return v;
-        };
-        const float mu = block_sum(s, red) * inv_n;
-        const float rs = 1.0f / sqrtf(block_sum(centred(mu), red) * inv_n + a.post_eps);
-#pragma unroll
-        for (int i = 0; i < kHold; ++i) {
-          const int c = 4 * (i * kGemvThreads + static_cast<int>(threadIdx.x));
-          if (c < n_out) {
-            const float4 w = *reinterpret_cast<const float4*>(a.post_w + c), b = *reinterpret_cast<const float4*>(a.post_b + c);
-            z[i] = make_float4(fmaf((z[i].x - mu) * rs, w.x, b.x), fmaf((z[i].y - mu) * rs, w.y, b.y),
-                               fmaf((z[i].z - mu) * rs, w.z, b.z), fmaf((z[i].w - mu) * rs, w.w, b.w));
-            *reinterpret_cast<float4*>(xrow + c) = z[i];
-            q += (z[i].x + z[i].y) + (z[i].z + z[i].w);
-          }
-        }
-        if (a.stats_out) {
-          mu2 = block_sum(q, red) * inv_n;
-          rs2 = 1.0f / sqrtf(block_sum(centred(mu2), red) * inv_n + a.post_eps);
-        }
-      } else {
-        float s = 0.f, v = 0.f;
-        for (int i = threadIdx.x; i < n_out; i += kGemvThreads) s += fmaf(a.post_mult, xrow[i], __ldcg(row + i));
-        const float mu = block_sum(s, red) * inv_n;
-        for (int i = threadIdx.x; i < n_out; i += kGemvThreads) {
-          const float z = fmaf(a.post_mult, xrow[i], __ldcg(row + i)) - mu;
-          v = fmaf(z, z, v);
-        }
-        const float rs = 1.0f / sqrtf(block_sum(v, red) * inv_n + a.post_eps);
-        s = v = 0.f;
-        for (int i = threadIdx.x; i < n_out; i += kGemvThreads) {
-          const float x = fmaf((fmaf(a.post_mult, xrow[i], __ldcg(row + i)) - mu) * rs, a.post_w[i], a.post_b[i]);
-          xrow[i] = x;                                  // each thread re-reads only what it wrote
-          s += x;
-        }
-        if (a.stats_out) {
-          mu2 = block_sum(s, red) * inv_n;
-          for (int i = threadIdx.x; i < n_out; i += kGemvThreads) v = fmaf(xrow[i] - mu2, xrow[i] - mu2, v);
-          rs2 = 1.0f / sqrtf(block_sum(v, red) * inv_n + a.post_eps);
-        }
+      for (int i = 0; i < kHold; ++i) {
+        const int c = column(i);
+        const bool in = c < n_out;
+        y[i] = in ? __ldcg(reinterpret_cast<const float4*>(row + c)) : zero;
+        z[i] = in ? *reinterpret_cast<const float4*>(xrow + c) : zero;
+        w[i] = in ? *reinterpret_cast<const float4*>(a.post_w + c) : zero;
+        if (in && a.post_b) prefetch_l2(a.post_b + c);
+        if (in && a.post_next_w) prefetch_l2(a.post_next_w + c);
+        if (in && a.post_next_b) prefetch_l2(a.post_next_b + c);
       }
-      if (threadIdx.x == 0 && a.stats_out) {
-        a.stats_out[2 * (m0 + bt)] = mu2;
-        a.stats_out[2 * (m0 + bt) + 1] = rs2;
-      }
-    }
-    return;
-  }
-  if (a.post_w) {
-    // norm after the sublayer, residual add, and the root mean square of the new residual row
-    const int n_out = a.n_valid > 0 ? a.n_valid : a.N;
-    // rows of up to kHold * 4 * 256 numbers live in registers: one round of loads for y and x together
-    constexpr int kHold = 4;
-    const int ldo = a.ld_out > 0 ? a.ld_out : a.N;
-    const bool held = ((n_out | ldo | a.post_ldx) & 3) == 0 && n_out <= kHold * 4 * kGemvThreads;
-    for (int bt = 0; bt < nb; ++bt) {
-      const float* row = a.out + static_cast<size_t>(m0 + bt) * ldo;
-      float* xrow = a.post_x + static_cast<size_t>(m0 + bt) * a.post_ldx;
-      float s = 0.f, q = 0.f;
-      if (held) {
-        float4 y4[kHold], x4[kHold];
+      auto total = [&]() {
+        float s = 0.f;
 #pragma unroll
-        for (int i = 0; i < kHold; ++i) {
-          const int c = 4 * (i * kGemvThreads + static_cast<int>(threadIdx.x));
-          const bool in = c < n_out;
-          y4[i] = in ? __ldcg(reinterpret_cast<const float4*>(row + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-          if (in) prefetch_l2(a.post_w + c);
-          x4[i] = in ? *reinterpret_cast<const float4*>(xrow + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        for (int i = 0; i < kHold; ++i) s += (z[i].x + z[i].y) + (z[i].z + z[i].w);
+        return block_sum(s, red);
+      };
+      auto centred = [&](float mu) {                    // sum of squared deviations
+        float v = 0.f;
 #pragma unroll
         for (int i = 0; i < kHold; ++i)
-          s += y4[i].x * y4[i].x + y4[i].y * y4[i].y + y4[i].z * y4[i].z + y4[i].w * y4[i].w;
+          if (column(i) < n_out) {
+            const float dx = z[i].x - mu, dy = z[i].y - mu, dz = z[i].z - mu, dw = z[i].w - mu;
+            v += (dx * dx + dy * dy) + (dz * dz + dw * dw);
+          }
+        return block_sum(v, red);
+      };
+      float mu2 = 0.f, rs2;
+      if (a.post_b) {
+        // layer norm of the residual sum
+#pragma unroll
+        for (int i = 0; i < kHold; ++i)
+          z[i] = make_float4(fmaf(a.post_mult, z[i].x, y[i].x), fmaf(a.post_mult, z[i].y, y[i].y), fmaf(a.post_mult, z[i].z, y[i].z), fmaf(a.post_mult, z[i].w, y[i].w));
+        const float mu = total() * inv_n;
+        const float rs = 1.0f / sqrtf(centred(mu) * inv_n + a.post_eps);
+#pragma unroll
+        for (int i = 0; i < kHold; ++i) {
+          const int c = column(i);
+          if (c < n_out) {
+            const float4 b = *reinterpret_cast<const float4*>(a.post_b + c);
+            z[i] = make_float4(fmaf((z[i].x - mu) * rs, w[i].x, b.x), fmaf((z[i].y - mu) * rs, w[i].y, b.y),
+                               fmaf((z[i].z - mu) * rs, w[i].z, b.z), fmaf((z[i].w - mu) * rs, w[i].w, b.w));
+            *reinterpret_cast<float4*>(xrow + c) = z[i];
+          } else {
+            z[i] = zero;
+          }
+        }
+        if (!a.post_next_w) continue;
+        mu2 = total() * inv_n;
+        rs2 = 1.0f / sqrtf(centred(mu2) * inv_n + a.post_eps);
+      } else {
+        // norm after the sublayer, residual add
+        float s = 0.f, q = 0.f;
+#pragma unroll
+        for (int i = 0; i < kHold; ++i) s += y[i].x * y[i].x + y[i].y * y[i].y + y[i].z * y[i].z + y[i].w * y[i].w;
         const float rs = a.post_mult / sqrtf(block_sum(s, red) / static_cast<float>(n_out) + a.post_eps);
 #pragma unroll
         for (int i = 0; i < kHold; ++i) {
-          const int c = 4 * (i * kGemvThreads + static_cast<int>(threadIdx.x));
-          float4 v = x4[i];
-          if (c < n_out) {
-            const float4 w = *reinterpret_cast<const float4*>(a.post_w + c);
-            v.x = fmaf(y4[i].x * rs, w.x, v.x);
-            v.y = fmaf(y4[i].y * rs, w.y, v.y);
-            v.z = fmaf(y4[i].z * rs, w.z, v.z);
-            v.w = fmaf(y4[i].w * rs, w.w, v.w);
-            *reinterpret_cast<float4*>(xrow + c) = v;
-          }
-          q += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+          z[i] = make_float4(fmaf(y[i].x * rs, w[i].x, z[i].x), fmaf(y[i].y * rs, w[i].y, z[i].y), fmaf(y[i].z * rs, w[i].z, z[i].z), fmaf(y[i].w * rs, w[i].w, z[i].w));
+          if (column(i) < n_out) *reinterpret_cast<float4*>(xrow + column(i)) = z[i];
+          q += z[i].x * z[i].x + z[i].y * z[i].y + z[i].z * z[i].z + z[i].w * z[i].w;
         }
-      } else {
-#pragma unroll 8
-        for (int i = threadIdx.x; i < n_out; i += kGemvThreads) {
-          const float y = __ldcg(row + i);
-          s = fmaf(y, y, s);
-        }
-        const float rs = a.post_mult / sqrtf(block_sum(s, red) / static_cast<float>(n_out) + a.post_eps);
-#pragma unroll 8
-        for (int i = threadIdx.x; i < n_out; i += kGemvThreads) {
-          const float v = fmaf(__ldcg(row + i) * rs, a.post_w[i], xrow[i]);
-          xrow[i] = v;
-          q = fmaf(v, v, q);
-        }
+        if (!a.post_next_w) continue;
+        rs2 = 1.0f / sqrtf(block_sum(q, red) / static_cast<float>(n_out) + a.post_eps);
       }
-      const float ms = block_sum(q, red) / static_cast<float>(n_out);
-      if (threadIdx.x == 0) {
-        a.stats_out[2 * (m0 + bt)] = 0.f;
-        a.stats_out[2 * (m0 + bt) + 1] = 1.0f / sqrtf(ms + a.post_eps);
+#pragma unroll
+      for (int i = 0; i < kHold; ++i) {
+        const int c = column(i);
+        if (c >= n_out) continue;
+        const float4 nw = *reinterpret_cast<const float4*>(a.post_next_w + c), o = a.post_next_b ? *reinterpret_cast<const float4*>(a.post_next_b + c) : zero;
+        *reinterpret_cast<float4*>(xn + c) = make_float4(fmaf(nw.x * rs2, z[i].x - mu2, o.x), fmaf(nw.y * rs2, z[i].y - mu2, o.y),
+                                                         fmaf(nw.z * rs2, z[i].z - mu2, o.z), fmaf(nw.w * rs2, z[i].w - mu2, o.w));
       }
+      continue;
     }
-    return;
+    // each thread re-reads only what it wrote
+    float mu2 = 0.f, rs2;
+    if (a.post_b) {
+      float s = 0.f, v = 0.f;
+      for (int i = threadIdx.x; i < n_out; i += kGemvThreads) s += fmaf(a.post_mult, xrow[i], __ldcg(row + i));
+      const float mu = block_sum(s, red) * inv_n;
+      for (int i = threadIdx.x; i < n_out; i += kGemvThreads) {
+        const float z = fmaf(a.post_mult, xrow[i], __ldcg(row + i)) - mu;
+        v = fmaf(z, z, v);
+      }
+      const float rs = 1.0f / sqrtf(block_sum(v, red) * inv_n + a.post_eps);
+      s = v = 0.f;
+      for (int i = threadIdx.x; i < n_out; i += kGemvThreads) {
+        const float x = fmaf((fmaf(a.post_mult, xrow[i], __ldcg(row + i)) - mu) * rs, a.post_w[i], a.post_b[i]);
+        xrow[i] = x;
+        s += x;
+      }
+      if (!a.post_next_w) continue;
+      mu2 = block_sum(s, red) * inv_n;
+      for (int i = threadIdx.x; i < n_out; i += kGemvThreads) v = fmaf(xrow[i] - mu2, xrow[i] - mu2, v);
+      rs2 = 1.0f / sqrtf(block_sum(v, red) * inv_n + a.post_eps);
+    } else {
+      float s = 0.f, q = 0.f;
+#pragma unroll 8
+      for (int i = threadIdx.x; i < n_out; i += kGemvThreads) {
+        const float y = __ldcg(row + i);
+        s = fmaf(y, y, s);
+      }
+      const float rs = a.post_mult / sqrtf(block_sum(s, red) / static_cast<float>(n_out) + a.post_eps);
+#pragma unroll 8
+      for (int i = threadIdx.x; i < n_out; i += kGemvThreads) {
+        const float v = fmaf(__ldcg(row + i) * rs, a.post_w[i], xrow[i]);
+        xrow[i] = v;
+        q = fmaf(v, v, q);
+      }
+      if (!a.post_next_w) continue;
+      rs2 = 1.0f / sqrtf(block_sum(q, red) / static_cast<float>(n_out) + a.post_eps);
+    }
+    for (int i = threadIdx.x; i < n_out; i += kGemvThreads)
+      xn[i] = fmaf(a.post_next_w[i] * rs2, xrow[i] - mu2, a.post_next_b ? a.post_next_b[i] : 0.f);
   }
 }
 

@@ -2,8 +2,7 @@
 //
 // gemv_kernel keeps 64 bytes per thread in flight and starts with an empty pipe in each of its waves of blocks; a product
 // of 50 to 180 MB is over after 10 to 30 us, so that ramps and last waves cost a third of it.  Here one block per SM owns a
-// run of rows, and each of its 8 warps the same eighth of the columns of all of them: the activations stay in registers
-// (normed once).  A ninth warp streams the rows, one bulk copy each, through a ring of 96 KB, filled from before the wait on
+// run of rows, and each of its 8 warps the same eighth of the columns of all of them: the activations stay in registers.  A ninth warp streams the rows, one bulk copy each, through a ring of 96 KB, filled from before the wait on
 // the predecessor (two such blocks fit an SM, so a kernel's ring fills while its predecessor ends).  Whole rows, because
 // the copy engine takes about 70 ns for a copy of 1 KB: with a ring per warp and 1 KB pieces 184 MB took 87 us.  No
 // block-wide barrier until the rows are done; the 8 partial sums of a row are added in order.
@@ -24,7 +23,6 @@ __device__ __forceinline__ void arrive(uint32_t bar) { asm volatile("mbarrier.ar
 
 template <int NCH, int EPI>
 __global__ void __launch_bounds__(kStreamThreads, 2) gemv_stream_kernel(const GemvArgs a, int ring) {
-  constexpr bool kNorm = EPI == kEpiLogits || EPI == kEpiSwiGLU;
   extern __shared__ __align__(128) unsigned char stream_smem[];
   __shared__ __align__(8) uint64_t bars[2 * kMaxRing];
   __shared__ float red[kGemvWarps];
@@ -75,26 +73,14 @@ __global__ void __launch_bounds__(kStreamThreads, 2) gemv_stream_kernel(const Ge
     const int v0 = warp * per, mine = max(0, min(per, vecs - v0));
     const int src = a.row_select ? a.row_select[0] : 0;
     const float* xp = a.x + static_cast<size_t>(src) * a.ldx + v0 * 8 + lane * 8;
-    const float* sc = a.ln_scale + v0 * 8 + lane * 8;
-    const float* of = a.ln_offset + v0 * 8 + lane * 8;
     float x[NCH][8];
-    float mean = 0.f, rstd = 0.f;
-    if (kNorm) {
-      mean = a.stats[2 * src];
-      rstd = a.stats[2 * src + 1];
-    }
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
       const bool in = c * 32 + lane < mine;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 v = in ? *reinterpret_cast<const float4*>(xp + c * 256 + 4 * h) : zero;
-        if (kNorm && in) {
-          const float4 s4 = *reinterpret_cast<const float4*>(sc + c * 256 + 4 * h), o4 = *reinterpret_cast<const float4*>(of + c * 256 + 4 * h);
-          v = make_float4(fmaf(s4.x * rstd, v.x - mean, o4.x), fmaf(s4.y * rstd, v.y - mean, o4.y), fmaf(s4.z * rstd, v.z - mean, o4.z),
-                          fmaf(s4.w * rstd, v.w - mean, o4.w));
-        }
+        const float4 v = in ? *reinterpret_cast<const float4*>(xp + c * 256 + 4 * h) : zero;
         x[c][4 * h] = v.x; x[c][4 * h + 1] = v.y; x[c][4 * h + 2] = v.z; x[c][4 * h + 3] = v.w;
       }
     }
@@ -165,13 +151,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) gemv_stream_kernel(const Ge
       const float y = fmaxf(val, 0.f);
       a.act2[n] = y * y;
     } else {
-      float y = a.bias ? val + a.bias[n] : val;
-      if (EPI == kEpiLogits) {
-        if (a.softcap > 0.f) y = a.softcap * tanhf(y / a.softcap);
-        a.logits[n] = y;
-      } else {
-        a.out[n] = y;
-      }
+      a.out[n] = EPI == kEpiSoftcap ? a.softcap * tanhf(val / a.softcap) : a.bias ? val + a.bias[n] : val;
     }
   }
   if (EPI == kEpiOut && a.post_w) {
@@ -218,8 +198,8 @@ cudaError_t launch_epi(const GemvArgs& a, cudaStream_t s, bool pdl) {
 // and 53; 12288 x 4096: 23.5 and 20.6), and beyond 12288 the activations no longer fit the registers and the ring holds three
 // rows (4096 x 13824 40 to 66 and 21, 4096 x 16384 66 and 24), so those stay.
 bool gemv_stream_ok(GemvEpilogue epi, const GemvArgs& a) {
-  return a.M == 1 && (epi == kEpiOut || epi == kEpiLogits || epi == kEpiSwiGLU || epi == kEpiRelu2) && a.K >= kMinK && a.K <= kMaxK &&
-         a.N >= 4 * 148 && a.N <= 148 * 2048 && !a.residual && !a.slot_sel && (a.post_w || !a.stats_out) && a.ks_override == 0;
+  return a.M == 1 && (epi == kEpiOut || epi == kEpiSoftcap || epi == kEpiSwiGLU || epi == kEpiRelu2) && a.K >= kMinK && a.K <= kMaxK &&
+         a.N >= 4 * 148 && a.N <= 148 * 2048 && !a.residual && !a.slot_sel && !a.stats_out && a.ks_override == 0;
 }
 
 cudaError_t launch_gemv_stream(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl) {
@@ -228,7 +208,7 @@ cudaError_t launch_gemv_stream(GemvEpilogue epi, const GemvArgs& a, cudaStream_t
     case kEpiOut: return launch_epi<kEpiOut>(a, s, pdl);
     case kEpiSwiGLU: return launch_epi<kEpiSwiGLU>(a, s, pdl);
     case kEpiRelu2: return launch_epi<kEpiRelu2>(a, s, pdl);
-    default: return launch_epi<kEpiLogits>(a, s, pdl);
+    default: return launch_epi<kEpiSoftcap>(a, s, pdl);
   }
 }
 

@@ -46,7 +46,7 @@ enum GemvEpilogue { kEpiInProj = 0, kEpiOut = 1, kEpiLogits = 2,
                     kEpiPlain = 4,        // fp32 and / or bf16 result (tensor-core GEMM only)
                     kEpiSwiGLU = 5,       // weight rows in (gate, up) pairs: silu(gate) * up
                     kEpiRelu2 = 6,        // squared relu
-                    kEpiSoftcap = 7 };    // cap * tanh(result / cap), fp32 (tensor-core GEMM; the GEMV takes GemvArgs.softcap)
+                    kEpiSoftcap = 7 };    // cap * tanh(result / cap), fp32
 
 struct GemvArgs {
   // y[m, n] = sum_k W[n, k] * act(x[m, k]);  W is bf16 [N, K] (K contiguous).
@@ -55,7 +55,7 @@ struct GemvArgs {
   int n0;                      // index of W's first row within the full projection (epilogue indexing)
   const float* x;              // [M, ldx] fp32
   int ldx;
-  // LayerNorm prologue (in-proj and logits): act(x) = scale*rstd*(x-mean)+offset
+  // LayerNorm prologue (in-proj and logits of the GEMV): act(x) = scale*rstd*(x-mean)+offset
   const float* ln_scale;
   const float* ln_offset;
   const float* stats;          // [M, 2] = (mean, rstd)
@@ -85,15 +85,18 @@ struct GemvArgs {
   int n_valid;                 // rows of W past this one are padding, nothing is stored for them (0 = N)
   int ld_out;                  // row stride of `out` (0 = N); SwiGLU: of `act2`
   // out-proj epilogue of layers with a norm after the sublayer: instead of the LayerNorm statistics of `out` the last
-  // block computes post_x += post_mult * RMSNorm(out) * post_w and, into stats_out, (0, 1 / rms) of the new post_x
+  // block computes post_x += post_mult * RMSNorm(out) * post_w and, with post_next_w, post_xn = RMSNorm(post_x) * post_next_w,
+  // what the next projection reads
   const float* post_w;         // [n_valid] or null
   float* post_x;               // [M, post_ldx]
   int post_ldx;
   float post_mult, post_eps;
-  // with post_b: post_x = LayerNorm(post_mult * post_x + out) * post_w + post_b instead, and stats_out, if given, takes
-  // the (mean, 1 / deviation) of the new post_x
+  // with post_b: post_x = LayerNorm(post_mult * post_x + out) * post_w + post_b instead, and, with post_next_w,
+  // post_xn = LayerNorm(post_x) * post_next_w + post_next_b
   const float* post_b;         // [n_valid] or null
-  float softcap;               // logits epilogue: cap * tanh(logit / cap); 0 = none
+  const float *post_next_w, *post_next_b;   // [n_valid] or null
+  float* post_xn;              // [M, post_ldx]
+  float softcap;               // kEpiSoftcap: cap * tanh(result / cap)
 };
 
 cudaError_t launch_gemv(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl);
@@ -101,8 +104,8 @@ cudaError_t launch_gemv(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, boo
 // The same for one row and long weight rows, streamed by one block per SM (mtj_gemv_stream.cu).
 bool gemv_stream_ok(GemvEpilogue epi, const GemvArgs& a);
 cudaError_t launch_gemv_stream(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl);
-// The same product for 2 rows and more, fp32 activations and sums (mtj_gemm_rows.cu): every epilogue but the
-// in-projection's, no residual, no norm behind it.  planes and counters (zero between launches) are scratch of
+// The same product for 2 rows and more, fp32 activations and sums (mtj_gemm_rows.cu): every epilogue but those with a norm in
+// front, no residual, no norm behind it.  planes and counters (zero between launches) are scratch of
 // kGemmRowsPlaneFloats and kGemmRowsCounters elements; one launch at a time may use them.
 // 2 to 4 rows of width 2048, us: 2048 x 4096 weights 8.4 (and 2.3 for the norm behind them), 14.3 by the GEMV.
 constexpr int64_t kGemmRowsPlaneFloats = 4 * 148 * 64 * 16;

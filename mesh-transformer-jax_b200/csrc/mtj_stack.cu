@@ -173,7 +173,6 @@ void LayerStack::carve_weights(Carver& c) {
   embed_ = c.take<__nv_bfloat16>(static_cast<int64_t>(V_) * d_);
   final_norm_ = c.take<float>(ld_);
   if (post_ln_) final_norm_b_ = c.take<float>(ld_);
-  zeros_ = c.take<float>(ld_);
   head_.take(c);
   if (loop_times_ > 0) loop_in_.take(c);
   tables_.clear();
@@ -274,7 +273,7 @@ void LayerStack::carve_workspace(Carver& c) {
   ld_act_ = static_cast<int>(act);
   lin_rows_ = static_cast<int>(R + hist);
   x_ = c.take<float>(R * ld_);
-  stats_ = c.take<float>(R * 2);
+  xn_ = c.take<float>(R * ld_);
   y_ = c.take<float>(R * ld_);
   p1_ = c.take<float>(R * p1);
   act_ = c.take<float>(R * act);
@@ -680,9 +679,8 @@ int32_t LayerStack::gemm_planes(mtj_handle* h, const Linear& l, const __nv_bfloa
   return MTJ_OK;
 }
 
-int32_t LayerStack::gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const float* x, int ldx, int M, const float* norm,
-                         float* out, int ld_out, const Post* post, bool pdl, cudaStream_t s, const int32_t* select,
-                         const float* stats) {
+int32_t LayerStack::gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const float* x, int ldx, int M, float* out, int ld_out,
+                         const Post* post, bool pdl, cudaStream_t s, const int32_t* select) {
   GemvArgs a = {};
   a.W = l.w;
   a.N = up4(l.N);
@@ -691,16 +689,13 @@ int32_t LayerStack::gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
   a.M = M;
   a.x = x;
   a.ldx = ldx;
-  a.ln_scale = norm;
-  a.ln_offset = norm == final_norm_ && final_norm_b_ ? final_norm_b_ : zeros_;
-  a.stats = stats ? stats : stats_;
   a.rows = {0, 1, 0, nullptr};
   a.row_select = select;
   a.dev_err = h->dev_err;
   a.ld_out = ld_out;
   if (epi == kEpiSwiGLU || epi == kEpiRelu2) a.act2 = out;
-  else if (epi == kEpiLogits) { a.logits = out; a.ld_logits = ld_out; a.softcap = l.w == head_.w ? softcap_ : 0.f; }
   else a.out = out;
+  a.softcap = softcap_;
   if (M >= kGemmRowsMin) {
     MTJ_CUDA(launch_gemm_rows(epi, a, rows_planes_, rows_counters_, s, pdl));
     h->launches++;
@@ -718,7 +713,9 @@ int32_t LayerStack::gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
       r.b = post->b;
       r.alpha = mult_;
       r.eps = eps_;
-      r.stats = post->stats ? stats_ : nullptr;
+      r.w_next = post->next_w;
+      r.b_next = post->next_b;
+      r.xn_f32 = xn_;
       MTJ_CUDA(launch_residual_layernorm(r, s, pdl));
     } else {
       ResidualNormArgs r = {};
@@ -731,7 +728,8 @@ int32_t LayerStack::gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
       r.w_post = post->w;
       r.mult = mult_;
       r.eps = eps_;
-      r.stats = stats_;
+      r.w_next = post->next_w;
+      r.xn_f32 = post->next_w ? xn_ : nullptr;
       MTJ_CUDA(launch_residual_norm(r, s, pdl));
     }
     h->launches++;
@@ -744,7 +742,9 @@ int32_t LayerStack::gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
     a.post_ldx = ld_;
     a.post_mult = mult_;
     a.post_eps = eps_;
-    a.stats_out = post->stats ? stats_ : nullptr;
+    a.post_next_w = post->next_w;
+    a.post_next_b = post->next_b;
+    a.post_xn = xn_;
     a.counters = counters_;
   }
   if (gemv_stream_ok(epi, a)) MTJ_CUDA(launch_gemv_stream(epi, a, s, pdl));
@@ -766,9 +766,8 @@ namespace {
 bool chained(const mtj_handle* h, bool tc, bool decode) { return h->use_pdl && (decode || !tc); }
 }  // namespace
 
-int32_t LayerStack::project_in(mtj_handle* h, const Linear& l, const float* norm, int M, float* out, int ld_out, bool pdl, cudaStream_t s) {
-  return post_ln_ ? gemv(h, kEpiOut, l, x_, ld_, M, nullptr, out, ld_out, nullptr, pdl, s)
-                  : gemv(h, kEpiLogits, l, x_, ld_, M, norm, out, ld_out, nullptr, pdl, s);
+int32_t LayerStack::project_in(mtj_handle* h, const Linear& l, int M, float* out, int ld_out, bool pdl, cudaStream_t s) {
+  return gemv(h, kEpiOut, l, post_ln_ ? x_ : xn_, ld_, M, out, ld_out, nullptr, pdl, s);
 }
 
 int32_t LayerStack::mamba(mtj_handle* h, const Run& r, int M, const RowMap& rows, bool tc, bool decode, const Post& post, cudaStream_t s) {
@@ -813,7 +812,7 @@ int32_t LayerStack::mamba(mtj_handle* h, const Run& r, int M, const RowMap& rows
     a.xz = p1_;
     a.u = u_;
     a.out = act_;
-    MTJ_DO(project_in(h, l.in, l.norm1, M, p1_, a.ld_xz, pdl, s));
+    MTJ_DO(project_in(h, l.in, M, p1_, a.ld_xz, pdl, s));
   }
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_ATTN, s);
@@ -826,9 +825,9 @@ int32_t LayerStack::mamba(mtj_handle* h, const Run& r, int M, const RowMap& rows
     MTJ_DO(gemm(h, kEpiPlain, l.dt, dtr_bf_, M, dt_raw_, l.ld_u, nullptr, 0, decode, s));
     a.dt_raw = dt_raw_;
   } else {
-    MTJ_DO(gemv(h, kEpiOut, l.x, u_, l.ld_u, M, nullptr, xp_, l.ld_xp, nullptr, pdl, s));
+    MTJ_DO(gemv(h, kEpiOut, l.x, u_, l.ld_u, M, xp_, l.ld_xp, nullptr, pdl, s));
     if (rows.Tc > 1) {
-      MTJ_DO(gemv(h, kEpiOut, l.dt, xp_, l.ld_xp, M, nullptr, dt_raw_, l.ld_u, nullptr, pdl, s));
+      MTJ_DO(gemv(h, kEpiOut, l.dt, xp_, l.ld_xp, M, dt_raw_, l.ld_u, nullptr, pdl, s));
       a.dt_raw = dt_raw_;
     }
   }
@@ -838,7 +837,7 @@ int32_t LayerStack::mamba(mtj_handle* h, const Run& r, int M, const RowMap& rows
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
   if (tc) MTJ_DO(gemm_out(h, l.out, M, decode, s));
-  else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, nullptr, y_, ld_, &post, pdl, s));
+  else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, y_, ld_, &post, pdl, s));
   h->prof_end(s);
   return MTJ_OK;
 }
@@ -873,7 +872,7 @@ int32_t LayerStack::latent(mtj_handle* h, const Run& r, int M, const RowMap& row
   a.ld_out = l.out.ld;
   h->prof_begin(MTJ_FAMILY_INPROJ, s);
   if (tc) MTJ_DO(gemm(h, kEpiPlain, l.in, xn_bf_, M, p1_, a.ld_p1, nullptr, 0, decode, s));
-  else MTJ_DO(project_in(h, l.in, l.norm1, M, p1_, a.ld_p1, pdl, s));
+  else MTJ_DO(project_in(h, l.in, M, p1_, a.ld_p1, pdl, s));
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_ATTN, s);
   if (tc && !decode && l.up.w) {
@@ -928,7 +927,7 @@ int32_t LayerStack::latent(mtj_handle* h, const Run& r, int M, const RowMap& row
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
   if (tc) MTJ_DO(gemm_out(h, l.out, M, decode, s));
-  else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, nullptr, y_, ld_, &post, pdl, s));
+  else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, y_, ld_, &post, pdl, s));
   h->prof_end(s);
   return MTJ_OK;
 }
@@ -965,7 +964,7 @@ int32_t LayerStack::grouped(mtj_handle* h, const Run& r, int M, const RowMap& ro
   a.ld_out = l.out.ld;
   h->prof_begin(MTJ_FAMILY_INPROJ, s);
   if (tc) MTJ_DO(gemm(h, kEpiPlain, l.in, xn_bf_, M, p1_, a.ld_p1, nullptr, 0, decode, s));
-  else MTJ_DO(project_in(h, l.in, l.norm1, M, p1_, a.ld_p1, pdl, s));
+  else MTJ_DO(project_in(h, l.in, M, p1_, a.ld_p1, pdl, s));
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_ATTN, s);
   MTJ_CUDA(launch_grouped_prep(a, s, pdl));
@@ -1011,7 +1010,7 @@ int32_t LayerStack::grouped(mtj_handle* h, const Run& r, int M, const RowMap& ro
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
   if (tc) MTJ_DO(gemm_out(h, l.out, M, decode, s));
-  else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, nullptr, y_, ld_, &post, pdl, s));
+  else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, y_, ld_, &post, pdl, s));
   h->prof_end(s);
   return MTJ_OK;
 }
@@ -1026,7 +1025,7 @@ int32_t LayerStack::matrix(mtj_handle* h, const Run& r, int M, const RowMap& row
   const int ld_aux = tc ? ld_aux_ : ld_p;
   h->prof_begin(MTJ_FAMILY_INPROJ, s);
   if (tc) MTJ_DO(gemm(h, kEpiPlain, l.in, xn_bf_, M, aux_, ld_aux_, xz_bf_, ld_p, decode, s, 0, 0, l.aux0));
-  else MTJ_DO(project_in(h, l.in, l.norm1, M, p1_, ld_p, pdl, s));
+  else MTJ_DO(project_in(h, l.in, M, p1_, ld_p, pdl, s));
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_ATTN, s);
   SsmArgs c = {};
@@ -1053,8 +1052,8 @@ int32_t LayerStack::matrix(mtj_handle* h, const Run& r, int M, const RowMap& row
       MTJ_DO(gemm(h, kEpiPlain, l.dt, xz_bf_ + l.a0, M, dt_raw_, up8(l.dt.N), nullptr, 0, decode, s, 0, ld_p));
       MTJ_DO(gemm(h, kEpiPlain, l.gate2, xz_bf_ + l.g0, M, nullptr, 0, gate_bf_, up8(inner), decode, s, 0, ld_p));
     } else {
-      MTJ_DO(gemv(h, kEpiOut, l.dt, p1_ + l.a0, ld_p, M, nullptr, dt_raw_, up8(l.dt.N), nullptr, pdl, s));
-      MTJ_DO(gemv(h, kEpiOut, l.gate2, p1_ + l.g0, ld_p, M, nullptr, gate_raw_, up8(inner), nullptr, pdl, s));
+      MTJ_DO(gemv(h, kEpiOut, l.dt, p1_ + l.a0, ld_p, M, dt_raw_, up8(l.dt.N), nullptr, pdl, s));
+      MTJ_DO(gemv(h, kEpiOut, l.gate2, p1_ + l.g0, ld_p, M, gate_raw_, up8(inner), nullptr, pdl, s));
     }
   }
   MatrixStateArgs a = {};
@@ -1112,7 +1111,7 @@ int32_t LayerStack::matrix(mtj_handle* h, const Run& r, int M, const RowMap& row
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
   if (tc) MTJ_DO(gemm_out(h, l.out, M, decode, s));
-  else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, nullptr, y_, ld_, &post, pdl, s));
+  else MTJ_DO(gemv(h, kEpiOut, l.out, act_, l.out.ld, M, y_, ld_, &post, pdl, s));
   h->prof_end(s);
   return MTJ_OK;
 }
@@ -1149,7 +1148,7 @@ int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, cons
     return {layers_[runs_[i].layer].norm1, runs_[i].first};
   };
   // residual add (y != null) and what the next sublayer reads; on the fp32 path the projections have done the add and
-  // the statistics themselves
+  // the norm themselves
   auto settle = [&](const float* y, const Post& post, const Next& n) -> int32_t {
     if (post_ln_) {
       ResidualLayerNormArgs a = {};
@@ -1167,7 +1166,6 @@ int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, cons
       if (n.last) {
         a.w_next = final_norm_;
         a.b_next = final_norm_b_;
-        a.stats = stats_;
       }
       MTJ_CUDA(launch_residual_layernorm(a, s, pdl));
       h->launches++;
@@ -1183,7 +1181,6 @@ int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, cons
     a.w_post = post.w;
     a.mult = mult_;
     a.eps = eps_;
-    a.stats = stats_;
     if (n.pass) {
       a.x0 = x0_;
       if (tc) a.cat_bf16 = cat_bf_;
@@ -1191,6 +1188,9 @@ int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, cons
     } else if (tc) {
       a.w_next = n.norm;
       a.xn = xn_bf_;
+    } else {
+      a.w_next = n.norm;
+      a.xn_f32 = xn_;
     }
     MTJ_CUDA(launch_residual_norm(a, s, pdl));
     h->launches++;
@@ -1206,13 +1206,17 @@ int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, cons
     const Layer& l = layers_[r.layer];
     if (r.first) {
       if (tc) MTJ_DO(gemm(h, kEpiPlain, loop_in_, cat_bf_, M, x_, ld_, nullptr, 0, decode, s));
-      else MTJ_DO(gemv(h, kEpiOut, loop_in_, cat_, 2 * ld_, M, nullptr, x_, ld_, nullptr, pdl, s));
+      else MTJ_DO(gemv(h, kEpiOut, loop_in_, cat_, 2 * ld_, M, x_, ld_, nullptr, pdl, s));
       MTJ_DO(settle(nullptr, Post{}, {l.norm1, false}));
     }
     const Next after_layer = next_run(i + 1), after_mixer = l.d.ff > 0 ? Next{l.norm2, false} : after_layer;
-    // statistics of the new residual row: the next prologue's; behind a layer norm only the final norm has one
-    const Post post1 = post_ln_ ? Post{l.norm1, l.norm1_b, after_mixer.last} : Post{l.norm1b, nullptr, true};
-    const Post post2 = post_ln_ ? Post{l.norm2, l.norm2_b, after_layer.last} : Post{l.norm2b, nullptr, true};
+    // the norm that the next projection reads the new residual row behind; behind a layer norm only the final one
+    auto post_of = [&](const float* w, const float* b, const Next& n) {
+      const bool normed = post_ln_ ? n.last : !n.pass;
+      return Post{w, b, normed ? n.norm : nullptr, normed && n.last ? final_norm_b_ : nullptr};
+    };
+    const Post post1 = post_ln_ ? post_of(l.norm1, l.norm1_b, after_mixer) : post_of(l.norm1b, nullptr, after_mixer);
+    const Post post2 = post_ln_ ? post_of(l.norm2, l.norm2_b, after_layer) : post_of(l.norm2b, nullptr, after_layer);
     switch (l.d.mixer) {
       case MTJ_MIXER_LATENT_ATTENTION: MTJ_DO(latent(h, r, M, rows, hist, tc, decode, post1, s)); break;
       case MTJ_MIXER_GROUPED_ATTENTION: MTJ_DO(grouped(h, r, M, rows, tc, decode, post1, s)); break;
@@ -1224,11 +1228,11 @@ int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, cons
       const GemvEpilogue act = l.d.ff_kind == MTJ_FF_SWIGLU ? kEpiSwiGLU : kEpiRelu2;
       h->prof_begin(MTJ_FAMILY_FFIN, s);
       if (tc) MTJ_DO(gemm(h, act, l.gate_up, xn_bf_, M, nullptr, 0, act_bf_, l.down.ld, decode, s));
-      else MTJ_DO(gemv(h, act, l.gate_up, x_, ld_, M, post_ln_ ? nullptr : l.norm2, act_, l.down.ld, nullptr, pdl, s));
+      else MTJ_DO(gemv(h, act, l.gate_up, post_ln_ ? x_ : xn_, ld_, M, act_, l.down.ld, nullptr, pdl, s));
       h->prof_end(s);
       h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
       if (tc) MTJ_DO(gemm_out(h, l.down, M, decode, s));
-      else MTJ_DO(gemv(h, kEpiOut, l.down, act_, l.down.ld, M, nullptr, y_, ld_, &post2, pdl, s));
+      else MTJ_DO(gemv(h, kEpiOut, l.down, act_, l.down.ld, M, y_, ld_, &post2, pdl, s));
       h->prof_end(s);
       MTJ_DO(after(post2, after_layer));
     }
@@ -1240,15 +1244,46 @@ int32_t LayerStack::logits(mtj_handle* h, int row0, int n, float* out, bool deco
   h->prof_begin(MTJ_FAMILY_LOGITS, s);
   if (last_tc_) MTJ_DO(gemm(h, softcap_ > 0.f ? kEpiSoftcap : kEpiPlain, head_, xn_bf_, n, out, V_, nullptr, 0, decode, s, row0));
   else
-    MTJ_DO(gemv(h, kEpiLogits, head_, x_ + static_cast<size_t>(row0) * ld_, ld_, n, final_norm_, out, V_, nullptr,
-                decode && h->use_pdl, s, nullptr, stats_ + 2 * static_cast<size_t>(row0)));
+    MTJ_DO(gemv(h, softcap_ > 0.f ? kEpiSoftcap : kEpiOut, head_, xn_ + static_cast<size_t>(row0) * ld_, ld_, n, out, V_, nullptr,
+                decode && h->use_pdl, s));
   h->prof_end(s);
   return MTJ_OK;
 }
 
 int32_t LayerStack::logits_select(mtj_handle* h, const int32_t* rows_dev, int n, float* out, cudaStream_t s) {
-  if (!last_tc_ || n <= kSelectGemvRows)
-    return gemv(h, kEpiLogits, head_, x_, ld_, n, final_norm_, out, V_, nullptr, false, s, rows_dev);
+  const GemvEpilogue epi = softcap_ > 0.f ? kEpiSoftcap : kEpiOut;
+  if (!last_tc_) return gemv(h, epi, head_, xn_, ld_, n, out, V_, nullptr, false, s, rows_dev);
+  if (n <= kSelectGemvRows) {
+    // a few rows of a pass on the tensor cores: in fp32 from the residual stream
+    if (post_ln_) {
+      ResidualLayerNormArgs a = {};
+      a.x = x_;
+      a.M = n;
+      a.d = d_;
+      a.ld = ld_;
+      a.planes = 1;
+      a.eps = eps_;
+      a.w_next = final_norm_;
+      a.b_next = final_norm_b_;
+      a.xn_f32 = xn_;
+      a.select = rows_dev;
+      MTJ_CUDA(launch_residual_layernorm(a, s, false));
+    } else {
+      ResidualNormArgs a = {};
+      a.x = x_;
+      a.M = n;
+      a.d = d_;
+      a.ld = ld_;
+      a.planes = 1;
+      a.eps = eps_;
+      a.w_next = final_norm_;
+      a.xn_f32 = xn_;
+      a.select = rows_dev;
+      MTJ_CUDA(launch_residual_norm(a, s, false));
+    }
+    h->launches++;
+    return gemv(h, epi, head_, xn_, ld_, n, out, V_, nullptr, h->use_pdl, s);
+  }
   MTJ_CUDA(launch_gather_rows_bf16(xn_bf_, ld_, rows_dev, n, sel_bf_, s));
   h->launches++;
   return gemm(h, softcap_ > 0.f ? kEpiSoftcap : kEpiPlain, head_, sel_bf_, n, out, V_, nullptr, 0, false, s);

@@ -94,8 +94,8 @@ class LayerStack {
   };
   // what follows a sublayer's projection on the few-row path
   struct Post {
-    const float *w, *b;
-    bool stats;
+    const float *w, *b;                // the norm of the sublayer's output or of the residual sum
+    const float *next_w, *next_b;      // the norm before the next projection, or null
   };
   enum { kRows, kF32, kNegExp, kTransposeF32 };
 
@@ -109,11 +109,10 @@ class LayerStack {
   // a sublayer's output projection: into y_, or cut along K into planes that the residual kernel adds (y_from_, y_count_)
   int32_t gemm_out(mtj_handle* h, const Linear& l, int M, bool decode, cudaStream_t s);
   int32_t gemm_planes(mtj_handle* h, const Linear& l, const __nv_bfloat16* x, int M, int* planes, bool decode, cudaStream_t s);
-  int32_t gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const float* x, int ldx, int M, const float* norm, float* out,
-               int ld_out, const Post* post, bool pdl, cudaStream_t s, const int32_t* select = nullptr,
-               const float* stats = nullptr);
+  int32_t gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const float* x, int ldx, int M, float* out, int ld_out,
+               const Post* post, bool pdl, cudaStream_t s, const int32_t* select = nullptr);
   // a sublayer's input projection: of the normed residual stream, or of the stream itself
-  int32_t project_in(mtj_handle* h, const Linear& l, const float* norm, int M, float* out, int ld_out, bool pdl, cudaStream_t s);
+  int32_t project_in(mtj_handle* h, const Linear& l, int M, float* out, int ld_out, bool pdl, cudaStream_t s);
   int32_t grouped(mtj_handle* h, const Run& r, int M, const RowMap& rows, bool tc, bool decode, const Post& post, cudaStream_t s);
   int32_t matrix(mtj_handle* h, const Run& r, int M, const RowMap& rows, bool tc, bool decode, const Post& post, cudaStream_t s);
   int32_t mamba(mtj_handle* h, const Run& r, int M, const RowMap& rows, bool tc, bool decode, const Post& post, cudaStream_t s);
@@ -131,7 +130,7 @@ class LayerStack {
   std::vector<Run> runs_;
   Linear loop_in_, head_;
   __nv_bfloat16* embed_ = nullptr;
-  float *final_norm_ = nullptr, *final_norm_b_ = nullptr, *zeros_ = nullptr;
+  float *final_norm_ = nullptr, *final_norm_b_ = nullptr;
   std::map<std::pair<double, int>, float2*> tables_;
   std::map<std::string, Leaf> leaf_map_;
   int64_t leaf_count_ = 0;
@@ -145,7 +144,7 @@ class LayerStack {
   uint32_t* rows_counters_ = nullptr;
   int y_count_ = 1;
   int64_t y_planes_elems_ = 0;
-  float *x_ = nullptr, *x0_ = nullptr, *stats_ = nullptr, *cat_ = nullptr, *y_ = nullptr, *y_planes_ = nullptr, *y_from_ = nullptr, *p1_ = nullptr, *u_ = nullptr, *xp_ = nullptr,
+  float *x_ = nullptr, *x0_ = nullptr, *xn_ = nullptr, *cat_ = nullptr, *y_ = nullptr, *y_planes_ = nullptr, *y_from_ = nullptr, *p1_ = nullptr, *u_ = nullptr, *xp_ = nullptr,
         *dt_raw_ = nullptr, *gate_raw_ = nullptr, *aux_ = nullptr, *mix_ = nullptr, *q_f32_ = nullptr, *act_ = nullptr, *xp_planes_ = nullptr, *q_abs_ = nullptr, *part_o_ = nullptr, *part_ml_ = nullptr;
   __nv_bfloat16 *xn_bf_ = nullptr, *cat_bf_ = nullptr, *xz_bf_ = nullptr, *u_bf_ = nullptr, *dtr_bf_ = nullptr, *act_bf_ = nullptr,
                 *sel_bf_ = nullptr, *q_pack_ = nullptr, *c_lin_ = nullptr, *kr_lin_ = nullptr, *kv_lin_ = nullptr, *gate_bf_ = nullptr;

@@ -74,11 +74,11 @@ __global__ void __launch_bounds__(kRegThreads) residual_norm_reg_kernel(const Re
   const size_t m = blockIdx.x;
   float4 wp[HOLD], wn[HOLD], x[HOLD];
   load_row<HOLD>(a.y ? a.w_post : nullptr, n4, wp);          // weights do not depend on the predecessor
-  load_row<HOLD>(a.xn ? a.w_next : nullptr, n4, wn);
+  load_row<HOLD>(a.xn || a.xn_f32 ? a.w_next : nullptr, n4, wn);
   pdl_wait();
   pdl_launch_dependents();
-  float4* xrow = reinterpret_cast<float4*>(a.x + m * a.ld);
-  load_row<HOLD>(a.x + m * a.ld, n4, x);
+  float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
+  load_row<HOLD>(reinterpret_cast<const float*>(xrow), n4, x);
   float ss = 0.f;
   if (a.y) {
     float4 y[HOLD];
@@ -98,15 +98,12 @@ __global__ void __launch_bounds__(kRegThreads) residual_norm_reg_kernel(const Re
 #pragma unroll
   for (int i = 0; i < HOLD; ++i) ss += dot4(x[i]);
   const float rs = 1.0f / sqrtf(rn_block_sum(ss, red) / static_cast<float>(a.d) + a.eps);
-  if (a.stats && threadIdx.x == 0) {
-    a.stats[2 * m] = 0.f;
-    a.stats[2 * m + 1] = rs;
-  }
 #pragma unroll
   for (int i = 0; i < HOLD; ++i) {
     const int c = i * kRegThreads + threadIdx.x;
     if (c >= n4) continue;
     const float4 v = x[i], w = wn[i];
+    if (a.xn_f32) reinterpret_cast<float4*>(a.xn_f32 + m * a.ld)[c] = keep(make_float4(w.x * rs * v.x, w.y * rs * v.y, w.z * rs * v.z, w.w * rs * v.w), a.d - 4 * c);
     if (a.xn) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(keep(make_float4(v.x * rs * w.x, v.y * rs * w.y, v.z * rs * w.z, v.w * rs * w.w), a.d - 4 * c));
     if (a.cat_f32 || a.cat_bf16) {
       const float4 e = reinterpret_cast<const float4*>(a.x0 + m * a.ld)[c];
@@ -135,7 +132,7 @@ __global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(con
   load_row<HOLD>(a.y ? a.b : nullptr, n4, b);
   pdl_wait();
   pdl_launch_dependents();
-  float4* xrow = reinterpret_cast<float4*>(a.x + m * a.ld);
+  float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
   auto norm = [&](float* mu, float* rs) {
     float s = 0.f, q = 0.f;
 #pragma unroll
@@ -152,8 +149,13 @@ __global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(con
     return keep(make_float4(fmaf((z.x - mu) * rs, w4.x, b4.x), fmaf((z.y - mu) * rs, w4.y, b4.y), fmaf((z.z - mu) * rs, w4.z, b4.z),
                             fmaf((z.w - mu) * rs, w4.w, b4.w)), a.d - 4 * c);
   };
+  // the products of the norm in the order of the fp32 path
+  auto rescaled = [&](int c, const float4& z, float mu, float rs, const float4& w4, const float4& b4) {
+    return keep(make_float4(fmaf(w4.x * rs, z.x - mu, b4.x), fmaf(w4.y * rs, z.y - mu, b4.y), fmaf(w4.z * rs, z.z - mu, b4.z),
+                            fmaf(w4.w * rs, z.w - mu, b4.w)), a.d - 4 * c);
+  };
   float mu, rs;
-  load_row<HOLD>(a.x + m * a.ld, n4, x);
+  load_row<HOLD>(reinterpret_cast<const float*>(xrow), n4, x);
   if (a.y) {
     float4 y[HOLD];
     load_planes<HOLD>(a.y, a.planes, m, a.M, a.ld, n4, y);
@@ -175,20 +177,16 @@ __global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(con
       if (c < n4) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(x[i]);
     }
   }
-  if (!a.w_next && !a.stats) return;
+  if (!a.w_next) return;
   norm(&mu, &rs);
-  if (a.stats && threadIdx.x == 0) {
-    a.stats[2 * m] = mu;
-    a.stats[2 * m + 1] = rs;
-  }
-  if (a.xn && a.w_next) {
-    load_row<HOLD>(a.w_next, n4, w);
-    load_row<HOLD>(a.b_next, n4, b);
+  load_row<HOLD>(a.w_next, n4, w);
+  load_row<HOLD>(a.b_next, n4, b);
 #pragma unroll
-    for (int i = 0; i < HOLD; ++i) {
-      const int c = i * kRegThreads + threadIdx.x;
-      if (c < n4) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(scaled(c, x[i], mu, rs, w[i], b[i]));
-    }
+  for (int i = 0; i < HOLD; ++i) {
+    const int c = i * kRegThreads + threadIdx.x;
+    if (c >= n4) continue;
+    if (a.xn) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(scaled(c, x[i], mu, rs, w[i], b[i]));
+    if (a.xn_f32) reinterpret_cast<float4*>(a.xn_f32 + m * a.ld)[c] = rescaled(c, x[i], mu, rs, w[i], b[i]);
   }
 }
 
@@ -201,7 +199,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const Residua
   pdl_launch_dependents();
   const int n4 = a.ld >> 2;
   const size_t m = blockIdx.x;
-  float4* xrow = reinterpret_cast<float4*>(a.x + m * a.ld);
+  float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
   float ss = 0.f;
   if (a.y) {
     float4* yrow = rn_row + n4;
@@ -238,15 +236,18 @@ __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const Residua
     }
   }
   const float rs = 1.0f / sqrtf(rn_block_sum(ss, red) / static_cast<float>(a.d) + a.eps);
-  if (a.stats && threadIdx.x == 0) {
-    a.stats[2 * m] = 0.f;
-    a.stats[2 * m + 1] = rs;
-  }
   if (a.xn) {
     uint2* o = reinterpret_cast<uint2*>(a.xn + m * a.ld);
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
       const float4 x = rn_row[i], w = reinterpret_cast<const float4*>(a.w_next)[i];
       o[i] = pack4(keep(make_float4(x.x * rs * w.x, x.y * rs * w.y, x.z * rs * w.z, x.w * rs * w.w), a.d - 4 * i));
+    }
+  }
+  if (a.xn_f32) {
+    float4* o = reinterpret_cast<float4*>(a.xn_f32 + m * a.ld);
+    for (int i = threadIdx.x; i < n4; i += kRnThreads) {
+      const float4 x = rn_row[i], w = reinterpret_cast<const float4*>(a.w_next)[i];
+      o[i] = keep(make_float4(w.x * rs * x.x, w.y * rs * x.y, w.z * rs * x.z, w.w * rs * x.w), a.d - 4 * i);
     }
   }
   if (a.cat_f32 || a.cat_bf16) {
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_layernorm_kernel(const Re
   pdl_launch_dependents();
   const int n4 = a.ld >> 2;
   const size_t m = blockIdx.x;
-  float4* xrow = reinterpret_cast<float4*>(a.x + m * a.ld);
+  float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
   const float inv_n = 1.0f / static_cast<float>(a.d);
   auto norm = [&](float sum, float* mu, float* rs) {
     *mu = rn_block_sum(sum, red) * inv_n;
@@ -320,15 +321,16 @@ __global__ void __launch_bounds__(kRnThreads) residual_layernorm_kernel(const Re
   } else if (a.xn && !a.w_next) {
     for (int i = threadIdx.x; i < n4; i += kRnThreads) reinterpret_cast<uint2*>(a.xn + m * a.ld)[i] = pack4(rn_row[i]);
   }
-  if (!a.w_next && !a.stats) return;
+  if (!a.w_next) return;
   norm(sum, &mu, &rs);
-  if (a.stats && threadIdx.x == 0) {
-    a.stats[2 * m] = mu;
-    a.stats[2 * m + 1] = rs;
+  for (int i = threadIdx.x; i < n4; i += kRnThreads) {
+    if (a.xn) reinterpret_cast<uint2*>(a.xn + m * a.ld)[i] = pack4(scaled(i, mu, rs, a.w_next, a.b_next));
+    if (!a.xn_f32) continue;
+    const float4 z = rn_row[i], w4 = reinterpret_cast<const float4*>(a.w_next)[i], b4 = reinterpret_cast<const float4*>(a.b_next)[i];
+    reinterpret_cast<float4*>(a.xn_f32 + m * a.ld)[i] =
+        keep(make_float4(fmaf(w4.x * rs, z.x - mu, b4.x), fmaf(w4.y * rs, z.y - mu, b4.y), fmaf(w4.z * rs, z.z - mu, b4.z),
+                         fmaf(w4.w * rs, z.w - mu, b4.w)), a.d - 4 * i);
   }
-  if (a.xn && a.w_next)
-    for (int i = threadIdx.x; i < n4; i += kRnThreads)
-      reinterpret_cast<uint2*>(a.xn + m * a.ld)[i] = pack4(scaled(i, mu, rs, a.w_next, a.b_next));
 }
 
 __global__ void gather_rows_bf16_kernel(const __nv_bfloat16* __restrict__ src, int ld, const int32_t* __restrict__ rows,

@@ -19,16 +19,17 @@ struct ResidualNormArgs {
   int planes;
   const float* w_post;         // [ld]
   float mult, eps;
-  float* stats;                // [M, 2] or null
-  const float* w_next;         // [ld], with xn
+  const float* w_next;         // [ld], with xn or xn_f32
   __nv_bfloat16* xn;           // [M, ld] or null
+  float* xn_f32;               // [M, ld] or null
+  const int32_t* select;       // optional [M], with y == null: source row of x
   const float* x0;             // [M, ld], with cat_*
   float* cat_f32;              // [M, 2 ld] or null
   __nv_bfloat16* cat_bf16;     // [M, 2 ld] or null
 };
 cudaError_t launch_residual_norm(const ResidualNormArgs& a, cudaStream_t s, bool pdl);
 // One row per block:  y = sum of the planes;  x = LayerNorm(alpha * x + y) * w + b;  then xn = x in bf16, or, with w_next, the layer norm of the
-// new x in bf16, and its (mean, 1 / deviation) into stats.  y == null: x stays, only what follows is done.
+// new x, in bf16 (xn) or fp32 (xn_f32).  y == null: x stays, only what follows is done.
 struct ResidualLayerNormArgs {
   float* x;                    // [M, ld]; columns d .. ld - 1 of every buffer here are zero
   int M, d, ld;
@@ -38,7 +39,8 @@ struct ResidualLayerNormArgs {
   float alpha, eps;
   __nv_bfloat16* xn;           // [M, ld] or null
   const float *w_next, *b_next;  // [ld] or null
-  float* stats;                // [M, 2] or null
+  float* xn_f32;               // [M, ld] or null, with w_next
+  const int32_t* select;       // optional [M], with y == null: source row of x
 };
 cudaError_t launch_residual_layernorm(const ResidualLayerNormArgs& a, cudaStream_t s, bool pdl);
 cudaError_t launch_gather_rows_bf16(const __nv_bfloat16* src, int ld, const int32_t* rows, int n, __nv_bfloat16* dst,
