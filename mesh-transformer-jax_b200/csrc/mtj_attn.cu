@@ -463,11 +463,15 @@ __global__ void __launch_bounds__(kStreamThreads) decode_attn_stream_kernel(cons
   if (threadIdx.x == 0) a.counters[b * a.heads + head] = 0u;
 }
 
-// Causal attention for a chunk of rows; one warp owns QPW consecutive queries
-// of one (sequence, head) and walks the keys once for all of them.
+// Causal attention for a chunk of rows on the CUDA cores, fp32 queries; one warp owns QPW consecutive queries of one
+// (sequence, head) and walks the keys 32 at a time, once for all of them.  For the scores a lane owns a key, whose row it
+// reads by itself (no sum across lanes, all of the row's loads in flight); for the outputs it owns DH / 32 columns.  A key at a
+// time with the columns over the lanes, every key cost its load latency and five shuffles: 99 rows of 4 heads of 64 columns
+// took 55 us.
 template <int DH, int QPW>
 __global__ void __launch_bounds__(kAttnThreads) prefill_attn_kernel(const PrefillAttnArgs a) {
   constexpr int EPL = DH / 32;
+  __shared__ __align__(16) float qs[kAttnWarps][QPW][DH];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int head = blockIdx.y, bi = blockIdx.z;
   const int tl0 = (blockIdx.x * kAttnWarps + warp) * QPW;   // first query of this warp in the chunk
@@ -480,57 +484,82 @@ __global__ void __launch_bounds__(kAttnThreads) prefill_attn_kernel(const Prefil
   const int klimit = a.key_limit ? a.key_limit[b] : 0x7fffffff;
 
   constexpr float scale = DH == 256 ? 0.0625f : 0.125f;   // 1 / sqrt(d_head), exact
-  float q[QPW][EPL], o[QPW][EPL], m[QPW], l[QPW];
+  float o[QPW][EPL], m[QPW], l[QPW];                        // l: of this lane's keys
 #pragma unroll
   for (int i = 0; i < QPW; ++i) {
     const int row = bi * a.rows.Tc + tl0 + (i < nq ? i : 0);
-    const float* qp = a.q + (static_cast<size_t>(row) * a.heads + head) * DH + lane * EPL;
+    const float* qp = a.q + (static_cast<size_t>(row) * a.heads + head) * DH;
 #pragma unroll
     for (int e = 0; e < EPL; ++e) {
-      q[i][e] = qp[e] * scale;
+      qs[warp][i][e * 32 + lane] = qp[e * 32 + lane] * scale;
       o[i][e] = 0.f;
     }
     m[i] = -INFINITY;
     l[i] = 0.f;
   }
+  __syncwarp();
   const int last_pos = min(pos0 + tl0 + nq - 1, klimit);
-  for (int kp = kstart; kp <= last_pos; ++kp) {
-    const size_t off = kv_offset(table, a.kv.ring_pages, a.heads, DH, head, kp) + lane * EPL;
-    KvVec<EPL> kv, vv;
-    kv.load(a.kv.kpool + off);
-    vv.load(a.kv.vpool + off);
-    float kf[EPL], vf[EPL];
-    kv.get(kf);
-    vv.get(vf);
+  for (int kp = kstart; kp <= last_pos; kp += 32) {
+    const int key = min(kp + lane, last_pos);
+    const int page = table[(key / kPageTokens) % a.kv.ring_pages];
+    const int krow = (page * a.heads + head) * kPageTokens + key % kPageTokens;
+    const uint4* kr = reinterpret_cast<const uint4*>(a.kv.kpool + static_cast<size_t>(krow) * DH);
     float s[QPW];
 #pragma unroll
-    for (int i = 0; i < QPW; ++i) {
-      float d = 0.f;
+    for (int i = 0; i < QPW; ++i) s[i] = 0.f;
+#pragma unroll 1
+    for (int c = 0; c < DH / 64; ++c) {
+      uint4 kv[8];
 #pragma unroll
-      for (int e = 0; e < EPL; ++e) d = fmaf(q[i][e], kf[e], d);
-      s[i] = d;
+      for (int u = 0; u < 8; ++u) kv[u] = kr[c * 8 + u];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        float kf[8];
+        unpack8(kv[u], kf);
+#pragma unroll
+        for (int i = 0; i < QPW; ++i) {
+          const float4 qa = *reinterpret_cast<const float4*>(&qs[warp][i][c * 64 + u * 8]), qb = *reinterpret_cast<const float4*>(&qs[warp][i][c * 64 + u * 8 + 4]);
+          s[i] = fmaf(kf[0], qa.x, s[i]); s[i] = fmaf(kf[1], qa.y, s[i]); s[i] = fmaf(kf[2], qa.z, s[i]); s[i] = fmaf(kf[3], qa.w, s[i]);
+          s[i] = fmaf(kf[4], qb.x, s[i]); s[i] = fmaf(kf[5], qb.y, s[i]); s[i] = fmaf(kf[6], qb.z, s[i]); s[i] = fmaf(kf[7], qb.w, s[i]);
+        }
+      }
     }
 #pragma unroll
-    for (int o2 = 16; o2 > 0; o2 >>= 1)
-#pragma unroll
-      for (int i = 0; i < QPW; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o2);
-#pragma unroll
     for (int i = 0; i < QPW; ++i) {
-      if (kp > pos0 + tl0 + i) continue;       // causal
-      const float mn = fmaxf(m[i], s[i]);
-      const float corr = __expf(m[i] - mn);
-      const float p = __expf(s[i] - mn);
-      l[i] = fmaf(l[i], corr, p);
+      const bool seen = kp + lane <= min(last_pos, pos0 + tl0 + i);      // causal, and not beyond the last key
+      const float v = seen ? s[i] : -INFINITY;
+      const float mn = fmaxf(m[i], warp_max(v));
+      const float corr = mn == -INFINITY ? 1.f : __expf(m[i] - mn);
+      s[i] = seen ? __expf(v - mn) : 0.f;
+      l[i] = fmaf(l[i], corr, s[i]);
 #pragma unroll
-      for (int e = 0; e < EPL; ++e) o[i][e] = fmaf(o[i][e], corr, p * vf[e]);
+      for (int e = 0; e < EPL; ++e) o[i][e] *= corr;
       m[i] = mn;
+    }
+    const int n = min(32, last_pos - kp + 1);
+    for (int j0 = 0; j0 < n; j0 += 8) {
+      KvVec<EPL> vv[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) vv[u].load(a.kv.vpool + static_cast<size_t>(__shfl_sync(0xffffffffu, krow, j0 + u)) * DH + lane * EPL);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        float vf[EPL];
+        vv[u].get(vf);
+#pragma unroll
+        for (int i = 0; i < QPW; ++i) {
+          const float p = __shfl_sync(0xffffffffu, s[i], j0 + u);
+          if (p == 0.f) continue;                            // a key that is not seen adds nothing, whatever its value holds
+#pragma unroll
+          for (int e = 0; e < EPL; ++e) o[i][e] = fmaf(p, vf[e], o[i][e]);
+        }
+      }
     }
   }
 #pragma unroll
   for (int i = 0; i < QPW; ++i) {
     if (i >= nq) break;
     const int row = bi * a.rows.Tc + tl0 + i;
-    const float inv = l[i] > 0.f ? 1.0f / l[i] : 0.f;   // rows with no visible key (left pad) give 0
+    const float sum = warp_sum(l[i]), inv = sum > 0.f ? 1.0f / sum : 0.f;   // rows with no visible key (left pad) give 0
     const size_t o_off = static_cast<size_t>(row) * a.ld_out + head * DH + lane * EPL;
     if (a.out_bf16) {
 #pragma unroll
@@ -642,12 +671,13 @@ cudaError_t launch_decode_attn(const DecodeAttnArgs& a, cudaStream_t s, bool pdl
 
 cudaError_t launch_prefill_attn(const PrefillAttnArgs& a, cudaStream_t s) {
   if (a.M <= 0 || a.rows.Tc <= 0 || a.M % a.rows.Tc != 0) return cudaErrorInvalidValue;
-  constexpr int QPW = 4;
-  const dim3 grid((a.rows.Tc + kAttnWarps * QPW - 1) / (kAttnWarps * QPW), a.heads, a.M / a.rows.Tc);
-  const dim3 block(kAttnThreads);
-  if (a.d_head == 256) return launch_cfg(prefill_attn_kernel<256, QPW>, grid, block, s, false, a);
-  if (a.d_head == 64) return launch_cfg(prefill_attn_kernel<64, QPW>, grid, block, s, false, a);
-  return cudaErrorInvalidValue;
+  if (a.d_head != 256 && a.d_head != 64) return cudaErrorInvalidValue;
+  // a query per warp while that leaves the SMs below two blocks each: short prompts are bound by a warp's chain of keys
+  const int qpw = static_cast<int64_t>(a.M) * a.heads <= 2 * 148 * kAttnWarps ? 1 : 4;
+  const dim3 grid((a.rows.Tc + kAttnWarps * qpw - 1) / (kAttnWarps * qpw), a.heads, a.M / a.rows.Tc), block(kAttnThreads);
+  if (a.d_head == 256)
+    return qpw == 1 ? launch_cfg(prefill_attn_kernel<256, 1>, grid, block, s, false, a) : launch_cfg(prefill_attn_kernel<256, 4>, grid, block, s, false, a);
+  return qpw == 1 ? launch_cfg(prefill_attn_kernel<64, 1>, grid, block, s, false, a) : launch_cfg(prefill_attn_kernel<64, 4>, grid, block, s, false, a);
 }
 
 }  // namespace mtj

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kPrepThreads) grouped_prep_kernel(const Groupe
 
 // ---- what the row-at-a-time kernels share: the key range of a block and the end of a (row, key head)
 struct Range {
-  int seq, k0, k1, lo;                // keys [max(k0, lo), k1)
+  int seq, k0, k1, lo, p;             // keys [max(k0, lo), k1); the query's position
 };
 __device__ __forceinline__ Range key_range(const GroupedAttnArgs& a, int m, int split) {
   Range r;
@@ -131,6 +131,7 @@ __device__ __forceinline__ Range key_range(const GroupedAttnArgs& a, int m, int 
   r.k0 = first + split * per;                          // pieces lie inside one page
   r.k1 = min(r.k0 + per, p + 1);
   r.lo = lo;
+  r.p = p;
   return r;
 }
 __device__ __forceinline__ float ex2(float x) {
@@ -342,8 +343,6 @@ __global__ void __launch_bounds__(32 * kWarps) grouped_attn_mma_kernel(const Gro
     if (kc < kd) *reinterpret_cast<uint4*>(ring + i * kst + kc) = make_uint4(0u, 0u, 0u, 0u);
     if (vc < vd) *reinterpret_cast<uint4*>(vring + i * vst + vc) = make_uint4(0u, 0u, 0u, 0u);
   }
-  pdl_wait();
-  pdl_launch_dependents();
   const Range r = key_range(a, m, split);
   const int n_pieces = r.k1 > r.k0 ? (r.k1 - r.k0 + kPiece - 1) / kPiece : 0;
   // a lane copies the same 16 bytes of every kper-th key
@@ -368,8 +367,16 @@ __global__ void __launch_bounds__(32 * kWarps) grouped_attn_mma_kernel(const Gro
     }
     cp_commit();                                            // always, so that groups count pieces
   };
-#pragma unroll
-  for (int i = 0; i < kStages - 1; ++i) fetch(warp + i * kWarps, i);
+  // decoding: this pass wrote one key, the last; the pieces in front of it are copied before the wait
+  const int settled = a.rows.pos0_dev ? r.p : 0;
+  int ahead = 0;
+  while (ahead < kStages - 1 && r.k0 + (warp + ahead * kWarps + 1) * kPiece <= min(settled, r.k1)) {
+    fetch(warp + ahead * kWarps, ahead);
+    ++ahead;
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  for (; ahead < kStages - 1; ++ahead) fetch(warp + ahead * kWarps, ahead);
   for (int i = threadIdx.x; i < kHM * (kd >> 3); i += 32 * kWarps) {
     const int h = i / (kd >> 3), c = i % (kd >> 3) * 8;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);

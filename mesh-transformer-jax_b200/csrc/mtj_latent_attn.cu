@@ -219,8 +219,6 @@ __global__ void __launch_bounds__(kThreads) latent_attn_kernel(const LatentArgs 
   extern __shared__ __align__(16) unsigned char la_smem[];
   __shared__ float s_corr[kHG];
   __shared__ __align__(16) float s_p[kTK][kHG];
-  pdl_wait();
-  pdl_launch_dependents();
   const int m = blockIdx.z, h0 = blockIdx.y * kHG, split = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ld = a.cache.row_ld, kv_ld = a.cache.kv_ld, tld = ld + Vec8<T>::kPad;
@@ -231,19 +229,9 @@ __global__ void __launch_bounds__(kThreads) latent_attn_kernel(const LatentArgs 
   const int lo = max(0, p - a.window + 1), n = p - lo + 1;            // n <= 0: a padding row
   const int per = (((max(n, 0) + a.splits - 1) / a.splits) + kTK - 1) / kTK * kTK;
   const int k0 = lo + split * per, k1 = min(k0 + per, p + 1);
-
-  for (int i = threadIdx.x; i < kHG * (ld >> 2); i += kThreads) {
-    const int h = i / (ld >> 2), c = i % (ld >> 2);
-    reinterpret_cast<float4*>(qs)[i] =
-        h0 + h < a.heads ? reinterpret_cast<const float4*>(a.q_abs + (static_cast<size_t>(m) * a.heads + h0 + h) * ld)[c]
-                         : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  float acc[NC][kHG][2] = {};
-  float mx = -INFINITY, l = 0.f;                                    // of head h0 + warp, the same in every lane
   constexpr int kVec = 16 / static_cast<int>(sizeof(T));
   const int nv = ld / kVec;
-  for (int kt = k0; kt < k1; kt += kTK) {
-    __syncthreads();                                                // the tile and the weights of the last round are read
+  auto fetch = [&](int kt) {
     for (int key = warp; key < kTK; key += kThreads / 32) {           // a warp per row, all copies in flight at once
       T* dst = cs + key * tld;
       if (kt + key < k1) {
@@ -254,6 +242,23 @@ __global__ void __launch_bounds__(kThreads) latent_attn_kernel(const LatentArgs 
       }
     }
     cp_commit();
+  };
+  // decoding: this pass wrote one key, the last; a first tile without it is copied before the wait
+  const bool ahead = a.rows.pos0_dev && k0 < k1 && min(k0 + kTK, k1) <= p;
+  if (ahead) fetch(k0);
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int i = threadIdx.x; i < kHG * (ld >> 2); i += kThreads) {
+    const int h = i / (ld >> 2), c = i % (ld >> 2);
+    reinterpret_cast<float4*>(qs)[i] =
+        h0 + h < a.heads ? reinterpret_cast<const float4*>(a.q_abs + (static_cast<size_t>(m) * a.heads + h0 + h) * ld)[c]
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float acc[NC][kHG][2] = {};
+  float mx = -INFINITY, l = 0.f;                                    // of head h0 + warp, the same in every lane
+  for (int kt = k0; kt < k1; kt += kTK) {
+    __syncthreads();                                                // the tile and the weights of the last round are read
+    if (!ahead || kt > k0) fetch(kt);
     cp_wait<0>();
     __syncthreads();
     float s = 0.f, s2 = 0.f;
@@ -357,8 +362,6 @@ __global__ void __launch_bounds__(kThreads) latent_attn_mma_kernel(const LatentA
   float* ss = reinterpret_cast<float*>(ps + HM * kPld);                     // [KH][HM][kSld]
   float* corr_s = ss + KH * HM * kSld;                                      // [HM]
   const int m = blockIdx.z, h0 = blockIdx.y * HM, split = blockIdx.x;
-  pdl_wait();
-  pdl_launch_dependents();
   int seq;
   const int p = own_pos(a.rows, a.pad, m, &seq);
   const int lo = max(0, p - a.window + 1), n = p - lo + 1;
@@ -377,7 +380,11 @@ __global__ void __launch_bounds__(kThreads) latent_attn_mma_kernel(const LatentA
     }
     cp_commit();
   };
-  if (k0 < k1) fetch(k0, 0);
+  const bool ahead = a.rows.pos0_dev && k0 < k1 && min(k0 + kTK, k1) <= p;   // as above
+  if (ahead) fetch(k0, 0);
+  pdl_wait();
+  pdl_launch_dependents();
+  if (!ahead && k0 < k1) fetch(k0, 0);
   for (int i = threadIdx.x; i < HM * (kd >> 3); i += kThreads) {
     const int h = i / (kd >> 3), c = i % (kd >> 3) * 8;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
