@@ -48,6 +48,21 @@ struct KvVec<2> {
   }
 };
 
+// sum over the splits of weight times one column, eight loads in flight (one at a time, each costs an L2 round trip)
+template <int DH>
+__device__ __forceinline__ float merge_column(const float* po, const float* wgt, int nsplit) {
+  float O = 0.f;
+  for (int s0 = 0; s0 < nsplit; s0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = __ldcg(po + static_cast<size_t>(min(s0 + u, nsplit - 1)) * DH);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (s0 + u < nsplit) O = fmaf(v[u], wgt[s0 + u], O);
+  }
+  return O;
+}
+
 template <int DH>
 __global__ void __launch_bounds__(kAttnThreads) decode_attn_kernel(const DecodeAttnArgs a) {
   constexpr int EPL = DH / 32;
@@ -66,7 +81,7 @@ __global__ void __launch_bounds__(kAttnThreads) decode_attn_kernel(const DecodeA
 
   // The step counter, the page table and every cached token except the newest
   // were written before the predecessor kernel started: the split geometry can
-  // be worked out, and all pages but the one holding the newest token fetched,
+  // be worked out, and everything but the newest token's row fetched,
   // before waiting for it.  One split = one 64-token page of one head, whose K
   // (and V) slab is contiguous: a single bulk copy each.
   const int cur = *a.cur_dev;
@@ -75,28 +90,29 @@ __global__ void __launch_bounds__(kAttnThreads) decode_attn_kernel(const DecodeA
   const int first_page = start / kPageTokens;
   const int nsplit = cur / kPageTokens - first_page + 1;
   const int page_pos0 = (first_page + split) * kPageTokens;
-  const bool active = split < nsplit;
+  if (split >= nsplit) return;      // most blocks of a grid made for the whole window: they must not hold an SM until the wait ends
   const bool newest_page = page_pos0 + kPageTokens > cur;
   const int t0 = max(start, page_pos0), t1 = min(end, page_pos0 + kPageTokens);
   const uint32_t bar_u32 = smem_u32(&bar);
-  auto fetch = [&]() {
+  // rows [0, old) were cached before this step; the newest page has one more, which the predecessor writes
+  const int old = newest_page ? cur - page_pos0 : kPageTokens;
+  auto fetch = [&](int row, int n) {
     const int32_t* table = a.kv.page_table + static_cast<size_t>(b) * a.kv.ring_pages;
     const int page = table[(first_page + split) % a.kv.ring_pages];
-    const size_t off = (static_cast<size_t>(page) * a.heads + head) * kPageTokens * DH;
+    const size_t off = ((static_cast<size_t>(page) * a.heads + head) * kPageTokens + row) * DH;
     const uint64_t pol = l2_evict_first_policy();
-    mbar_expect_tx(bar_u32, 2 * kSlab);
-    bulk_load(smem_u32(sk), a.kv.kpool + off, kSlab, bar_u32, pol);
-    bulk_load(smem_u32(sv), a.kv.vpool + off, kSlab, bar_u32, pol);
+    bulk_load(smem_u32(sk) + row * DH * 2, a.kv.kpool + off, n * DH * 2, bar_u32, pol);
+    bulk_load(smem_u32(sv) + row * DH * 2, a.kv.vpool + off, n * DH * 2, bar_u32, pol);
   };
   if (threadIdx.x == 0) {
     mbar_init(bar_u32, 1);
     mbar_fence_init();
-    if (active && !newest_page) fetch();
+    mbar_expect_tx(bar_u32, 2 * (old + (newest_page ? 1 : 0)) * DH * 2);
+    if (old > 0) fetch(0, old);
   }
   pdl_wait();
   pdl_launch_dependents();
-  if (!active) return;
-  if (threadIdx.x == 0 && newest_page) fetch();
+  if (threadIdx.x == 0 && newest_page) fetch(old, 1);
 
   constexpr float scale = DH == 256 ? 0.0625f : 0.125f;   // 1 / sqrt(d_head), exact
   float q[EPL];
@@ -215,16 +231,7 @@ __global__ void __launch_bounds__(kAttnThreads) decode_attn_kernel(const DecodeA
     __syncthreads();
     if (threadIdx.x < DH) {
       const float* po = a.part_o + base * DH + threadIdx.x;
-      float O = 0.f;
-      int sidx = 0;
-      for (; sidx + 8 <= nsplit; sidx += 8) {
-        float v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = __ldcg(po + static_cast<size_t>(sidx + u) * DH);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) O = fmaf(v[u], wgt[sidx + u], O);
-      }
-      for (; sidx < nsplit; ++sidx) O = fmaf(__ldcg(po + static_cast<size_t>(sidx) * DH), wgt[sidx], O);
+      const float O = merge_column<DH>(po, wgt, nsplit);
       const size_t oi = static_cast<size_t>(b) * a.ld_out + head * DH + threadIdx.x;
       if (a.out_bf16) {
         const float y = O * inv_l;
@@ -240,14 +247,14 @@ __global__ void __launch_bounds__(kAttnThreads) decode_attn_kernel(const DecodeA
 }
 
 // The same decode attention for many sequences: one block walks a.stream_pages (1-4) consecutive pages of one
-// (sequence, head) as half-page tiles (32 keys: 16 KB of K + 16 KB of V) through a 3-stage ring fed by a
+// (sequence, head) as half-page tiles (32 keys: 16 KB of K + 16 KB of V) through a 2-stage ring (three blocks per SM) fed by a
 // producer warp, so the block's loads stay in flight while its eight consumer warps work, and the
 // per-block costs (launch, warp merge, partial write, ticket) are spread over up to 256 keys.  Each
 // consumer warp keeps its own running (max, sum, weighted V) over the 4 keys it takes from every tile.
 // The launcher picks the pages per block so that the grid fills whole waves of resident blocks: with few
 // heads per GPU (tensor-parallel shards) four pages per block leave the last wave mostly empty.
 constexpr int kStreamPages = 4;                            // most pages a block walks
-constexpr int kStreamStages = 3;
+constexpr int kStreamStages = 2;
 constexpr int kTileTokens = 32;
 constexpr int kStreamThreads = kAttnThreads + 32;
 
@@ -447,8 +454,7 @@ __global__ void __launch_bounds__(kStreamThreads) decode_attn_stream_kernel(cons
     __syncthreads();
     if (threadIdx.x < DH) {
       const float* po = a.part_o + base * DH + threadIdx.x;
-      float O = 0.f;
-      for (int sidx = 0; sidx < nsplit; ++sidx) O = fmaf(__ldcg(po + static_cast<size_t>(sidx) * DH), wgt[sidx], O);
+      const float O = merge_column<DH>(po, wgt, nsplit);
       const size_t oi = static_cast<size_t>(b) * a.ld_out + head * DH + threadIdx.x;
       if (a.out_bf16) {
         const float y = O * inv_l;
