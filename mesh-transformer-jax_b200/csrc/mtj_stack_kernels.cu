@@ -11,6 +11,7 @@ namespace {
 
 constexpr int kRnThreads = 256;
 
+template <int THREADS>
 __device__ __forceinline__ float rn_block_sum(float v, float* red) {
   v = warp_sum(v);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -18,7 +19,7 @@ __device__ __forceinline__ float rn_block_sum(float v, float* red) {
   __syncthreads();
   float t = 0.f;
 #pragma unroll
-  for (int i = 0; i < kRnThreads / 32; ++i) t += red[i];
+  for (int i = 0; i < THREADS / 32; ++i) t += red[i];
   __syncthreads();
   return t;
 }
@@ -39,57 +40,60 @@ __device__ __forceinline__ float4 keep(float4 v, int left) {
 // of the planes issued before the first sum, because with few rows the kernel is nothing but the latency of its loads
 // and sums (8 rows of 4096 in 8 planes: 12.4 us through shared memory); wider rows in shared memory.  Both add in the
 // same order.
-constexpr int kRegThreads = 256, kRegHold = 8;
+//
+// Rows of up to as many blocks as SMs take 512 threads, twice the loads in flight (24 rows of 2048 in 8 planes 6.1 us with 256
+// threads, 5.1 with 512); above, the SMs hold fewer such blocks (1794 rows of 2048 10 us and 15.7).
+constexpr int kRegCols = 8192, kFewRows = 148;
 
 // the sum of the planes of row m, in order
-template <int HOLD>
+template <int THREADS, int HOLD>
 __device__ __forceinline__ void load_planes(const float* y, int planes, size_t m, int M, int ld, int n4, float4 (&v)[HOLD]) {
   const size_t step = static_cast<size_t>(M) * ld / 4;
   const float4* src = reinterpret_cast<const float4*>(y + m * ld);
 #pragma unroll
   for (int i = 0; i < HOLD; ++i) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
+#pragma unroll(HOLD > 2 ? 4 : 8)
   for (int p = 0; p < planes; ++p) {
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
-      const int c = i * kRegThreads + threadIdx.x;
+      const int c = i * THREADS + threadIdx.x;
       const float4 w = c < n4 ? __ldcg(src + p * step + c) : make_float4(0.f, 0.f, 0.f, 0.f);
       v[i].x += w.x; v[i].y += w.y; v[i].z += w.z; v[i].w += w.w;
     }
   }
 }
-template <int HOLD>
+template <int THREADS, int HOLD>
 __device__ __forceinline__ void load_row(const float* row, int n4, float4 (&v)[HOLD]) {
 #pragma unroll
   for (int i = 0; i < HOLD; ++i) {
-    const int c = i * kRegThreads + threadIdx.x;
+    const int c = i * THREADS + threadIdx.x;
     v[i] = row && c < n4 ? reinterpret_cast<const float4*>(row)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
-template <int HOLD>
-__global__ void __launch_bounds__(kRegThreads) residual_norm_reg_kernel(const ResidualNormArgs a) {
-  __shared__ float red[kRegThreads / 32];
+template <int THREADS, int HOLD>
+__global__ void __launch_bounds__(THREADS) residual_norm_reg_kernel(const ResidualNormArgs a) {
+  __shared__ float red[THREADS / 32];
   const int n4 = a.ld >> 2;
   const size_t m = blockIdx.x;
   float4 wp[HOLD], wn[HOLD], x[HOLD];
-  load_row<HOLD>(a.y ? a.w_post : nullptr, n4, wp);          // weights do not depend on the predecessor
-  load_row<HOLD>(a.xn || a.xn_f32 ? a.w_next : nullptr, n4, wn);
+  load_row<THREADS, HOLD>(a.y ? a.w_post : nullptr, n4, wp);          // weights do not depend on the predecessor
+  load_row<THREADS, HOLD>(a.xn || a.xn_f32 ? a.w_next : nullptr, n4, wn);
   pdl_wait();
   pdl_launch_dependents();
   float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
-  load_row<HOLD>(reinterpret_cast<const float*>(xrow), n4, x);
+  load_row<THREADS, HOLD>(reinterpret_cast<const float*>(xrow), n4, x);
   float ss = 0.f;
   if (a.y) {
     float4 y[HOLD];
-    load_planes<HOLD>(a.y, a.planes, m, a.M, a.ld, n4, y);
+    load_planes<THREADS, HOLD>(a.y, a.planes, m, a.M, a.ld, n4, y);
     float ys = 0.f;
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) ys += dot4(y[i]);
-    const float rs = a.mult / sqrtf(rn_block_sum(ys, red) / static_cast<float>(a.d) + a.eps);
+    const float rs = a.mult / sqrtf(rn_block_sum<THREADS>(ys, red) / static_cast<float>(a.d) + a.eps);
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
-      const int c = i * kRegThreads + threadIdx.x;
+      const int c = i * THREADS + threadIdx.x;
       x[i] = keep(make_float4(fmaf(y[i].x * rs, wp[i].x, x[i].x), fmaf(y[i].y * rs, wp[i].y, x[i].y), fmaf(y[i].z * rs, wp[i].z, x[i].z),
                               fmaf(y[i].w * rs, wp[i].w, x[i].w)), a.d - 4 * c);
       if (c < n4) xrow[c] = x[i];
@@ -97,10 +101,10 @@ __global__ void __launch_bounds__(kRegThreads) residual_norm_reg_kernel(const Re
   }
 #pragma unroll
   for (int i = 0; i < HOLD; ++i) ss += dot4(x[i]);
-  const float rs = 1.0f / sqrtf(rn_block_sum(ss, red) / static_cast<float>(a.d) + a.eps);
+  const float rs = 1.0f / sqrtf(rn_block_sum<THREADS>(ss, red) / static_cast<float>(a.d) + a.eps);
 #pragma unroll
   for (int i = 0; i < HOLD; ++i) {
-    const int c = i * kRegThreads + threadIdx.x;
+    const int c = i * THREADS + threadIdx.x;
     if (c >= n4) continue;
     const float4 v = x[i], w = wn[i];
     if (a.xn_f32) reinterpret_cast<float4*>(a.xn_f32 + m * a.ld)[c] = keep(make_float4(w.x * rs * v.x, w.y * rs * v.y, w.z * rs * v.z, w.w * rs * v.w), a.d - 4 * c);
@@ -121,15 +125,15 @@ __global__ void __launch_bounds__(kRegThreads) residual_norm_reg_kernel(const Re
   }
 }
 
-template <int HOLD>
-__global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(const ResidualLayerNormArgs a) {
-  __shared__ float red[kRegThreads / 32];
+template <int THREADS, int HOLD>
+__global__ void __launch_bounds__(THREADS) residual_layernorm_reg_kernel(const ResidualLayerNormArgs a) {
+  __shared__ float red[THREADS / 32];
   const int n4 = a.ld >> 2;
   const size_t m = blockIdx.x;
   const float inv_n = 1.0f / static_cast<float>(a.d);
   float4 w[HOLD], b[HOLD], x[HOLD];
-  load_row<HOLD>(a.y ? a.w : nullptr, n4, w);                // weights do not depend on the predecessor
-  load_row<HOLD>(a.y ? a.b : nullptr, n4, b);
+  load_row<THREADS, HOLD>(a.y ? a.w : nullptr, n4, w);                // weights do not depend on the predecessor
+  load_row<THREADS, HOLD>(a.y ? a.b : nullptr, n4, b);
   pdl_wait();
   pdl_launch_dependents();
   float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
@@ -137,13 +141,13 @@ __global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(con
     float s = 0.f, q = 0.f;
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) s += (x[i].x + x[i].y) + (x[i].z + x[i].w);
-    *mu = rn_block_sum(s, red) * inv_n;
+    *mu = rn_block_sum<THREADS>(s, red) * inv_n;
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
-      const int left = a.d - 4 * (i * kRegThreads + static_cast<int>(threadIdx.x));      // columns that exist
+      const int left = a.d - 4 * (i * THREADS + static_cast<int>(threadIdx.x));      // columns that exist
       q += dot4(make_float4(left > 0 ? x[i].x - *mu : 0.f, left > 1 ? x[i].y - *mu : 0.f, left > 2 ? x[i].z - *mu : 0.f, left > 3 ? x[i].w - *mu : 0.f));
     }
-    *rs = 1.0f / sqrtf(rn_block_sum(q, red) * inv_n + a.eps);
+    *rs = 1.0f / sqrtf(rn_block_sum<THREADS>(q, red) * inv_n + a.eps);
   };
   auto scaled = [&](int c, const float4& z, float mu, float rs, const float4& w4, const float4& b4) {
     return keep(make_float4(fmaf((z.x - mu) * rs, w4.x, b4.x), fmaf((z.y - mu) * rs, w4.y, b4.y), fmaf((z.z - mu) * rs, w4.z, b4.z),
@@ -155,17 +159,17 @@ __global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(con
                             fmaf(w4.w * rs, z.w - mu, b4.w)), a.d - 4 * c);
   };
   float mu, rs;
-  load_row<HOLD>(reinterpret_cast<const float*>(xrow), n4, x);
+  load_row<THREADS, HOLD>(reinterpret_cast<const float*>(xrow), n4, x);
   if (a.y) {
     float4 y[HOLD];
-    load_planes<HOLD>(a.y, a.planes, m, a.M, a.ld, n4, y);
+    load_planes<THREADS, HOLD>(a.y, a.planes, m, a.M, a.ld, n4, y);
 #pragma unroll
     for (int i = 0; i < HOLD; ++i)
       x[i] = make_float4(fmaf(a.alpha, x[i].x, y[i].x), fmaf(a.alpha, x[i].y, y[i].y), fmaf(a.alpha, x[i].z, y[i].z), fmaf(a.alpha, x[i].w, y[i].w));
     norm(&mu, &rs);
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
-      const int c = i * kRegThreads + threadIdx.x;
+      const int c = i * THREADS + threadIdx.x;
       x[i] = scaled(c, x[i], mu, rs, w[i], b[i]);
       if (c < n4) xrow[c] = x[i];
     }
@@ -173,17 +177,17 @@ __global__ void __launch_bounds__(kRegThreads) residual_layernorm_reg_kernel(con
   if (a.xn && !a.w_next) {
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
-      const int c = i * kRegThreads + threadIdx.x;
+      const int c = i * THREADS + threadIdx.x;
       if (c < n4) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(x[i]);
     }
   }
   if (!a.w_next) return;
   norm(&mu, &rs);
-  load_row<HOLD>(a.w_next, n4, w);
-  load_row<HOLD>(a.b_next, n4, b);
+  load_row<THREADS, HOLD>(a.w_next, n4, w);
+  load_row<THREADS, HOLD>(a.b_next, n4, b);
 #pragma unroll
   for (int i = 0; i < HOLD; ++i) {
-    const int c = i * kRegThreads + threadIdx.x;
+    const int c = i * THREADS + threadIdx.x;
     if (c >= n4) continue;
     if (a.xn) reinterpret_cast<uint2*>(a.xn + m * a.ld)[c] = pack4(scaled(c, x[i], mu, rs, w[i], b[i]));
     if (a.xn_f32) reinterpret_cast<float4*>(a.xn_f32 + m * a.ld)[c] = rescaled(c, x[i], mu, rs, w[i], b[i]);
@@ -215,7 +219,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const Residua
       rn_row[i] = xrow[i];
       ys += dot4(v);
     }
-    const float rs = a.mult / sqrtf(rn_block_sum(ys, red) / static_cast<float>(a.d) + a.eps);
+    const float rs = a.mult / sqrtf(rn_block_sum<kRnThreads>(ys, red) / static_cast<float>(a.d) + a.eps);
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
       const float4 y = yrow[i], w = reinterpret_cast<const float4*>(a.w_post)[i];
       float4 x = rn_row[i];
@@ -235,7 +239,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const Residua
       ss += dot4(x);
     }
   }
-  const float rs = 1.0f / sqrtf(rn_block_sum(ss, red) / static_cast<float>(a.d) + a.eps);
+  const float rs = 1.0f / sqrtf(rn_block_sum<kRnThreads>(ss, red) / static_cast<float>(a.d) + a.eps);
   if (a.xn) {
     uint2* o = reinterpret_cast<uint2*>(a.xn + m * a.ld);
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
@@ -279,14 +283,14 @@ __global__ void __launch_bounds__(kRnThreads) residual_layernorm_kernel(const Re
   float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
   const float inv_n = 1.0f / static_cast<float>(a.d);
   auto norm = [&](float sum, float* mu, float* rs) {
-    *mu = rn_block_sum(sum, red) * inv_n;
+    *mu = rn_block_sum<kRnThreads>(sum, red) * inv_n;
     float v = 0.f;
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
       const float4 z = rn_row[i];
       const int left = a.d - 4 * i;                       // columns that exist
       v += dot4(make_float4(left > 0 ? z.x - *mu : 0.f, left > 1 ? z.y - *mu : 0.f, left > 2 ? z.z - *mu : 0.f, left > 3 ? z.w - *mu : 0.f));
     }
-    *rs = 1.0f / sqrtf(rn_block_sum(v, red) * inv_n + a.eps);
+    *rs = 1.0f / sqrtf(rn_block_sum<kRnThreads>(v, red) * inv_n + a.eps);
   };
   auto scaled = [&](int i, float mu, float rs, const float* w, const float* b) {
     const float4 z = rn_row[i], w4 = reinterpret_cast<const float4*>(w)[i], b4 = reinterpret_cast<const float4*>(b)[i];
@@ -379,10 +383,11 @@ int load_grid(int64_t n) { return static_cast<int>(std::min<int64_t>((n + 255) /
 
 cudaError_t launch_residual_norm(const ResidualNormArgs& a, cudaStream_t s, bool pdl) {
   if (a.M <= 0 || a.d <= 0 || a.ld < a.d || (a.ld & 3)) return cudaErrorInvalidValue;
-  const dim3 grid(a.M), block(kRegThreads);
-  if (a.ld <= 8 * kRegThreads) return launch_pdl(residual_norm_reg_kernel<2>, grid, block, 0, s, pdl, a);
-  if (a.ld <= 16 * kRegThreads) return launch_pdl(residual_norm_reg_kernel<4>, grid, block, 0, s, pdl, a);
-  if (a.ld <= 4 * kRegHold * kRegThreads) return launch_pdl(residual_norm_reg_kernel<kRegHold>, grid, block, 0, s, pdl, a);
+  auto go = [&](auto kernel, int threads) { return launch_pdl(kernel, dim3(a.M), dim3(threads), 0, s, pdl, a); };
+  const bool few = a.M <= kFewRows;
+  if (a.ld <= 2048) return few ? go(residual_norm_reg_kernel<512, 1>, 512) : go(residual_norm_reg_kernel<256, 2>, 256);
+  if (a.ld <= 4096) return few ? go(residual_norm_reg_kernel<512, 2>, 512) : go(residual_norm_reg_kernel<256, 4>, 256);
+  if (a.ld <= kRegCols) return few ? go(residual_norm_reg_kernel<512, 4>, 512) : go(residual_norm_reg_kernel<256, 8>, 256);
   const size_t smem = static_cast<size_t>(a.ld) * sizeof(float) * (a.y ? 2 : 1);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   static DeviceOnce once;
@@ -395,13 +400,14 @@ cudaError_t launch_residual_norm(const ResidualNormArgs& a, cudaStream_t s, bool
 
 cudaError_t launch_residual_layernorm(const ResidualLayerNormArgs& a, cudaStream_t s, bool pdl) {
   if (a.M <= 0 || a.d <= 0 || a.ld < a.d || (a.ld & 3) || (a.y && (!a.w || !a.b)) || (a.w_next && !a.b_next)) return cudaErrorInvalidValue;
-  const dim3 grid(a.M), block(kRegThreads);
+  auto go = [&](auto kernel, int threads) { return launch_pdl(kernel, dim3(a.M), dim3(threads), 0, s, pdl, a); };
+  const bool few = a.M <= kFewRows;
   // many short rows are bound by how many blocks an SM holds, not by the latency of one row's loads: in shared memory (1500
   // rows of 512: 5.6 us there, 7.6 in registers)
   const bool many = a.M > 512 && a.ld <= 1024;
-  if (!many && a.ld <= 8 * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<2>, grid, block, 0, s, pdl, a);
-  if (!many && a.ld <= 16 * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<4>, grid, block, 0, s, pdl, a);
-  if (!many && a.ld <= 4 * kRegHold * kRegThreads) return launch_pdl(residual_layernorm_reg_kernel<kRegHold>, grid, block, 0, s, pdl, a);
+  if (!many && a.ld <= 2048) return few ? go(residual_layernorm_reg_kernel<512, 1>, 512) : go(residual_layernorm_reg_kernel<256, 2>, 256);
+  if (!many && a.ld <= 4096) return few ? go(residual_layernorm_reg_kernel<512, 2>, 512) : go(residual_layernorm_reg_kernel<256, 4>, 256);
+  if (!many && a.ld <= kRegCols) return few ? go(residual_layernorm_reg_kernel<512, 4>, 512) : go(residual_layernorm_reg_kernel<256, 8>, 256);
   const size_t smem = static_cast<size_t>(a.ld) * sizeof(float);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   static DeviceOnce once;
