@@ -480,6 +480,8 @@ __global__ void __launch_bounds__(kAttnThreads) prefill_attn_kernel(const Prefil
   __shared__ __align__(16) float qs[kAttnWarps][QPW][DH];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int head = blockIdx.y, bi = blockIdx.z;
+  pdl_wait();
+  pdl_launch_dependents();
   const int tl0 = (blockIdx.x * kAttnWarps + warp) * QPW;   // first query of this warp in the chunk
   if (tl0 >= a.rows.Tc) return;
   const int b = a.rows.b0 + bi;
@@ -675,15 +677,15 @@ cudaError_t launch_decode_attn(const DecodeAttnArgs& a, cudaStream_t s, bool pdl
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_prefill_attn(const PrefillAttnArgs& a, cudaStream_t s) {
+cudaError_t launch_prefill_attn(const PrefillAttnArgs& a, cudaStream_t s, bool pdl) {
   if (a.M <= 0 || a.rows.Tc <= 0 || a.M % a.rows.Tc != 0) return cudaErrorInvalidValue;
   if (a.d_head != 256 && a.d_head != 64) return cudaErrorInvalidValue;
   // a query per warp while that leaves the SMs below two blocks each: short prompts are bound by a warp's chain of keys
   const int qpw = static_cast<int64_t>(a.M) * a.heads <= 2 * 148 * kAttnWarps ? 1 : 4;
   const dim3 grid((a.rows.Tc + kAttnWarps * qpw - 1) / (kAttnWarps * qpw), a.heads, a.M / a.rows.Tc), block(kAttnThreads);
   if (a.d_head == 256)
-    return qpw == 1 ? launch_cfg(prefill_attn_kernel<256, 1>, grid, block, s, false, a) : launch_cfg(prefill_attn_kernel<256, 4>, grid, block, s, false, a);
-  return qpw == 1 ? launch_cfg(prefill_attn_kernel<64, 1>, grid, block, s, false, a) : launch_cfg(prefill_attn_kernel<64, 4>, grid, block, s, false, a);
+    return qpw == 1 ? launch_cfg(prefill_attn_kernel<256, 1>, grid, block, s, pdl, a) : launch_cfg(prefill_attn_kernel<256, 4>, grid, block, s, pdl, a);
+  return qpw == 1 ? launch_cfg(prefill_attn_kernel<64, 1>, grid, block, s, pdl, a) : launch_cfg(prefill_attn_kernel<64, 4>, grid, block, s, pdl, a);
 }
 
 }  // namespace mtj

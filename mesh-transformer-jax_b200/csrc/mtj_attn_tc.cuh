@@ -212,6 +212,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_attn_tc_kernel(const __
   __syncthreads();
   fence_after();
   const uint32_t tmem = tmem_slot;
+  pdl_wait();
+  pdl_launch_dependents();                             // behind the allocation of tensor memory: no later kernel takes it first
 
   // causal: later query tiles walk more key blocks; the block order is longest tile first, heads
   // within a tile, so the tail of the grid is made of the short tiles
@@ -517,10 +519,9 @@ cudaError_t launch_attn_tc(const void* map_q, const void* map_k, const void* map
     if (e != cudaSuccess) return e;
   }
   const dim3 grid(a.heads, (a.rows.Tc + kQT - 1) / kQT, a.M / a.rows.Tc);
-  prefill_attn_tc_kernel<QA, VA, SRC><<<grid, kThreadsTc, smem, s>>>(
-      *static_cast<const CUtensorMap*>(map_q), *static_cast<const CUtensorMap*>(map_k),
-      *static_cast<const CUtensorMap*>(map_ks), *static_cast<const CUtensorMap*>(map_v), a);
-  return cudaGetLastError();
+  return launch_pdl(prefill_attn_tc_kernel<QA, VA, SRC>, grid, dim3(kThreadsTc), smem, s, a.chained != 0,
+                    *static_cast<const CUtensorMap*>(map_q), *static_cast<const CUtensorMap*>(map_k),
+                    *static_cast<const CUtensorMap*>(map_ks), *static_cast<const CUtensorMap*>(map_v), a);
 }
 
 }  // namespace

@@ -14,7 +14,7 @@ MTJ_WEAK cudaError_t launch_gemm_tc_gptj(GemvEpilogue, bool, const CUtensorMap&,
 MTJ_WEAK cudaError_t launch_decode_mega(const MegaArgs&, cudaStream_t, int*) MTJ_ABSENT
 MTJ_WEAK cudaError_t launch_decode_attn(const DecodeAttnArgs&, cudaStream_t, bool) MTJ_ABSENT
 MTJ_WEAK int decode_attn_splits(int) { return 1 << 20; }      // more than mtj_create accepts: no GPT-J handles
-MTJ_WEAK cudaError_t launch_prefill_attn(const PrefillAttnArgs&, cudaStream_t) MTJ_ABSENT
+MTJ_WEAK cudaError_t launch_prefill_attn(const PrefillAttnArgs&, cudaStream_t, bool) MTJ_ABSENT
 MTJ_WEAK cudaError_t launch_prefill_attn_tc(const void*, const void*, const void*, const PrefillAttnTcArgs&,
                                             cudaStream_t) MTJ_ABSENT
 MTJ_WEAK int32_t comm_unique_id(uint8_t*, std::string* err) MTJ_NO_COMM

@@ -612,9 +612,6 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
   tc_fence_after();
   const uint32_t tmem_acc = tmem_slot;
 
-  pdl_launch_dependents();
-  pdl_wait();
-
   const int m_tiles = (a.M + bn - 1) / bn;
   const int n_tiles = (a.N + kTileN - 1) / kTileN;
   // split-K (PAIR, a.partial): piece z of a tile covers k-blocks [z * per_z, + per_z) and leaves a plane of partial sums
@@ -632,9 +629,26 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
   const int tile_first = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
   const int tile_step = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
+  const uint32_t box_bytes = static_cast<uint32_t>(a.x_box) * kBK * 2;       // rows past bn / 2 are not multiplied
+  // the bytes of a stage are expected and its weights fetched; PAIR: block 0's barrier counts the bytes of both blocks
+  auto load_w = [&](int s, int kb, int n0) {
+    if (!PAIR || crank == 0) mbar_expect_tx(full_bar(s), PAIR ? 2 * (kABytes + box_bytes) : kStageBytes);
+    if (PAIR) tma_load_2d_pair(smem_base + s * kStageBytes, &map_w, kb * kBK, n0, tc_map_to_rank(full_bar(s), 0));
+    else tma_load_2d(smem_base + s * kStageBytes, &map_w, kb * kBK, n0, full_bar(s));
+  };
+  // the first tile's weights do not depend on the predecessor: the ring is full of them before the wait
+  int ahead = 0;
+  if (threadIdx.x == 0 && tile_first < total) {
+    int m0, n0, z, kb0, nk;
+    piece(tile_first, m0, n0, z, kb0, nk);
+    ahead = min(nk, kStages);
+    for (int s = 0; s < ahead; ++s) load_w(s, kb0 + s, n0);
+  }
+  pdl_wait();                                        // the activations come from the predecessor kernel
+  pdl_launch_dependents();                           // behind the allocation of tensor memory: no later kernel takes it first
+
   if (warp == 0) {
     if (lane == 0) {
-      const uint32_t box_bytes = static_cast<uint32_t>(a.x_box) * kBK * 2;   // rows past bn / 2 are not multiplied
       int s = 0;
       uint32_t phase = 0;
       bool alive = true;
@@ -642,21 +656,21 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
         int m0, n0, z, kb0, nk;
         piece(t, m0, n0, z, kb0, nk);
         for (int kb = 0; kb < nk; ++kb) {
-          if (!mbar_wait(empty_bar(s), phase ^ 1u)) {        // passes in the ring's first round
-            atomicOr(&failed, 1u);
-            alive = false;
-            break;
+          if (ahead > 0) {
+            --ahead;
+          } else {
+            if (!mbar_wait(empty_bar(s), phase ^ 1u)) {      // passes in the ring's first round
+              atomicOr(&failed, 1u);
+              alive = false;
+              break;
+            }
+            load_w(s, kb0 + kb, n0);
           }
           const uint32_t dst = smem_base + s * kStageBytes;
           if (PAIR) {
-            // block 0's barrier counts the bytes of both blocks
-            if (crank == 0) mbar_expect_tx(full_bar(s), 2 * (kABytes + box_bytes));
-            const uint32_t fb = tc_map_to_rank(full_bar(s), 0);
-            tma_load_2d_pair(dst, &map_w, (kb0 + kb) * kBK, n0, fb);
-            tma_load_2d_pair(dst + kABytes, &map_x, (kb0 + kb) * kBK, a.x_row0 + m0 + static_cast<int>(crank) * (bn / 2), fb);
+            tma_load_2d_pair(dst + kABytes, &map_x, (kb0 + kb) * kBK, a.x_row0 + m0 + static_cast<int>(crank) * (bn / 2),
+                             tc_map_to_rank(full_bar(s), 0));
           } else {
-            mbar_expect_tx(full_bar(s), kStageBytes);
-            tma_load_2d(dst, &map_w, kb * kBK, n0, full_bar(s));
             tma_load_2d(dst + kABytes, &map_x, kb * kBK, a.x_row0 + m0, full_bar(s));
             tma_load_2d(dst + kABytes + (kPBN / 2) * kBK * 2, &map_x, kb * kBK, a.x_row0 + m0 + kPBN / 2, full_bar(s));
           }
@@ -1034,24 +1048,25 @@ cudaError_t launch_tc_persist(const CUtensorMap& mw, const CUtensorMap& mx, cons
     const int nk = (a.K + kBK - 1) / kBK, ks = a.partial ? a.ksplit : 1;
     if (ks < 1 || (ks - 1) * ((nk + ks - 1) / ks) >= nk) return cudaErrorInvalidValue;
     const int total = (a.M + b.bn - 1) / b.bn * ((a.N + 2 * kBM - 1) / (2 * kBM)) * ks;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(2 * std::min(total, sms_of[dev] / 2)));
     cfg.blockDim = dim3(kPThreads);
     cfg.dynamicSmemBytes = smem_pair;
     cfg.stream = s;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = a.chained ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, gemm_tc_persist_kernel<EPI, true>, mw, b.x_box == 64 ? *mx64 : mx, b);
   }
   if (a.partial) return cudaErrorInvalidValue;
   const int total = (a.M + kPBN - 1) / kPBN * ((a.N + kBM - 1) / kBM);
-  gemm_tc_persist_kernel<EPI, false><<<std::min(total, sms_of[dev]), kPThreads, smem, s>>>(mw, mx, a);
-  return cudaGetLastError();
+  return launch_pdl(gemm_tc_persist_kernel<EPI, false>, dim3(std::min(total, sms_of[dev])), dim3(kPThreads), smem, s, a.chained != 0, mw, mx, a);
 }
 
 }  // namespace

@@ -161,7 +161,7 @@ struct PrefillAttnArgs {
   __nv_bfloat16* out_bf16;     // bf16 destination (operand of the tensor-core out-proj); exactly one is set
   int ld_out;
 };
-cudaError_t launch_prefill_attn(const PrefillAttnArgs& a, cudaStream_t s);
+cudaError_t launch_prefill_attn(const PrefillAttnArgs& a, cudaStream_t s, bool pdl);
 
 // Tensor-core causal attention for prefill / eval, d_head = 256 (see mtj_attn_tc.cu).
 struct PrefillAttnTcArgs {
@@ -182,6 +182,7 @@ struct PrefillAttnTcArgs {
   // paged rows (launch_prefill_attn_tc_grouped): kv.page_table, kv.ring_pages and kv.pad, window, v_cols, scale_log2, and
   int kv_group;                // query heads per key head
   int k_cols, v_ld;            // columns of a key head in the key and value rows, multiples of 8
+  int chained;                 // launched programmatically behind the kernel before it
 };
 cudaError_t launch_prefill_attn_tc(const void* map_q, const void* map_k, const void* map_v,
                                    const PrefillAttnTcArgs& a, cudaStream_t s);
@@ -301,6 +302,7 @@ struct GemmTcArgs {
                                // to out_bf16; 0: every row to both
   float softcap;               // kEpiSoftcap
   int pair;                    // wide kernel only: 1 = clusters of 2 blocks on 256 x 256 tiles (tcgen05 cta_group::2)
+  int chained;                 // wide kernel only: launched programmatically behind the kernel before it
   int bn, x_box, stages;       // wide kernel with pair: token rows per tile and of the activation box, ring stages; set by the launch
   uint32_t* dev_err;
 };

@@ -614,6 +614,8 @@ __global__ void __launch_bounds__(kThreads, RT > 1 && RT <= 4 && KC <= 2 ? 3 : 1
 // [own columns, padded | rotated columns, padded].
 template <typename T>
 __global__ void __launch_bounds__(kThreads) latent_pack_kernel(const LatentArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float red[kThreads / 32];
   const int m = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hd = a.dim + a.rot;
   int seq;
@@ -660,6 +662,8 @@ __global__ void __launch_bounds__(kThreads) latent_pack_kernel(const LatentArgs 
 
 template <typename T>
 __global__ void __launch_bounds__(128) latent_history_kernel(const LatentArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int i = blockIdx.x, b = blockIdx.y, seq = a.rows.b0 + b;
   const int p = a.rows.pos0_host - a.hist + i - a.pad[seq];
   const size_t lin = static_cast<size_t>(b) * a.key_rows + i;
@@ -760,19 +764,17 @@ cudaError_t launch_latent_out(const LatentArgs& a, cudaStream_t s, bool pdl) {
   return kc == 1 ? go(latent_out_kernel<16, 1>, 16) : go(latent_out_kernel<16, 2>, 16);
 }
 
-cudaError_t launch_latent_pack(const LatentArgs& a, cudaStream_t s) {
+cudaError_t launch_latent_pack(const LatentArgs& a, cudaStream_t s, bool pdl) {
   if (!latent_ok(a) || a.kr_ld < a.rot || a.key_rows < a.hist + a.rows.Tc) return cudaErrorInvalidValue;
-  if (a.cache.f32) latent_pack_kernel<float><<<a.M, kThreads, 0, s>>>(a);
-  else latent_pack_kernel<__nv_bfloat16><<<a.M, kThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  return a.cache.f32 ? launch_pdl(latent_pack_kernel<float>, dim3(a.M), dim3(kThreads), 0, s, pdl, a)
+                     : launch_pdl(latent_pack_kernel<__nv_bfloat16>, dim3(a.M), dim3(kThreads), 0, s, pdl, a);
 }
 
-cudaError_t launch_latent_history(const LatentArgs& a, cudaStream_t s) {
+cudaError_t launch_latent_history(const LatentArgs& a, cudaStream_t s, bool pdl) {
   if (a.hist <= 0) return cudaSuccess;
   if (!latent_ok(a) || a.nseq <= 0 || a.rows.pos0_dev) return cudaErrorInvalidValue;
-  if (a.cache.f32) latent_history_kernel<float><<<dim3(a.hist, a.nseq), 128, 0, s>>>(a);
-  else latent_history_kernel<__nv_bfloat16><<<dim3(a.hist, a.nseq), 128, 0, s>>>(a);
-  return cudaGetLastError();
+  return a.cache.f32 ? launch_pdl(latent_history_kernel<float>, dim3(a.hist, a.nseq), dim3(128), 0, s, pdl, a)
+                     : launch_pdl(latent_history_kernel<__nv_bfloat16>, dim3(a.hist, a.nseq), dim3(128), 0, s, pdl, a);
 }
 
 }  // namespace mtj

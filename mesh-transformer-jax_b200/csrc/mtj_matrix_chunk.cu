@@ -152,6 +152,8 @@ __device__ __forceinline__ float4 four(const __nv_bfloat16* p, int n, int have, 
 // One block of 4 warps per (chunk, head).
 template <int DP>
 __global__ void __launch_bounds__(128) delta_prep_kernel(const MatrixStateArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   using Rec = Record<DP>;
   extern __shared__ __align__(16) unsigned char dp_smem[];
   PrepSmem<DP>& sm = *reinterpret_cast<PrepSmem<DP>*>(dp_smem);
@@ -345,6 +347,8 @@ __global__ void __launch_bounds__(32 * (2 * NG + 1)) delta_chunk_kernel(const Ma
     failed = 0;
   }
   __syncthreads();
+  pdl_wait();
+  pdl_launch_dependents();
   const MsSpan sp = ms_span(a, blockIdx.z);
   const int chunks = (sp.n + kC - 1) / kC, c0 = blockIdx.y * 16 * NG;
   if (warp == NW) {
@@ -526,6 +530,8 @@ __device__ __forceinline__ void fetch_rows(__nv_bfloat16* dst, int LD, const __n
 // One block of 4 warps per (chunk, key head): C B^T once, then the records of the heads that share it.
 template <int DP>
 __global__ void __launch_bounds__(128) ssd_prep_kernel(const MatrixStateArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   constexpr int LD = DP + 8;
   __shared__ __align__(16) __nv_bfloat16 tile[2][kC * LD];           // B, C
   const int chunk = blockIdx.x, kh = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -624,6 +630,8 @@ __global__ void __launch_bounds__(32 * (2 * NG + 1)) ssd_chunk_kernel(const Matr
     failed = 0;
   }
   __syncthreads();
+  pdl_wait();
+  pdl_launch_dependents();
   const MsSpan sp = ms_span(a, blockIdx.z);
   const int chunks = (sp.n + kC - 1) / kC, c0 = blockIdx.y * 16 * NG;
   if (warp == NW) {
@@ -741,50 +749,46 @@ cudaError_t allow_smem(DeviceOnce& once, K kernel, int bytes) {
 }
 
 template <int DP, int NG>
-cudaError_t delta_cols(const MatrixStateArgs& a, int chunks, cudaStream_t s) {
+cudaError_t delta_cols(const MatrixStateArgs& a, int chunks, cudaStream_t s, bool pdl) {
   constexpr int smem = kRing * Record<DP>::kBytes;
   static_assert(smem <= 200 * 1024 && Record<DP>::kBytes % 16 == 0, "shared memory");
   static DeviceOnce once;
   cudaError_t e = allow_smem(once, delta_chunk_kernel<DP, NG>, smem);
   if (e != cudaSuccess) return e;
-  delta_chunk_kernel<DP, NG><<<dim3(a.heads, (a.vdim + 16 * NG - 1) / (16 * NG), a.nseq), 32 * (2 * NG + 1), smem, s>>>(a, chunks);
-  return cudaGetLastError();
+  return launch_pdl(delta_chunk_kernel<DP, NG>, dim3(a.heads, (a.vdim + 16 * NG - 1) / (16 * NG), a.nseq), dim3(32 * (2 * NG + 1)), smem, s, pdl, a, chunks);
 }
 
 template <int DP>
-cudaError_t delta(const MatrixStateArgs& a, cudaStream_t s) {
+cudaError_t delta(const MatrixStateArgs& a, cudaStream_t s, bool pdl) {
   constexpr int prep = static_cast<int>(sizeof(PrepSmem<DP>));
   static DeviceOnce once;
   cudaError_t e = allow_smem(once, delta_prep_kernel<DP>, prep);
   if (e != cudaSuccess) return e;
   const int chunks = (a.rows.Tc + kC - 1) / kC;
-  delta_prep_kernel<DP><<<dim3(chunks, a.heads, a.nseq), 128, prep, s>>>(a);
-  e = cudaGetLastError();
+  e = launch_pdl(delta_prep_kernel<DP>, dim3(chunks, a.heads, a.nseq), dim3(128), prep, s, pdl, a);
   if (e != cudaSuccess) return e;
   // as few columns per block as still give every SM a block
   const int64_t cols = static_cast<int64_t>(a.heads) * a.nseq * ((a.vdim + 15) / 16);
-  return cols <= 148 * 2 ? delta_cols<DP, 2>(a, chunks, s) : delta_cols<DP, 4>(a, chunks, s);
+  return cols <= 148 * 2 ? delta_cols<DP, 2>(a, chunks, s, pdl) : delta_cols<DP, 4>(a, chunks, s, pdl);
 }
 
 template <int DP, int NG>
-cudaError_t ssd_cols(const MatrixStateArgs& a, int chunks, cudaStream_t s) {
+cudaError_t ssd_cols(const MatrixStateArgs& a, int chunks, cudaStream_t s, bool pdl) {
   constexpr int smem = 4 * (SsdTiles<DP>::kBytes + SsdRecord::kBytes);
   static_assert(smem <= 200 * 1024 && SsdTiles<DP>::kBytes % 16 == 0, "shared memory");
   static DeviceOnce once;
   cudaError_t e = allow_smem(once, ssd_chunk_kernel<DP, NG>, smem);
   if (e != cudaSuccess) return e;
-  ssd_chunk_kernel<DP, NG><<<dim3(a.heads, (a.vdim + 16 * NG - 1) / (16 * NG), a.nseq), 32 * (2 * NG + 1), smem, s>>>(a, chunks);
-  return cudaGetLastError();
+  return launch_pdl(ssd_chunk_kernel<DP, NG>, dim3(a.heads, (a.vdim + 16 * NG - 1) / (16 * NG), a.nseq), dim3(32 * (2 * NG + 1)), smem, s, pdl, a, chunks);
 }
 
 template <int DP>
-cudaError_t ssd(const MatrixStateArgs& a, cudaStream_t s) {
+cudaError_t ssd(const MatrixStateArgs& a, cudaStream_t s, bool pdl) {
   const int chunks = (a.rows.Tc + kC - 1) / kC;
-  ssd_prep_kernel<DP><<<dim3(chunks, a.key_heads, a.nseq), 128, 0, s>>>(a);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pdl(ssd_prep_kernel<DP>, dim3(chunks, a.key_heads, a.nseq), dim3(128), 0, s, pdl, a);
   if (e != cudaSuccess) return e;
   const int64_t cols = static_cast<int64_t>(a.heads) * a.nseq * ((a.vdim + 15) / 16);
-  return cols <= 148 * 2 ? ssd_cols<DP, 2>(a, chunks, s) : ssd_cols<DP, 4>(a, chunks, s);
+  return cols <= 148 * 2 ? ssd_cols<DP, 2>(a, chunks, s, pdl) : ssd_cols<DP, 4>(a, chunks, s, pdl);
 }
 
 }  // namespace
@@ -795,11 +799,11 @@ int64_t matrix_chunk_bytes(int heads, int key_heads, int dim, int delta) {
   return h * SsdRecord::kBytes + g * (dim <= 32 ? SsdTiles<32>::kBytes : dim <= 64 ? SsdTiles<64>::kBytes : dim <= 128 ? SsdTiles<128>::kBytes : SsdTiles<256>::kBytes);
 }
 
-cudaError_t launch_matrix_chunks(const MatrixStateArgs& a, cudaStream_t s) {
+cudaError_t launch_matrix_chunks(const MatrixStateArgs& a, cudaStream_t s, bool pdl) {
   if (!matrix_state_ok(a) || !a.u_bf16 || a.nseq > 65535 || a.heads > 65535) return cudaErrorInvalidValue;
   if (!a.chunk_records || (reinterpret_cast<uintptr_t>(a.chunk_records) & 15)) return cudaErrorInvalidValue;
-  if (a.delta) return a.dim <= 32 ? delta<32>(a, s) : a.dim <= 64 ? delta<64>(a, s) : a.dim <= 128 ? delta<128>(a, s) : delta<256>(a, s);
-  return a.dim <= 32 ? ssd<32>(a, s) : a.dim <= 64 ? ssd<64>(a, s) : a.dim <= 128 ? ssd<128>(a, s) : ssd<256>(a, s);
+  if (a.delta) return a.dim <= 32 ? delta<32>(a, s, pdl) : a.dim <= 64 ? delta<64>(a, s, pdl) : a.dim <= 128 ? delta<128>(a, s, pdl) : delta<256>(a, s, pdl);
+  return a.dim <= 32 ? ssd<32>(a, s, pdl) : a.dim <= 64 ? ssd<64>(a, s, pdl) : a.dim <= 128 ? ssd<128>(a, s, pdl) : ssd<256>(a, s, pdl);
 }
 
 }  // namespace mtj

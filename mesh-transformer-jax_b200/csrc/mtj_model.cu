@@ -204,7 +204,7 @@ int32_t run_layer(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, bool
     p.out = h->act2;
     p.ld_out = h->dl + h->ffl;
     h->prof_begin(MTJ_FAMILY_ATTN, s);
-    MTJ_CUDA(mtj::launch_prefill_attn(p, s));
+    MTJ_CUDA(mtj::launch_prefill_attn(p, s, false));
     h->prof_end(s);
   }
   h->launches++;
@@ -281,9 +281,9 @@ OutPlan plan_out(const mtj_handle* h, int M, bool wide, bool to_slot, bool detac
 int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, const int32_t* key_limit,
                      cudaStream_t s, float* detached_out = nullptr, bool decode = false, bool defer_reduce = false, bool chain = false) {
   LayerWeights& lw = h->layers[layer];
-  // decode (graph-replayed, launch-latency sensitive): every kernel of the chain waits on its predecessor with
-  // griddepcontrol.wait, so each may be scheduled while the previous one drains
-  const bool pdl = h->use_pdl && h->tc_pdl && decode;
+  // every kernel of the chain waits on its predecessor with griddepcontrol.wait, so each may be scheduled while the previous
+  // one drains (prompts too: 2 us less between their kernels; shards run prompts on two streams, there kernels meet by events)
+  const bool pdl = h->use_pdl && h->tc_pdl && (decode || h->mp == 1);
   // few sequences: activations go through the GEMMs as hi + lo bf16 pairs
   const bool hilo = decode && h->hilo_ok && M <= h->tc_hilo_max_b;
   if (h->xn_ready) {
@@ -314,6 +314,7 @@ int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, c
   h->prof_begin(MTJ_FAMILY_INPROJ, s);
   const bool wide = !decode && use_tc_wide(h, M, h->same_sums);
   a.pair = h->tc_pair & 1;
+  a.chained = pdl;
   if (wide)
     MTJ_CUDA(mtj::launch_gemm_tc_wide(mtj::kEpiInProj, &lw.map_in, &h->map_xn_wide, &h->map_xn[1], a, s));
   else
@@ -353,6 +354,7 @@ int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, c
     p.out_bf16 = h->act_bf16;
     p.ld_out = h->dl + h->ffl;
     p.dev_err = h->dev_err;
+    p.chained = pdl;
     MTJ_CUDA(mtj::launch_prefill_attn_tc(&h->map_q, &lw.map_k, &lw.map_v, p, s));
   } else {
     mtj::PrefillAttnArgs p = {};
@@ -365,7 +367,7 @@ int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, c
     p.key_limit = key_limit;
     p.out_bf16 = h->act_bf16;
     p.ld_out = h->dl + h->ffl;
-    MTJ_CUDA(mtj::launch_prefill_attn(p, s));
+    MTJ_CUDA(mtj::launch_prefill_attn(p, s, pdl));
   }
   h->prof_end(s);
 
@@ -379,6 +381,7 @@ int32_t run_layer_tc(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, c
   o.out = h->mp == 1 ? (detached_out ? detached_out : h->x) : (to_slot ? partial_dst(h, M) : h->part);
   o.ld_out = h->d;
   o.dev_err = h->dev_err;
+  o.chained = pdl;
   const OutPlan plan = plan_out(h, M, wide, to_slot, detached_out != nullptr, h->same_sums);
   const bool wide_out = plan.wide;
   const int ksplit = plan.pieces;
@@ -538,7 +541,7 @@ int32_t run_embed(mtj_handle* h, const uint32_t* ids, int ids_ld, int M, const m
     e.slot_stride = partial_slot_stride(h);
   }
   e.stats = h->mp == 1 ? h->stats : nullptr;
-  MTJ_CUDA(mtj::launch_embed(e, s, h->use_pdl && decode));
+  MTJ_CUDA(mtj::launch_embed(e, s, h->use_pdl && (decode || h->mp == 1)));
   h->launches++;
   if (push) {
     const bool hilo = h->hilo_ok && M <= h->tc_hilo_max_b;

@@ -331,6 +331,8 @@ __global__ void __launch_bounds__(96) ssm_scan_kernel(const SsmArgs a) {
   const int c0 = blockIdx.x * CW;
   const int tiles = (sp.n + kTT - 1) / kTT;
   for (int i = threadIdx.x; i < static_cast<int>(sizeof(sm.tile) / 4); i += 96) reinterpret_cast<float*>(sm.tile)[i] = 0.f;   // padded states stay zero
+  pdl_wait();
+  pdl_launch_dependents();
   __syncthreads();
   if (warp == 0) {
     const int ch = lane / G, g = lane % G, c = c0 + ch;
@@ -576,7 +578,7 @@ bool conv_ok(const SsmArgs& a) {
 bool ssm_ok(const SsmArgs& a) { return conv_ok(a) && a.state > 0 && a.state <= kSsmMaxState; }
 
 template <typename T, int G, int NS>
-cudaError_t scan(const SsmArgs& a, cudaStream_t s) {
+cudaError_t scan(const SsmArgs& a, cudaStream_t s, bool pdl) {
   constexpr int smem = static_cast<int>(sizeof(ScanSmem<T, G, NS>)), CW = 32 / G;
   static_assert(smem <= 220 * 1024, "shared memory");
   static DeviceOnce once;
@@ -584,17 +586,16 @@ cudaError_t scan(const SsmArgs& a, cudaStream_t s) {
     return cudaFuncSetAttribute(ssm_scan_kernel<T, G, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   });
   if (e != cudaSuccess) return e;
-  ssm_scan_kernel<T, G, NS><<<dim3((a.inner + CW - 1) / CW, a.nseq), 96, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_pdl(ssm_scan_kernel<T, G, NS>, dim3((a.inner + CW - 1) / CW, a.nseq), dim3(96), smem, s, pdl, a);
 }
 
 template <typename T>
-cudaError_t scan_states(const SsmArgs& a, cudaStream_t s) {
-  if (a.state <= 16) return scan<T, 4, 4>(a, s);
-  if (a.state <= 32) return scan<T, 8, 4>(a, s);
-  if (a.state <= 64) return scan<T, 16, 4>(a, s);
-  if (a.state <= 128) return scan<T, 32, 4>(a, s);
-  return scan<T, 32, 8>(a, s);
+cudaError_t scan_states(const SsmArgs& a, cudaStream_t s, bool pdl) {
+  if (a.state <= 16) return scan<T, 4, 4>(a, s, pdl);
+  if (a.state <= 32) return scan<T, 8, 4>(a, s, pdl);
+  if (a.state <= 64) return scan<T, 16, 4>(a, s, pdl);
+  if (a.state <= 128) return scan<T, 32, 4>(a, s, pdl);
+  return scan<T, 32, 8>(a, s, pdl);
 }
 
 template <typename T, int G, bool VEC>
@@ -654,9 +655,9 @@ cudaError_t launch_ssm_split(const SsmArgs& a, cudaStream_t s, bool pdl) {
   return launch_pdl(ssm_split_kernel, dim3(a.M, (a.dt_rank + 2 * a.state + 63) / 64), dim3(64), 0, s, pdl, a);
 }
 
-cudaError_t launch_ssm_scan(const SsmArgs& a, cudaStream_t s) {
+cudaError_t launch_ssm_scan(const SsmArgs& a, cudaStream_t s, bool pdl) {
   if (!ssm_ok(a) || !a.dt_raw || (a.ld_u & 7) || (a.ld_xz & 7) || (a.z0 & 7)) return cudaErrorInvalidValue;
-  return a.xz_bf16 ? scan_states<__nv_bfloat16>(a, s) : scan_states<float>(a, s);
+  return a.xz_bf16 ? scan_states<__nv_bfloat16>(a, s, pdl) : scan_states<float>(a, s, pdl);
 }
 
 cudaError_t launch_ssm_step(const SsmArgs& a, cudaStream_t s, bool pdl) {

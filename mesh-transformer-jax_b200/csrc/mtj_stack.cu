@@ -556,6 +556,11 @@ int32_t LayerStack::load_param(mtj_handle* h, const std::string& name, const voi
   return MTJ_OK;
 }
 
+namespace {
+// Kernels chained by programmatic launch (without it, 2 to 3 us between the kernels of a pass).
+bool chained(const mtj_handle* h, bool tc) { return h->use_pdl && (!tc || h->tc_pdl); }
+}  // namespace
+
 // ------------------------------------------------------------------------------------------------- linear maps
 bool LayerStack::use_tc(const mtj_handle* h, int M, bool decode) const {
   return !f32_ && M >= (decode ? h->tc_decode_min_b : tc_min_rows_);
@@ -603,9 +608,10 @@ int32_t LayerStack::gemm(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
   a.softcap = softcap_;
   a.f32_from = f32_from;
   a.pair = 1;
+  a.chained = chained(h, true);
   a.cluster_k = h->tc_cluster_k ? gemm_tc_decode_cluster_k(l.N, M, l.K) : 1;
   if (wide) MTJ_CUDA(launch_gemm_tc_wide(epi, &l.map, mx, xmap(x, l.K, ldx, 64), a, s));
-  else MTJ_CUDA(launch_gemm_tc(epi, &l.map, mx, a, s, decode && h->use_pdl && h->tc_pdl));
+  else MTJ_CUDA(launch_gemm_tc(epi, &l.map, mx, a, s, chained(h, true)));
   h->launches++;
   return MTJ_OK;
 }
@@ -652,8 +658,9 @@ int32_t LayerStack::gemm_out(mtj_handle* h, const Linear& l, int M, bool decode,
   a.ksplit = ks;
   a.dev_err = h->dev_err;
   a.pair = 1;
+  a.chained = chained(h, true);
   if (wide) MTJ_CUDA(launch_gemm_tc_wide(kEpiPlain, &l.map, mx, xmap(act_bf_, l.K, l.ld, 64), a, s));
-  else MTJ_CUDA(launch_gemm_tc(kEpiPlain, &l.map, mx, a, s, decode && h->use_pdl && h->tc_pdl));
+  else MTJ_CUDA(launch_gemm_tc(kEpiPlain, &l.map, mx, a, s, chained(h, true)));
   h->launches++;
   return MTJ_OK;
 }
@@ -673,7 +680,7 @@ int32_t LayerStack::gemm_planes(mtj_handle* h, const Linear& l, const __nv_bfloa
   a.partial = xp_planes_;
   a.ksplit = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({fit, 296 / tiles, (l.K + 127) / 128, 16})));
   a.dev_err = h->dev_err;
-  MTJ_CUDA(launch_gemm_tc(kEpiPlain, &l.map, key, a, s, decode && h->use_pdl && h->tc_pdl));
+  MTJ_CUDA(launch_gemm_tc(kEpiPlain, &l.map, key, a, s, chained(h, true)));
   h->launches++;
   *planes = a.ksplit;
   return MTJ_OK;
@@ -760,11 +767,6 @@ int32_t LayerStack::gemv(mtj_handle* h, GemvEpilogue epi, const Linear& l, const
     if (_rc) return _rc;                   \
   } while (0)
 
-namespace {
-// Kernels chained by programmatic launch: in decode, and wherever few rows make a pass of 47 short kernels (5 to 20 rows of
-// width 2048: 3 us between kernels without).
-bool chained(const mtj_handle* h, bool tc, bool decode) { return h->use_pdl && (decode || !tc); }
-}  // namespace
 
 int32_t LayerStack::project_in(mtj_handle* h, const Linear& l, int M, float* out, int ld_out, bool pdl, cudaStream_t s) {
   return gemv(h, kEpiOut, l, post_ln_ ? x_ : xn_, ld_, M, out, ld_out, nullptr, pdl, s);
@@ -773,7 +775,7 @@ int32_t LayerStack::project_in(mtj_handle* h, const Linear& l, int M, float* out
 int32_t LayerStack::mamba(mtj_handle* h, const Run& r, int M, const RowMap& rows, bool tc, bool decode, const Post& post, cudaStream_t s) {
   Layer& l = layers_[r.layer];
   const mtj_layer_desc& m = l.d;
-  const bool pdl = chained(h, tc, decode);
+  const bool pdl = chained(h, tc);
   SsmArgs a = {};
   a.M = M;
   a.inner = m.inner;
@@ -832,7 +834,7 @@ int32_t LayerStack::mamba(mtj_handle* h, const Run& r, int M, const RowMap& rows
     }
   }
   if (rows.Tc == 1) MTJ_CUDA(launch_ssm_step(a, s, pdl));
-  else MTJ_CUDA(launch_ssm_scan(a, s));
+  else MTJ_CUDA(launch_ssm_scan(a, s, pdl));
   h->launches++;
   h->prof_end(s);
   h->prof_begin(MTJ_FAMILY_OUTPROJ, s);
@@ -846,7 +848,7 @@ int32_t LayerStack::latent(mtj_handle* h, const Run& r, int M, const RowMap& row
                            cudaStream_t s) {
   Layer& l = layers_[r.layer];
   const mtj_layer_desc& m = l.d;
-  const bool pdl = chained(h, tc, decode);
+  const bool pdl = chained(h, tc);
   LatentArgs a = {};
   a.M = M;
   a.heads = m.heads;
@@ -885,8 +887,8 @@ int32_t LayerStack::latent(mtj_handle* h, const Run& r, int M, const RowMap& row
     a.nseq = M / rows.Tc;
     a.hist = std::min(hist, m.window - 1);
     a.key_rows = a.hist + rows.Tc;
-    MTJ_CUDA(launch_latent_pack(a, s));
-    MTJ_CUDA(launch_latent_history(a, s));
+    MTJ_CUDA(launch_latent_pack(a, s, pdl));
+    MTJ_CUDA(launch_latent_history(a, s, pdl));
     MTJ_DO(gemm(h, kEpiPlain, l.up, c_lin_, a.nseq * a.key_rows, nullptr, 0, kv_lin_, l.up.N, decode, s));
     PrefillAttnTcArgs p = {};
     p.kv.pad = h->pad;
@@ -902,6 +904,7 @@ int32_t LayerStack::latent(mtj_handle* h, const Run& r, int M, const RowMap& row
     p.k_own = l.k_own;
     p.v_cols = m.vdim;
     p.scale_log2 = m.scale * 1.4426950408889634f;
+    p.chained = pdl;
     MTJ_CUDA(launch_prefill_attn_tc_linear(&l.map_q, &l.map_k, &l.map_kr, &l.map_v, l.key_blocks, l.value_blocks, p, s));
     h->launches += a.hist > 0 ? 3 : 2;
   } else {
@@ -935,7 +938,7 @@ int32_t LayerStack::latent(mtj_handle* h, const Run& r, int M, const RowMap& row
 int32_t LayerStack::grouped(mtj_handle* h, const Run& r, int M, const RowMap& rows, bool tc, bool decode, const Post& post, cudaStream_t s) {
   Layer& l = layers_[r.layer];
   const mtj_layer_desc& m = l.d;
-  const bool pdl = chained(h, tc, decode);
+  const bool pdl = chained(h, tc);
   GroupedAttnArgs a = {};
   a.M = M;
   a.heads = m.heads;
@@ -986,6 +989,7 @@ int32_t LayerStack::grouped(mtj_handle* h, const Run& r, int M, const RowMap& ro
     p.v_ld = l.v_cols;
     p.v_cols = m.vdim;
     p.scale_log2 = m.scale * 1.4426950408889634f;
+    p.chained = pdl;
     MTJ_CUDA(launch_prefill_attn_tc_grouped(&l.map_q, &r.map_k, &r.map_v, l.key_blocks, l.value_blocks, p, s));
     h->launches++;
   } else {
@@ -1018,7 +1022,7 @@ int32_t LayerStack::grouped(mtj_handle* h, const Run& r, int M, const RowMap& ro
 int32_t LayerStack::matrix(mtj_handle* h, const Run& r, int M, const RowMap& rows, bool tc, bool decode, const Post& post, cudaStream_t s) {
   Layer& l = layers_[r.layer];
   const mtj_layer_desc& m = l.d;
-  const bool pdl = chained(h, tc, decode), ssd = m.mixer == MTJ_MIXER_MATRIX_STATE_SSD;
+  const bool pdl = chained(h, tc), ssd = m.mixer == MTJ_MIXER_MATRIX_STATE_SSD;
   const int ld_p = up8(l.in.N), inner = m.heads * m.vdim, keys = m.kv_heads * m.dim;
   // the input projection: convolution inputs, gates and low-rank parts in bf16, step sizes and update strengths in fp32
   const float* aux = tc ? aux_ : p1_ + l.aux0;
@@ -1104,7 +1108,7 @@ int32_t LayerStack::matrix(mtj_handle* h, const Run& r, int M, const RowMap& row
   g.ld_out = l.out.ld;
   const bool step = matrix_step_ok(a), normed = step && matrix_step_norms(a);
   if (step) MTJ_CUDA(launch_matrix_step(a, normed ? &g : nullptr, s, pdl));
-  else if (tc && rows.Tc >= kChunkedRows) MTJ_CUDA(launch_matrix_chunks(a, s));
+  else if (tc && rows.Tc >= kChunkedRows) MTJ_CUDA(launch_matrix_chunks(a, s, pdl));
   else MTJ_CUDA(launch_matrix_scan(a, s, pdl));
   if (!normed) MTJ_CUDA(launch_gated_norm(g, s, pdl));
   h->launches += (normed ? 1 : 2) + (!step && tc && rows.Tc >= kChunkedRows ? 1 : 0);
@@ -1120,7 +1124,7 @@ int32_t LayerStack::matrix(mtj_handle* h, const Run& r, int M, const RowMap& row
 int32_t LayerStack::forward(mtj_handle* h, const uint32_t* ids, int ids_ld, const RowMap& id_rows, int M, const RowMap& rows,
                             int hist, bool decode, cudaStream_t s) {
   if (M <= 0 || M > R_ || M % rows.Tc) return fail(MTJ_ERR_INVALID, "rows exceed max_rows");
-  const bool tc = use_tc(h, M, decode), pdl = chained(h, tc, decode);
+  const bool tc = use_tc(h, M, decode), pdl = chained(h, tc);
   last_tc_ = tc;
   EmbedArgs e = {};
   e.ids = ids;

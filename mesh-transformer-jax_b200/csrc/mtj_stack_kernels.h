@@ -97,8 +97,8 @@ cudaError_t launch_latent_attn(const LatentArgs& a, cudaStream_t s, bool pdl);
 cudaError_t launch_latent_out(const LatentArgs& a, cudaStream_t s, bool pdl);
 // the same caching, with the queries packed for the tensor-core attention and the latents copied to c_lin / kr_lin;
 // the second fills the history rows from the cache
-cudaError_t launch_latent_pack(const LatentArgs& a, cudaStream_t s);
-cudaError_t launch_latent_history(const LatentArgs& a, cudaStream_t s);
+cudaError_t launch_latent_pack(const LatentArgs& a, cudaStream_t s, bool pdl);
+cudaError_t launch_latent_history(const LatentArgs& a, cudaStream_t s, bool pdl);
 constexpr int kLatentMaxRank = 1024;
 constexpr int kLatentBlocks = 592;       // most (rows x splits x head groups) a call spreads over beyond one per row
 int latent_attn_splits(int M, int heads, int row_ld, int tensor_cores, int window);
@@ -191,7 +191,7 @@ bool matrix_step_norms(const MatrixStateArgs& a);
 // ---- mtj_matrix_chunk.cu: the same over long prompts, in chunks on the tensor cores (bf16 operands)
 constexpr int kMatrixChunk = 16;
 int64_t matrix_chunk_bytes(int heads, int key_heads, int dim, int delta);     // of chunk_records, per chunk of a sequence
-cudaError_t launch_matrix_chunks(const MatrixStateArgs& a, cudaStream_t s);
+cudaError_t launch_matrix_chunks(const MatrixStateArgs& a, cudaStream_t s, bool pdl);
 cudaError_t launch_gated_norm(const GatedNormArgs& a, cudaStream_t s, bool pdl);
 constexpr int kMatrixMaxDim = 256;
 
@@ -231,7 +231,7 @@ struct SsmArgs {
 cudaError_t launch_ssm_conv(const SsmArgs& a, cudaStream_t s, bool pdl);
 cudaError_t launch_ssm_split(const SsmArgs& a, cudaStream_t s, bool pdl);
 // the recurrence over the rows of every sequence, from and to ssm_state, with the gate
-cudaError_t launch_ssm_scan(const SsmArgs& a, cudaStream_t s);
+cudaError_t launch_ssm_scan(const SsmArgs& a, cudaStream_t s, bool pdl);
 // one row per sequence: step size, recurrence and gate in one kernel
 cudaError_t launch_ssm_step(const SsmArgs& a, cudaStream_t s, bool pdl);
 constexpr int kSsmMaxState = 256;
