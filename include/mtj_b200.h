@@ -304,7 +304,9 @@ int32_t mtj_profile_read(mtj_handle* h, double* ms_sum, int64_t* count, mtj_stre
  * counterpart): enable != 0 makes later steps record, for block 0, the
  * %globaltimer value (ns) at 6 points per layer (before / after the wait for
  * the residual stream, after its in-projection rows, after its attention units,
- * after the wait for all attention + FF-in, after its out-projection rows) and 3
+ * after the wait for all attention + FF-in, after its out-projection rows; where
+ * attention runs beside the products: ..., twice at the start of the FF columns of
+ * the out-projection, at the start of its attention columns, after them) and 3
  * at the end; out (host, n entries, may be NULL) receives the last step's record. */
 int32_t mtj_mega_trace(mtj_handle* h, int32_t enable, uint64_t* out_host, int32_t n, mtj_stream s);
 

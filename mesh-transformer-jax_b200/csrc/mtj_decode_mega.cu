@@ -29,7 +29,7 @@ namespace mtj {
 namespace {
 
 // This file is compiled twice: with 256 threads per block (two blocks per SM), and with MTJ_MEGA_MT=512 (one block
-// of 16 warps per SM) for one sequence on one GPU, where halving the arrivals per grid-wide hand-over is worth
+// of 16 warps per SM) for one sequence on one GPU at widths that mtj_decode_stream.cu leaves to it, where halving the arrivals per grid-wide hand-over is worth
 // 1.2 % of the step; with tensor-parallel slices the wider block loses more in the attention phase than it gains.
 #ifndef MTJ_MEGA_MT
 #define MTJ_MEGA_MT 256
@@ -1042,7 +1042,8 @@ cudaError_t launch_decode_mega(const MegaArgs& a, cudaStream_t s, int* grid_out)
   if (a.world < 1 || a.world > 8 || a.B < 1 || a.B > 4 || (a.d & 255) || a.d > 8192 || (a.dl & 1) || (a.V & 1) || ((3 * a.dl + a.ffl) & 1) ||
       ((a.dl + a.ffl) & 7) || a.max_splits < 1 || (a.dl + a.ffl) * 4 > 200 * 1024)
     return cudaErrorInvalidValue;
-  if (a.world == 1 && a.B == 1 && !getenv("MTJ_MEGA_NARROW")) return launch_decode_mega_wide(a, s, grid_out);
+  if (a.world == 1 && a.B == 1 && !getenv("MTJ_MEGA_NARROW"))
+    return decode_stream_ok(a) ? launch_decode_stream(a, s, grid_out) : launch_decode_mega_wide(a, s, grid_out);
   if (a.dh == 256) {
     if (a.B == 1) return launch_mega_t<1, 256>(a, s, grid_out);
     if (a.B == 2) return launch_mega_t<2, 256>(a, s, grid_out);

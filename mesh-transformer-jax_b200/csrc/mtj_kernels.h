@@ -252,10 +252,14 @@ struct MegaArgs {
   unsigned long long* trace;   // optional [6 L + 3] phase time stamps of block 0 (ns)
   uint32_t* dev_err;
   int wait_limit;              // spins before a wait on a phase counter, flag or packet gives up
+  int part_rows[2];            // set by launch_decode_stream: most FF-in rows or logits, and Q/K/V rows, of a block
 };
 cudaError_t launch_decode_mega(const MegaArgs& a, cudaStream_t s, int* grid_out);
-// the same kernel built with one 512-thread block per SM (one sequence only); launch_decode_mega picks it on one GPU
+// the same kernel built with one 512-thread block per SM (one sequence only); launch_decode_mega picks it on one GPU where decode_stream_ok says no
 cudaError_t launch_decode_mega_wide(const MegaArgs& a, cudaStream_t s, int* grid_out);
+// The same for one sequence on one GPU with the weights on a stream of their own (mtj_decode_stream.cu)
+bool decode_stream_ok(const MegaArgs& a);
+cudaError_t launch_decode_stream(const MegaArgs& a, cudaStream_t s, int* grid_out);
 
 struct ArgmaxArgs {
   const float* logits;         // [B, V]
