@@ -101,7 +101,7 @@ struct GemvArgs {
 
 cudaError_t launch_gemv(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl);
 
-// The same for one row and long weight rows, streamed by one block per SM (mtj_gemv_stream.cu).
+// The same for one row and weights of 25 MB and more, streamed by one block per SM (mtj_gemv_stream.cu).
 bool gemv_stream_ok(GemvEpilogue epi, const GemvArgs& a);
 cudaError_t launch_gemv_stream(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl);
 // The same product for 2 rows and more, fp32 activations and sums (mtj_gemm_rows.cu): every epilogue but those with a norm in
