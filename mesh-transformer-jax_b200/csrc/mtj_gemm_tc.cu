@@ -186,7 +186,7 @@ int gemm_tc_decode_cluster_k(int weight_rows, int M, int K) {
   return ck;
 }
 
-int gemm_tc_token_tile_for(int M) { return M <= 32 ? 32 : (M <= 64 ? 64 : 128); }
+int gemm_tc_token_tile_for(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : (M <= 64 ? 64 : 128); }
 // Rows from which the pair kernel takes over: above 192 always, and from 33 on where a prompt is read (not `same_sums`:
 // decoding, whose kernels are chained, and evaluation, whose sums keep their order).  GPT-J-6B's two projections, us a layer:
 // 56 rows 126 with the small tiles and 87 with it, 136 rows 356 and 98.

@@ -158,14 +158,16 @@ __device__ __forceinline__ float swiglu(float g, float u) { return __fdividef(g,
 // HILO: the activations arrive as two bf16 operands, x = hi + lo (lo = the rounding error of hi), both
 // multiplied into the same accumulator: the product carries the activations to about 16 mantissa bits,
 // which is what keeps few-sequence decode on the tensor cores as accurate as the fp32-activation path.
-template <int BN, int STAGES, int EPI, bool HILO>
+// XR: rows of the activation tile, as many as BN or 16: up to 16 rows (M of UMMA's N = 16; the accumulator's other 16 columns are
+// never stored), which leaves room for one more stage of weights.
+template <int BN, int XR, int STAGES, int EPI, bool HILO>
 __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,
                                                              const __grid_constant__ CUtensorMap map_x,
                                                              const __grid_constant__ CUtensorMap map_xlo,
                                                              const GemmTcArgs a) {
-  constexpr uint32_t kABytes = kBM * kBK * 2, kBBytes = BN * kBK * 2,
+  constexpr uint32_t kABytes = kBM * kBK * 2, kBBytes = XR * kBK * 2,
                      kStageBytes = kABytes + (HILO ? 2 : 1) * kBBytes;
-  constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) |
+  constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(XR >> 3) << 17) |
                               (static_cast<uint32_t>(kBM >> 4) << 24);
   extern __shared__ unsigned char tc_smem_raw[];
   const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;   // swizzled tiles need 1024-byte alignment
@@ -976,13 +978,13 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_persist_kernel(const __g
   if (threadIdx.x == 0 && failed && a.dev_err) atomicOr(a.dev_err, kDevErrTimeout);
 }
 
-template <int BN, int STAGES, int EPI, bool HILO = false>
+template <int XR, int STAGES, int EPI, bool HILO = false>
 cudaError_t launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTcArgs& a, cudaStream_t s, bool pdl,
                       const CUtensorMap* mxlo = nullptr) {
-  constexpr int smem = STAGES * (kBM * kBK * 2 + (HILO ? 2 : 1) * BN * kBK * 2) + 1024;
+  constexpr int BN = XR == 16 ? 32 : XR, smem = STAGES * (kBM * kBK * 2 + (HILO ? 2 : 1) * XR * kBK * 2) + 1024;
   static DeviceOnce once;
   {
-    cudaError_t e = once.run([&] { return cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, EPI, HILO>,
+    cudaError_t e = once.run([&] { return cudaFuncSetAttribute(gemm_tc_kernel<BN, XR, STAGES, EPI, HILO>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
     if (e != cudaSuccess) return e;
   }
@@ -1009,7 +1011,7 @@ cudaError_t launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTc
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, STAGES, EPI, HILO>, mw, mx, mxlo ? *mxlo : mx, a);
+  return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, XR, STAGES, EPI, HILO>, mw, mx, mxlo ? *mxlo : mx, a);
 }
 
 // Token rows per tile of the pair kernel: the fewest tiles of at most 256, as even as 32-row chunks allow.  A k-block

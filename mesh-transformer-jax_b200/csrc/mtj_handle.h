@@ -128,14 +128,14 @@ struct mtj_handle {
   bool tc_ok = false;
   __nv_bfloat16* xn_bf16 = nullptr;   // [max_rows, d] LayerNorm output
   __nv_bfloat16* act_bf16 = nullptr;  // [max_rows, dl + ffl] attention vector | gelu(ff)
-  mtj::TensorMap map_xn[3], map_act[3], map_proj, map_q;   // activation views with 32 / 64 / 128-row boxes
+  mtj::TensorMap map_xn[4], map_act[4], map_proj, map_q;   // activation views with 32 / 64 / 128 / 16-row boxes
   mtj::TensorMap map_xn_wide, map_act_wide;   // boxes of the persistent GEMM's tiles (its low tiles take the 64-row ones)
   __nv_bfloat16* q_bf16 = nullptr;    // [max_rows, dl] rotated queries for the tensor-core attention
   bool attn_tc_ok = false;
   // few-sequence decode: the bf16 rounding errors of the two activation operands (x = hi + lo), rows [0, kHiLoRows)
   __nv_bfloat16* xn_lo = nullptr;
   __nv_bfloat16* act_lo = nullptr;
-  mtj::TensorMap map_xn_lo[2], map_act_lo[2];   // 32 / 64-row boxes
+  mtj::TensorMap map_xn_lo[4], map_act_lo[4];   // the same, without 128 rows
   bool hilo_ok = false;
   int tc_hilo_max_b = mtj::kHiLoRows;    // up to this many sequences the activations travel as hi + lo (mtj_config.hilo_max_batch)
   int wait_limit = 1 << 22;         // iteration limit of the bounded device-side waits (mtj_config.wait_limit)
@@ -213,7 +213,7 @@ struct mtj_handle {
   struct ActView {
     float *x, *stats, *part, *q;
     __nv_bfloat16 *xn_bf16, *act_bf16, *q_bf16;
-    mtj::TensorMap map_xn[3], map_act[3], map_xn_wide, map_act_wide, map_q;
+    mtj::TensorMap map_xn[4], map_act[4], map_xn_wide, map_act_wide, map_q;
   };
   ActView views[2];
   bool views_ok = false;
@@ -225,13 +225,13 @@ struct mtj_handle {
   void save_view(int i) {
     ActView& v = views[i];
     v.x = x; v.stats = stats; v.part = part; v.q = q; v.xn_bf16 = xn_bf16; v.act_bf16 = act_bf16; v.q_bf16 = q_bf16;
-    for (int k = 0; k < 3; ++k) { v.map_xn[k] = map_xn[k]; v.map_act[k] = map_act[k]; }
+    for (int k = 0; k < 4; ++k) { v.map_xn[k] = map_xn[k]; v.map_act[k] = map_act[k]; }
     v.map_xn_wide = map_xn_wide; v.map_act_wide = map_act_wide; v.map_q = map_q;
   }
   void use_view(int i) {
     const ActView& v = views[i];
     x = v.x; stats = v.stats; part = v.part; q = v.q; xn_bf16 = v.xn_bf16; act_bf16 = v.act_bf16; q_bf16 = v.q_bf16;
-    for (int k = 0; k < 3; ++k) { map_xn[k] = v.map_xn[k]; map_act[k] = v.map_act[k]; }
+    for (int k = 0; k < 4; ++k) { map_xn[k] = v.map_xn[k]; map_act[k] = v.map_act[k]; }
     map_xn_wide = v.map_xn_wide; map_act_wide = v.map_act_wide; map_q = v.map_q;
   }
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;

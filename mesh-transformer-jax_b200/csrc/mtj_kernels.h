@@ -312,7 +312,7 @@ struct GemmTcArgs {
 };
 constexpr int64_t kWidePlaneFloats = 148LL * 256 * 256;   // most partial sums of any split launch_gemm_tc_wide: two waves of tiles
 int gemm_tc_token_tile();                 // widest token tile of launch_gemm_tc (128)
-// Token tile launch_gemm_tc uses for M rows (32, 64 or 128): map_x must have been made with this box_rows.
+// Token tile launch_gemm_tc uses for M rows (16, 32, 64 or 128): map_x must have been made with this box_rows.
 int gemm_tc_token_tile_for(int M);
 // Whether M rows go through launch_gemm_tc_wide.
 bool gemm_tc_use_wide(int M, bool same_sums);

@@ -244,7 +244,8 @@ int32_t run_layer(mtj_handle* h, int layer, int M, const mtj::RowMap& rows, bool
   return MTJ_OK;
 }
 
-int tc_tile_index(int M) { return mtj::gemm_tc_token_tile_for(M) == 32 ? 0 : (mtj::gemm_tc_token_tile_for(M) == 64 ? 1 : 2); }
+constexpr int kTileBoxes[4] = {32, 64, 128, 16};                // rows of the boxes of map_xn and its like
+int tc_tile_index(int M) { return static_cast<int>(std::find(kTileBoxes, kTileBoxes + 3, mtj::gemm_tc_token_tile_for(M)) - kTileBoxes); }
 bool use_tc_wide(const mtj_handle* h, int M, bool same_sums) { return h->tc_wide_ok && mtj::gemm_tc_use_wide(M, same_sums); }
 
 // Evaluation's products (mtj_handle::same_sums) for the length of a call, however it ends.
@@ -950,8 +951,8 @@ int32_t mtj_bind_arenas(mtj_handle* h, void* wdev, int64_t wbytes, void* sdev, i
       ok = ok && mtj::make_tensor_map_bf16(&lw.map_out, lw.w_out, h->d, h->dl + h->ffl, 128) == cudaSuccess;
     }
     ok = ok && mtj::make_tensor_map_bf16(&h->map_proj, h->proj_w, h->Vl, h->d, 128) == cudaSuccess;
-    for (int i = 0; i < 3; ++i) {
-      const int box = 32 << i;
+    for (int i = 0; i < 4; ++i) {
+      const int box = kTileBoxes[i];
       ok = ok && mtj::make_tensor_map_bf16(&h->map_xn[i], h->xn_bf16, h->max_rows, h->d, box) == cudaSuccess;
       ok = ok && mtj::make_tensor_map_bf16(&h->map_act[i], h->act_bf16, h->max_rows, h->dl + h->ffl, box) == cudaSuccess;
     }
@@ -962,9 +963,9 @@ int32_t mtj_bind_arenas(mtj_handle* h, void* wdev, int64_t wbytes, void* sdev, i
     {
       const int64_t rl = std::min<int64_t>(h->max_rows, kHiLoRows);
       bool okl = ok;
-      for (int i = 0; i < 2 && okl; ++i) {
-        okl = okl && mtj::make_tensor_map_bf16(&h->map_xn_lo[i], h->xn_lo, rl, h->d, 32 << i) == cudaSuccess;
-        okl = okl && mtj::make_tensor_map_bf16(&h->map_act_lo[i], h->act_lo, rl, h->dl + h->ffl, 32 << i) == cudaSuccess;
+      for (int i : {0, 1, 3}) {
+        okl = okl && mtj::make_tensor_map_bf16(&h->map_xn_lo[i], h->xn_lo, rl, h->d, kTileBoxes[i]) == cudaSuccess;
+        okl = okl && mtj::make_tensor_map_bf16(&h->map_act_lo[i], h->act_lo, rl, h->dl + h->ffl, kTileBoxes[i]) == cudaSuccess;
       }
       h->hilo_ok = okl;
     }
@@ -998,8 +999,8 @@ int32_t mtj_bind_arenas(mtj_handle* h, void* wdev, int64_t wbytes, void* sdev, i
     v.act_bf16 = h->act_bf16 + r0 * (h->dl + h->ffl);
     v.q_bf16 = h->q_bf16 + r0 * h->dl;
     bool ok = r1 >= 1;
-    for (int i = 0; i < 3 && ok; ++i) {
-      const int box = 32 << i;
+    for (int i = 0; i < 4 && ok; ++i) {
+      const int box = kTileBoxes[i];
       ok = ok && mtj::make_tensor_map_bf16(&v.map_xn[i], v.xn_bf16, r1, h->d, box) == cudaSuccess;
       ok = ok && mtj::make_tensor_map_bf16(&v.map_act[i], v.act_bf16, r1, h->dl + h->ffl, box) == cudaSuccess;
     }

@@ -570,13 +570,13 @@ const TensorMap* LayerStack::xmap(const __nv_bfloat16* buf, int K, int ld, int t
   const auto key = std::make_tuple(static_cast<const void*>(buf), K, ld);
   auto it = xmaps_.find(key);
   if (it == xmaps_.end()) {
-    std::array<TensorMap, 3> maps;
+    std::array<TensorMap, 4> maps;                 // boxes of 32, 64, 128 and 16 rows
     const int rows = buf == c_lin_ ? lin_rows_ : R_;
-    for (int i = 0; i < 3; ++i)
-      if (make_tensor_map_bf16(&maps[i], buf, rows, K, 32 << i, ld) != cudaSuccess) return nullptr;
+    for (int i = 0; i < 4; ++i)
+      if (make_tensor_map_bf16(&maps[i], buf, rows, K, i < 3 ? 32 << i : 16, ld) != cudaSuccess) return nullptr;
     it = xmaps_.emplace(key, maps).first;
   }
-  return &it->second[tile == 32 ? 0 : tile == 64 ? 1 : 2];
+  return &it->second[tile == 32 ? 0 : tile == 64 ? 1 : tile == 128 ? 2 : 3];
 }
 
 namespace {

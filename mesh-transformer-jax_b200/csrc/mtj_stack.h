@@ -151,7 +151,7 @@ class LayerStack {
   char* chunk_records_ = nullptr;
   uint32_t *counters_ = nullptr, *attn_counters_ = nullptr;
   int ld_aux_ = 0, ld_mix_ = 0;
-  std::map<std::tuple<const void*, int, int>, std::array<TensorMap, 3>> xmaps_;
+  std::map<std::tuple<const void*, int, int>, std::array<TensorMap, 4>> xmaps_;
 };
 
 }  // namespace mtj
