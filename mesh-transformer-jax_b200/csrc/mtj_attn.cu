@@ -387,8 +387,10 @@ __global__ void __launch_bounds__(kStreamThreads) decode_attn_stream_kernel(cons
         }
         m = m_new;
       }
-      __syncwarp();
-      if (lane == 0) {
+      // the tile is in every lane's registers: which lane hands it back hangs on what the lanes made of it, because an arrival
+      // alone does not wait for loads that nothing has used yet
+      const int by = __any_sync(0xffffffffu, __float_as_uint(o[0]) == 0x7fc0dead || __float_as_uint(m) == 0x7fc0dead) ? 1 : 0;
+      if (lane == by) {
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty_bar(st)) : "memory");
       }
     }

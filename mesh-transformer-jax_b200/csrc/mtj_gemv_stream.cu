@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const Ge
     }
     uint32_t phase = 0;
     int left = 0;                                                // rows of this group in the current stage
+    float before = 0.f;                                          // the sum of the row before
     auto dot = [&]() {
       if (left == 0) {
         ok = __all_sync(0xffffffffu, mbar_wait(full(slot), phase));
@@ -129,17 +130,21 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const Ge
       uint4 v[NCH];
 #pragma unroll
       for (int c = 0; c < NCH; ++c) v[c] = c * 32 + lane < mine ? row[c * 32] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) dot8(c & 1 ? t1 : t0, v[c], x[c]);
+      const float sum = sum2(t0) + sum2(t1);
       if (--left == 0) {
-        __syncwarp();                                            // every lane has read the stage
-        if (lane == 0) arrive(empty(slot));
+        // Every lane has the stage in its registers: which lane hands it back hangs on every lane's sums, because an arrival
+        // alone does not wait for loads that nothing has used yet, and the next rows would land under them.
+        const int by = __any_sync(0xffffffffu, __float_as_uint(sum) == 0x7fc0dead || __float_as_uint(before) == 0x7fc0dead) ? 1 : 0;
+        if (lane == by) arrive(empty(slot));
         if (++slot == ring) {
           slot = 0;
           phase ^= 1u;
         }
       }
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) dot8(c & 1 ? t1 : t0, v[c], x[c]);
-      return sum2(t0) + sum2(t1);
+      before = sum;
+      return sum;
     };
     // two rows' sums at a time: the first in lanes 0 to 15, the second in lanes 16 to 31; a wait that ran out ends the loop
     for (int r = r0 + grp; r < r1; r += 2 * GROUPS) {
