@@ -323,7 +323,12 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ void arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// Hands a stage of a ring back.  a and b are numbers that the warp has made of the stage's last loads: which lane arrives hangs on
+// every lane's, because an arrival alone does not wait for loads that nothing has used yet, and the next copy would land under them.
+__device__ __forceinline__ void hand_back(uint32_t bar, int lane, float a, float b) {
+  const int by = __any_sync(0xffffffffu, __float_as_uint(a) == 0x7fc0dead || __float_as_uint(b) == 0x7fc0dead) ? 1 : 0;
+  if (lane == by) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 
 constexpr int kRing = 3;
 
@@ -471,8 +476,6 @@ __global__ void __launch_bounds__(32 * (2 * NG + 1)) delta_chunk_kernel(const Ma
       }
       ldsm4(bh, r + Rec::kM + os);
       ldsm4(bl, r + Rec::kM + Rec::kSmall + os);
-      __syncwarp();
-      if (lane == 0) arrive(empty + 8 * s);              // the record is read
       float y[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) y[e] = half ? O[0][1][e] : O[0][0][e];
@@ -481,6 +484,7 @@ __global__ void __launch_bounds__(32 * (2 * NG + 1)) delta_chunk_kernel(const Ma
       mma(y, hi, mh);
       mma(y, hi, ml);
       mma(y, lo, mh);
+      hand_back(empty + 8 * s, lane, y[0], S[NT - 1][0]);   // the record is read: M for y, K^ and the decays for the state
       store_tile(out + static_cast<size_t>(k) * kC * a.ld_out, a.ld_out, half * 8, nt, left, lane, y);
     }
     if (!ok) atomicOr(&failed, 1u);
@@ -721,8 +725,6 @@ __global__ void __launch_bounds__(32 * (2 * NG + 1)) ssd_chunk_kernel(const Matr
       ldsm4(mh, rr + os);
       ldsm4(ml, rr + SsdRecord::kSmall + os);
       const float2 eg = *reinterpret_cast<const float2*>(fl + 8 * half + (lane & 3) * 2);
-      __syncwarp();
-      if (lane == 0) arrive(empty + 8 * s);                // the stage is read
       pair_sync(1 + grp);
       const float4 po = swap[k & 1][warp ^ 1][lane];
       const uint32_t x0 = half ? x[2] : x[0], x1 = half ? x[3] : x[1];
@@ -734,6 +736,7 @@ __global__ void __launch_bounds__(32 * (2 * NG + 1)) ssd_chunk_kernel(const Matr
       const uint32_t th[2] = {half ? mh[2] : mh[0], half ? mh[3] : mh[1]}, tl[2] = {half ? ml[2] : ml[0], half ? ml[3] : ml[1]};
       mma(y, x, th);
       mma(y, x, tl);
+      hand_back(empty + 8 * s, lane, y[0], S[NT - 1][0]);   // the stage is read: the masked products for y, B for the state
       store_tile(out + static_cast<size_t>(k) * kC * a.ld_out, a.ld_out, half * 8, nt, left, lane, y);
     }
     if (!ok) atomicOr(&failed, 1u);
