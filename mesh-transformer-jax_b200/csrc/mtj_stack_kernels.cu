@@ -11,7 +11,6 @@ namespace {
 
 constexpr int kRnThreads = 256;
 
-template <int THREADS>
 __device__ __forceinline__ float rn_block_sum(float v, float* red) {
   v = warp_sum(v);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -19,10 +18,45 @@ __device__ __forceinline__ float rn_block_sum(float v, float* red) {
   __syncthreads();
   float t = 0.f;
 #pragma unroll
-  for (int i = 0; i < THREADS / 32; ++i) t += red[i];
+  for (int i = 0; i < kRnThreads / 32; ++i) t += red[i];
   __syncthreads();
   return t;
 }
+// The same of the row kernels' partial sums, one per float4 of a thread.  512 threads add in the order of 256, of which a thread has
+// the numbers of threads t and t + 256 in turn: a row's bits do not depend on how many rows a call has.
+template <int THREADS, int HOLD>
+struct RowSum {
+  float red[kRnThreads / 32], upper[THREADS == kRnThreads ? 1 : HOLD][kRnThreads];
+  __device__ __forceinline__ float operator()(const float (&part)[HOLD]) {
+    const int t = threadIdx.x;
+    float v = 0.f;
+    if constexpr (THREADS == kRnThreads) {
+#pragma unroll
+      for (int i = 0; i < HOLD; ++i) v += part[i];
+      return rn_block_sum(v, red);
+    }
+    static_assert(THREADS == kRnThreads || THREADS == 2 * kRnThreads, "thread t adds the numbers of t + 256");
+    if (t >= kRnThreads) {
+#pragma unroll
+      for (int i = 0; i < HOLD; ++i) upper[i][t - kRnThreads] = part[i];
+    }
+    __syncthreads();
+    if (t < kRnThreads) {
+#pragma unroll
+      for (int i = 0; i < HOLD; ++i) {
+        v += part[i];
+        v += upper[i][t];
+      }
+      v = warp_sum(v);
+      if ((t & 31) == 0) red[t >> 5] = v;
+    }
+    __syncthreads();                                         // `upper` is read; `red` is before the next sum's first barrier
+    v = 0.f;
+#pragma unroll
+    for (int i = 0; i < kRnThreads / 32; ++i) v += red[i];
+    return v;
+  }
+};
 
 __device__ __forceinline__ float dot4(const float4& a) { return a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w; }
 __device__ __forceinline__ uint2 pack4(const float4& v) {
@@ -73,7 +107,8 @@ __device__ __forceinline__ void load_row(const float* row, int n4, float4 (&v)[H
 
 template <int THREADS, int HOLD>
 __global__ void __launch_bounds__(THREADS) residual_norm_reg_kernel(const ResidualNormArgs a) {
-  __shared__ float red[THREADS / 32];
+  __shared__ RowSum<THREADS, HOLD> row_sum;
+  float part[HOLD];
   const int n4 = a.ld >> 2;
   const size_t m = blockIdx.x;
   float4 wp[HOLD], wn[HOLD], x[HOLD];
@@ -83,14 +118,12 @@ __global__ void __launch_bounds__(THREADS) residual_norm_reg_kernel(const Residu
   pdl_launch_dependents();
   float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
   load_row<THREADS, HOLD>(reinterpret_cast<const float*>(xrow), n4, x);
-  float ss = 0.f;
   if (a.y) {
     float4 y[HOLD];
     load_planes<THREADS, HOLD>(a.y, a.planes, m, a.M, a.ld, n4, y);
-    float ys = 0.f;
 #pragma unroll
-    for (int i = 0; i < HOLD; ++i) ys += dot4(y[i]);
-    const float rs = a.mult / sqrtf(rn_block_sum<THREADS>(ys, red) / static_cast<float>(a.d) + a.eps);
+    for (int i = 0; i < HOLD; ++i) part[i] = dot4(y[i]);
+    const float rs = a.mult / sqrtf(row_sum(part) / static_cast<float>(a.d) + a.eps);
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
       const int c = i * THREADS + threadIdx.x;
@@ -100,8 +133,8 @@ __global__ void __launch_bounds__(THREADS) residual_norm_reg_kernel(const Residu
     }
   }
 #pragma unroll
-  for (int i = 0; i < HOLD; ++i) ss += dot4(x[i]);
-  const float rs = 1.0f / sqrtf(rn_block_sum<THREADS>(ss, red) / static_cast<float>(a.d) + a.eps);
+  for (int i = 0; i < HOLD; ++i) part[i] = dot4(x[i]);
+  const float rs = 1.0f / sqrtf(row_sum(part) / static_cast<float>(a.d) + a.eps);
 #pragma unroll
   for (int i = 0; i < HOLD; ++i) {
     const int c = i * THREADS + threadIdx.x;
@@ -127,7 +160,8 @@ __global__ void __launch_bounds__(THREADS) residual_norm_reg_kernel(const Residu
 
 template <int THREADS, int HOLD>
 __global__ void __launch_bounds__(THREADS) residual_layernorm_reg_kernel(const ResidualLayerNormArgs a) {
-  __shared__ float red[THREADS / 32];
+  __shared__ RowSum<THREADS, HOLD> row_sum;
+  float part[HOLD];
   const int n4 = a.ld >> 2;
   const size_t m = blockIdx.x;
   const float inv_n = 1.0f / static_cast<float>(a.d);
@@ -138,16 +172,15 @@ __global__ void __launch_bounds__(THREADS) residual_layernorm_reg_kernel(const R
   pdl_launch_dependents();
   float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
   auto norm = [&](float* mu, float* rs) {
-    float s = 0.f, q = 0.f;
 #pragma unroll
-    for (int i = 0; i < HOLD; ++i) s += (x[i].x + x[i].y) + (x[i].z + x[i].w);
-    *mu = rn_block_sum<THREADS>(s, red) * inv_n;
+    for (int i = 0; i < HOLD; ++i) part[i] = (x[i].x + x[i].y) + (x[i].z + x[i].w);
+    *mu = row_sum(part) * inv_n;
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
       const int left = a.d - 4 * (i * THREADS + static_cast<int>(threadIdx.x));      // columns that exist
-      q += dot4(make_float4(left > 0 ? x[i].x - *mu : 0.f, left > 1 ? x[i].y - *mu : 0.f, left > 2 ? x[i].z - *mu : 0.f, left > 3 ? x[i].w - *mu : 0.f));
+      part[i] = dot4(make_float4(left > 0 ? x[i].x - *mu : 0.f, left > 1 ? x[i].y - *mu : 0.f, left > 2 ? x[i].z - *mu : 0.f, left > 3 ? x[i].w - *mu : 0.f));
     }
-    *rs = 1.0f / sqrtf(rn_block_sum<THREADS>(q, red) * inv_n + a.eps);
+    *rs = 1.0f / sqrtf(row_sum(part) * inv_n + a.eps);
   };
   auto scaled = [&](int c, const float4& z, float mu, float rs, const float4& w4, const float4& b4) {
     return keep(make_float4(fmaf((z.x - mu) * rs, w4.x, b4.x), fmaf((z.y - mu) * rs, w4.y, b4.y), fmaf((z.z - mu) * rs, w4.z, b4.z),
@@ -219,7 +252,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const Residua
       rn_row[i] = xrow[i];
       ys += dot4(v);
     }
-    const float rs = a.mult / sqrtf(rn_block_sum<kRnThreads>(ys, red) / static_cast<float>(a.d) + a.eps);
+    const float rs = a.mult / sqrtf(rn_block_sum(ys, red) / static_cast<float>(a.d) + a.eps);
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
       const float4 y = yrow[i], w = reinterpret_cast<const float4*>(a.w_post)[i];
       float4 x = rn_row[i];
@@ -239,7 +272,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const Residua
       ss += dot4(x);
     }
   }
-  const float rs = 1.0f / sqrtf(rn_block_sum<kRnThreads>(ss, red) / static_cast<float>(a.d) + a.eps);
+  const float rs = 1.0f / sqrtf(rn_block_sum(ss, red) / static_cast<float>(a.d) + a.eps);
   if (a.xn) {
     uint2* o = reinterpret_cast<uint2*>(a.xn + m * a.ld);
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
@@ -283,14 +316,14 @@ __global__ void __launch_bounds__(kRnThreads) residual_layernorm_kernel(const Re
   float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
   const float inv_n = 1.0f / static_cast<float>(a.d);
   auto norm = [&](float sum, float* mu, float* rs) {
-    *mu = rn_block_sum<kRnThreads>(sum, red) * inv_n;
+    *mu = rn_block_sum(sum, red) * inv_n;
     float v = 0.f;
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
       const float4 z = rn_row[i];
       const int left = a.d - 4 * i;                       // columns that exist
       v += dot4(make_float4(left > 0 ? z.x - *mu : 0.f, left > 1 ? z.y - *mu : 0.f, left > 2 ? z.z - *mu : 0.f, left > 3 ? z.w - *mu : 0.f));
     }
-    *rs = 1.0f / sqrtf(rn_block_sum<kRnThreads>(v, red) * inv_n + a.eps);
+    *rs = 1.0f / sqrtf(rn_block_sum(v, red) * inv_n + a.eps);
   };
   auto scaled = [&](int i, float mu, float rs, const float* w, const float* b) {
     const float4 z = rn_row[i], w4 = reinterpret_cast<const float4*>(w)[i], b4 = reinterpret_cast<const float4*>(b)[i];
