@@ -58,7 +58,9 @@ struct RowSum {
   }
 };
 
-__device__ __forceinline__ float dot4(const float4& a) { return a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w; }
+// Spelled out, because the compiler may fuse the sum of two products in either order and does so differently from one template to
+// the next: a row's bits would depend on which of the row kernels finishes it.
+__device__ __forceinline__ float dot4(const float4& a) { return fmaf(a.w, a.w, fmaf(a.z, a.z, fmaf(a.x, a.x, a.y * a.y))); }
 __device__ __forceinline__ uint2 pack4(const float4& v) {
   return make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
 }
@@ -72,8 +74,8 @@ __device__ __forceinline__ float4 keep(float4 v, int left) {
 
 // The row kernels in two forms: rows of up to 8192 columns in registers (HOLD float4 a thread), every load of the row and
 // of the planes issued before the first sum, because with few rows the kernel is nothing but the latency of its loads
-// and sums (8 rows of 4096 in 8 planes: 12.4 us through shared memory); wider rows in shared memory.  Both add in the
-// same order.
+// and sums (8 rows of 4096 in 8 planes: 12.4 us through shared memory); wider rows in shared memory.  Both add a row in the same
+// order, except that the layer norm in shared memory begins a float4's squares with its second column.
 //
 // Rows of up to as many blocks as SMs take 512 threads, twice the loads in flight (24 rows of 2048 in 8 planes 6.1 us with 256
 // threads, 5.1 with 512); above, the SMs hold fewer such blocks (1794 rows of 2048 10 us and 15.7).
@@ -321,7 +323,8 @@ __global__ void __launch_bounds__(kRnThreads) residual_layernorm_kernel(const Re
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
       const float4 z = rn_row[i];
       const int left = a.d - 4 * i;                       // columns that exist
-      v += dot4(make_float4(left > 0 ? z.x - *mu : 0.f, left > 1 ? z.y - *mu : 0.f, left > 2 ? z.z - *mu : 0.f, left > 3 ? z.w - *mu : 0.f));
+      const float dx = left > 0 ? z.x - *mu : 0.f, dy = left > 1 ? z.y - *mu : 0.f, dz = left > 2 ? z.z - *mu : 0.f, dw = left > 3 ? z.w - *mu : 0.f;
+      v += fmaf(dw, dw, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));                      // (not dot4's order)
     }
     *rs = 1.0f / sqrtf(rn_block_sum(v, red) * inv_n + a.eps);
   };
