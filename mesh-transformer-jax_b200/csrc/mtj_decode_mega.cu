@@ -968,6 +968,7 @@ __global__ void __launch_bounds__(kMT, (BT == 1 && kMT == 256) ? 2 : 1) decode_m
   __syncthreads();
   if (is_last) {
     for (int i = threadIdx.x; i < 5 * L + 3; i += kMT) a.sync[i] = 0u;
+    for (int i = threadIdx.x; i < B * a.heads; i += kMT) a.head_counters[i] = 0u;   // zero, unless a merge has run out of its wait
     if (tp && threadIdx.x == 0) *a.seq = seq0 + 1 + L;
     if (a.amax) {
       // every block's maxima were published before its ticket: the token of the step, then the position moves on

@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(const MegaAr
   constexpr int kSide = 256 / DH, kParts = kAttW * kSide;        // keys side by side in a warp (a lane holds 8 columns), partial results
   __shared__ float sm_m[kParts], sm_l[kParts], sm_o[kParts][DH];
   __shared__ float wgt[64], inv_l;
-  __shared__ bool is_last;
+  __shared__ bool is_last, merges;                               // the step's last block; the last block of a head
   __shared__ unsigned long long blk_amax;
   __shared__ uint32_t failed;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -446,23 +446,6 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(const MegaAr
     }
     ebar();
     stamp(a.trace, 6 * L + 2);
-    // the last block to finish resets the arrival counters, writes the token and moves the position on
-    if (t == 0) {
-      if (*failed_v && a.dev_err) atomicOr(a.dev_err, kDevErrTimeout);
-      if (a.amax && blk_amax) atomicMax(a.amax, blk_amax);
-      __threadfence();
-      is_last = atomicAdd(a.sync + (4 * L + 1), 1u) == target - 1;
-    }
-    ebar();
-    if (is_last) {
-      for (int i = t; i < 5 * L + 3; i += kEpiT) a.sync[i] = 0u;
-      if (a.amax && t == 0) {
-        __threadfence();
-        a.tokens_out[0] = static_cast<uint32_t>(*reinterpret_cast<volatile unsigned long long*>(a.amax));
-        a.amax[0] = 0ull;
-        if (a.cur_out) *a.cur_out += 1;
-      }
-    }
   } else {
     // ------------------------------------------------------------------------------------ attending warps
     // block = (head, one of `splits` ranges of the keys that are there), all blocks as far as there are keys
@@ -563,9 +546,9 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(const MegaAr
         }
         __threadfence();
         abar();
-        if (t == 0) is_last = atomicAdd(a.head_counters + head, 1u) == static_cast<uint32_t>(nsplit - 1);
+        if (t == 0) merges = atomicAdd(a.head_counters + head, 1u) == static_cast<uint32_t>(nsplit - 1);
         abar();
-        if (is_last) {                                           // merge the head's ranges
+        if (merges) {                                            // merge the head's ranges
           __threadfence();
           if (sw == 0) {
             float ms[2], ls[2];
@@ -608,14 +591,33 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(const MegaAr
       if (t == 0) phase_arrive(c_af + l);
     }
   }
+  // The last block to finish resets the counters, writes the token and moves the position on.  A block takes its ticket when all of
+  // its warps are here: once a wait has run out they are no longer in step, and an arrival behind the reset would be the next step's.
   __syncthreads();
-  if (*failed_v && threadIdx.x == 0)
-    // some wait ran out: what is still in flight gets another bounded chance to land before the block leaves
-    for (int i = 0; i < kRing; ++i) {
-      mbar_wait(full(i), 0);
-      mbar_wait(full(i), 1);
+  if (threadIdx.x == 0) {
+    if (*failed_v) {
+      // what is still in flight gets another bounded chance to land before the block leaves
+      for (int i = 0; i < kRing; ++i) {
+        mbar_wait(full(i), 0);
+        mbar_wait(full(i), 1);
+      }
+      if (a.dev_err) atomicOr(a.dev_err, kDevErrTimeout);
     }
+    if (a.amax && blk_amax) atomicMax(a.amax, blk_amax);
+    __threadfence();
+    is_last = atomicAdd(a.sync + (4 * L + 1), 1u) == target - 1;
+  }
   __syncthreads();
+  if (is_last) {
+    for (int i = threadIdx.x; i < 5 * L + 3; i += kThreads) a.sync[i] = 0u;
+    for (int i = threadIdx.x; i < a.heads; i += kThreads) a.head_counters[i] = 0u;
+    if (a.amax && threadIdx.x == 0) {
+      __threadfence();
+      a.tokens_out[0] = static_cast<uint32_t>(*reinterpret_cast<volatile unsigned long long*>(a.amax));
+      a.amax[0] = 0ull;
+      if (a.cur_out) *a.cur_out += 1;
+    }
+  }
 }
 
 // shared memory of a block of G: the ring and the partial sums of the most rows that a block has (two lots of them in `rows`)
