@@ -33,14 +33,14 @@ struct KvVec;
 template <>
 struct KvVec<8> {
   uint4 v;
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = ld_stream16(p); }
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = ld_cached16(p); }
   __device__ __forceinline__ void load_shared(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint4*>(p); }
   __device__ __forceinline__ void get(float* f) const { unpack8(v, f); }
 };
 template <>
 struct KvVec<2> {
   uint32_t v;
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = ld_stream4(p); }
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = ld_cached4(p); }
   __device__ __forceinline__ void load_shared(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint32_t*>(p); }
   __device__ __forceinline__ void get(float* f) const {
     f[0] = bf16_lo(v);

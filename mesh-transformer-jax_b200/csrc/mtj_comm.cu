@@ -72,7 +72,7 @@ __device__ __forceinline__ float block_sum256(float v, float* red) {
 // x[m] = (accumulate ? x[m] : 0) + reduced[m], then the LayerNorm statistics of
 // the row (layers.py:18-19,32): what follows every g_psum on the residual path.
 __global__ void __launch_bounds__(kThreads) residual_stats_kernel(float* __restrict__ x,
-                                                                  const float* __restrict__ reduced,
+                                                                  const float* reduced,
                                                                   float* __restrict__ stats, int d,
                                                                   int accumulate) {
   __shared__ float red[kThreads / 32];

@@ -30,8 +30,8 @@ struct DeviceOnce {
   }
 };
 
-// 16-byte streaming load of read-only data that is touched once per pass
-// (weights, KV pages): bypass L1 so the activations stay resident there.
+// 16-byte streaming load of data that nobody writes while the kernel is there (weights) and that is touched once per pass: bypass
+// L1 so the activations stay resident there.
 __device__ __forceinline__ uint4 ld_stream16(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -39,9 +39,18 @@ __device__ __forceinline__ uint4 ld_stream16(const void* p) {
                : "l"(p));
   return v;
 }
-__device__ __forceinline__ uint32_t ld_stream4(const void* p) {
+// The same for cached keys and values, whose newest rows other blocks or the predecessor of a chained launch write while the kernel
+// is there: a coherent load.
+__device__ __forceinline__ uint4 ld_cached16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_cached4(const void* p) {
   uint32_t v;
-  asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 

@@ -720,11 +720,11 @@ __global__ void __launch_bounds__(kMT, (BT == 1 && kMT == 256) ? 2 : 1) decode_m
             ok[t] = tt < w1;
             const size_t off = kv_offset(table, a.ring_pages, a.heads, DH, head, ok[t] ? tt : tb) + lane * EPL;
             if (EPL == 8) {
-              kraw[t] = ld_stream16(lw.kpool + off);
-              vraw[t] = ld_stream16(lw.vpool + off);
+              kraw[t] = ld_cached16(lw.kpool + off);
+              vraw[t] = ld_cached16(lw.vpool + off);
             } else {
-              kraw[t].x = ld_stream4(lw.kpool + off);
-              vraw[t].x = ld_stream4(lw.vpool + off);
+              kraw[t].x = ld_cached4(lw.kpool + off);
+              vraw[t].x = ld_cached4(lw.vpool + off);
             }
           }
           float sc[TB];

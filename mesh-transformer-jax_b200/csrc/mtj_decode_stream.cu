@@ -484,8 +484,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(const MegaAr
 #pragma unroll
           for (int k = 0; k < TB; ++k) {
             const size_t off = kv_offset(a.page_table, a.ring_pages, a.heads, DH, head, min(tb + k * kSide + side, w1 - 1)) + col;
-            kraw[k] = ld_stream16(lw.kpool + off);
-            vraw[k] = ld_stream16(lw.vpool + off);
+            kraw[k] = ld_cached16(lw.kpool + off);
+            vraw[k] = ld_cached16(lw.vpool + off);
           }
           float sc[TB];
 #pragma unroll

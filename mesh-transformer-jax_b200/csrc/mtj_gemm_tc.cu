@@ -21,9 +21,10 @@ __device__ __forceinline__ float row_sum(float v, float* red) {
 // LayerNorm of fp32 rows into bf16 (the GEMM's activation operand: hi, and lo where asked for), layers.py:17-36.  HOLD > 0:
 // rows of up to 256 HOLD columns stay in registers, one read of the row with all loads in flight instead of three, and the
 // weights before it; 0: wider rows, three reads.  Both add in the same order.  Few rows are bound by the loads' latency (33 of
-// 4096: 5.2 us in three reads, 3.0 from registers; 33 of 1024: 2.7 and 2.2), many by how many blocks an SM holds.
+// 4096: 5.2 us in three reads, 3.0 from registers; 33 of 1024: 2.7 and 2.2), many by how many blocks an SM holds.  (The predecessor
+// of a chained launch writes x while this kernel is there: not __restrict__, which would let its loads be read-only ones.)
 template <int HOLD>
-__global__ void __launch_bounds__(256) ln_rows_kernel(const float* __restrict__ x, const float* __restrict__ scale,
+__global__ void __launch_bounds__(256) ln_rows_kernel(const float* x, const float* __restrict__ scale,
                                                       const float* __restrict__ offset,
                                                       __nv_bfloat16* __restrict__ out, __nv_bfloat16* out_lo, int d) {
   __shared__ float red[8];
@@ -265,7 +266,7 @@ cudaError_t launch_gemm_tc(GemvEpilogue epi, const void* map_w, const void* map_
 
 namespace {
 // out[m, n] = sum_z partial[z, m, n] + bias[n] (+ residual[m, n]); fixed summation order
-__global__ void splitk_reduce_kernel(const float* __restrict__ partial, int ksplit, int M, int N,
+__global__ void splitk_reduce_kernel(const float* partial, int ksplit, int M, int N,
                                      const float* __restrict__ bias, const float* residual, float* out, int ld_out,
                                      const uint32_t* slot_sel, size_t slot_stride) {
   const size_t total = static_cast<size_t>(M) * N;

@@ -380,7 +380,7 @@ __global__ void gather_rows_bf16_kernel(const __nv_bfloat16* __restrict__ src, i
   for (int i = threadIdx.x; i < ld / 8; i += blockDim.x) d[i] = s[i];
 }
 
-__global__ void copy_rows_kernel(const float4* __restrict__ src, float4* __restrict__ dst, int64_t n4) {
+__global__ void copy_rows_kernel(const float4* src, float4* __restrict__ dst, int64_t n4) {
   pdl_wait();
   pdl_launch_dependents();
   const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
