@@ -254,12 +254,13 @@ cudaError_t launch_epi(const GemvArgs& a, cudaStream_t s, bool pdl) {
 // this way too: a reply of a model of width 1024 12.0 ms against 11.8, of 2048 17.0 against 16.8 or 18.0 against 18.2).  The
 // columns are what the warps' registers hold.
 bool gemv_stream_ok(GemvEpilogue epi, const GemvArgs& a) {
+  if ((a.K & 7) || (a.N & 1) || (a.ldx & 3)) return false;      // 16-byte pieces of both operands, pairs of rows
   return a.M == 1 && (epi == kEpiOut || epi == kEpiSoftcap || epi == kEpiSwiGLU || epi == kEpiRelu2) && a.K >= kMinK && a.K <= kMaxK &&
          static_cast<int64_t>(a.N) * a.K >= kMinWeights && !a.residual && !a.slot_sel && !a.stats_out && a.ks_override == 0 && plan_of(epi, a).smem <= kMaxSmem;
 }
 
 cudaError_t launch_gemv_stream(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl) {
-  if (!gemv_stream_ok(epi, a) || (a.K & 7) || (a.N & 1) || (a.ldx & 3)) return cudaErrorInvalidValue;
+  if (!gemv_stream_ok(epi, a)) return cudaErrorInvalidValue;
   switch (epi) {
     case kEpiOut: return launch_epi<kEpiOut>(a, s, pdl);
     case kEpiSwiGLU: return launch_epi<kEpiSwiGLU>(a, s, pdl);
