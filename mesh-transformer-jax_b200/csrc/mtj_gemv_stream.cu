@@ -23,6 +23,7 @@ namespace {
 
 constexpr int kMinK = 1024, kMaxK = 16384;               // columns of a weight row
 constexpr int64_t kMinWeights = 12 << 20;
+constexpr int kLongK = 8192, kLeastN = 4 * 148;          // columns and rows from which fewer weights will do
 constexpr int kRingBytes = 128 * 1024, kStage = 32 * 1024, kMaxRing = 8;
 constexpr int kMaxSmem = 224 * 1024;
 constexpr int kW = 16, kStreamThreads = 32 * kW + 32;
@@ -251,12 +252,14 @@ cudaError_t launch_epi(const GemvArgs& a, cudaStream_t s, bool pdl) {
 }  // namespace
 
 // One row and weights of 25 MB and more: below, the stream is over before its ring has paid for its setup (products of 8 to 24 MB
-// this way too: a reply of a model of width 1024 12.0 ms against 11.8, of 2048 17.0 against 16.8 or 18.0 against 18.2).  The
-// columns are what the warps' registers hold.
+// this way too: a reply of a model of width 1024 12.0 ms against 11.8, of 2048 17.0 against 16.8 or 18.0 against 18.2).  Rows of
+// 8192 columns and more earlier, from four a block on: gemv_kernel has few such rows to spread (down projections of six layers, us a
+// step by gemv_kernel and this way: 600 x 8192 167 and 163, 600 x 12288 186 and 174, 768 x 12288 186 and 176, 1024 x 8192 171 and
+// 174 with one family, 190 and 187 with the other).  The columns are what the warps' registers hold.
 bool gemv_stream_ok(GemvEpilogue epi, const GemvArgs& a) {
   if ((a.K & 7) || (a.N & 1) || (a.ldx & 3)) return false;      // 16-byte pieces of both operands, pairs of rows
   return a.M == 1 && (epi == kEpiOut || epi == kEpiSoftcap || epi == kEpiSwiGLU || epi == kEpiRelu2) && a.K >= kMinK && a.K <= kMaxK &&
-         static_cast<int64_t>(a.N) * a.K >= kMinWeights && !a.residual && !a.slot_sel && !a.stats_out && a.ks_override == 0 && plan_of(epi, a).smem <= kMaxSmem;
+         (static_cast<int64_t>(a.N) * a.K >= kMinWeights || (a.K >= kLongK && a.N >= kLeastN)) && !a.residual && !a.slot_sel && !a.stats_out && a.ks_override == 0 && plan_of(epi, a).smem <= kMaxSmem;
 }
 
 cudaError_t launch_gemv_stream(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl) {

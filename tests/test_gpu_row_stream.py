@@ -29,6 +29,13 @@ def test_single_tokens(cuda_device, family, width, ff):
     rt.close()
 
 
+@pytest.mark.parametrize("width,ff", [(592, 8192), (600, 12296), (604, 16384), (588, 8192)])
+@pytest.mark.parametrize("family", ["keselix", "bavutar"])
+def test_long_rows_of_few_weights(cuda_device, family, width, ff):
+    """From four rows a block on, rows of 8192 columns and more are streamed however few the weights are; with one row less not."""
+    test_single_tokens(cuda_device, family, width, ff)
+
+
 @pytest.mark.parametrize("family", ["keselix", "bavutar"])
 def test_the_same_tokens_give_the_same_bits(cuda_device, family):
     """A stage of weights is handed back before it is read if nothing has waited for its loads: most stages in the ring at once, the

@@ -38,7 +38,7 @@ def rule(tmp_path_factory):
 
 
 def test_only_what_the_kernel_takes(rule):
-    yes = [(32768, 4096, 4096), (4096, 16384, 16384), (12304, 1024, 1024), (3072, 4104, 4108)]
+    yes = [(32768, 4096, 4096), (4096, 16384, 16384), (12304, 1024, 1024), (3072, 4104, 4108), (592, 8192, 8192), (600, 16384, 16384)]
     no = [(n + dn, k + dk, ldx + dx) for n, k, ldx in yes for dn, dk, dx in ((1, 0, 0), (0, 4, 0), (0, 1, 0), (0, 0, 2), (0, 0, 1))]
-    got = rule(yes + no + [(2048, 4096, 4096), (65536, 1016, 1016), (4096, 16392, 16392)])
+    got = rule(yes + no + [(2048, 4096, 4096), (65536, 1016, 1016), (4096, 16392, 16392), (588, 8192, 8192), (592, 8184, 8184)])
     assert all(got[s] == ("1111" if s in yes else "0000") for s in got), got
