@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kGemvThreads, BT == 1 ? (EPI == kEpiOut ? 4 : 
     if (!is_last) return;
     __threadfence();
     if (a.post_w) {
-      finish_rows(a, m0, nb, red);
+      finish_row(a, red);
       if (threadIdx.x == 0) a.counters[blockIdx.y] = 0u;
       return;
     }
@@ -291,6 +291,7 @@ cudaError_t launch_epi(const GemvArgs& a, cudaStream_t s, bool pdl) {
 
 cudaError_t launch_gemv(GemvEpilogue epi, const GemvArgs& a, cudaStream_t s, bool pdl) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || (a.K & 7) != 0 || (a.N & 3) != 0) return cudaErrorInvalidValue;
+  if (a.post_w && a.M != 1) return cudaErrorInvalidValue;
   if (a.ks_override != 0 && a.ks_override != 1 && a.ks_override != 2 && a.ks_override != 4 &&
       a.ks_override != 8)
     return cudaErrorInvalidValue;

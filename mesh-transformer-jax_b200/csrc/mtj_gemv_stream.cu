@@ -2,8 +2,8 @@
 //
 // gemv_kernel keeps 64 bytes per thread in flight and starts with an empty pipe in each of its waves of blocks; a product
 // of 25 to 260 MB is over after 4 to 40 us, so that ramps and last waves cost a third of it.  Here one block per SM owns a
-// run of rows.  A seventeenth warp streams them in stages of up to 32 KB, whole rows that touch in one bulk copy, through a ring
-// of 128 KB, filled from before the wait on the predecessor.  One block per SM: with a ring of 96 KB the next product's block
+// run of rows.  A seventeenth warp streams them in stages of 16 to 32 KB, one row for each group of warps in one bulk copy (rows
+// touch), through a ring of 128 KB, filled from before the wait on the predecessor.  One block per SM: with a ring of 96 KB the next product's block
 // came in beside this one's, and both streams got slower (a reply of width 4096 24.4 ms, 20.2 with 160 KB, 19.6 with 128).
 // The 16 others hold the activations in registers, a warp the same 512 to 1024 columns of every row that its group takes.  No
 // block-wide barrier until the rows are done; the partial sums of a row are added in order.  What bounds it beside HBM is the
@@ -24,7 +24,7 @@ namespace {
 constexpr int kMinK = 1024, kMaxK = 16384;               // columns of a weight row
 constexpr int64_t kMinWeights = 12 << 20;
 constexpr int kLongK = 8192, kLeastN = 4 * 148;          // columns and rows from which fewer weights will do
-constexpr int kRingBytes = 128 * 1024, kStage = 32 * 1024, kMaxRing = 8;
+constexpr int kRingBytes = 128 * 1024, kMaxRing = 8;
 constexpr int kMaxSmem = 224 * 1024;
 constexpr int kW = 16, kStreamThreads = 32 * kW + 32;
 
@@ -55,7 +55,7 @@ __device__ __forceinline__ float sum2(F2 v) {
 
 // pieces of 8 columns of a lane, groups of warps that take the rows in turn
 template <int NCH, int GROUPS, int EPI>
-__global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const GemvArgs a, int ring, int stage_rows) {
+__global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const GemvArgs a, int ring) {
   extern __shared__ __align__(128) unsigned char stream_smem[];
   __shared__ __align__(8) uint64_t bars[2 * kMaxRing];
   __shared__ float red[kW];
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const Ge
   const int units = a.N / kUnit;
   const int r0 = kUnit * static_cast<int>(static_cast<int64_t>(blockIdx.x) * units / gridDim.x);
   const int r1 = kUnit * static_cast<int>(static_cast<int64_t>(blockIdx.x + 1) * units / gridDim.x);
-  const uint32_t row_bytes = static_cast<uint32_t>(a.K) * 2u, stage = row_bytes * stage_rows;
+  const uint32_t row_bytes = static_cast<uint32_t>(a.K) * 2u, stage = row_bytes * GROUPS;
   float* part = reinterpret_cast<float*>(stream_smem + static_cast<size_t>(ring) * stage);   // [row][kPitch]
   const uint32_t bar0 = smem_u32(bars), ring0 = smem_u32(stream_smem);
   auto full = [&](int i) { return bar0 + 8u * i; };
@@ -89,10 +89,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const Ge
       // weights do not depend on the predecessor
       const uint64_t pol = l2_evict_first_policy();
       uint32_t phase = 1;                                        // the first round passes
-      for (int r = r0; r < r1 && ok; r += stage_rows) {
+      for (int r = r0; r < r1 && ok; r += GROUPS) {
         ok = mbar_wait(empty(slot), phase);
         if (!ok) break;
-        const uint32_t bytes = row_bytes * min(stage_rows, r1 - r);
+        const uint32_t bytes = row_bytes * min(GROUPS, r1 - r);
         mbar_expect_tx(full(slot), bytes);
         bulk_load(ring0 + slot * stage, a.W + static_cast<size_t>(r) * a.K, bytes, full(slot), pol);
         if (++slot == ring) {
@@ -118,15 +118,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const Ge
       x[c][0] = pack2(lo.x, lo.y); x[c][1] = pack2(lo.z, lo.w); x[c][2] = pack2(hi.x, hi.y); x[c][3] = pack2(hi.z, hi.w);
     }
     uint32_t phase = 0;
-    int left = 0;                                                // rows of this group in the current stage
-    float before = 0.f;                                          // the sum of the row before
-    auto dot = [&]() {
-      if (left == 0) {
-        ok = __all_sync(0xffffffffu, mbar_wait(full(slot), phase));
-        left = stage_rows / GROUPS;
-      }
-      const int at = (stage_rows / GROUPS - left) * GROUPS + grp;
-      const uint4* row = reinterpret_cast<const uint4*>(stream_smem + static_cast<size_t>(slot) * stage) + at * vecs + v0 + lane;
+    auto dot = [&]() {                                           // this group's row of the next stage
+      ok = __all_sync(0xffffffffu, mbar_wait(full(slot), phase));
+      const uint4* row = reinterpret_cast<const uint4*>(stream_smem + static_cast<size_t>(slot) * stage) + grp * vecs + v0 + lane;
       F2 t0 = 0ull, t1 = 0ull;
       uint4 v[NCH];
 #pragma unroll
@@ -134,17 +128,14 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const Ge
 #pragma unroll
       for (int c = 0; c < NCH; ++c) dot8(c & 1 ? t1 : t0, v[c], x[c]);
       const float sum = sum2(t0) + sum2(t1);
-      if (--left == 0) {
-        // Every lane has the stage in its registers: which lane hands it back hangs on every lane's sums, because an arrival
-        // alone does not wait for loads that nothing has used yet, and the next rows would land under them.
-        const int by = __any_sync(0xffffffffu, __float_as_uint(sum) == 0x7fc0dead || __float_as_uint(before) == 0x7fc0dead) ? 1 : 0;
-        if (lane == by) arrive(empty(slot));
-        if (++slot == ring) {
-          slot = 0;
-          phase ^= 1u;
-        }
+      // Every lane has the row in its registers: which lane hands the stage back hangs on every lane's sum, because an arrival
+      // alone does not wait for loads that nothing has used yet, and the next rows would land under them.
+      const int by = __any_sync(0xffffffffu, __float_as_uint(sum) == 0x7fc0dead) ? 1 : 0;
+      if (lane == by) arrive(empty(slot));
+      if (++slot == ring) {
+        slot = 0;
+        phase ^= 1u;
       }
-      before = sum;
       return sum;
     };
     // two rows' sums at a time: the first in lanes 0 to 15, the second in lanes 16 to 31; a wait that ran out ends the loop
@@ -199,7 +190,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const Ge
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    if (warp < kW) finish_rows<32 * kW>(a, 0, 1, red);
+    if (warp < kW) finish_row<32 * kW>(a, red);
     if (threadIdx.x == 0) a.counters[0] = 0u;
   }
 }
@@ -215,16 +206,15 @@ int blocks_of() {
 int groups_of(int K) { return K <= 1024 ? 16 : K <= 2048 ? 8 : K <= 4096 ? 4 : K <= 8192 ? 2 : 1; }
 
 struct StreamPlan {
-  int grid, ring, rows, smem;                                    // rows of a stage
+  int grid, ring, smem;
 };
 StreamPlan plan_of(GemvEpilogue epi, const GemvArgs& a) {
   const int unit = epi == kEpiSwiGLU ? 2 : 1, groups = groups_of(a.K);
   StreamPlan p;
   p.grid = std::min(blocks_of(), a.N / unit);
-  p.rows = std::max(1, kStage / (2 * a.K * groups)) * groups;
-  p.ring = std::min(kMaxRing, kRingBytes / (2 * a.K * p.rows));
+  p.ring = std::min(kMaxRing, kRingBytes / (2 * a.K * groups));
   const int most = unit * ((a.N / unit + p.grid - 1) / p.grid);
-  p.smem = p.ring * p.rows * a.K * 2 + (kW / groups + 1) * most * 4;
+  p.smem = p.ring * groups * a.K * 2 + (kW / groups + 1) * most * 4;
   p.smem = std::max(p.smem, 116 * 1024);                         // one block per SM
   return p;
 }
@@ -234,7 +224,7 @@ cudaError_t launch_one(const GemvArgs& a, const StreamPlan& p, cudaStream_t s, b
   static DeviceOnce once;
   const cudaError_t e = once.run([&] { return cudaFuncSetAttribute(gemv_stream_kernel<NCH, GROUPS, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem); });
   if (e != cudaSuccess) return e;
-  return launch_pdl(gemv_stream_kernel<NCH, GROUPS, EPI>, dim3(p.grid), dim3(kStreamThreads), p.smem, s, pdl, a, p.ring, p.rows);
+  return launch_pdl(gemv_stream_kernel<NCH, GROUPS, EPI>, dim3(p.grid), dim3(kStreamThreads), p.smem, s, pdl, a, p.ring);
 }
 
 template <int EPI>
