@@ -353,7 +353,8 @@ def run_mtj(args):
         decode(None, tok_out)
     prof = rt.profile_read()
     rt.profile_enable(False)
-    # phase time stamps of the persistent decode kernel (when it is the path in use)
+    # phase time stamps of the persistent decode kernel (when it is the path in use; where attention runs beside the products,
+    # attention_us is 0 and what is felt of it stands under the attention columns)
     phases = None
     if B <= max(1, rt.tuning["mega_max_batch"]) and os.environ.get("MTJ_NO_MEGA") != "1" \
             and os.environ.get("MTJ_NO_P2P") != "1":
@@ -544,7 +545,9 @@ def run_mtj(args):
     if phases is not None:
         # one persistent kernel does the whole step: it is the dominant kernel
         top = "mega"
-        fam_kernel["mega"] = ("decode_mega_kernel (whole decode step: embedding, L x [LN + in-proj, attention, "
+        streamed = world == 1 and B == 1 and 1024 <= d <= 4096 and not os.environ.get("MTJ_MEGA_NARROW")
+        fam_kernel["mega"] = (("decode_stream_kernel" if streamed else "decode_mega_kernel") +
+                              " (whole decode step: embedding, L x [LN + in-proj, attention, "
                               "out-proj + residual], final LN + logits)")
         fam["mega"] = {"ms_per_launch": ms_step, "launches": K, "bytes_per_launch": rank_bytes,
                        "gbs": rank_bytes / (ms_step * 1e-3) / 1e9, "ms_per_step": ms_step}
