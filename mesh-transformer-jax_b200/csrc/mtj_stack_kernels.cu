@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(THREADS) residual_layernorm_reg_kernel(const R
   auto norm = [&](float* mu, float* rs) {
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) part[i] = (x[i].x + x[i].y) + (x[i].z + x[i].w);
-    *mu = row_sum(part) * inv_n;
+    *mu = __fmul_rn(row_sum(part), inv_n);               // never fused into the differences below, in no template
 #pragma unroll
     for (int i = 0; i < HOLD; ++i) {
       const int left = a.d - 4 * (i * THREADS + static_cast<int>(threadIdx.x));      // columns that exist
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_layernorm_kernel(const Re
   float4* xrow = reinterpret_cast<float4*>(a.x + (a.select ? a.select[m] : m) * a.ld);
   const float inv_n = 1.0f / static_cast<float>(a.d);
   auto norm = [&](float sum, float* mu, float* rs) {
-    *mu = rn_block_sum(sum, red) * inv_n;
+    *mu = __fmul_rn(rn_block_sum(sum, red), inv_n);
     float v = 0.f;
     for (int i = threadIdx.x; i < n4; i += kRnThreads) {
       const float4 z = rn_row[i];
