@@ -31,7 +31,7 @@ namespace {
 constexpr int kW = 16, kT = 32 * kW;                          // streaming warps and threads
 constexpr int kEpiW = 3, kEpiT = 32 * kEpiW;                  // finishing warps and threads
 constexpr int kAttW = 8, kAttT = 32 * kAttW;                  // attending warps and threads
-constexpr int kThreads = kT + kEpiT + kAttT + 32;             // 28 warps: 72 registers a thread
+constexpr int kThreads = kT + kEpiT + kAttT + 32;             // 28 warps: 72 registers a thread, no spills
 constexpr int kRing = 5;
 constexpr uint32_t kStage = 32 * 1024;
 constexpr int kMaxD = 4096, kMaxFf = 16384;                   // columns that the warps' registers hold
@@ -226,8 +226,11 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(const MegaAr
       if (!mbar_ready(full(slot), phase) && !*failed_v && !mbar_wait(full(slot), phase)) *failed_v = 1;
       return ds_smem + slot * kStage;
     };
+    // Hands the stage back.  In front of it stands the store of the last sums, which hangs on a shuffle over what every lane has made
+    // of the stage: that, and not the barrier, has waited for the loads (an arrival alone does not wait for loads that nothing has
+    // used yet), so the reduction has to stay in front.
     auto release = [&]() {
-      __syncwarp();                                              // every lane has read the stage
+      __syncwarp();
       if (lane == 0) arrive(empty(slot));
       if (++slot == kRing) {
         slot = 0;

@@ -11,7 +11,7 @@ namespace mtj {
 
 // ---- mtj_stack_kernels.cu
 // One row per block:  y = sum of the planes;  x += mult * RMSNorm(y) * w_post (y may be null);  then, of the new x:
-// stats = (0, 1 / rms), xn = RMSNorm(x) * w_next in bf16, and cat = [x | x0] for the projection at the start of a pass.
+// RMSNorm(x) * w_next in bf16 (xn) or fp32 (xn_f32), and cat = [x | x0] for the projection at the start of a pass.
 struct ResidualNormArgs {
   float* x;                    // [M, ld]; columns d .. ld - 1 of every buffer here are zero
   int M, d, ld;
